@@ -1,0 +1,693 @@
+// Delta rules over prompt portions, 32 tokens at a time.
+//
+// Token by token a portion costs tokens x the latency of one step, however few columns a head's state has. Over a chunk of tokens
+// the rule S <- g S; u = beta (v - S^T k); S <- S + k u^T; o = S^T q is a handful of small matrix products (the chunkwise form of
+// delta rules: Yang, Kautz and Hatamizadeh, "Gated Delta Networks: Improving Mamba2 with Delta Rule"; with a decay per key channel
+// every product over channels carries the decays between its two tokens). With S the state in front of the chunk, G_ij the product
+// of the decays of tokens j + 1 .. i (per channel), e_i the product up to token i:
+//   u_i = beta_i (v_i - S^T (e_i k_i) - sum_{j < i} (k_i . G_ij k_j) u_j),   o_i = S^T (e_i q_i) + sum_{j <= i} (q_i . G_ij k_j) u_j,
+//   S <- e_last S + sum_j (G_last,j k_j) u_j^T.
+// With L_ij = beta_i k_i . G_ij k_j (j < i): U = W + Y S, W = (I + L)^-1 diag(beta) V, Y = -(I + L)^-1 diag(beta) (e K).
+// Three kernels:
+//   chunk_prepare    all chunks side by side: A = (q_i . G_ij k_j), W, Y and the scaled e Q and G_last K;
+//   chunk_walk       a head's chunks one after another, a tile of 16 columns of S per block: U = W + Y S, S <- e S + (G_last K)^T U;
+//   chunk_out        all chunks side by side again: O = (e Q) S + A U, from the states that the walk left at each chunk's start.
+// Only what the next chunk waits for is in the walk. Everything is 32-bit FMAs (no reduced-precision tensor-core mode): state,
+// decays and gates stay what they are token by token, up to the order of sums. Decays enter as products (or sums of their logarithms)
+// from token j on, never as quotients of products from the chunk's start, so strong decays in front of a pair cost it no digits.
+//
+// What bounds it: the walk, a chain of chunks in which a block does 2 x 32 x dk x 16 FMAs per chunk (1,024 cycles of an SM's FMA pipe
+// at dk = 128) and takes about twice as many cycles' worth of operands out of shared memory, between two block-wide barriers.
+// Measured on a B200 (one request of 2,048 tokens, heads of 128 x 128; all three kernels): a decay per channel, 12 heads: 731 us token
+// by token -> 252 us (prepare 60, walk 130, out 60), 28 heads: 941 -> 449; one decay per head (before: outputs and triangular products
+// inside the walk): 305 -> 252 and 525 -> 450.
+#include "common.cuh"
+
+namespace {
+
+constexpr int C = 32;            // tokens per chunk
+constexpr int kColumns = 16;     // columns of the state per block of the walk
+constexpr int kThreads = 256;
+constexpr int kWarps = kThreads / 32;
+constexpr int kMaxRows = 256;    // key channels per head
+
+__host__ __device__ constexpr int padded_rows(int dk) { return dk <= 64 ? 64 : (dk <= 128 ? 128 : 256); }
+__host__ __device__ constexpr int padded_columns(int dv) { return (dv + kColumns - 1) / kColumns * kColumns; }
+// A chunk's place among all chunks of the step: different for all (request, chunk), below tokens / C + requests + 1.
+__device__ __forceinline__ int64_t chunk_place(int start, int seq, int chunk) { return static_cast<int64_t>(start / C) + seq + chunk; }
+
+template <int kBytes>
+__device__ __forceinline__ void stage_copy(float* smem, const float* gmem, bool valid) {
+  const uint32_t s = static_cast<uint32_t>(__cvta_generic_to_shared(smem));
+  const int bytes = valid ? kBytes : 0;
+  asm volatile("cp.async.ca.shared.global [%0], [%1], %2, %3;" ::"r"(s), "l"(gmem), "n"(kBytes), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ void commit_copies() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int LEFT>
+__device__ __forceinline__ void wait_copies() {
+  asm volatile("cp.async.wait_group %0;" ::"n"(LEFT) : "memory");
+}
+
+// Rows `first .. first + n` of src [tokens][ld] from column `at` on, `width` numbers each, to dst [C][dst_ld], a warp per row; rows
+// past n and columns from `width` to `padded` become zeros. W numbers a copy.
+template <int W>
+__device__ __forceinline__ void stage_rows(float* dst, int dst_ld, const float* src, int64_t first, int n, int64_t ld, int64_t at, int width, int padded) {
+  const int lane = threadIdx.x & 31;
+  for (int r = threadIdx.x >> 5; r < C; r += kWarps) {
+    const float* from = src + (r < n ? (first + r) * ld + at : 0);
+    for (int c = lane * W; c < padded; c += 32 * W) {
+      const bool valid = r < n && c < width;
+      stage_copy<4 * W>(dst + r * dst_ld + c, valid ? from + c : src, valid);
+    }
+  }
+}
+
+// Two 32-bit numbers in one register pair, multiplied and added as such (two FMAs an instruction).
+using pair_t = unsigned long long;
+__device__ __forceinline__ pair_t fma_pair(pair_t a, pair_t b, pair_t c) {
+  pair_t d;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+  return d;
+}
+__device__ __forceinline__ pair_t mul_pair(pair_t a, pair_t b) {
+  pair_t d;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+  return d;
+}
+__device__ __forceinline__ float sum_pair(pair_t a) {
+  float x, y;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(x), "=f"(y) : "l"(a));
+  return x + y;
+}
+struct quad_t {  // four neighbouring numbers
+  pair_t lo, hi;
+};
+__device__ __forceinline__ quad_t load_quad(const float* p) {
+  const ulonglong2 v = *reinterpret_cast<const ulonglong2*>(p);
+  return {v.x, v.y};
+}
+
+// What `chunk_prepare` hands on, and the walk's result. Rows of `padded_rows(dk)` and `padded_columns(dv)` numbers, so all copies
+// are whole 16-byte steps whatever the sizes.
+struct Scratch {
+  float* y;   // [tokens][heads][rows]
+  float* kd;  // [tokens][heads][rows]: G_last,j k_j
+  float* qt;  // [tokens][heads][rows]: e_i q_i
+  float* x;   // [tokens][heads][columns]: W, then U
+  float* a;   // [tokens][heads][C]
+  float* e;   // [chunks][heads][rows]: e_last
+  float* s;   // [chunks][heads][rows][columns]: the state in front of each chunk
+};
+
+// Solves (I + l) x = rhs in place, row after row: x_i = rhs_i - sum_{j < i} l[i][j] x_j.
+__device__ __forceinline__ void substitute(const float* l, float (&x)[C]) {
+#pragma unroll
+  for (int i = 1; i < C; ++i) {
+    float sum0 = x[i], sum1 = 0.f;
+#pragma unroll
+    for (int j = 0; j < i; j += 4) {
+      const float4 row = *reinterpret_cast<const float4*>(l + i * C + j);
+      sum0 = fmaf(-row.x, x[j], sum0);
+      if (j + 1 < i) sum1 = fmaf(-row.y, x[j + 1], sum1);
+      if (j + 2 < i) sum0 = fmaf(-row.z, x[j + 2], sum0);
+      if (j + 3 < i) sum1 = fmaf(-row.w, x[j + 3], sum1);
+    }
+    x[i] = sum0 + sum1;
+  }
+}
+
+// --- what does not depend on the state -------------------------------------------------------------------------------------------
+//
+// One block per (chunk, head, request). Pairs of tokens: the chunk's rows form four groups of eight. Inside a group a lane has a token
+// j and carries p = G_ij k_j from row to row. Between groups every decay product splits at the group's border, G_ij = (product up
+// to i inside i's group) (whole groups between) (product from j + 1 to the end of j's group), three factors without a quotient, so
+// those pairs are plain products of scaled rows. A warp has an eighth of the channels; the warps' sums meet in shared memory.
+// PER_HEAD: one decay per head, given as its logarithm; pairs are products of the raw rows and G_ij = exp of the sum of logarithms.
+// Columns: a thread per column of [e K | V] solves the triangular system by substitution.
+constexpr int kGroup = 8, kGroups = C / kGroup;
+constexpr int kBetween = 6;                                  // pairs of groups
+constexpr int kWarpSums = (kBetween * 4 + 2 * kGroup) * 32;  // numbers that a warp hands on
+
+size_t prepare_smem(int rows) {
+  return sizeof(float) * (3 * C * (rows + 4) + kGroups * rows + kWarps * kWarpSums + 2 * C * (C + 1) + C * C + 3 * C);
+}
+
+template <int W, bool PER_HEAD>
+__global__ void __launch_bounds__(kThreads, 2)
+chunk_prepare_kernel(const float* q, const float* k, const float* v, const float* beta, const float* decay, const int* __restrict__ seq_q_start,
+                     const int* __restrict__ seq_q_len, int heads, int kv_heads, int dk, int dv, Scratch to) {
+  extern __shared__ __align__(16) float chunk_smem[];
+  let_successor_start();
+  const int seq = blockIdx.z, head = blockIdx.y, chunk = blockIdx.x;
+  const int n = min(C, seq_q_len[seq] - chunk * C);
+  if (n <= 0) return;
+  const int start = seq_q_start[seq], kvh = head / (heads / kv_heads);
+  const int64_t first = static_cast<int64_t>(start) + chunk * C;
+  const int rows = padded_rows(dk), columns = padded_columns(dv), ld = rows + 4;
+  float* ks = chunk_smem;                     // [C][ld]: keys, then times the decays of their group up to their own token
+  float* qs = ks + C * ld;                    // [C][ld]: queries, then likewise
+  float* gs = qs + C * ld;                    // [C][ld]: decays, then keys times the decays from the next token to their group's end
+  float* whole = gs + C * ld;                 // [groups][rows]: each group's decays multiplied
+  float* ls = whole + kGroups * rows;         // [C][C]
+  float* sums = ls + C * C;                   // [warps][kWarpSums]
+  float* kk = sums + kWarps * kWarpSums;      // [C][C + 1]: k_i . G_ij k_j
+  float* qk = kk + C * (C + 1);               // [C][C + 1]: q_i . G_ij k_j
+  float* bs = qk + C * (C + 1);               // [C]: beta
+  float* es = bs + C;                         // [C]: PER_HEAD: e_i
+  float* fs = es + C;                         // [C]: PER_HEAD: G_last,j
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  wait_for_predecessor();
+  stage_rows<W>(ks, ld, k, first, n, static_cast<int64_t>(kv_heads) * dk, static_cast<int64_t>(kvh) * dk, dk, rows);
+  stage_rows<W>(qs, ld, q, first, n, static_cast<int64_t>(kv_heads) * dk, static_cast<int64_t>(kvh) * dk, dk, rows);
+  if (!PER_HEAD) stage_rows<W>(gs, ld, decay, first, n, static_cast<int64_t>(heads) * dk, static_cast<int64_t>(head) * dk, dk, rows);
+  if (tid < C) bs[tid] = tid < n ? beta[(first + tid) * heads + head] : 0.f;
+  commit_copies();
+  wait_copies<0>();
+  __syncthreads();
+  const int slice = rows / kWarps, c0 = warp * slice;
+  float* mine = sums + warp * kWarpSums;
+  {  // pairs inside a group: lane j, rows i = 8 (j / 8) + r
+    const int own = lane & 7;
+    const float* group = ks + (lane & ~7) * ld;
+    pair_t acc[kGroup][2];
+#pragma unroll
+    for (int r = 0; r < kGroup; ++r) acc[r][0] = acc[r][1] = 0;
+    for (int c = c0; c < c0 + slice; c += 4) {
+      const quad_t kj = load_quad(ks + lane * ld + c);
+      quad_t p = kj;
+      if (!PER_HEAD) p = {0, 0};
+#pragma unroll
+      for (int r = 0; r < kGroup; ++r) {
+        if (!PER_HEAD) {
+          const quad_t g = load_quad(group + 2 * C * ld + r * ld + c);
+          p.lo = r == own ? kj.lo : mul_pair(p.lo, g.lo);
+          p.hi = r == own ? kj.hi : mul_pair(p.hi, g.hi);
+        }
+        const quad_t ki = load_quad(group + r * ld + c), qi = load_quad(group + C * ld + r * ld + c);
+        acc[r][0] = fma_pair(ki.hi, p.hi, fma_pair(ki.lo, p.lo, acc[r][0]));
+        acc[r][1] = fma_pair(qi.hi, p.hi, fma_pair(qi.lo, p.lo, acc[r][1]));
+      }
+    }
+#pragma unroll
+    for (int r = 0; r < kGroup; ++r) {
+      mine[(kBetween * 4 + r * 2) * 32 + lane] = sum_pair(acc[r][0]);
+      mine[(kBetween * 4 + r * 2 + 1) * 32 + lane] = sum_pair(acc[r][1]);
+    }
+  }
+  if (!PER_HEAD) {
+    __syncthreads();
+    for (int item = tid; item < kGroups * rows; item += kThreads) {  // a thread per (group, channel)
+      const int c = item % rows, at = item / rows * kGroup * ld + c;
+      float key[kGroup], g[kGroup];
+      float run = 1.f;
+#pragma unroll
+      for (int r = 0; r < kGroup; ++r) {
+        key[r] = ks[at + r * ld];
+        g[r] = item / rows * kGroup + r < n ? gs[at + r * ld] : 1.f;
+        run *= g[r];
+        ks[at + r * ld] = key[r] * run;
+        qs[at + r * ld] *= run;
+      }
+      whole[item] = run;
+      run = 1.f;
+#pragma unroll
+      for (int r = kGroup - 1; r >= 0; --r) {
+        gs[at + r * ld] = key[r] * run;
+        run *= g[r];
+      }
+    }
+    __syncthreads();
+  }
+  {  // pairs of two groups, b before g: lane = token 8 b + lane % 8, rows 8 g + 2 (lane / 8) and the next one
+    const float* ends = (PER_HEAD ? ks : gs) + (lane & 7) * ld;
+    const float* left = ks + (lane >> 3) * 2 * ld;
+    pair_t acc[kBetween][4];
+#pragma unroll
+    for (int x = 0; x < kBetween; ++x) acc[x][0] = acc[x][1] = acc[x][2] = acc[x][3] = 0;
+    for (int c = c0; c < c0 + slice; c += 4) {
+      quad_t p[kGroups - 1];
+#pragma unroll
+      for (int b = 0; b < kGroups - 1; ++b) p[b] = load_quad(ends + b * kGroup * ld + c);
+      int x = 0;
+#pragma unroll
+      for (int g = 1; g < kGroups; ++g) {
+        if (!PER_HEAD && g > 1) {  // the groups that are now whole ones between
+          const quad_t between = load_quad(whole + (g - 1) * rows + c);
+#pragma unroll
+          for (int b = 0; b < g - 1; ++b) p[b].lo = mul_pair(p[b].lo, between.lo), p[b].hi = mul_pair(p[b].hi, between.hi);
+        }
+        const float* at = left + g * kGroup * ld + c;
+        const quad_t k0 = load_quad(at), k1 = load_quad(at + ld), q0 = load_quad(at + C * ld), q1 = load_quad(at + C * ld + ld);
+#pragma unroll
+        for (int b = 0; b < g; ++b, ++x) {
+          acc[x][0] = fma_pair(k0.hi, p[b].hi, fma_pair(k0.lo, p[b].lo, acc[x][0]));
+          acc[x][1] = fma_pair(q0.hi, p[b].hi, fma_pair(q0.lo, p[b].lo, acc[x][1]));
+          acc[x][2] = fma_pair(k1.hi, p[b].hi, fma_pair(k1.lo, p[b].lo, acc[x][2]));
+          acc[x][3] = fma_pair(q1.hi, p[b].hi, fma_pair(q1.lo, p[b].lo, acc[x][3]));
+        }
+      }
+    }
+#pragma unroll
+    for (int x = 0; x < kBetween; ++x)
+#pragma unroll
+      for (int o = 0; o < 4; ++o) mine[(x * 4 + o) * 32 + lane] = sum_pair(acc[x][o]);
+  }
+  __syncthreads();
+  for (int idx = tid; idx < kWarpSums; idx += kThreads) {
+    float sum = 0.f;
+#pragma unroll
+    for (int w = 0; w < kWarps; ++w) sum += sums[w * kWarpSums + idx];
+    const int o = idx / 32, l = idx % 32;
+    int i, j;
+    if (o < kBetween * 4) {
+      const int x = o / 4, g = x == 0 ? 1 : (x < 3 ? 2 : 3), b = x - (g == 1 ? 0 : (g == 2 ? 1 : 3));
+      i = g * kGroup + (l >> 3) * 2 + (o & 3) / 2, j = b * kGroup + (l & 7);
+    } else {
+      i = (l & ~7) + (o - kBetween * 4) / 2, j = l;
+    }
+    (o & 1 ? qk : kk)[i * (C + 1) + j] = sum;
+  }
+  __syncthreads();
+  {
+    float own = 0.f, d = 0.f, prefix = 0.f, e = 0.f;
+    if (PER_HEAD) own = lane < n ? decay[(first + lane) * heads + head] : 0.f;
+    float* a = to.a + (first * heads + head) * C + lane;
+    for (int i = 0; i < C; ++i) {
+      if (PER_HEAD) {  // D_ij of column j = lane, the sum of the logarithms from token j + 1 on, grows with i from zero at i = j
+        const float gi = __shfl_sync(0xffffffffu, own, i);
+        d = i > lane ? d + gi : 0.f;
+        prefix += gi;
+        if (i == lane) e = prefix;
+      }
+      if ((i & 7) == warp) {
+        const float between = PER_HEAD ? expf(d) : 1.f;
+        ls[i * C + lane] = lane < i ? bs[i] * between * kk[i * (C + 1) + lane] : 0.f;
+        if (i < n) a[static_cast<int64_t>(i) * heads * C] = lane <= i ? between * qk[i * (C + 1) + lane] : 0.f;
+      }
+    }
+    if (PER_HEAD && warp == 0) es[lane] = expf(e), fs[lane] = expf(d);  // d is now D_last,j: tokens past n added nothing
+  }
+  __syncthreads();
+  for (int column = tid; column < rows + columns; column += kThreads) {
+    float x[C];
+    float* to_x;
+    const int64_t stride = static_cast<int64_t>(heads) * (column < rows ? rows : columns);
+    if (column < rows) {
+      const int64_t at = (first * heads + head) * rows + column;
+      float* qt = to.qt + at;
+      float* kd = to.kd + at;
+      to_x = to.y + at;
+      float before[kGroups], after[kGroups];  // whole groups in front of and behind a token's own
+      if (!PER_HEAD) {
+        before[0] = after[kGroups - 1] = 1.f;
+#pragma unroll
+        for (int g = 1; g < kGroups; ++g) before[g] = before[g - 1] * whole[(g - 1) * rows + column];
+#pragma unroll
+        for (int g = kGroups - 2; g >= 0; --g) after[g] = after[g + 1] * whole[(g + 1) * rows + column];
+      }
+#pragma unroll
+      for (int i = 0; i < C; ++i) {
+        const float key = ks[i * ld + column], e = PER_HEAD ? es[i] : before[i / kGroup];
+        if (i < n) {
+          *qt = e * qs[i * ld + column];
+          *kd = PER_HEAD ? fs[i] * key : after[i / kGroup] * gs[i * ld + column];
+        }
+        qt += stride, kd += stride;
+        x[i] = -bs[i] * e * key;
+      }
+      to.e[(chunk_place(start, seq, chunk) * heads + head) * rows + column] =
+          PER_HEAD ? es[n - 1] : before[kGroups - 1] * whole[(kGroups - 1) * rows + column];
+    } else {
+      const int c = column - rows;
+      const float* value = v + (first * heads + head) * dv + c;
+      to_x = to.x + (first * heads + head) * columns + c;
+#pragma unroll
+      for (int i = 0; i < C; ++i) x[i] = i < n && c < dv ? value[static_cast<int64_t>(i) * heads * dv] : 0.f;
+#pragma unroll
+      for (int i = 0; i < C; ++i) x[i] *= bs[i];
+    }
+    substitute(ls, x);
+#pragma unroll
+    for (int i = 0; i < C; ++i) {
+      if (i < n) *to_x = x[i];
+      to_x += stride;
+    }
+  }
+}
+
+// --- the walk ------------------------------------------------------------------------------------------------------------------------
+//
+// One block per (16 columns of the state, head, request). U = W + Y S: a warp has four tokens, its lanes four groups of columns times
+// eight parts of the rows, whose sums meet by shuffles. S <- e S + Kd^T U: a warp has an eighth of the rows, a lane four rows by four
+// columns over every kSplit-th token; after the shuffles it keeps its kPer rows of S in registers, with a transposed copy in shared
+// memory for the next chunk's first product.
+__host__ __device__ constexpr int walk_stage(int rows) { return 2 * C * (rows + 4) + C * kColumns + rows; }
+__host__ __device__ constexpr int walk_tile(int rows) { return kColumns * (rows + 8); }
+constexpr int kMaxRowX = 24;
+constexpr size_t walk_smem(int rows) { return sizeof(float) * (2 * walk_stage(rows) + walk_tile(rows) + C * kMaxRowX); }
+
+__device__ __forceinline__ float from_pair(float give, float keep, int with) { return keep + __shfl_xor_sync(0xffffffffu, give, with); }
+
+template <int ROWS>
+__global__ void __launch_bounds__(kThreads, ROWS <= 128 ? 2 : 1)
+chunk_walk_kernel(const int* __restrict__ seq_q_start, const int* __restrict__ seq_q_len, const int* __restrict__ seq_slot, int heads, int dk, int dv,
+                  Scratch from, float* state) {
+  extern __shared__ __align__(16) float chunk_smem[];
+  constexpr int kSplit = kThreads / ROWS;         // lanes that share a tile of S: 4, 2 or 1
+  constexpr int kPer = 4 / kSplit;                // rows of S that a lane keeps
+  constexpr int kLd = ROWS + 4;
+  constexpr int kLdS = ROWS + 8;                  // 8 banks from column to column
+  constexpr int kRowX = kSplit == 4 ? 24 : 16;    // the rows that lanes read side by side in different banks
+  let_successor_start();
+  const int col0 = blockIdx.x * kColumns, head = blockIdx.y, seq = blockIdx.z;
+  const int start = seq_q_start[seq], len = seq_q_len[seq];
+  const int columns = padded_columns(dv);
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  float* tile = chunk_smem + 2 * walk_stage(ROWS);  // [16 columns][kLdS]: S, transposed
+  float* xs = tile + walk_tile(ROWS);               // [C][kRowX]: U
+  const int chunks = (len + C - 1) / C;
+  auto fetch = [&](int chunk) {
+    float* ys = chunk_smem + (chunk & 1) * walk_stage(ROWS);
+    float* kds = ys + C * kLd;
+    float* ws = kds + C * kLd;
+    float* es = ws + C * kColumns;
+    const int n = min(C, len - chunk * C);
+    const int64_t first = static_cast<int64_t>(start) + chunk * C;
+#pragma unroll
+    for (int idx = tid; idx < C * ROWS / 4; idx += kThreads) {
+      const int r = idx / (ROWS / 4), c = idx % (ROWS / 4) * 4;
+      const int64_t at = r < n ? ((first + r) * heads + head) * ROWS + c : 0;
+      stage_copy<16>(ys + r * kLd + c, from.y + at, r < n);
+      stage_copy<16>(kds + r * kLd + c, from.kd + at, r < n);
+    }
+    if (tid < C * kColumns / 4) {
+      const int r = tid / 4, c = tid % 4 * 4;
+      stage_copy<16>(ws + r * kColumns + c, from.x + (r < n ? ((first + r) * heads + head) * columns + col0 + c : 0), r < n);
+    } else if (tid < C * kColumns / 4 + ROWS / 4) {
+      const int c = (tid - C * kColumns / 4) * 4;
+      stage_copy<16>(es + c, from.e + (chunk_place(start, seq, chunk) * heads + head) * ROWS + c, true);
+    }
+    commit_copies();
+  };
+  const int jp = lane % kSplit, cg = lane / kSplit % 4;
+  const int quad = warp * (ROWS / kWarps) + lane / (4 * kSplit) * 4;  // the lane's tile: rows quad .. + 3, columns 4 cg .. + 3
+  const int row0 = quad + jp * kPer;                                  // the rows it keeps
+  float* s_base = state + (static_cast<int64_t>(seq_slot[seq]) * heads + head) * dk * dv + col0;
+  float s[kPer][4];
+  wait_for_predecessor();
+  if (chunks > 0) fetch(0);
+#pragma unroll
+  for (int r = 0; r < kPer; ++r)
+#pragma unroll
+    for (int c = 0; c < 4; ++c)
+      s[r][c] = row0 + r < dk && col0 + cg * 4 + c < dv ? s_base[static_cast<int64_t>(row0 + r) * dv + cg * 4 + c] : 0.f;
+  for (int chunk = 0; chunk < chunks; ++chunk) {
+    const int n = min(C, len - chunk * C);
+    const int64_t first = static_cast<int64_t>(start) + chunk * C;
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+      float* to = tile + (cg * 4 + c) * kLdS + row0;
+      if (kPer == 4) *reinterpret_cast<float4*>(to) = make_float4(s[0][c], s[kPer / 4][c], s[kPer / 2][c], s[kPer - 1][c]);
+      else if (kPer == 2) *reinterpret_cast<float2*>(to) = make_float2(s[0][c], s[kPer - 1][c]);
+      else *to = s[0][c];
+    }
+    wait_copies<0>();
+    __syncthreads();  // S and the chunk's operands are there, and nobody reads the other stage any more
+    if (chunk + 1 < chunks) fetch(chunk + 1);
+    const float* ys = chunk_smem + (chunk & 1) * walk_stage(ROWS);
+    const float* kds = ys + C * kLd;
+    const float* ws = kds + C * kLd;
+    const float* es = ws + C * kColumns;
+    {
+      // Tokens 4 warp .. + 3, columns ct, ct + 4, .., every eighth group of four rows; sums over even and odd rows side by side.
+      const int ct = lane & 3, part = lane >> 2;
+      const float* y = ys + warp * 4 * kLd + part * 4;
+      const float* t = tile + ct * kLdS + part * 4;
+      pair_t acc[4][4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int c = 0; c < 4; ++c) acc[i][c] = 0;
+#pragma unroll
+      for (int k = 0; k < ROWS; k += 32) {
+        quad_t a[4], b[4];
+#pragma unroll
+        for (int x = 0; x < 4; ++x) {
+          a[x] = load_quad(y + x * kLd + k);
+          b[x] = load_quad(t + x * 4 * kLdS + k);
+        }
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+          for (int c = 0; c < 4; ++c) acc[i][c] = fma_pair(a[i].hi, b[c].hi, fma_pair(a[i].lo, b[c].lo, acc[i][c]));
+      }
+      // The eight parts meet: a lane ends with two columns of one token.
+      const bool b2 = lane & 4, b3 = lane & 8, b4 = lane & 16;
+      float sum[4][4], two[2][4], row[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int c = 0; c < 4; ++c) sum[i][c] = sum_pair(acc[i][c]);
+#pragma unroll
+      for (int i = 0; i < 2; ++i)
+#pragma unroll
+        for (int c = 0; c < 4; ++c) two[i][c] = from_pair(b2 ? sum[i][c] : sum[i + 2][c], b2 ? sum[i + 2][c] : sum[i][c], 4);
+#pragma unroll
+      for (int c = 0; c < 4; ++c) row[c] = from_pair(b3 ? two[0][c] : two[1][c], b3 ? two[1][c] : two[0][c], 8);
+      const int i = warp * 4 + (b2 ? 2 : 0) + (b3 ? 1 : 0), c = ct + (b4 ? 8 : 0);
+      const float u0 = from_pair(b4 ? row[0] : row[2], b4 ? row[2] : row[0], 16) + ws[i * kColumns + c];
+      const float u1 = from_pair(b4 ? row[1] : row[3], b4 ? row[3] : row[1], 16) + ws[i * kColumns + c + 4];
+      xs[i * kRowX + c] = u0, xs[i * kRowX + c + 4] = u1;
+      if (i < n) {
+        float* to = from.x + ((first + i) * heads + head) * columns + col0 + c;
+        to[0] = u0, to[4] = u1;
+      }
+    }
+    // The state in front of the chunk, for `chunk_out`.
+    float* s_out = from.s + ((chunk_place(start, seq, chunk) * heads + head) * ROWS + row0) * columns + col0 + cg * 4;
+#pragma unroll
+    for (int r = 0; r < kPer; ++r) *reinterpret_cast<float4*>(s_out + static_cast<int64_t>(r) * columns) = make_float4(s[r][0], s[r][1], s[r][2], s[r][3]);
+    __syncthreads();
+    {
+      float add[4][4];  // summed apart from the state, which is rounded once a chunk
+#pragma unroll
+      for (int r = 0; r < 4; ++r) add[r][0] = add[r][1] = add[r][2] = add[r][3] = 0.f;
+      const float* kd = kds + jp * kLd + quad;
+      const float* x = xs + jp * kRowX + cg * 4;
+#pragma unroll 4
+      for (int j = 0; j < C; j += kSplit) {
+        const float4 u = *reinterpret_cast<const float4*>(x + j * kRowX);
+        const float4 kj = *reinterpret_cast<const float4*>(kd + j * kLd);
+        const float f[4] = {kj.x, kj.y, kj.z, kj.w};
+#pragma unroll
+        for (int r = 0; r < 4; ++r) {
+          add[r][0] = fmaf(f[r], u.x, add[r][0]), add[r][1] = fmaf(f[r], u.y, add[r][1]);
+          add[r][2] = fmaf(f[r], u.z, add[r][2]), add[r][3] = fmaf(f[r], u.w, add[r][3]);
+        }
+      }
+      // The lanes of a tile meet, each keeping kPer rows.
+      if (kSplit == 4) {
+        const bool high = jp & 2;
+#pragma unroll
+        for (int r = 0; r < 2; ++r)
+#pragma unroll
+          for (int c = 0; c < 4; ++c) add[r][c] = from_pair(high ? add[r][c] : add[r + 2][c], high ? add[r + 2][c] : add[r][c], 2);
+      }
+      if (kSplit >= 2) {
+        const bool high = jp & 1;
+#pragma unroll
+        for (int r = 0; r < kPer; ++r)
+#pragma unroll
+          for (int c = 0; c < 4; ++c) add[r][c] = from_pair(high ? add[r][c] : add[r + kPer][c], high ? add[r + kPer][c] : add[r][c], 1);
+      }
+#pragma unroll
+      for (int r = 0; r < kPer; ++r) {
+        const float e = es[row0 + r];
+#pragma unroll
+        for (int c = 0; c < 4; ++c) s[r][c] = fmaf(e, s[r][c], add[r][c]);
+      }
+    }
+  }
+  if (chunks > 0) {
+#pragma unroll
+    for (int r = 0; r < kPer; ++r)
+#pragma unroll
+      for (int c = 0; c < 4; ++c)
+        if (row0 + r < dk && col0 + cg * 4 + c < dv) s_base[static_cast<int64_t>(row0 + r) * dv + cg * 4 + c] = s[r][c];
+  }
+}
+
+// --- outputs ---------------------------------------------------------------------------------------------------------------------------
+//
+// One block per (chunk, head, request and 128 columns): O = Qt S + A U as one product over rows + 32 numbers, 32 of them at a time
+// by cp.async in two stages. A thread has eight tokens and four neighbouring columns: 12 numbers read for 32 FMAs, since what an SM
+// takes out of shared memory (32 numbers a cycle, however many lanes want the same one) bounds this kernel.
+constexpr int kOutColumns = 128;
+constexpr int kOutThreads = 128;
+constexpr int kLdOut = kOutColumns + 4;
+constexpr int kLdSlab = C + 4;
+constexpr size_t kOutSmem = sizeof(float) * 2 * (C * kLdSlab + C * kLdOut);
+
+__global__ void __launch_bounds__(kOutThreads)
+chunk_out_kernel(const int* __restrict__ seq_q_start, const int* __restrict__ seq_q_len, int heads, int dv, int rows, int tiles, Scratch from, float* out) {
+  extern __shared__ __align__(16) float chunk_smem[];
+  let_successor_start();
+  const int seq = blockIdx.z / tiles, col0 = blockIdx.z % tiles * kOutColumns, head = blockIdx.y, chunk = blockIdx.x;
+  const int start = seq_q_start[seq], n = min(C, seq_q_len[seq] - chunk * C);
+  if (n <= 0) return;
+  const int64_t first = static_cast<int64_t>(start) + chunk * C;
+  const int columns = padded_columns(dv), width = min(kOutColumns, columns - col0);
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const float* states = from.s + (chunk_place(start, seq, chunk) * heads + head) * rows * columns + col0;
+  const int slabs = rows / C + 1;
+  wait_for_predecessor();
+  auto fetch = [&](int slab) {
+    float* left = chunk_smem + (slab & 1) * (C * kLdSlab + C * kLdOut);
+    float* right = left + C * kLdSlab;
+    const bool last = slab == slabs - 1;
+#pragma unroll
+    for (int half = 0; half < 2; ++half) {
+      const int r = (tid >> 3) + 16 * half, c = (tid & 7) * 4;
+      const int64_t row = (first + r) * heads + head;
+      stage_copy<16>(left + r * kLdSlab + c, r < n ? (last ? from.a + row * C + c : from.qt + row * rows + slab * C + c) : from.a, r < n);
+    }
+    const int c = lane * 4;
+#pragma unroll
+    for (int r = warp; r < C; r += kOutThreads / 32) {
+      const bool valid = c < width && (!last || r < n);
+      const float* at = last ? from.x + ((first + r) * heads + head) * columns + col0 + c : states + static_cast<int64_t>(slab * C + r) * columns + c;
+      stage_copy<16>(right + r * kLdOut + c, valid ? at : from.a, valid);
+    }
+    commit_copies();
+  };
+  const int ct = (lane & 7) + 8 * warp, it = lane >> 3;  // columns 4 ct .. + 3, tokens it, it + 4, ..
+  float acc[8][4];
+#pragma unroll
+  for (int i = 0; i < 8; ++i) acc[i][0] = acc[i][1] = acc[i][2] = acc[i][3] = 0.f;
+  fetch(0);
+  for (int slab = 0; slab < slabs; ++slab) {
+    if (slab + 1 < slabs) {
+      fetch(slab + 1);
+      wait_copies<1>();
+    } else {
+      wait_copies<0>();
+    }
+    __syncthreads();
+    const float* left = chunk_smem + (slab & 1) * (C * kLdSlab + C * kLdOut) + it * kLdSlab;
+    const float* right = chunk_smem + (slab & 1) * (C * kLdSlab + C * kLdOut) + C * kLdSlab + ct * 4;
+    float sum[8][4];  // one slab's sum by itself: fewer roundings of the whole
+#pragma unroll
+    for (int i = 0; i < 8; ++i) sum[i][0] = sum[i][1] = sum[i][2] = sum[i][3] = 0.f;
+#pragma unroll 2
+    for (int k = 0; k < C; k += 4) {
+      float4 b[4];
+#pragma unroll
+      for (int x = 0; x < 4; ++x) b[x] = *reinterpret_cast<const float4*>(right + (k + x) * kLdOut);
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        const float4 a = *reinterpret_cast<const float4*>(left + i * 4 * kLdSlab + k);
+        const float f[4] = {a.x, a.y, a.z, a.w};
+#pragma unroll
+        for (int x = 0; x < 4; ++x) {
+          sum[i][0] = fmaf(f[x], b[x].x, sum[i][0]), sum[i][1] = fmaf(f[x], b[x].y, sum[i][1]);
+          sum[i][2] = fmaf(f[x], b[x].z, sum[i][2]), sum[i][3] = fmaf(f[x], b[x].w, sum[i][3]);
+        }
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < 8; ++i) acc[i][0] += sum[i][0], acc[i][1] += sum[i][1], acc[i][2] += sum[i][2], acc[i][3] += sum[i][3];
+    __syncthreads();
+  }
+  const int c = col0 + ct * 4;
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    const int row = it + 4 * i;
+    if (row >= n) continue;
+    float* to = out + ((first + row) * heads + head) * dv + c;
+    if (dv % 4 == 0 && (reinterpret_cast<uintptr_t>(out) & 15) == 0) {
+      if (c < dv) *reinterpret_cast<float4*>(to) = make_float4(acc[i][0], acc[i][1], acc[i][2], acc[i][3]);
+    } else {
+#pragma unroll
+      for (int x = 0; x < 4; ++x)
+        if (c + x < dv) to[x] = acc[i][x];
+    }
+  }
+}
+
+// --- host ------------------------------------------------------------------------------------------------------------------------------
+
+struct Sizes {
+  int tokens, seqs, heads, dk, dv;
+};
+
+int64_t aligned_floats(int64_t n) { return (n + 3) / 4 * 4; }
+
+// The scratch's arrays one after another in `base` (null pointers with a null base); returns the numbers they need.
+int64_t lay_out(const Sizes& z, float* base, Scratch* to) {
+  const int64_t rows = padded_rows(z.dk), columns = padded_columns(z.dv), per_head = static_cast<int64_t>(z.tokens) * z.heads;
+  const int64_t chunks = (static_cast<int64_t>(z.tokens) / C + z.seqs + 1) * z.heads;
+  const int64_t sizes[7] = {per_head * rows, per_head * rows, per_head * rows, per_head * columns, per_head * C, chunks * rows, chunks * rows * columns};
+  float** arrays[7] = {&to->y, &to->kd, &to->qt, &to->x, &to->a, &to->e, &to->s};
+  int64_t at = 0;
+  for (int i = 0; i < 7; ++i) {
+    *arrays[i] = base == nullptr ? nullptr : base + at;
+    at += aligned_floats(sizes[i]);
+  }
+  return at;
+}
+
+template <typename Kernel>
+bool raise_smem(Kernel kernel, size_t bytes) {
+  return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(bytes)) == cudaSuccess;
+}
+
+bool raise_all() {
+  static const bool raised =
+      raise_smem(chunk_prepare_kernel<1, false>, prepare_smem(kMaxRows)) && raise_smem(chunk_prepare_kernel<4, false>, prepare_smem(kMaxRows)) &&
+      raise_smem(chunk_prepare_kernel<1, true>, prepare_smem(kMaxRows)) && raise_smem(chunk_prepare_kernel<4, true>, prepare_smem(kMaxRows)) &&
+      raise_smem(chunk_walk_kernel<64>, walk_smem(64)) && raise_smem(chunk_walk_kernel<128>, walk_smem(128)) && raise_smem(chunk_walk_kernel<256>, walk_smem(256));
+  return raised;
+}
+
+bool aligned16(const void* p) { return reinterpret_cast<uintptr_t>(p) % 16 == 0; }
+
+}  // namespace
+
+// Sizes the chunked form takes; the caller walks token by token otherwise.
+B200_API int b200_delta_chunks_supported(int heads, int kv_heads, int dk, int dv) {
+  return heads > 0 && heads <= 65535 && kv_heads > 0 && heads % kv_heads == 0 && dk > 0 && dk <= kMaxRows && dv > 0 && dv <= 65536;
+}
+
+// Numbers of scratch (32-bit, aligned to 16 bytes) that a call needs.
+B200_API int64_t b200_delta_chunks_scratch(int tokens, int seqs, int heads, int dk, int dv) {
+  Scratch scratch;
+  return lay_out({tokens, seqs, heads, dk, dv}, nullptr, &scratch);
+}
+
+// The delta rule over every request's new tokens; operands as `delta_prepare` leaves them. per_head = 0: `decay` [tokens][heads][dk]
+// holds factors; per_head = 1: [tokens][heads] logarithms.
+B200_API int b200_delta_chunks(const float* q, const float* k, const float* v, const float* beta, const float* decay, int per_head, const int* seq_q_start,
+                               const int* seq_q_len, const int* seq_slot, int tokens, int seqs, int max_q_len, int heads, int kv_heads, int dk, int dv,
+                               float* scratch, int64_t scratch_floats, float* state, float* out, cudaStream_t stream) {
+  if (seqs == 0 || tokens == 0) return 0;
+  B200_REQUIRE(tokens > 0 && seqs > 0 && max_q_len > 0 && b200_delta_chunks_supported(heads, kv_heads, dk, dv), "delta_chunks: shape not taken");
+  const Sizes z = {tokens, seqs, heads, dk, dv};
+  Scratch parts;
+  B200_REQUIRE(aligned16(scratch) && lay_out(z, scratch, &parts) <= scratch_floats, "delta_chunks: scratch too small or not aligned to 16 bytes");
+  const int rows = padded_rows(dk), columns = padded_columns(dv), chunks = (max_q_len + C - 1) / C, tiles = (columns + kOutColumns - 1) / kOutColumns;
+  B200_REQUIRE(static_cast<int64_t>(seqs) * tiles <= 65535, "delta_chunks: too many requests");
+  B200_REQUIRE(raise_all(), "delta_chunks: cannot size shared memory");
+  const bool wide = dk % 4 == 0 && aligned16(q) && aligned16(k) && (per_head || aligned16(decay));
+  auto prepare = per_head ? (wide ? chunk_prepare_kernel<4, true> : chunk_prepare_kernel<1, true>) : (wide ? chunk_prepare_kernel<4, false> : chunk_prepare_kernel<1, false>);
+  launch_kernel(prepare, dim3(chunks, heads, seqs), dim3(kThreads), prepare_smem(rows), stream, q, k, v, beta, decay, seq_q_start, seq_q_len, heads, kv_heads,
+                dk, dv, parts);
+  if (int status = b200_check_launch("chunk_prepare")) return status;
+  auto walk = rows == 64 ? chunk_walk_kernel<64> : (rows == 128 ? chunk_walk_kernel<128> : chunk_walk_kernel<256>);
+  // The ordinary way, not early: the few long-lived blocks should spread over all SMs, not over those the kernel in front leaves first.
+  launch_kernel_as(true, walk, dim3(columns / kColumns, heads, seqs), dim3(kThreads), walk_smem(rows), stream, seq_q_start, seq_q_len, seq_slot, heads, dk, dv,
+                   parts, state);
+  if (int status = b200_check_launch("chunk_walk")) return status;
+  launch_kernel(chunk_out_kernel, dim3(chunks, heads, seqs * tiles), dim3(kOutThreads), kOutSmem, stream, seq_q_start, seq_q_len, heads, dv, rows, tiles, parts,
+                out);
+  return b200_check_launch("chunk_out");
+}

@@ -869,12 +869,45 @@ def delta_prepare(
     ctx.lib.calls += 1  # the slot update is a launch of its own
 
 
+# Longest portion that is walked token by token. One request, 12 heads of 128 x 128 on a B200, chunks against tokens: 49 and 39 us at
+# 64 tokens, 53 and 52 us at 100, 64 and 87 us at 200, 252 and 731 us at 2,048 (one decay per head within 4 us of the same).
+DELTA_CHUNK_FROM = 112
+
+
+def _delta_chunks(
+    ctx: StepContext, q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, beta: torch.Tensor, decay: torch.Tensor, per_head: bool,
+    state: torch.Tensor, out: torch.Tensor, heads: int, kv_heads: int, dk: int, dv: int,
+) -> bool:
+    """Portions of more than ``DELTA_CHUNK_FROM`` tokens run chunk by chunk (csrc/kernels/state_chunks.cu); returns False, doing
+    nothing, for shorter ones and for sizes the chunked form does not take. ``options["delta_portions"]``: ``"chunks"`` or
+    ``"tokens"`` forces one of the two."""
+    choice = ctx.options.get("delta_portions", "auto")
+    if choice == "tokens" or (choice == "auto" and not (
+        ctx.max_q_len > DELTA_CHUNK_FROM and ctx.lib.lib.b200_delta_chunks_supported(heads, kv_heads, dk, dv)
+    )):
+        return False
+    tokens = q.shape[0]
+    floats = int(ctx.lib.lib.b200_delta_chunks_scratch(tokens, ctx.num_seqs, heads, dk, dv))
+    scratch = ctx.buffer("delta_chunks", (floats,), torch.float32, per_token=False)
+    ctx.lib.call(
+        "b200_delta_chunks", ptr(q), ptr(k), ptr(v), ptr(beta), ptr(decay), c_int(1 if per_head else 0), ptr(ctx.seq_q_start), ptr(ctx.seq_q_len),
+        ptr(ctx.seq_slot), c_int(tokens), c_int(ctx.num_seqs), c_int(ctx.max_q_len), c_int(heads), c_int(kv_heads), c_int(dk), c_int(dv),
+        ptr(scratch), c_int64(floats), ptr(state), ptr(out), ctx.stream,
+    )
+    ctx.lib.calls += 2  # three kernels
+    return True
+
+
 def delta_recurrence(
     ctx: StepContext, q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, beta: torch.Tensor, decay: torch.Tensor,
     state: torch.Tensor, out: torch.Tensor, heads: int, kv_heads: int, dk: int, dv: int,
 ) -> torch.Tensor:
+    """The delta rule with a decay per head and key channel over every request's new tokens: chunk by chunk or token by token
+    (see ``_delta_chunks``)."""
     _need(state.dtype == torch.float32 and tuple(state.shape[1:]) == (heads, dk, dv) and state.is_contiguous(), "delta_recurrence: the state is float32 [slots, heads, dk, dv]")
     _need(out.dtype == torch.float32 and tuple(out.shape) == (q.shape[0], heads * dv) and out.is_contiguous(), "delta_recurrence: bad output")
+    if _delta_chunks(ctx, q, k, v, beta, decay, False, state, out, heads, kv_heads, dk, dv):
+        return out
     ctx.lib.call(
         "b200_delta_recurrence", ptr(q), ptr(k), ptr(v), ptr(beta), ptr(decay), ptr(ctx.seq_q_start), ptr(ctx.seq_q_len),
         ptr(ctx.seq_slot), c_int(ctx.num_seqs), c_int(heads), c_int(kv_heads), c_int(dk), c_int(dv), ptr(state), ptr(out),
@@ -899,30 +932,17 @@ def delta_output(
     return out
 
 
-DELTA_CHUNK_FROM = 64  # longest portion that is walked token by token: two more launches and a whole chunk a block cost about as much
-
-
 def delta_head_recurrence(
     ctx: StepContext, q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, beta: torch.Tensor, log_decay: torch.Tensor, kq: torch.Tensor,
     state: torch.Tensor, out: torch.Tensor, heads: int, kv_heads: int, dk: int, dv: int,
 ) -> torch.Tensor:
-    """The delta rule with one decay per head over every request's new tokens (operands as :func:`delta_prepare` leaves them).
-    Portions of more than ``DELTA_CHUNK_FROM`` tokens run chunk by chunk (two kernels, the 32 x 32 matrices of all chunks in
-    between), shorter ones token by token; ``options["delta_portions"]``: ``"chunks"`` or ``"tokens"`` forces one of them."""
+    """The delta rule with one decay per head over every request's new tokens (operands as :func:`delta_prepare` leaves them):
+    chunk by chunk or token by token (see ``_delta_chunks``)."""
     tokens = q.shape[0]
     _need(state.dtype == torch.float32 and tuple(state.shape[1:]) == (heads, dk, dv) and state.is_contiguous(), "delta_head_recurrence: the state is float32 [slots, heads, dk, dv]")
     for tensor, width in ((q, kv_heads * dk), (k, kv_heads * dk), (v, heads * dv), (beta, heads), (log_decay, heads), (kq, kv_heads), (out, heads * dv)):
         _need(tensor.dtype == torch.float32 and tuple(tensor.shape) == (tokens, width) and tensor.is_contiguous(), "delta_head_recurrence: bad operands")
-    choice = ctx.options.get("delta_portions", "auto")
-    if choice == "chunks" or (choice == "auto" and ctx.max_q_len > DELTA_CHUNK_FROM and ctx.lib.lib.b200_delta_chunks_supported(heads, kv_heads, dk, dv)):
-        attn, solve = (ctx.buffer("delta_" + name, (tokens, heads * 32), torch.float32) for name in ("chunk_attn", "chunk_solve"))
-        factors = ctx.buffer("delta_chunk_factors", (tokens, heads * 2), torch.float32)
-        ctx.lib.call(
-            "b200_delta_chunks", ptr(q), ptr(k), ptr(v), ptr(beta), ptr(log_decay), ptr(ctx.seq_q_start), ptr(ctx.seq_q_len), ptr(ctx.seq_slot),
-            c_int(ctx.num_seqs), c_int(ctx.max_q_len), c_int(heads), c_int(kv_heads), c_int(dk), c_int(dv), ptr(attn), ptr(solve), ptr(factors),
-            ptr(state), ptr(out), ctx.stream,
-        )
-        ctx.lib.calls += 1  # two kernels
+    if _delta_chunks(ctx, q, k, v, beta, log_decay, True, state, out, heads, kv_heads, dk, dv):
         return out
     ctx.lib.call(
         "b200_delta_head_recurrence", ptr(q), ptr(k), ptr(v), ptr(beta), ptr(log_decay), ptr(kq), ptr(ctx.seq_q_start), ptr(ctx.seq_q_len),

@@ -1,0 +1,90 @@
+"""Recurrent rules over prompt portions chunk by chunk and token by token, against the recurrences themselves in 64 bits, at the
+sizes where a chunk, a tile of the state or a wide copy ends: portions around multiples of 32 tokens, key and value sizes that are
+multiples of nothing, decays from one down to zero, states that come in."""
+
+from __future__ import annotations
+
+import numpy as np
+import pytest
+import torch
+
+from test_parts import context_for
+
+pytestmark = pytest.mark.gpu
+
+# All arithmetic is 32-bit: a sum of n products carries about sqrt(n) roundings of 6e-8, and a state here adds up at most a few hundred
+# unit-sized terms.
+CLOSE = dict(atol=2e-5, rtol=2e-5)
+
+
+def device_context(runs, slots, state_shapes, options):
+    from llm_inference_b200.parts import StateSpec
+
+    runner, cache, ctx = context_for({0: StateSpec(state_shapes, (torch.float32,) * len(state_shapes))}, torch.float32, [1] * len(runs))
+    ctx.options = options
+    as_device = lambda values: torch.tensor(values, dtype=torch.int32, device="cuda")
+    ctx.num_tokens, ctx.num_seqs, ctx.max_q_len = sum(runs), len(runs), max(runs)
+    ctx.seq_q_start, ctx.seq_q_len = as_device(np.concatenate([[0], np.cumsum(runs)[:-1]]).tolist()), as_device(list(runs))
+    ctx.seq_slot = as_device(list(slots))
+    return runner, cache, ctx
+
+
+def on_device(array):
+    return torch.from_numpy(np.ascontiguousarray(array.reshape(array.shape[0], -1))).cuda()
+
+
+DELTA_SIZES = [
+    (2, 1, 128, 128, (113, 32, 1)),
+    (3, 3, 64, 16, (31, 65)),
+    (2, 2, 33, 17, (64, 33)),
+    (1, 1, 256, 40, (127,)),
+    (2, 2, 72, 130, (96, 95, 97)),
+]
+
+
+@pytest.mark.parametrize("heads,kv_heads,dk,dv,runs", DELTA_SIZES)
+@pytest.mark.parametrize("portions", ["chunks", "tokens"])
+@pytest.mark.parametrize("per_head", [False, True])
+def test_delta_rules(heads, kv_heads, dk, dv, runs, portions, per_head):
+    from llm_inference_b200.parts import ops
+
+    n = sum(runs)
+    rng = np.random.default_rng(dk + dv)
+    unit = lambda x: x / np.linalg.norm(x, axis=-1, keepdims=True)
+    q, k = unit(rng.normal(size=(n, kv_heads, dk))), unit(rng.normal(size=(n, kv_heads, dk)))
+    k[5:20] = k[5]  # keys that repeat, with beta near one: the triangular system at its stiffest
+    v, beta = rng.normal(size=(n, heads, dv)), rng.uniform(0.9, 1.0, (n, heads))
+    logs = -np.exp(rng.normal(-4, 3, (n, heads, 1 if per_head else dk)))
+    logs[3::29] = 0.0
+    logs[17::41, 0] = -400.0  # a memory that ends at once
+    start = rng.normal(size=(len(runs), heads, dk, dv))
+    q, k, v, beta, logs, start = (a.astype(np.float32) for a in (q, k, v, beta, logs, start))
+    decay = logs if per_head else np.exp(logs)
+    factors = np.broadcast_to(np.exp(logs.astype(np.float64)) if per_head else decay.astype(np.float64), (n, heads, dk))
+    states, want, at = start.astype(np.float64), np.zeros((n, heads, dv)), 0
+    share = heads // kv_heads
+    for s, run in enumerate(runs):
+        for t in range(at, at + run):
+            key, query = (x[t].repeat(share, axis=0).astype(np.float64) for x in (k, q))
+            S = states[s] * factors[t][..., None]
+            u = beta[t].astype(np.float64)[:, None] * (v[t] - np.einsum("hkv,hk->hv", S, key))
+            states[s] = S + key[..., None] * u[:, None]
+            want[t] = np.einsum("hkv,hk->hv", states[s], query)
+        at += run
+    slots = [4, 0, 2][: len(runs)]
+    runner, cache, ctx = device_context(runs, slots, ((heads, dk, dv),), {"delta_portions": portions})
+    state = cache.states[0][0]
+    untouched = state.clone().normal_()
+    state.copy_(untouched)
+    state[slots] = torch.from_numpy(start).cuda()
+    out = torch.full((n, heads * dv), float("nan"), device="cuda")
+    device = [on_device(a) for a in (q, k, v, beta, decay)]
+    if per_head:
+        ops.delta_head_recurrence(ctx, *device, on_device((q * k).sum(-1)), state, out, heads, kv_heads, dk, dv)
+    else:
+        ops.delta_recurrence(ctx, *device, state, out, heads, kv_heads, dk, dv)
+    runner.check()
+    np.testing.assert_allclose(out.double().cpu().numpy().reshape(want.shape), want, **CLOSE)
+    np.testing.assert_allclose(state[slots].double().cpu().numpy(), states, **CLOSE)
+    others = [slot for slot in range(state.shape[0]) if slot not in slots]
+    assert torch.equal(state[others], untouched[others])
