@@ -118,3 +118,14 @@ def build_part(kind: str, spec: PartSpec, **extra: Any) -> Part:
 
 def registered_parts(kind: str) -> tuple[str, ...]:
     return tuple(sorted(n for k, n in _PARTS if k == kind))
+
+
+def whole_steps(weight: torch.Tensor) -> torch.Tensor:
+    """The rows of several bfloat16 projections of one input, filled up with zero rows to a multiple of eight, so that the rows of
+    their common product are whole 16-byte steps apart (the added columns are read by nobody). With 4,620 columns the library's
+    product of 2,048 rows of 1,536 fell back to narrow copies and took 103 us on a B200, with 4,624 it takes 28. The 32-bit
+    product is this engine's own and takes any row length."""
+    short = -weight.shape[0] % 8
+    if weight.dtype == torch.bfloat16 and short:
+        weight = torch.cat([weight, weight.new_zeros((short, weight.shape[1]))])
+    return weight.contiguous()

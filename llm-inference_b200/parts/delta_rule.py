@@ -6,7 +6,7 @@ import torch
 
 from ..weights.loader import TensorSpec
 from . import ops
-from .base import Part, StateSpec, register_part
+from .base import Part, StateSpec, register_part, whole_steps
 from .context import CacheView, StepContext
 
 
@@ -73,7 +73,7 @@ class ChannelDeltaRule(Part):
         def get(name: str, to=dtype) -> torch.Tensor:
             return tensors[p + name].to(device=device, dtype=to)
 
-        self.w_main = torch.cat([get("q"), get("k"), get("v"), get("b")]).contiguous()
+        self.w_main = whole_steps(torch.cat([get("q"), get("k"), get("v"), get("b")]))
         a1, a2, g1, g2 = get("a1"), get("a2"), get("g1"), get("g2")
         self.w_low = torch.cat([a1, g1]).contiguous()
         ra, rg = a1.shape[0], g1.shape[0]
@@ -152,7 +152,7 @@ class HeadDeltaRule(Part):
         def get(name: str, to=dtype) -> torch.Tensor:
             return tensors[p + name].to(device=device, dtype=to).contiguous()
 
-        self.w_in = torch.cat([get(n) for n in ("q", "k", "v", "b", "a", "g")]).contiguous()
+        self.w_in = whole_steps(torch.cat([get(n) for n in ("q", "k", "v", "b", "a", "g")]))
         self.w_o = get("o")
         self.taps_w = torch.cat([get(n + ".conv", f32) for n in ("q", "k", "v")]).contiguous()
         self.a_log, self.dt_bias, self.norm_weight = get("A_log", f32), get("dt_bias", f32), get("norm", f32)
@@ -178,7 +178,7 @@ class HeadDeltaRule(Part):
             ops.delta_prepare(ctx, proj, proj[:, a_at : a_at + heads], self.taps_w, conv_state, self.a_log, self.dt_bias, heads, kvh, dk, dv,
                               q, k, v, beta, decay, kq)
             o = ops.delta_head_recurrence(ctx, q, k, v, beta, decay, kq, state, ctx.buffer("delta_o", (t, heads * dv), f32), heads, kvh, dk, dv)
-            ops.delta_output(ctx, o, self.norm_weight, proj[:, a_at + heads :], heads, dv, self.eps, y, silu=True)
+            ops.delta_output(ctx, o, self.norm_weight, proj[:, a_at + heads : a_at + heads + heads * dv], heads, dv, self.eps, y, silu=True)
         return y
 
 

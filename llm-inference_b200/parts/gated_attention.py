@@ -6,7 +6,7 @@ import torch
 
 from ..weights.loader import TensorSpec
 from . import ops
-from .base import KVCacheSpec, Part, register_part
+from .base import KVCacheSpec, Part, register_part, whole_steps
 from .context import CacheView, StepContext
 
 
@@ -69,7 +69,7 @@ class GatedAttention(Part):
     def load(self, tensors, dtype, device) -> None:
         p = self.prefix
         names = ["q", "k", "v"] + (["g"] if self.gate else [])
-        self.w_in = torch.cat([tensors[p + n].to(device=device, dtype=dtype) for n in names]).contiguous()
+        self.w_in = whole_steps(torch.cat([tensors[p + n].to(device=device, dtype=dtype) for n in names]))
         self.w_o = tensors[p + "o"].to(device=device, dtype=dtype).contiguous()
         if self.values == "blend":
             self.blend = tensors[p + "vmix"].to(device=device, dtype=torch.float32).reshape(1).contiguous()

@@ -6,7 +6,7 @@ import torch
 
 from ..weights.loader import TensorSpec
 from . import ops
-from .base import KVCacheSpec, Part, PartSpec, build_part, register_part
+from .base import KVCacheSpec, Part, PartSpec, build_part, register_part, whole_steps
 from .context import CacheView, StepContext
 
 
@@ -82,7 +82,7 @@ class LatentAttention(Part):
         if self.q_rank:
             self.w_uq = tensors[p + "uq"].to(device=device, dtype=dtype).contiguous()
             self.q_norm_weight = tensors[p + "dq.norm"].to(device=device, dtype=torch.float32).contiguous()
-        self.w_in = torch.cat([tensors[p + n].to(device=device, dtype=dtype) for n in names]).contiguous()
+        self.w_in = whole_steps(torch.cat([tensors[p + n].to(device=device, dtype=dtype) for n in names]))
         # [heads, rank, dim]: the product that carries a query into the latent space reads W_uk[n]^T.
         self.w_uk_t = tensors[p + "uk"].to(device=device, dtype=dtype).view(self.heads, self.dim, self.rank).transpose(1, 2).contiguous()
         self.w_uv = tensors[p + "uv"].to(device=device, dtype=dtype).view(self.heads, self.vdim, self.rank).contiguous()
@@ -118,7 +118,8 @@ class LatentAttention(Part):
             self.position.apply_latent(ctx, cache, proj, 0, kv_offset, heads, self.dim, rank, self.norm_weight, self.eps, q_rot)
         q_plain = queries.view(t, heads, self.dim + rot)[:, :, : self.dim].transpose(0, 1)
         q_lat = ops.linear_per_head(ctx, q_plain, self.w_uk_t, ctx.buffer("latent_q", (heads, t, rank)))
-        gate = proj[:, kv_offset + rank + rot :] if self.has_gate else None
+        gate_at, gates = kv_offset + rank + rot, heads * (self.vdim if self.gate_per_element else 1)
+        gate = proj[:, gate_at : gate_at + gates] if self.has_gate else None
         mixed = ctx.buffer("latent_out", (heads, t, rank))
         self.attend(ctx, cache, q_lat, q_rot, None if self.gate_per_element else gate, mixed)
         attn = ctx.buffer("attn", (t, heads * self.vdim))
