@@ -1,4 +1,5 @@
-// Delta rules over prompt portions, 32 tokens at a time.
+// Recurrent matrix states over prompt portions, 32 tokens at a time: the delta rule (one decay per head, or one per head and key
+// channel), the generalized delta rule, and the rule with a decay per channel and a bonus for the current token.
 //
 // Token by token a portion costs tokens x the latency of one step, however few columns a head's state has. Over a chunk of tokens
 // the rule S <- g S; u = beta (v - S^T k); S <- S + k u^T; o = S^T q is a handful of small matrix products (the chunkwise form of
@@ -8,10 +9,15 @@
 //   u_i = beta_i (v_i - S^T (e_i k_i) - sum_{j < i} (k_i . G_ij k_j) u_j),   o_i = S^T (e_i q_i) + sum_{j <= i} (q_i . G_ij k_j) u_j,
 //   S <- e_last S + sum_j (G_last,j k_j) u_j^T.
 // With L_ij = beta_i k_i . G_ij k_j (j < i): U = W + Y S, W = (I + L)^-1 diag(beta) V, Y = -(I + L)^-1 diag(beta) (e K).
-// Three kernels:
-//   chunk_prepare    all chunks side by side: A = (q_i . G_ij k_j), W, Y and the scaled e Q and G_last K;
+// The generalized rule S <- w S + b (u^T S) + k v^T (b = -a u), o = S^T r, has the same form in X_i = u_i^T S_{i-1}: with
+// N_ij = u_i . G_{i-1,j} b_j and M_ij = u_i . G_{i-1,j} k_j (j < i), X = W + Y S, W = (I - N)^-1 M V, Y = (I - N)^-1 (e_{i-1} u_i), and what
+// the values alone add to S and to o is known in front of the walk. Without the removal (S <- w S + k v^T, o = S^T r read before the
+// update) nothing is left of a walk but sums of whole chunks.
+// Kernels:
+//   chunk_prepare, linear_chunk_prepare   all chunks side by side: pairs of tokens, W, Y, scaled rows, the values' own sums;
 //   chunk_walk       a head's chunks one after another, a tile of 16 columns of S per block: U = W + Y S, S <- e S + (G_last K)^T U;
-//   chunk_out        all chunks side by side again: O = (e Q) S + A U, from the states that the walk left at each chunk's start.
+//   chunk_scan       the same without U: S <- e S + the chunk's own sum, element by element;
+//   chunk_out        all chunks side by side again: O = (e Q) S + A U, from the states left at each chunk's start.
 // Only what the next chunk waits for is in the walk. Everything is 32-bit FMAs (no reduced-precision tensor-core mode): state,
 // decays and gates stay what they are token by token, up to the order of sums. Decays enter as products (or sums of their logarithms)
 // from token j on, never as quotients of products from the chunk's start, so strong decays in front of a pair cost it no digits.
@@ -20,7 +26,8 @@
 // at dk = 128) and takes about twice as many cycles' worth of operands out of shared memory, between two block-wide barriers.
 // Measured on a B200 (one request of 2,048 tokens, heads of 128 x 128; all three kernels): a decay per channel, 12 heads: 731 us token
 // by token -> 252 us (prepare 60, walk 130, out 60), 28 heads: 941 -> 449; one decay per head (before: outputs and triangular products
-// inside the walk): 305 -> 252 and 525 -> 450.
+// inside the walk): 305 -> 252 and 525 -> 450. 24 heads of 64 x 64: the generalized rule 473 -> 244 us (prepare 100, walk 90, out 35), the
+// rule without a removal 564 -> 101 us (prepare 51, scan 16, out 27).
 #include "common.cuh"
 
 namespace {
@@ -94,9 +101,10 @@ struct Scratch {
   float* kd;  // [tokens][heads][rows]: G_last,j k_j
   float* qt;  // [tokens][heads][rows]: e_i q_i
   float* x;   // [tokens][heads][columns]: W, then U
-  float* a;   // [tokens][heads][C]
+  float* a;   // [tokens][heads][C]: what reads out U
+  float* av;  // [tokens][heads][C]: what reads out V
   float* e;   // [chunks][heads][rows]: e_last
-  float* s;   // [chunks][heads][rows][columns]: the state in front of each chunk
+  float* s;   // [chunks][heads][rows][columns]: what the values alone add, then the state in front of each chunk
 };
 
 // Solves (I + l) x = rhs in place, row after row: x_i = rhs_i - sum_{j < i} l[i][j] x_j.
@@ -125,14 +133,123 @@ __device__ __forceinline__ void substitute(const float* l, float (&x)[C]) {
 // PER_HEAD: one decay per head, given as its logarithm; pairs are products of the raw rows and G_ij = exp of the sum of logarithms.
 // Columns: a thread per column of [e K | V] solves the triangular system by substitution.
 constexpr int kGroup = 8, kGroups = C / kGroup;
-constexpr int kBetween = 6;                                  // pairs of groups
-constexpr int kWarpSums = (kBetween * 4 + 2 * kGroup) * 32;  // numbers that a warp hands on
+constexpr int kBetween = 6;  // pairs of groups
+__host__ __device__ constexpr int inside_sums(int lefts) { return kGroup * lefts * 32; }  // numbers that a warp hands on
+__host__ __device__ constexpr int between_sums(int lefts) { return kBetween * 2 * lefts * 32; }
 
+// left_i . G_ij right_j for i, j in one group, over the warp's eighth of the channels: lane j, rows i = 8 (j / 8) + r. BEFORE: the first left
+// row meets the decays of tokens j + 1 .. i - 1 only. Without DECAYS: left_i . right_j.
+template <int ROWS, int LEFTS, bool DECAYS, bool BEFORE>
+__device__ __forceinline__ void pairs_inside(const float* left0, const float* left1, const float* right, const float* decays, float* sums) {
+  constexpr int ld = ROWS + 4, slice = ROWS / kWarps;
+  const int c0 = threadIdx.x / 32 * slice;
+  const int lane = threadIdx.x & 31, own = lane & 7, group = (lane & ~7) * ld;
+  pair_t acc[kGroup][LEFTS];
+#pragma unroll
+  for (int r = 0; r < kGroup; ++r)
+#pragma unroll
+    for (int x = 0; x < LEFTS; ++x) acc[r][x] = 0;
+#pragma unroll 2
+  for (int c = c0; c < c0 + slice; c += 4) {
+    const quad_t mine = load_quad(right + lane * ld + c);
+    quad_t p = mine;
+    if (DECAYS) p = {0, 0};
+#pragma unroll
+    for (int r = 0; r < kGroup; ++r) {
+      const int at = group + r * ld + c;
+      const quad_t a = load_quad(left0 + at);
+      if (BEFORE) acc[r][0] = fma_pair(a.hi, p.hi, fma_pair(a.lo, p.lo, acc[r][0]));
+      if (DECAYS) {
+        const quad_t g = load_quad(decays + at);
+        p.lo = r == own ? mine.lo : mul_pair(p.lo, g.lo);
+        p.hi = r == own ? mine.hi : mul_pair(p.hi, g.hi);
+      }
+      if (!BEFORE) acc[r][0] = fma_pair(a.hi, p.hi, fma_pair(a.lo, p.lo, acc[r][0]));
+      if (LEFTS == 2) {
+        const quad_t b = load_quad(left1 + at);
+        acc[r][LEFTS - 1] = fma_pair(b.hi, p.hi, fma_pair(b.lo, p.lo, acc[r][LEFTS - 1]));
+      }
+    }
+  }
+#pragma unroll
+  for (int r = 0; r < kGroup; ++r)
+#pragma unroll
+    for (int x = 0; x < LEFTS; ++x) sums[(r * LEFTS + x) * 32 + lane] = sum_pair(acc[r][x]);
+}
+
+// The same for j in a group b before i's group g, from rows that carry their decays inside their own groups: lane = token 8 b + lane % 8,
+// rows 8 g + 2 (lane / 8) and the next one; `whole` holds the groups' decays multiplied.
+template <int ROWS, int LEFTS, bool DECAYS>
+__device__ __forceinline__ void pairs_between(const float* left0, const float* left1, const float* ends, const float* whole, float* sums) {
+  constexpr int rows = ROWS, ld = ROWS + 4, slice = ROWS / kWarps;
+  const int c0 = threadIdx.x / 32 * slice;
+  const int lane = threadIdx.x & 31, at0 = (lane >> 3) * 2 * ld;
+  const float* right = ends + (lane & 7) * ld;
+  pair_t acc[kBetween][2][LEFTS];
+#pragma unroll
+  for (int x = 0; x < kBetween; ++x)
+#pragma unroll
+    for (int y = 0; y < LEFTS; ++y) acc[x][0][y] = acc[x][1][y] = 0;
+  for (int c = c0; c < c0 + slice; c += 4) {
+    quad_t p[kGroups - 1];
+#pragma unroll
+    for (int b = 0; b < kGroups - 1; ++b) p[b] = load_quad(right + b * kGroup * ld + c);
+    int x = 0;
+#pragma unroll
+    for (int g = 1; g < kGroups; ++g) {
+      if (DECAYS && g > 1) {  // the groups that are now whole ones between
+        const quad_t between = load_quad(whole + (g - 1) * rows + c);
+#pragma unroll
+        for (int b = 0; b < g - 1; ++b) p[b].lo = mul_pair(p[b].lo, between.lo), p[b].hi = mul_pair(p[b].hi, between.hi);
+      }
+      quad_t left[2][LEFTS];
+#pragma unroll
+      for (int r = 0; r < 2; ++r) {
+        const int at = at0 + (g * kGroup + r) * ld + c;
+        left[r][0] = load_quad(left0 + at);
+        if (LEFTS == 2) left[r][LEFTS - 1] = load_quad(left1 + at);
+      }
+#pragma unroll
+      for (int b = 0; b < g; ++b, ++x)
+#pragma unroll
+        for (int r = 0; r < 2; ++r)
+#pragma unroll
+          for (int y = 0; y < LEFTS; ++y) acc[x][r][y] = fma_pair(left[r][y].hi, p[b].hi, fma_pair(left[r][y].lo, p[b].lo, acc[x][r][y]));
+    }
+  }
+#pragma unroll
+  for (int x = 0; x < kBetween; ++x)
+#pragma unroll
+    for (int r = 0; r < 2; ++r)
+#pragma unroll
+      for (int y = 0; y < LEFTS; ++y) sums[((x * 2 + r) * LEFTS + y) * 32 + lane] = sum_pair(acc[x][r][y]);
+}
+
+// The warps' sums of either kind, `stride` numbers from warp to warp, added up into the [C][C + 1] matrices of the left rows.
+template <int LEFTS, bool INSIDE>
+__device__ __forceinline__ void add_up(const float* sums, int stride, float* to0, float* to1) {
+  for (int idx = threadIdx.x; idx < (INSIDE ? inside_sums(LEFTS) : between_sums(LEFTS)); idx += kThreads) {
+    float sum = 0.f;
+#pragma unroll
+    for (int w = 0; w < kWarps; ++w) sum += sums[w * stride + idx];
+    const int l = idx % 32, y = idx / 32 % LEFTS, o = idx / 32 / LEFTS;
+    int i, j;
+    if (INSIDE) {
+      i = (l & ~7) + o, j = l;
+    } else {
+      const int x = o / 2, g = x == 0 ? 1 : (x < 3 ? 2 : 3), b = x - (g == 1 ? 0 : (g == 2 ? 1 : 3));
+      i = g * kGroup + (l >> 3) * 2 + (o & 1), j = b * kGroup + (l & 7);
+    }
+    (y == 0 ? to0 : to1)[i * (C + 1) + j] = sum;
+  }
+}
+
+constexpr int kWarpSums = inside_sums(2) + between_sums(2);
 size_t prepare_smem(int rows) {
   return sizeof(float) * (3 * C * (rows + 4) + kGroups * rows + kWarps * kWarpSums + 2 * C * (C + 1) + C * C + 3 * C);
 }
 
-template <int W, bool PER_HEAD>
+template <int ROWS, int W, bool PER_HEAD>
 __global__ void __launch_bounds__(kThreads, 2)
 chunk_prepare_kernel(const float* q, const float* k, const float* v, const float* beta, const float* decay, const int* __restrict__ seq_q_start,
                      const int* __restrict__ seq_q_len, int heads, int kv_heads, int dk, int dv, Scratch to) {
@@ -143,7 +260,8 @@ chunk_prepare_kernel(const float* q, const float* k, const float* v, const float
   if (n <= 0) return;
   const int start = seq_q_start[seq], kvh = head / (heads / kv_heads);
   const int64_t first = static_cast<int64_t>(start) + chunk * C;
-  const int rows = padded_rows(dk), columns = padded_columns(dv), ld = rows + 4;
+  constexpr int rows = ROWS, ld = ROWS + 4;
+  const int columns = padded_columns(dv);
   float* ks = chunk_smem;                     // [C][ld]: keys, then times the decays of their group up to their own token
   float* qs = ks + C * ld;                    // [C][ld]: queries, then likewise
   float* gs = qs + C * ld;                    // [C][ld]: decays, then keys times the decays from the next token to their group's end
@@ -164,36 +282,8 @@ chunk_prepare_kernel(const float* q, const float* k, const float* v, const float
   commit_copies();
   wait_copies<0>();
   __syncthreads();
-  const int slice = rows / kWarps, c0 = warp * slice;
   float* mine = sums + warp * kWarpSums;
-  {  // pairs inside a group: lane j, rows i = 8 (j / 8) + r
-    const int own = lane & 7;
-    const float* group = ks + (lane & ~7) * ld;
-    pair_t acc[kGroup][2];
-#pragma unroll
-    for (int r = 0; r < kGroup; ++r) acc[r][0] = acc[r][1] = 0;
-    for (int c = c0; c < c0 + slice; c += 4) {
-      const quad_t kj = load_quad(ks + lane * ld + c);
-      quad_t p = kj;
-      if (!PER_HEAD) p = {0, 0};
-#pragma unroll
-      for (int r = 0; r < kGroup; ++r) {
-        if (!PER_HEAD) {
-          const quad_t g = load_quad(group + 2 * C * ld + r * ld + c);
-          p.lo = r == own ? kj.lo : mul_pair(p.lo, g.lo);
-          p.hi = r == own ? kj.hi : mul_pair(p.hi, g.hi);
-        }
-        const quad_t ki = load_quad(group + r * ld + c), qi = load_quad(group + C * ld + r * ld + c);
-        acc[r][0] = fma_pair(ki.hi, p.hi, fma_pair(ki.lo, p.lo, acc[r][0]));
-        acc[r][1] = fma_pair(qi.hi, p.hi, fma_pair(qi.lo, p.lo, acc[r][1]));
-      }
-    }
-#pragma unroll
-    for (int r = 0; r < kGroup; ++r) {
-      mine[(kBetween * 4 + r * 2) * 32 + lane] = sum_pair(acc[r][0]);
-      mine[(kBetween * 4 + r * 2 + 1) * 32 + lane] = sum_pair(acc[r][1]);
-    }
-  }
+  pairs_inside<ROWS, 2, !PER_HEAD, false>(ks, qs, ks, gs, mine);
   if (!PER_HEAD) {
     __syncthreads();
     for (int item = tid; item < kGroups * rows; item += kThreads) {  // a thread per (group, channel)
@@ -218,55 +308,10 @@ chunk_prepare_kernel(const float* q, const float* k, const float* v, const float
     }
     __syncthreads();
   }
-  {  // pairs of two groups, b before g: lane = token 8 b + lane % 8, rows 8 g + 2 (lane / 8) and the next one
-    const float* ends = (PER_HEAD ? ks : gs) + (lane & 7) * ld;
-    const float* left = ks + (lane >> 3) * 2 * ld;
-    pair_t acc[kBetween][4];
-#pragma unroll
-    for (int x = 0; x < kBetween; ++x) acc[x][0] = acc[x][1] = acc[x][2] = acc[x][3] = 0;
-    for (int c = c0; c < c0 + slice; c += 4) {
-      quad_t p[kGroups - 1];
-#pragma unroll
-      for (int b = 0; b < kGroups - 1; ++b) p[b] = load_quad(ends + b * kGroup * ld + c);
-      int x = 0;
-#pragma unroll
-      for (int g = 1; g < kGroups; ++g) {
-        if (!PER_HEAD && g > 1) {  // the groups that are now whole ones between
-          const quad_t between = load_quad(whole + (g - 1) * rows + c);
-#pragma unroll
-          for (int b = 0; b < g - 1; ++b) p[b].lo = mul_pair(p[b].lo, between.lo), p[b].hi = mul_pair(p[b].hi, between.hi);
-        }
-        const float* at = left + g * kGroup * ld + c;
-        const quad_t k0 = load_quad(at), k1 = load_quad(at + ld), q0 = load_quad(at + C * ld), q1 = load_quad(at + C * ld + ld);
-#pragma unroll
-        for (int b = 0; b < g; ++b, ++x) {
-          acc[x][0] = fma_pair(k0.hi, p[b].hi, fma_pair(k0.lo, p[b].lo, acc[x][0]));
-          acc[x][1] = fma_pair(q0.hi, p[b].hi, fma_pair(q0.lo, p[b].lo, acc[x][1]));
-          acc[x][2] = fma_pair(k1.hi, p[b].hi, fma_pair(k1.lo, p[b].lo, acc[x][2]));
-          acc[x][3] = fma_pair(q1.hi, p[b].hi, fma_pair(q1.lo, p[b].lo, acc[x][3]));
-        }
-      }
-    }
-#pragma unroll
-    for (int x = 0; x < kBetween; ++x)
-#pragma unroll
-      for (int o = 0; o < 4; ++o) mine[(x * 4 + o) * 32 + lane] = sum_pair(acc[x][o]);
-  }
+  pairs_between<ROWS, 2, !PER_HEAD>(ks, qs, PER_HEAD ? ks : gs, whole, mine + inside_sums(2));
   __syncthreads();
-  for (int idx = tid; idx < kWarpSums; idx += kThreads) {
-    float sum = 0.f;
-#pragma unroll
-    for (int w = 0; w < kWarps; ++w) sum += sums[w * kWarpSums + idx];
-    const int o = idx / 32, l = idx % 32;
-    int i, j;
-    if (o < kBetween * 4) {
-      const int x = o / 4, g = x == 0 ? 1 : (x < 3 ? 2 : 3), b = x - (g == 1 ? 0 : (g == 2 ? 1 : 3));
-      i = g * kGroup + (l >> 3) * 2 + (o & 3) / 2, j = b * kGroup + (l & 7);
-    } else {
-      i = (l & ~7) + (o - kBetween * 4) / 2, j = l;
-    }
-    (o & 1 ? qk : kk)[i * (C + 1) + j] = sum;
-  }
+  add_up<2, true>(sums, kWarpSums, kk, qk);
+  add_up<2, false>(sums + inside_sums(2), kWarpSums, kk, qk);
   __syncthreads();
   {
     float own = 0.f, d = 0.f, prefix = 0.f, e = 0.f;
@@ -335,6 +380,292 @@ chunk_prepare_kernel(const float* q, const float* k, const float* v, const float
   }
 }
 
+// --- the same for rules in which the values enter as they are ---------------------------------------------------------------------------
+//
+// GENERAL: S <- w S + b (u^T S) + k v^T, o = S^T r, with b = -au. Otherwise S <- w S + k v^T, o = S^T r + bonus v read before the update.
+// One block per (chunk, head, request); the sums of the values (G_last K)^T V go where the chunk's state will be.
+constexpr int kValueTile = 64;
+constexpr int kLdV = kValueTile + 4;
+constexpr int kMaxLinearRows = 128;
+
+__host__ __device__ constexpr int linear_warp_sums(bool general) { return general ? 2 * inside_sums(2) : between_sums(1); }
+size_t linear_prepare_smem(int rows, bool general) {
+  return sizeof(float) * ((general ? 5 : 3) * C * (rows + 4) + C * kLdV + kGroups * rows + kWarps * linear_warp_sums(general) + (general ? 4 : 1) * C * (C + 1) +
+                          (general ? 2 : 0) * C * C);
+}
+
+struct LinearRule {
+  const float* r;
+  const float* k;
+  const float* v;
+  const float* w;
+  const float* au;     // GENERAL
+  const float* u;      // GENERAL
+  const float* bonus;  // otherwise: [tokens][heads]
+};
+
+template <int ROWS, int W, bool GENERAL>
+__global__ void __launch_bounds__(kThreads, 2)
+linear_chunk_prepare_kernel(LinearRule in, const int* __restrict__ seq_q_start, const int* __restrict__ seq_q_len, int heads, int dk, int dv, Scratch to) {
+  extern __shared__ __align__(16) float chunk_smem[];
+  let_successor_start();
+  const int seq = blockIdx.z, head = blockIdx.y, chunk = blockIdx.x;
+  const int n = min(C, seq_q_len[seq] - chunk * C);
+  if (n <= 0) return;
+  const int start = seq_q_start[seq];
+  const int64_t first = static_cast<int64_t>(start) + chunk * C, place = chunk_place(start, seq, chunk) * heads + head;
+  constexpr int rows = ROWS, ld = ROWS + 4;
+  const int columns = padded_columns(dv);
+  constexpr int kSums = linear_warp_sums(GENERAL);
+  float* ls = chunk_smem;                                // GENERAL: [C][C]: -N
+  float* ms = ls + (GENERAL ? C * C : 0);                // GENERAL: [C][C]: M
+  float* rs = ms + (GENERAL ? C * C : 0);                // [C][ld]: r, then times the decays of its group in front of (GENERAL: up to) its token
+  float* ks = rs + C * ld;                               // [C][ld]: k, then times the decays from the next token to its group's end
+  float* gs = ks + C * ld;                               // [C][ld]
+  float* us = gs + C * ld;                               // GENERAL: [C][ld]: u, then times the decays of its group in front of its token
+  float* bb = us + (GENERAL ? C * ld : 0);               // GENERAL: [C][ld]: -au, then as k
+  float* vs = bb + (GENERAL ? C * ld : 0);               // [C][kLdV]: a tile of the values
+  float* whole = vs + C * kLdV;                          // [groups][rows]
+  float* sums = whole + kGroups * rows;                  // [warps][kSums]
+  float* rk = sums + kWarps * kSums;                     // [C][C + 1]: r_i . G k_j
+  float* uk = rk + C * (C + 1);
+  float* rb = uk + C * (C + 1);
+  float* ub = rb + C * (C + 1);
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int64_t ld_in = static_cast<int64_t>(heads) * dk, at_in = static_cast<int64_t>(head) * dk;
+  auto stage_values = [&](int col0) {
+    for (int r = warp; r < C; r += kWarps)
+      for (int c = lane * W; c < kValueTile; c += 32 * W) {
+        const bool valid = r < n && col0 + c < dv;
+        stage_copy<4 * W>(vs + r * kLdV + c, valid ? in.v + ((first + r) * heads + head) * dv + col0 + c : in.v, valid);
+      }
+  };
+  wait_for_predecessor();
+  stage_rows<W>(rs, ld, in.r, first, n, ld_in, at_in, dk, rows);
+  stage_rows<W>(ks, ld, in.k, first, n, ld_in, at_in, dk, rows);
+  stage_rows<W>(gs, ld, in.w, first, n, ld_in, at_in, dk, rows);
+  if (GENERAL) {
+    stage_rows<W>(us, ld, in.u, first, n, ld_in, at_in, dk, rows);
+    stage_rows<W>(bb, ld, in.au, first, n, ld_in, at_in, dk, rows);
+  }
+  stage_values(0);
+  commit_copies();
+  wait_copies<0>();
+  __syncthreads();
+  float* mine = sums + warp * kSums;
+  if (GENERAL) {
+    pairs_inside<ROWS, 2, true, true>(us, rs, ks, gs, mine);
+    pairs_inside<ROWS, 2, true, true>(us, rs, bb, gs, mine + inside_sums(2));
+  } else {
+    pairs_inside<ROWS, 1, true, true>(rs, nullptr, ks, gs, mine);
+  }
+  __syncthreads();
+  if (GENERAL) {
+    add_up<2, true>(sums, kSums, uk, rk);
+    add_up<2, true>(sums + inside_sums(2), kSums, ub, rb);
+  } else {
+    add_up<1, true>(sums, kSums, rk, nullptr);
+  }
+  for (int item = tid; item < kGroups * rows; item += kThreads) {  // a thread per (group, channel)
+    const int c = item % rows, at = item / rows * kGroup * ld + c;
+    float g[kGroup];
+    float run = 1.f;
+#pragma unroll
+    for (int r = 0; r < kGroup; ++r) {
+      g[r] = item / rows * kGroup + r < n ? gs[at + r * ld] : 1.f;
+      if (GENERAL) us[at + r * ld] *= run;
+      else rs[at + r * ld] *= run;
+      run *= g[r];
+      if (GENERAL) rs[at + r * ld] *= run;
+    }
+    whole[item] = run;
+    run = 1.f;
+#pragma unroll
+    for (int r = kGroup - 1; r >= 0; --r) {
+      ks[at + r * ld] *= run;
+      if (GENERAL) bb[at + r * ld] *= run;
+      run *= g[r];
+    }
+  }
+  __syncthreads();
+  if (GENERAL) {
+    pairs_between<ROWS, 2, true>(us, rs, ks, whole, mine);
+    __syncthreads();
+    add_up<2, false>(sums, kSums, uk, rk);
+    __syncthreads();
+    pairs_between<ROWS, 2, true>(us, rs, bb, whole, mine);
+    __syncthreads();
+    add_up<2, false>(sums, kSums, ub, rb);
+  } else {
+    pairs_between<ROWS, 1, true>(rs, nullptr, ks, whole, mine);
+    __syncthreads();
+    add_up<1, false>(sums, kSums, rk, nullptr);
+  }
+  __syncthreads();
+  for (int i = warp; i < C; i += kWarps) {
+    const int at = i * (C + 1) + lane;
+    const int64_t row = ((first + i) * heads + head) * C + lane;
+    if (GENERAL) {  // au came in with its own sign: b = -au
+      ls[i * C + lane] = lane < i ? ub[at] : 0.f;
+      ms[i * C + lane] = lane < i ? uk[at] : 0.f;
+      if (i < n) {
+        to.a[row] = lane <= i ? -rb[at] : 0.f;
+        to.av[row] = lane <= i ? rk[at] : 0.f;
+      }
+    } else if (i < n) {
+      to.av[row] = lane < i ? rk[at] : (lane == i ? in.bonus[(first + i) * heads + head] : 0.f);
+    }
+  }
+  // Scaled rows: r times all decays in front of (or up to) its token, b times all decays behind its token; a thread per (group, channel).
+  for (int item = tid; item < kGroups * rows; item += kThreads) {
+    const int c = item % rows, group = item / rows;
+    float before = 1.f, after = 1.f;
+#pragma unroll
+    for (int g = 0; g < kGroups - 1; ++g) {
+      before *= g < group ? whole[g * rows + c] : 1.f;
+      after *= g + 1 > group ? whole[(g + 1) * rows + c] : 1.f;
+    }
+    const int64_t at = ((first + group * kGroup) * heads + head) * rows + c, step = static_cast<int64_t>(heads) * rows;
+    float* qt = to.qt + at;
+    float* kd = to.kd + at;
+#pragma unroll
+    for (int r = 0; r < kGroup; ++r) {
+      const int from = (group * kGroup + r) * ld + c;
+      if (group * kGroup + r < n) {
+        *qt = before * rs[from];
+        if (GENERAL) *kd = -after * bb[from];
+      }
+      qt += step, kd += step;
+    }
+  }
+  for (int c = tid; c < rows; c += kThreads) to.e[place * rows + c] = whole[c] * whole[rows + c] * whole[2 * rows + c] * whole[3 * rows + c];
+  if (GENERAL) __syncthreads();
+  for (int col0 = 0; col0 < columns; col0 += kValueTile) {
+    if (col0 > 0) {
+      __syncthreads();
+      stage_values(col0);
+      commit_copies();
+      wait_copies<0>();
+      __syncthreads();
+    }
+    if (GENERAL && tid < kValueTile + (col0 == 0 ? rows : 0)) {  // a thread per column of [M V | e U]
+      float x[C];
+      float* to_x;
+      int64_t stride;
+      const int c = tid;
+      if (tid < kValueTile) {
+        float value[C];
+#pragma unroll
+        for (int i = 0; i < C; ++i) value[i] = vs[i * kLdV + c];
+#pragma unroll
+        for (int i = 0; i < C; ++i) {
+          float sum0 = 0.f, sum1 = 0.f;
+#pragma unroll
+          for (int j = 0; j < i; j += 4) {
+            const float4 row = *reinterpret_cast<const float4*>(ms + i * C + j);
+            sum0 = fmaf(row.x, value[j], sum0);
+            if (j + 1 < i) sum1 = fmaf(row.y, value[j + 1], sum1);
+            if (j + 2 < i) sum0 = fmaf(row.z, value[j + 2], sum0);
+            if (j + 3 < i) sum1 = fmaf(row.w, value[j + 3], sum1);
+          }
+          x[i] = sum0 + sum1;
+        }
+        stride = static_cast<int64_t>(heads) * columns;
+        to_x = to.x + (first * heads + head) * columns + col0 + c;
+      } else {
+        const int channel = c - kValueTile;
+        float before = 1.f;
+#pragma unroll
+        for (int i = 0; i < C; ++i) {
+          if (i > 0 && i % kGroup == 0) before *= whole[(i / kGroup - 1) * rows + channel];
+          x[i] = before * us[i * ld + channel];
+        }
+        stride = static_cast<int64_t>(heads) * rows;
+        to_x = to.y + (first * heads + head) * rows + channel;
+      }
+      substitute(ls, x);
+      if (tid >= kValueTile || col0 + c < columns) {
+#pragma unroll
+        for (int i = 0; i < C; ++i) {
+          if (i < n) *to_x = x[i];
+          to_x += stride;
+        }
+      }
+    }
+    // (G_last K)^T V over the tile: four rows by four columns a thread, group after group of tokens.
+    const int rt = (tid & 15) * 4, ct = (tid >> 4) * 4;
+    for (int row = rt; row < rows; row += 64) {
+      float acc[4][4];
+#pragma unroll
+      for (int r = 0; r < 4; ++r) acc[r][0] = acc[r][1] = acc[r][2] = acc[r][3] = 0.f;
+#pragma unroll
+      for (int g = 0; g < kGroups; ++g) {
+        const float4 scale = *reinterpret_cast<const float4*>(whole + g * rows + row);
+        const float f[4] = {scale.x, scale.y, scale.z, scale.w};
+#pragma unroll
+        for (int r = 0; r < 4; ++r) acc[r][0] *= f[r], acc[r][1] *= f[r], acc[r][2] *= f[r], acc[r][3] *= f[r];
+#pragma unroll
+        for (int j = g * kGroup; j < (g + 1) * kGroup; ++j) {
+          const float4 key = *reinterpret_cast<const float4*>(ks + j * ld + row), value = *reinterpret_cast<const float4*>(vs + j * kLdV + ct);
+          const float a[4] = {key.x, key.y, key.z, key.w};
+#pragma unroll
+          for (int r = 0; r < 4; ++r) {
+            acc[r][0] = fmaf(a[r], value.x, acc[r][0]), acc[r][1] = fmaf(a[r], value.y, acc[r][1]);
+            acc[r][2] = fmaf(a[r], value.z, acc[r][2]), acc[r][3] = fmaf(a[r], value.w, acc[r][3]);
+          }
+        }
+      }
+      if (col0 + ct < columns) {
+#pragma unroll
+        for (int r = 0; r < 4; ++r)
+          *reinterpret_cast<float4*>(to.s + (place * rows + row + r) * columns + col0 + ct) = make_float4(acc[r][0], acc[r][1], acc[r][2], acc[r][3]);
+      }
+    }
+  }
+}
+
+// Four neighbouring numbers of a head's state a thread, from chunk to chunk: eight chunks' sums are asked for at a time.
+__global__ void __launch_bounds__(kThreads)
+chunk_scan_kernel(const int* __restrict__ seq_q_start, const int* __restrict__ seq_q_len, const int* __restrict__ seq_slot, int heads, int dk, int dv, Scratch from,
+                  float* state) {
+  let_successor_start();
+  const int seq = blockIdx.z, head = blockIdx.y;
+  const int start = seq_q_start[seq], len = seq_q_len[seq], chunks = (len + C - 1) / C;
+  const int rows = padded_rows(dk), columns = padded_columns(dv);
+  const int item = (blockIdx.x * kThreads + threadIdx.x) * 4;
+  if (item >= rows * columns) return;
+  const int row = item / columns, col = item % columns;
+  float* base = state + (static_cast<int64_t>(seq_slot[seq]) * heads + head) * dk * dv + static_cast<int64_t>(row) * dv + col;
+  float s[4];
+  wait_for_predecessor();
+#pragma unroll
+  for (int x = 0; x < 4; ++x) s[x] = row < dk && col + x < dv ? base[x] : 0.f;
+  const int64_t place = chunk_place(start, seq, 0) * heads + head;
+  const float* e = from.e + place * rows + row;
+  float* sums = from.s + place * rows * columns + item;
+  const int64_t step_e = static_cast<int64_t>(heads) * rows, step = step_e * columns;
+  constexpr int kAhead = 8;
+  for (int chunk = 0; chunk < chunks; chunk += kAhead) {
+    float4 add[kAhead];
+    float keep[kAhead];
+#pragma unroll
+    for (int i = 0; i < kAhead; ++i)
+      if (chunk + i < chunks) add[i] = *reinterpret_cast<const float4*>(sums + (chunk + i) * step), keep[i] = e[(chunk + i) * step_e];
+#pragma unroll
+    for (int i = 0; i < kAhead; ++i)
+      if (chunk + i < chunks) {
+        *reinterpret_cast<float4*>(sums + (chunk + i) * step) = make_float4(s[0], s[1], s[2], s[3]);
+        s[0] = fmaf(keep[i], s[0], add[i].x), s[1] = fmaf(keep[i], s[1], add[i].y);
+        s[2] = fmaf(keep[i], s[2], add[i].z), s[3] = fmaf(keep[i], s[3], add[i].w);
+      }
+  }
+  if (chunks > 0) {
+#pragma unroll
+    for (int x = 0; x < 4; ++x)
+      if (row < dk && col + x < dv) base[x] = s[x];
+  }
+}
+
 // --- the walk ------------------------------------------------------------------------------------------------------------------------
 //
 // One block per (16 columns of the state, head, request). U = W + Y S: a warp has four tokens, its lanes four groups of columns times
@@ -348,7 +679,7 @@ constexpr size_t walk_smem(int rows) { return sizeof(float) * (2 * walk_stage(ro
 
 __device__ __forceinline__ float from_pair(float give, float keep, int with) { return keep + __shfl_xor_sync(0xffffffffu, give, with); }
 
-template <int ROWS>
+template <int ROWS, bool ADD>  // ADD: what the values alone add to S stands where the chunk's state goes
 __global__ void __launch_bounds__(kThreads, ROWS <= 128 ? 2 : 1)
 chunk_walk_kernel(const int* __restrict__ seq_q_start, const int* __restrict__ seq_q_len, const int* __restrict__ seq_slot, int heads, int dk, int dv,
                   Scratch from, float* state) {
@@ -404,6 +735,12 @@ chunk_walk_kernel(const int* __restrict__ seq_q_start, const int* __restrict__ s
   for (int chunk = 0; chunk < chunks; ++chunk) {
     const int n = min(C, len - chunk * C);
     const int64_t first = static_cast<int64_t>(start) + chunk * C;
+    float* s_out = from.s + ((chunk_place(start, seq, chunk) * heads + head) * ROWS + row0) * columns + col0 + cg * 4;
+    float4 own[kPer];
+    if (ADD) {
+#pragma unroll
+      for (int r = 0; r < kPer; ++r) own[r] = *reinterpret_cast<const float4*>(s_out + static_cast<int64_t>(r) * columns);
+    }
 #pragma unroll
     for (int c = 0; c < 4; ++c) {
       float* to = tile + (cg * 4 + c) * kLdS + row0;
@@ -464,7 +801,6 @@ chunk_walk_kernel(const int* __restrict__ seq_q_start, const int* __restrict__ s
       }
     }
     // The state in front of the chunk, for `chunk_out`.
-    float* s_out = from.s + ((chunk_place(start, seq, chunk) * heads + head) * ROWS + row0) * columns + col0 + cg * 4;
 #pragma unroll
     for (int r = 0; r < kPer; ++r) *reinterpret_cast<float4*>(s_out + static_cast<int64_t>(r) * columns) = make_float4(s[r][0], s[r][1], s[r][2], s[r][3]);
     __syncthreads();
@@ -503,6 +839,7 @@ chunk_walk_kernel(const int* __restrict__ seq_q_start, const int* __restrict__ s
 #pragma unroll
       for (int r = 0; r < kPer; ++r) {
         const float e = es[row0 + r];
+        if (ADD) add[r][0] += own[r].x, add[r][1] += own[r].y, add[r][2] += own[r].z, add[r][3] += own[r].w;
 #pragma unroll
         for (int c = 0; c < 4; ++c) s[r][c] = fmaf(e, s[r][c], add[r][c]);
       }
@@ -519,44 +856,59 @@ chunk_walk_kernel(const int* __restrict__ seq_q_start, const int* __restrict__ s
 
 // --- outputs ---------------------------------------------------------------------------------------------------------------------------
 //
-// One block per (chunk, head, request and 128 columns): O = Qt S + A U as one product over rows + 32 numbers, 32 of them at a time
-// by cp.async in two stages. A thread has eight tokens and four neighbouring columns: 12 numbers read for 32 FMAs, since what an SM
-// takes out of shared memory (32 numbers a cycle, however many lanes want the same one) bounds this kernel.
-constexpr int kOutColumns = 128;
-constexpr int kOutThreads = 128;
-constexpr int kLdOut = kOutColumns + 4;
+// One block per (chunk, head, request and COLS columns): O = Qt S (+ A U) (+ Av V) as one product over rows + 32 (+ 32) numbers, 32 of
+// them at a time by cp.async in two stages. A thread has eight tokens and four neighbouring columns: 12 numbers read for 32 FMAs, since
+// what an SM takes out of shared memory (32 numbers a cycle, however many lanes want the same one) bounds this kernel.
 constexpr int kLdSlab = C + 4;
-constexpr size_t kOutSmem = sizeof(float) * 2 * (C * kLdSlab + C * kLdOut);
+constexpr size_t out_smem(int cols) { return sizeof(float) * 2 * (C * kLdSlab + C * (cols + 4)); }
 
-__global__ void __launch_bounds__(kOutThreads)
-chunk_out_kernel(const int* __restrict__ seq_q_start, const int* __restrict__ seq_q_len, int heads, int dv, int rows, int tiles, Scratch from, float* out) {
+template <int COLS, bool WITH_U, bool WITH_V>
+__global__ void __launch_bounds__(COLS)
+chunk_out_kernel(const int* __restrict__ seq_q_start, const int* __restrict__ seq_q_len, int heads, int dv, int rows, int tiles, Scratch from, const float* v,
+                 int v_wide, float* out) {
   extern __shared__ __align__(16) float chunk_smem[];
+  constexpr int kLdOut = COLS + 4, kStage = C * kLdSlab + C * kLdOut;
   let_successor_start();
-  const int seq = blockIdx.z / tiles, col0 = blockIdx.z % tiles * kOutColumns, head = blockIdx.y, chunk = blockIdx.x;
+  const int seq = blockIdx.z / tiles, col0 = blockIdx.z % tiles * COLS, head = blockIdx.y, chunk = blockIdx.x;
   const int start = seq_q_start[seq], n = min(C, seq_q_len[seq] - chunk * C);
   if (n <= 0) return;
   const int64_t first = static_cast<int64_t>(start) + chunk * C;
-  const int columns = padded_columns(dv), width = min(kOutColumns, columns - col0);
+  const int columns = padded_columns(dv), width = min(COLS, columns - col0);
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const float* states = from.s + (chunk_place(start, seq, chunk) * heads + head) * rows * columns + col0;
-  const int slabs = rows / C + 1;
+  const int state_slabs = rows / C, slabs = state_slabs + (WITH_U ? 1 : 0) + (WITH_V ? 1 : 0);
   wait_for_predecessor();
   auto fetch = [&](int slab) {
-    float* left = chunk_smem + (slab & 1) * (C * kLdSlab + C * kLdOut);
+    float* left = chunk_smem + (slab & 1) * kStage;
     float* right = left + C * kLdSlab;
-    const bool last = slab == slabs - 1;
+    const bool in_state = slab < state_slabs, is_u = WITH_U && slab == state_slabs;
+    const float* pairs = is_u ? from.a : from.av;
 #pragma unroll
-    for (int half = 0; half < 2; ++half) {
-      const int r = (tid >> 3) + 16 * half, c = (tid & 7) * 4;
+    for (int r = tid >> 3; r < C; r += COLS / 8) {
+      const int c = (tid & 7) * 4;
       const int64_t row = (first + r) * heads + head;
-      stage_copy<16>(left + r * kLdSlab + c, r < n ? (last ? from.a + row * C + c : from.qt + row * rows + slab * C + c) : from.a, r < n);
+      stage_copy<16>(left + r * kLdSlab + c, r < n ? (in_state ? from.qt + row * rows + slab * C + c : pairs + row * C + c) : from.qt, r < n);
     }
-    const int c = lane * 4;
+    if (in_state || is_u) {
 #pragma unroll
-    for (int r = warp; r < C; r += kOutThreads / 32) {
-      const bool valid = c < width && (!last || r < n);
-      const float* at = last ? from.x + ((first + r) * heads + head) * columns + col0 + c : states + static_cast<int64_t>(slab * C + r) * columns + c;
-      stage_copy<16>(right + r * kLdOut + c, valid ? at : from.a, valid);
+      for (int r = tid / (COLS / 4); r < C; r += 4) {
+        const int c = tid % (COLS / 4) * 4;
+        const bool valid = c < width && (in_state || r < n);
+        const float* at = in_state ? states + static_cast<int64_t>(slab * C + r) * columns + c : from.x + ((first + r) * heads + head) * columns + col0 + c;
+        stage_copy<16>(right + r * kLdOut + c, valid ? at : from.qt, valid);
+      }
+    } else if (v_wide) {
+#pragma unroll
+      for (int r = tid / (COLS / 4); r < C; r += 4) {
+        const int c = tid % (COLS / 4) * 4;
+        const bool valid = col0 + c < dv && r < n;
+        stage_copy<16>(right + r * kLdOut + c, valid ? v + ((first + r) * heads + head) * dv + col0 + c : v, valid);
+      }
+    } else {
+      for (int r = 0; r < C; ++r) {
+        const bool valid = col0 + tid < dv && r < n;
+        stage_copy<4>(right + r * kLdOut + tid, valid ? v + ((first + r) * heads + head) * dv + col0 + tid : v, valid);
+      }
     }
     commit_copies();
   };
@@ -573,8 +925,8 @@ chunk_out_kernel(const int* __restrict__ seq_q_start, const int* __restrict__ se
       wait_copies<0>();
     }
     __syncthreads();
-    const float* left = chunk_smem + (slab & 1) * (C * kLdSlab + C * kLdOut) + it * kLdSlab;
-    const float* right = chunk_smem + (slab & 1) * (C * kLdSlab + C * kLdOut) + C * kLdSlab + ct * 4;
+    const float* left = chunk_smem + (slab & 1) * kStage + it * kLdSlab;
+    const float* right = chunk_smem + (slab & 1) * kStage + C * kLdSlab + ct * 4;
     float sum[8][4];  // one slab's sum by itself: fewer roundings of the whole
 #pragma unroll
     for (int i = 0; i < 8; ++i) sum[i][0] = sum[i][1] = sum[i][2] = sum[i][3] = 0.f;
@@ -616,20 +968,24 @@ chunk_out_kernel(const int* __restrict__ seq_q_start, const int* __restrict__ se
 
 // --- host ------------------------------------------------------------------------------------------------------------------------------
 
+enum Rule { kDelta = 0, kGeneralDelta = 1, kLinear = 2 };
+
 struct Sizes {
-  int tokens, seqs, heads, dk, dv;
+  int tokens, seqs, max_q_len, heads, dk, dv;
 };
 
 int64_t aligned_floats(int64_t n) { return (n + 3) / 4 * 4; }
 
 // The scratch's arrays one after another in `base` (null pointers with a null base); returns the numbers they need.
-int64_t lay_out(const Sizes& z, float* base, Scratch* to) {
+int64_t lay_out(int rule, const Sizes& z, float* base, Scratch* to) {
   const int64_t rows = padded_rows(z.dk), columns = padded_columns(z.dv), per_head = static_cast<int64_t>(z.tokens) * z.heads;
   const int64_t chunks = (static_cast<int64_t>(z.tokens) / C + z.seqs + 1) * z.heads;
-  const int64_t sizes[7] = {per_head * rows, per_head * rows, per_head * rows, per_head * columns, per_head * C, chunks * rows, chunks * rows * columns};
-  float** arrays[7] = {&to->y, &to->kd, &to->qt, &to->x, &to->a, &to->e, &to->s};
+  const int64_t with_u = rule != kLinear ? 1 : 0, with_v = rule != kDelta ? 1 : 0;
+  const int64_t sizes[8] = {with_u * per_head * rows, with_u * per_head * rows, per_head * rows, with_u * per_head * columns,
+                            with_u * per_head * C, with_v * per_head * C, chunks * rows, chunks * rows * columns};
+  float** arrays[8] = {&to->y, &to->kd, &to->qt, &to->x, &to->a, &to->av, &to->e, &to->s};
   int64_t at = 0;
-  for (int i = 0; i < 7; ++i) {
+  for (int i = 0; i < 8; ++i) {
     *arrays[i] = base == nullptr ? nullptr : base + at;
     at += aligned_floats(sizes[i]);
   }
@@ -641,27 +997,80 @@ bool raise_smem(Kernel kernel, size_t bytes) {
   return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(bytes)) == cudaSuccess;
 }
 
+template <int ROWS>
+bool raise_prepares() {
+  const size_t delta = prepare_smem(ROWS);
+  bool ok = raise_smem(chunk_prepare_kernel<ROWS, 1, false>, delta) && raise_smem(chunk_prepare_kernel<ROWS, 4, false>, delta) &&
+            raise_smem(chunk_prepare_kernel<ROWS, 1, true>, delta) && raise_smem(chunk_prepare_kernel<ROWS, 4, true>, delta) &&
+            raise_smem(chunk_walk_kernel<ROWS, false>, walk_smem(ROWS));
+  if constexpr (ROWS <= kMaxLinearRows) {
+    const size_t general = linear_prepare_smem(ROWS, true), linear = linear_prepare_smem(ROWS, false);
+    ok = ok && raise_smem(linear_chunk_prepare_kernel<ROWS, 1, false>, linear) && raise_smem(linear_chunk_prepare_kernel<ROWS, 4, false>, linear) &&
+         raise_smem(linear_chunk_prepare_kernel<ROWS, 1, true>, general) && raise_smem(linear_chunk_prepare_kernel<ROWS, 4, true>, general) &&
+         raise_smem(chunk_walk_kernel<ROWS, true>, walk_smem(ROWS));
+  }
+  return ok;
+}
+
 bool raise_all() {
-  static const bool raised =
-      raise_smem(chunk_prepare_kernel<1, false>, prepare_smem(kMaxRows)) && raise_smem(chunk_prepare_kernel<4, false>, prepare_smem(kMaxRows)) &&
-      raise_smem(chunk_prepare_kernel<1, true>, prepare_smem(kMaxRows)) && raise_smem(chunk_prepare_kernel<4, true>, prepare_smem(kMaxRows)) &&
-      raise_smem(chunk_walk_kernel<64>, walk_smem(64)) && raise_smem(chunk_walk_kernel<128>, walk_smem(128)) && raise_smem(chunk_walk_kernel<256>, walk_smem(256));
+  static const bool raised = raise_prepares<64>() && raise_prepares<128>() && raise_prepares<256>();
   return raised;
+}
+
+template <int ROWS>
+auto delta_prepare_form(bool wide, bool per_head) {
+  return per_head ? (wide ? chunk_prepare_kernel<ROWS, 4, true> : chunk_prepare_kernel<ROWS, 1, true>)
+                  : (wide ? chunk_prepare_kernel<ROWS, 4, false> : chunk_prepare_kernel<ROWS, 1, false>);
+}
+
+template <int ROWS>
+auto linear_prepare_form(bool wide, bool general) {
+  return general ? (wide ? linear_chunk_prepare_kernel<ROWS, 4, true> : linear_chunk_prepare_kernel<ROWS, 1, true>)
+                 : (wide ? linear_chunk_prepare_kernel<ROWS, 4, false> : linear_chunk_prepare_kernel<ROWS, 1, false>);
 }
 
 bool aligned16(const void* p) { return reinterpret_cast<uintptr_t>(p) % 16 == 0; }
 
+struct Requests {
+  const int* q_start;
+  const int* q_len;
+  const int* slot;
+};
+
+int launch_walk(const Sizes& z, const Requests& req, bool add, const Scratch& scratch, float* state, cudaStream_t stream) {
+  const int rows = padded_rows(z.dk);
+  auto walk = add ? (rows == 64 ? chunk_walk_kernel<64, true> : chunk_walk_kernel<128, true>)
+                  : (rows == 64 ? chunk_walk_kernel<64, false> : (rows == 128 ? chunk_walk_kernel<128, false> : chunk_walk_kernel<256, false>));
+  // The ordinary way, not early: the few long-lived blocks should spread over all SMs, not over those the kernel in front leaves first.
+  launch_kernel_as(true, walk, dim3(padded_columns(z.dv) / kColumns, z.heads, z.seqs), dim3(kThreads), walk_smem(rows), stream, req.q_start, req.q_len, req.slot,
+                   z.heads, z.dk, z.dv, scratch, state);
+  return b200_check_launch("chunk_walk");
+}
+
+template <bool WITH_U, bool WITH_V>
+int launch_out(const Sizes& z, const Requests& req, const Scratch& scratch, const float* v, float* out, cudaStream_t stream) {
+  const int columns = padded_columns(z.dv), cols = columns <= 64 ? 64 : 128, tiles = (columns + cols - 1) / cols;
+  launch_kernel(cols == 64 ? chunk_out_kernel<64, WITH_U, WITH_V> : chunk_out_kernel<128, WITH_U, WITH_V>, dim3((z.max_q_len + C - 1) / C, z.heads, z.seqs * tiles),
+                dim3(cols), out_smem(cols), stream, req.q_start, req.q_len, z.heads, z.dv, padded_rows(z.dk), tiles, scratch, v,
+                z.dv % 4 == 0 && aligned16(v) ? 1 : 0, out);
+  return b200_check_launch("chunk_out");
+}
+
+bool too_many_requests(const Sizes& z) { return static_cast<int64_t>(z.seqs) * ((padded_columns(z.dv) + 127) / 128) > 65535; }
+
 }  // namespace
 
-// Sizes the chunked form takes; the caller walks token by token otherwise.
-B200_API int b200_delta_chunks_supported(int heads, int kv_heads, int dk, int dv) {
-  return heads > 0 && heads <= 65535 && kv_heads > 0 && heads % kv_heads == 0 && dk > 0 && dk <= kMaxRows && dv > 0 && dv <= 65536;
+// Sizes the chunked form takes (`rule`: 0 the delta rule, 1 the generalized one, 2 the one without a removal); the caller walks token by
+// token otherwise.
+B200_API int b200_state_chunks_supported(int rule, int heads, int kv_heads, int dk, int dv) {
+  return heads > 0 && heads <= 65535 && kv_heads > 0 && heads % kv_heads == 0 && dk > 0 && dk <= (rule == kDelta ? kMaxRows : kMaxLinearRows) && dv > 0 &&
+         dv <= 65536;
 }
 
 // Numbers of scratch (32-bit, aligned to 16 bytes) that a call needs.
-B200_API int64_t b200_delta_chunks_scratch(int tokens, int seqs, int heads, int dk, int dv) {
+B200_API int64_t b200_state_chunks_scratch(int rule, int tokens, int seqs, int heads, int dk, int dv) {
   Scratch scratch;
-  return lay_out({tokens, seqs, heads, dk, dv}, nullptr, &scratch);
+  return lay_out(rule, {tokens, seqs, 0, heads, dk, dv}, nullptr, &scratch);
 }
 
 // The delta rule over every request's new tokens; operands as `delta_prepare` leaves them. per_head = 0: `decay` [tokens][heads][dk]
@@ -670,24 +1079,52 @@ B200_API int b200_delta_chunks(const float* q, const float* k, const float* v, c
                                const int* seq_q_len, const int* seq_slot, int tokens, int seqs, int max_q_len, int heads, int kv_heads, int dk, int dv,
                                float* scratch, int64_t scratch_floats, float* state, float* out, cudaStream_t stream) {
   if (seqs == 0 || tokens == 0) return 0;
-  B200_REQUIRE(tokens > 0 && seqs > 0 && max_q_len > 0 && b200_delta_chunks_supported(heads, kv_heads, dk, dv), "delta_chunks: shape not taken");
-  const Sizes z = {tokens, seqs, heads, dk, dv};
+  B200_REQUIRE(tokens > 0 && seqs > 0 && max_q_len > 0 && b200_state_chunks_supported(kDelta, heads, kv_heads, dk, dv), "delta_chunks: shape not taken");
+  const Sizes z = {tokens, seqs, max_q_len, heads, dk, dv};
+  const Requests req = {seq_q_start, seq_q_len, seq_slot};
   Scratch parts;
-  B200_REQUIRE(aligned16(scratch) && lay_out(z, scratch, &parts) <= scratch_floats, "delta_chunks: scratch too small or not aligned to 16 bytes");
-  const int rows = padded_rows(dk), columns = padded_columns(dv), chunks = (max_q_len + C - 1) / C, tiles = (columns + kOutColumns - 1) / kOutColumns;
-  B200_REQUIRE(static_cast<int64_t>(seqs) * tiles <= 65535, "delta_chunks: too many requests");
+  B200_REQUIRE(aligned16(scratch) && lay_out(kDelta, z, scratch, &parts) <= scratch_floats, "delta_chunks: scratch too small or not aligned to 16 bytes");
+  B200_REQUIRE(seqs <= 65535 && !too_many_requests(z), "delta_chunks: too many requests");
   B200_REQUIRE(raise_all(), "delta_chunks: cannot size shared memory");
   const bool wide = dk % 4 == 0 && aligned16(q) && aligned16(k) && (per_head || aligned16(decay));
-  auto prepare = per_head ? (wide ? chunk_prepare_kernel<4, true> : chunk_prepare_kernel<1, true>) : (wide ? chunk_prepare_kernel<4, false> : chunk_prepare_kernel<1, false>);
-  launch_kernel(prepare, dim3(chunks, heads, seqs), dim3(kThreads), prepare_smem(rows), stream, q, k, v, beta, decay, seq_q_start, seq_q_len, heads, kv_heads,
-                dk, dv, parts);
+  const int rows = padded_rows(dk);
+  auto prepare = rows == 64 ? delta_prepare_form<64>(wide, per_head) : (rows == 128 ? delta_prepare_form<128>(wide, per_head) : delta_prepare_form<256>(wide, per_head));
+  launch_kernel(prepare, dim3((max_q_len + C - 1) / C, heads, seqs), dim3(kThreads), prepare_smem(rows), stream, q, k, v, beta, decay, seq_q_start,
+                seq_q_len, heads, kv_heads, dk, dv, parts);
   if (int status = b200_check_launch("chunk_prepare")) return status;
-  auto walk = rows == 64 ? chunk_walk_kernel<64> : (rows == 128 ? chunk_walk_kernel<128> : chunk_walk_kernel<256>);
-  // The ordinary way, not early: the few long-lived blocks should spread over all SMs, not over those the kernel in front leaves first.
-  launch_kernel_as(true, walk, dim3(columns / kColumns, heads, seqs), dim3(kThreads), walk_smem(rows), stream, seq_q_start, seq_q_len, seq_slot, heads, dk, dv,
-                   parts, state);
-  if (int status = b200_check_launch("chunk_walk")) return status;
-  launch_kernel(chunk_out_kernel, dim3(chunks, heads, seqs * tiles), dim3(kOutThreads), kOutSmem, stream, seq_q_start, seq_q_len, heads, dv, rows, tiles, parts,
-                out);
-  return b200_check_launch("chunk_out");
+  if (int status = launch_walk(z, req, false, parts, state, stream)) return status;
+  return launch_out<true, false>(z, req, parts, v, out, stream);
+}
+
+// The rules in which the values enter as they are. With `u` the generalized delta rule S <- w S - au (u^T S) + k v^T, o = S^T r; with
+// `bonus` [tokens][heads] instead S <- w S + k v^T, o = (S in front of the token)^T r + bonus v. Operands [tokens][heads * dk], v
+// [tokens][heads * dv].
+B200_API int b200_linear_chunks(const float* r, const float* k, const float* v, const float* w, const float* au, const float* u, const float* bonus,
+                                const int* seq_q_start, const int* seq_q_len, const int* seq_slot, int tokens, int seqs, int max_q_len, int heads, int dk, int dv,
+                                float* scratch, int64_t scratch_floats, float* state, float* out, cudaStream_t stream) {
+  if (seqs == 0 || tokens == 0) return 0;
+  const int rule = u != nullptr ? kGeneralDelta : kLinear;
+  B200_REQUIRE((u != nullptr) == (au != nullptr) && (u != nullptr) != (bonus != nullptr), "linear_chunks: either u and au or a bonus");
+  B200_REQUIRE(tokens > 0 && seqs > 0 && max_q_len > 0 && b200_state_chunks_supported(rule, heads, heads, dk, dv), "linear_chunks: shape not taken");
+  const Sizes z = {tokens, seqs, max_q_len, heads, dk, dv};
+  const Requests req = {seq_q_start, seq_q_len, seq_slot};
+  Scratch parts;
+  B200_REQUIRE(aligned16(scratch) && lay_out(rule, z, scratch, &parts) <= scratch_floats, "linear_chunks: scratch too small or not aligned to 16 bytes");
+  B200_REQUIRE(seqs <= 65535 && !too_many_requests(z), "linear_chunks: too many requests");
+  B200_REQUIRE(raise_all(), "linear_chunks: cannot size shared memory");
+  const bool wide = dk % 4 == 0 && dv % 4 == 0 && aligned16(r) && aligned16(k) && aligned16(v) && aligned16(w) && aligned16(au) && aligned16(u);
+  const bool general = rule == kGeneralDelta;
+  const int rows = padded_rows(dk), columns = padded_columns(dv);
+  auto prepare = rows == 64 ? linear_prepare_form<64>(wide, general) : linear_prepare_form<128>(wide, general);
+  launch_kernel(prepare, dim3((max_q_len + C - 1) / C, heads, seqs), dim3(kThreads), linear_prepare_smem(rows, general), stream, LinearRule{r, k, v, w, au, u, bonus},
+                seq_q_start, seq_q_len, heads, dk, dv, parts);
+  if (int status = b200_check_launch("linear_chunk_prepare")) return status;
+  if (general) {
+    if (int status = launch_walk(z, req, true, parts, state, stream)) return status;
+    return launch_out<true, true>(z, req, parts, v, out, stream);
+  }
+  launch_kernel(chunk_scan_kernel, dim3((rows * columns / 4 + kThreads - 1) / kThreads, heads, seqs), dim3(kThreads), 0, stream, seq_q_start, seq_q_len, seq_slot, heads,
+                dk, dv, parts, state);
+  if (int status = b200_check_launch("chunk_scan")) return status;
+  return launch_out<false, true>(z, req, parts, v, out, stream);
 }

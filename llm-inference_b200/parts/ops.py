@@ -874,27 +874,59 @@ def delta_prepare(
 DELTA_CHUNK_FROM = 112
 
 
+# The same for the rules in which the values enter as they are, one request, 24 heads of 64 x 64. Without a removal: 39 us in chunks and
+# 33 token by token at 64 tokens, 38 and 43 at 100, 40 and 69 at 200, 101 and 564 at 2,048. Generalized delta rule: 51 and 39 us at 100
+# tokens, 61 and 62 at 200, 244 and 473 at 2,048.
+LINEAR_CHUNK_FROM = 80
+GENERAL_DELTA_CHUNK_FROM = 192
+_DELTA, _GENERAL_DELTA, _LINEAR = 0, 1, 2  # csrc/kernels/state_chunks.cu
+
+
+def _chunk_scratch(ctx: StepContext, rule: int, longer_than: int, tokens: int, heads: int, kv_heads: int, dk: int, dv: int) -> torch.Tensor | None:
+    """Scratch for a recurrence that runs chunk by chunk (csrc/kernels/state_chunks.cu), or None where it runs token by token:
+    portions of at most ``longer_than`` tokens and sizes the chunked form does not take. ``options["delta_portions"]``:
+    ``"chunks"`` or ``"tokens"`` forces one of the two."""
+    choice = ctx.options.get("delta_portions", "auto")
+    if choice == "tokens" or (choice == "auto" and not (
+        ctx.max_q_len > longer_than and ctx.lib.lib.b200_state_chunks_supported(rule, heads, kv_heads, dk, dv)
+    )):
+        return None
+    floats = int(ctx.lib.lib.b200_state_chunks_scratch(rule, tokens, ctx.num_seqs, heads, dk, dv))
+    return ctx.buffer("state_chunks", (floats,), torch.float32, per_token=False)
+
+
 def _delta_chunks(
     ctx: StepContext, q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, beta: torch.Tensor, decay: torch.Tensor, per_head: bool,
     state: torch.Tensor, out: torch.Tensor, heads: int, kv_heads: int, dk: int, dv: int,
 ) -> bool:
-    """Portions of more than ``DELTA_CHUNK_FROM`` tokens run chunk by chunk (csrc/kernels/state_chunks.cu); returns False, doing
-    nothing, for shorter ones and for sizes the chunked form does not take. ``options["delta_portions"]``: ``"chunks"`` or
-    ``"tokens"`` forces one of the two."""
-    choice = ctx.options.get("delta_portions", "auto")
-    if choice == "tokens" or (choice == "auto" and not (
-        ctx.max_q_len > DELTA_CHUNK_FROM and ctx.lib.lib.b200_delta_chunks_supported(heads, kv_heads, dk, dv)
-    )):
-        return False
     tokens = q.shape[0]
-    floats = int(ctx.lib.lib.b200_delta_chunks_scratch(tokens, ctx.num_seqs, heads, dk, dv))
-    scratch = ctx.buffer("delta_chunks", (floats,), torch.float32, per_token=False)
+    scratch = _chunk_scratch(ctx, _DELTA, DELTA_CHUNK_FROM, tokens, heads, kv_heads, dk, dv)
+    if scratch is None:
+        return False
     ctx.lib.call(
         "b200_delta_chunks", ptr(q), ptr(k), ptr(v), ptr(beta), ptr(decay), c_int(1 if per_head else 0), ptr(ctx.seq_q_start), ptr(ctx.seq_q_len),
         ptr(ctx.seq_slot), c_int(tokens), c_int(ctx.num_seqs), c_int(ctx.max_q_len), c_int(heads), c_int(kv_heads), c_int(dk), c_int(dv),
-        ptr(scratch), c_int64(floats), ptr(state), ptr(out), ctx.stream,
+        ptr(scratch), c_int64(scratch.numel()), ptr(state), ptr(out), ctx.stream,
     )
-    ctx.lib.calls += 2  # three kernels
+    ctx.lib.calls += 2  # further kernels of the call
+    return True
+
+
+def _linear_chunks(
+    ctx: StepContext, r: torch.Tensor, k: torch.Tensor, v: torch.Tensor, w: torch.Tensor, au: torch.Tensor | None, u: torch.Tensor | None,
+    bonus: torch.Tensor | None, state: torch.Tensor, out: torch.Tensor, heads: int, dk: int, dv: int,
+) -> bool:
+    tokens = r.shape[0]
+    rule, longer_than = (_LINEAR, LINEAR_CHUNK_FROM) if u is None else (_GENERAL_DELTA, GENERAL_DELTA_CHUNK_FROM)
+    scratch = _chunk_scratch(ctx, rule, longer_than, tokens, heads, heads, dk, dv)
+    if scratch is None:
+        return False
+    ctx.lib.call(
+        "b200_linear_chunks", ptr(r), ptr(k), ptr(v), ptr(w), ptr(au), ptr(u), ptr(bonus), ptr(ctx.seq_q_start), ptr(ctx.seq_q_len),
+        ptr(ctx.seq_slot), c_int(tokens), c_int(ctx.num_seqs), c_int(ctx.max_q_len), c_int(heads), c_int(dk), c_int(dv),
+        ptr(scratch), c_int64(scratch.numel()), ptr(state), ptr(out), ctx.stream,
+    )
+    ctx.lib.calls += 3 if u is None else 2  # further kernels of the call
     return True
 
 
@@ -903,7 +935,7 @@ def delta_recurrence(
     state: torch.Tensor, out: torch.Tensor, heads: int, kv_heads: int, dk: int, dv: int,
 ) -> torch.Tensor:
     """The delta rule with a decay per head and key channel over every request's new tokens: chunk by chunk or token by token
-    (see ``_delta_chunks``)."""
+    (see ``_chunk_scratch``)."""
     _need(state.dtype == torch.float32 and tuple(state.shape[1:]) == (heads, dk, dv) and state.is_contiguous(), "delta_recurrence: the state is float32 [slots, heads, dk, dv]")
     _need(out.dtype == torch.float32 and tuple(out.shape) == (q.shape[0], heads * dv) and out.is_contiguous(), "delta_recurrence: bad output")
     if _delta_chunks(ctx, q, k, v, beta, decay, False, state, out, heads, kv_heads, dk, dv):
@@ -937,7 +969,7 @@ def delta_head_recurrence(
     state: torch.Tensor, out: torch.Tensor, heads: int, kv_heads: int, dk: int, dv: int,
 ) -> torch.Tensor:
     """The delta rule with one decay per head over every request's new tokens (operands as :func:`delta_prepare` leaves them):
-    chunk by chunk or token by token (see ``_delta_chunks``)."""
+    chunk by chunk or token by token (see ``_chunk_scratch``)."""
     tokens = q.shape[0]
     _need(state.dtype == torch.float32 and tuple(state.shape[1:]) == (heads, dk, dv) and state.is_contiguous(), "delta_head_recurrence: the state is float32 [slots, heads, dk, dv]")
     for tensor, width in ((q, kv_heads * dk), (k, kv_heads * dk), (v, heads * dv), (beta, heads), (log_decay, heads), (kq, kv_heads), (out, heads * dv)):
@@ -1087,6 +1119,8 @@ def wkv_recurrence(
 ) -> torch.Tensor:
     _need(state.dtype == torch.float32 and tuple(state.shape[1:]) == (heads, dk, dv) and state.is_contiguous(), "wkv_recurrence: the state is float32 [slots, heads, dk, dv]")
     _need(out.dtype == torch.float32 and tuple(out.shape) == (r.shape[0], heads * dv) and out.is_contiguous(), "wkv_recurrence: bad output")
+    if _linear_chunks(ctx, r, k, v, decay, None, None, bonus, state, out, heads, dk, dv):
+        return out
     ctx.lib.call(
         "b200_wkv_recurrence", ptr(r), ptr(k), ptr(v), ptr(bonus), ptr(decay), ptr(ctx.seq_q_start), ptr(ctx.seq_q_len), ptr(ctx.seq_slot),
         c_int(ctx.num_seqs), c_int(heads), c_int(dk), c_int(dv), ptr(state), ptr(out), ctx.stream,
@@ -1334,6 +1368,8 @@ def delta_general_recurrence(
     """``S <- diag(w) S - au (u^T S) + k v^T``, ``o = S^T r`` per head and token, each request from its slot of ``state``."""
     _need(state.dtype == torch.float32 and tuple(state.shape[1:]) == (heads, dk, dv) and state.is_contiguous(), "delta_general_recurrence: the state is float32 [slots, heads, dk, dv]")
     _need(out.dtype == torch.float32 and tuple(out.shape) == (r.shape[0], heads * dv) and out.is_contiguous(), "delta_general_recurrence: bad output")
+    if _linear_chunks(ctx, r, k, v, w, au, u, None, state, out, heads, dk, dv):
+        return out
     ctx.lib.call(
         "b200_delta_general_recurrence", ptr(r), ptr(k), ptr(v), ptr(w), ptr(au), ptr(u), ptr(ctx.seq_q_start), ptr(ctx.seq_q_len),
         ptr(ctx.seq_slot), c_int(ctx.num_seqs), c_int(max(ctx.max_q_len, 1)), c_int(heads), c_int(dk), c_int(dv), ptr(state), ptr(out), ctx.stream,

@@ -88,3 +88,61 @@ def test_delta_rules(heads, kv_heads, dk, dv, runs, portions, per_head):
     np.testing.assert_allclose(state[slots].double().cpu().numpy(), states, **CLOSE)
     others = [slot for slot in range(state.shape[0]) if slot not in slots]
     assert torch.equal(state[others], untouched[others])
+
+
+LINEAR_SIZES = [
+    (2, 64, 64, (81, 32, 1)),
+    (3, 33, 17, (31, 65)),
+    (1, 128, 70, (127,)),
+    (2, 16, 130, (96, 95, 97)),
+]
+
+
+@pytest.mark.parametrize("heads,dk,dv,runs", LINEAR_SIZES)
+@pytest.mark.parametrize("portions", ["chunks", "tokens"])
+@pytest.mark.parametrize("general", [False, True])
+def test_rules_in_which_the_values_enter_as_they_are(heads, dk, dv, runs, portions, general):
+    from llm_inference_b200.parts import ops
+
+    n = sum(runs)
+    rng = np.random.default_rng(dk + dv)
+    r, k, v = (rng.normal(size=(n, heads, width)) for width in (dk, dk, dv))
+    k[5:20] = k[5]
+    w = np.exp(-np.exp(rng.normal(-3, 2, (n, heads, dk))))
+    w[3::29], w[17::41, 0] = 1.0, 0.0
+    start, bonus = rng.normal(size=(len(runs), heads, dk, dv)), rng.normal(size=(n, heads))
+    u = k / np.linalg.norm(k, axis=-1, keepdims=True)
+    if general:  # decays of this rule are bounded from below
+        w = np.maximum(w, 0.545)
+    au = u * rng.uniform(0.0, 1.0, (n, heads, dk))
+    r, k, v, w, start, bonus, u, au = (a.astype(np.float32) for a in (r, k, v, w, start, bonus, u, au))
+    states, want, at = start.astype(np.float64), np.zeros((n, heads, dv)), 0
+    for s, run in enumerate(runs):
+        for t in range(at, at + run):
+            R, K, V, D, U, A = (x[t].astype(np.float64) for x in (r, k, v, w, u, au))
+            old = states[s]
+            added = K[..., None] * V[:, None]
+            if general:
+                states[s] = D[..., None] * old - A[..., None] * np.einsum("hkv,hk->hv", old, U)[:, None] + added
+                want[t] = np.einsum("hkv,hk->hv", states[s], R)
+            else:
+                want[t] = np.einsum("hkv,hk->hv", old, R) + bonus[t][:, None] * V
+                states[s] = D[..., None] * old + added
+        at += run
+    slots = [4, 0, 2][: len(runs)]
+    runner, cache, ctx = device_context(runs, slots, ((heads, dk, dv),), {"delta_portions": portions})
+    state = cache.states[0][0]
+    untouched = state.clone().normal_()
+    state.copy_(untouched)
+    state[slots] = torch.from_numpy(start).cuda()
+    out = torch.full((n, heads * dv), float("nan"), device="cuda")
+    if general:
+        ops.delta_general_recurrence(ctx, *(on_device(a) for a in (r, k, v, w, au, u)), state, out, heads, dk, dv)
+    else:
+        ops.wkv_recurrence(ctx, *(on_device(a) for a in (r, k, v, bonus, w)), state, out, heads, dk, dv)
+    runner.check()
+    # States and read-outs here are sums of a few hundred products of order one over dk channels: errors go with the whole's size.
+    for got, wanted in ((out.double().cpu().numpy().reshape(want.shape), want), (state[slots].double().cpu().numpy(), states)):
+        np.testing.assert_allclose(got, wanted, rtol=2e-5, atol=2e-6 * np.sqrt(np.mean(wanted**2)) * np.sqrt(dk) + 2e-5)
+    others = [slot for slot in range(state.shape[0]) if slot not in slots]
+    assert torch.equal(state[others], untouched[others])
