@@ -57,6 +57,7 @@ _SIGNATURES: dict[str, list] = {
     + [c_int, c_int, c_void_p]
     + [c_int] * 7
     + [c_float, c_int, c_float, c_void_p, c_int, c_int, c_void_p, c_void_p, c_int, c_void_p, c_void_p],
+    "b200_portion_attention_f32": [c_void_p] * 4 + [c_int] * 2 + [c_void_p] * 3 + [c_int] * 3 + [c_void_p] * 2 + [c_int] * 5 + [c_float, c_void_p, c_void_p],
     "b200_gemm_f32": [c_void_p] * 4 + [c_int] * 6 + [c_void_p],
     "b200_paged_flash_attention": [c_void_p] * 8 + [c_int] * 12 + [c_float, c_int, c_int, c_int, c_float, c_void_p, c_int, c_int, c_void_p,
                                    c_void_p, c_void_p, c_void_p, c_void_p],
@@ -167,6 +168,8 @@ class KernelLibrary:
         self.lib.b200_latent_attention_mma_supported.restype = c_int
         self.lib.b200_latent_attention_mma_scratch.argtypes = [c_int] * 5
         self.lib.b200_latent_attention_mma_scratch.restype = c_int64
+        self.lib.b200_portion_attention_f32_supported.argtypes = [c_int] * 3
+        self.lib.b200_portion_attention_f32_supported.restype = c_int
         self.lib.b200_state_chunks_supported.argtypes = [c_int] * 5
         self.lib.b200_state_chunks_supported.restype = c_int
         self.lib.b200_state_chunks_scratch.argtypes = [c_int] * 6

@@ -50,6 +50,12 @@ def attend(
     if not tuned:
         if choice in ("flash", "tcgen05"):
             raise ops.KernelError("the tensor-core attention kernels do not take this shape or dtype")
+        if choice != "plain" and ops.portion_attention_f32_takes(ctx, cache, q, q_heads, kv_heads, head_dim, value_head, shape):
+            decode = ctx.num_decode_seqs  # single tokens lead the batch
+            if decode:
+                ops.paged_attention_plain(ctx, cache, q, out, q_heads, kv_heads, head_dim, scale, num_tokens=decode, shape=shape)
+            ops.portion_attention_f32(ctx, cache, q, out, q_heads, kv_heads, head_dim, scale, first_seq=decode, shape=shape)
+            return
         ops.paged_attention_plain(ctx, cache, q, out, q_heads, kv_heads, head_dim, scale, value_head=value_head, shape=shape)
         return
     decode_seqs = ctx.num_decode_seqs

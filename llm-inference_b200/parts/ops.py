@@ -433,6 +433,34 @@ def paged_attention_plain(
     return out
 
 
+def portion_attention_f32_takes(ctx: StepContext, cache: CacheView, q: torch.Tensor, q_heads: int, kv_heads: int, head_dim: int, value_head: int,
+                                shape: ScoreShape) -> bool:
+    """Whether the step's prompt portions run the tiled 32-bit kernel (csrc/kernels/attention_f32.cu): float32, unshaped scores (a window
+    and a sink are taken). Only portions of a few tokens with few keys stay with the plain kernel, whose blocks start sooner
+    (one request, 12 heads of 128 on 2 kv heads, plain and tiled: 16 tokens 28 and 30 us, 32 tokens 30 and 28, 500 tokens 325 and
+    88; 8 tokens behind 1,000 others 191 and 128)."""
+    return (
+        q.dtype == torch.float32 and value_head < 0 and not shape.changes_scores() and shape.sigmoid_bias is None
+        and not (cache.window and cache.keep_first) and ctx.num_seqs > ctx.num_decode_seqs
+        and (ctx.max_q_len >= 32 or ctx.max_kv_len >= 256)
+        and bool(ctx.lib.lib.b200_portion_attention_f32_supported(q_heads, kv_heads, head_dim))
+    )
+
+
+def portion_attention_f32(ctx: StepContext, cache: CacheView, q: torch.Tensor, out: torch.Tensor, q_heads: int, kv_heads: int, head_dim: int, scale: float,
+                          *, first_seq: int, shape: ScoreShape = NO_SHAPE) -> torch.Tensor:
+    """Attention of the requests from ``first_seq`` on (float32)."""
+    _need(q.is_contiguous() and out.is_contiguous() and q.dtype == torch.float32 == out.dtype == cache.keys.dtype, "portion_attention_f32: bad operands")
+    sink = shape.arguments(q_heads)[-1]
+    ctx.lib.call(
+        "b200_portion_attention_f32", ptr(q), ptr(cache.keys), ptr(cache.values), ptr(cache.block_table), c_int(cache.max_pages), c_int(cache.num_pages),
+        ptr(ctx.seq_q_start), ptr(ctx.seq_q_len), ptr(ctx.seq_kv_len), c_int(first_seq), c_int(ctx.num_seqs - first_seq), c_int(ctx.max_q_len),
+        sink, ptr(out), c_int(q_heads), c_int(kv_heads), c_int(head_dim), c_int(cache.page_size), c_int(cache.window), c_float(scale),
+        ptr(ctx.err), ctx.stream,
+    )
+    return out
+
+
 NUM_SMS = 148  # a B200; only what `decode_splits` assumes when no device is asked (tests on the CPU)
 DECODE_STAGES = 3  # pieces in flight per warp of the TMA decode kernel
 MAX_DECODE_SPLITS = 64  # what the merge kernel takes in one round trip

@@ -1,0 +1,82 @@
+"""Prompt portions in true 32-bit attention (the tiled kernel): against the plain kernel's formulas in 64 bits at the ends of its tiles
+(32 rows of tokens and heads, 64 keys), with windows, sinks, ragged requests beside single tokens, odd head and page sizes, and values
+of later tokens that are not finite."""
+
+from __future__ import annotations
+
+import numpy as np
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+CASES = [
+    # q heads, kv heads, head size, page size, window, sink, (new tokens, tokens before) per request
+    (12, 2, 128, 64, 0, False, ((1, 40), (1, 0), (43, 0), (33, 200))),
+    (5, 5, 64, 16, 0, True, ((32, 0), (65, 31))),
+    (6, 2, 24, 7, 20, False, ((1, 300), (64, 300), (97, 5))),
+    (16, 1, 100, 32, 64, True, ((2, 254), (40, 64))),
+    (3, 3, 128, 128, 1, False, ((63, 129),)),
+]
+
+
+@pytest.mark.parametrize("q_heads,kv_heads,dim,page,window,with_sink,requests", CASES)
+def test_portions_against_64_bits(q_heads, kv_heads, dim, page, window, with_sink, requests):
+    from llm_inference_b200.cli.microbench import make_ctx
+    from llm_inference_b200.parts import attention_dispatch, ops
+    from llm_inference_b200.parts.context import CacheView
+
+    rng = np.random.default_rng(q_heads * dim + window)
+    runs, starts = [r for r, _ in requests], [s for _, s in requests]
+    lengths = [r + s for r, s in requests]
+    need = [-(-n // page) for n in lengths]
+    order = rng.permutation(sum(need) + 2)
+    tables, at = np.zeros((len(runs), max(need)), dtype=np.int32), 0
+    for row, count in zip(tables, need):
+        row[:count] = order[at : at + count]
+        at += count
+    keys, values = (rng.normal(size=(sum(need) + 2, kv_heads, page, dim)).astype(np.float32) for _ in range(2))
+    q = (3.0 * rng.normal(size=(sum(runs), q_heads, dim))).astype(np.float32)
+    sink = rng.normal(size=q_heads).astype(np.float32)
+    last = len(runs) - 1  # the last token of the last request has values that are not finite: nobody before it sees them
+    where = lengths[last] - 1
+    values[tables[last][where // page], :, where % page] = np.nan
+    scale, share = dim**-0.5, q_heads // kv_heads
+    want, row = np.zeros((sum(runs), q_heads, dim)), 0
+    for i, (run, start) in enumerate(requests):
+        flat = [a[tables[i][: need[i]]].transpose(0, 2, 1, 3).reshape(-1, kv_heads, dim)[: lengths[i]].astype(np.float64) for a in (keys, values)]
+        for t in range(run):
+            pos = start + t
+            lo = max(0, pos - window + 1) if window else 0
+            for h in range(q_heads):
+                s = flat[0][lo : pos + 1, h // share] @ q[row, h].astype(np.float64) * scale
+                top = max(s.max(), sink[h]) if with_sink else s.max()
+                p = np.exp(s - top)
+                want[row, h] = (p @ flat[1][lo : pos + 1, h // share]) / (p.sum() + (np.exp(sink[h] - top) if with_sink else 0.0))
+            row += 1
+    ctx = make_ctx([p for r, s in requests for p in range(s, s + r)], [i for i, r in enumerate(runs) for _ in range(r)], starts, runs)
+    ctx.num_decode_seqs = sum(1 for r in runs if r == 1)
+    view = CacheView(0, True, torch.from_numpy(keys).cuda(), torch.from_numpy(values).cuda(), torch.from_numpy(tables).cuda(), len(order), tables.shape[1], page, window)
+    shape = ops.ScoreShape(sink=torch.from_numpy(sink).cuda()) if with_sink else ops.NO_SHAPE
+    rows = torch.from_numpy(q.reshape(sum(runs), -1)).cuda()
+    assert ops.portion_attention_f32_takes(ctx, view, rows, q_heads, kv_heads, dim, -1, shape)
+    out = torch.full_like(rows, 7.0)
+    attention_dispatch.attend(ctx, view, rows, out, q_heads, kv_heads, dim, scale, shape=shape)
+    assert int(ctx.err.item()) == 0
+    got = out.double().cpu().numpy().reshape(want.shape)
+    assert np.isnan(got[-1]).all() and np.isnan(want[-1]).all()
+    # 32-bit: a score is a sum of dim products of size up to ten, its error enters the weights as it is
+    np.testing.assert_allclose(got[:-1], want[:-1], atol=3e-5, rtol=3e-5)
+
+
+def test_a_bad_page_is_flagged_and_not_read():
+    from llm_inference_b200.cli.microbench import make_ctx
+    from llm_inference_b200.parts import ops
+    from llm_inference_b200.parts.context import CacheView
+
+    ctx = make_ctx(list(range(70)), [0] * 70, [0], [70])
+    arena = torch.randn(3, 1, 64, 16, device="cuda")
+    q = torch.randn(70, 16, device="cuda")
+    view = CacheView(0, True, arena, arena, torch.tensor([[1, 9]], dtype=torch.int32, device="cuda"), 3, 2, 64, 0)
+    out = ops.portion_attention_f32(ctx, view, q, torch.empty_like(q), 1, 1, 16, 0.25, first_seq=0)
+    assert int(ctx.err.item()) == 1 and torch.isfinite(out).all()
