@@ -1236,6 +1236,15 @@ def moe_route(ctx: StepContext, logits: torch.Tensor, groups: int, keep: int, to
     )
 
 
+# Where tall tiles on tcgen05 beat short ones on mma.sync before an expert fills two of them: its tile of 128 places has to be a quarter
+# full, and the whole work large enough to pay for the gather pass and the longer pipeline. Both products on a B200, mma.sync and tcgen05
+# in us: 32 experts of 1,120 x 1,536, four a token: 256 tokens 137 and 134, 512 tokens 186 and 138, 1,777 tokens 413 and 190; of 2,368 x
+# 3,584: 192 tokens 352 and 378, 256 tokens 391 and 385, 1,024 tokens 999 and 463; 16 experts of 512 x 2,048, two a token: 512 tokens 83
+# and 98, 1,024 tokens 116 and 106; of 256 x 512: 2,048 tokens 63 and 79. Both form the same sums in the same order, to the bit.
+MOE_TALL_SLOTS = 32
+MOE_TALL_PRODUCTS = 1_750_000_000  # slots x width x inner width
+
+
 def moe_tile_rows(ctx: StepContext) -> int:
     return int(ctx.lib.lib.b200_moe_tile_rows())
 
@@ -1263,7 +1272,9 @@ def moe_experts(
     choice = ctx.options.get("moe", "auto")
     tensor_cores = h.dtype == torch.bfloat16 and choice != "plain" and bool(ctx.lib.lib.b200_moe_mma_supported(width, ff))
     tile = moe_tile_rows(ctx)
-    tall = tensor_cores and slots >= 2 * 4 * tile * experts
+    tall = tensor_cores and (
+        slots >= 2 * 4 * tile * experts or (slots >= MOE_TALL_SLOTS * experts and slots * width * ff >= MOE_TALL_PRODUCTS)
+    )
     if tall:
         tile *= 4
     max_tiles = (slots + experts * (tile - 1)) // tile + 1
