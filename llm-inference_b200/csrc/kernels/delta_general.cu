@@ -11,6 +11,7 @@
 // `delta_general_recurrence` (the columns of S are independent: column c follows
 // s <- w (.) s - (a (.) u) (u . s) + k v_c, so a thread group owns a column and walks the request's tokens).
 #include "common.cuh"
+#include "packs.cuh"
 
 namespace {
 
@@ -48,6 +49,36 @@ __global__ void delta_general_prepare_kernel(const T* proj, int ld, int r_at, in
       u_out[base + c] = u;
     }
   }
+}
+
+// The same with four numbers a thread: 2^n lanes hold one (token, head), dim = 4 x 2^n up to 128. 2,048 tokens of 24 heads of 64: 30 -> 17 us.
+template <typename T>
+__global__ void __launch_bounds__(256)
+delta_general_prepare_wide_kernel(const T* proj, int ld, int r_at, int k_at, int v_at, int a_at, const float* lw, const float* __restrict__ w0,
+                                  const float* __restrict__ a_bias, int tokens, int heads, int dim, float* r_out, float* k_out, float* v_out, float* w_out,
+                                  float* au_out, float* u_out) {
+  wait_for_predecessor();
+  let_successor_start();
+  const int lanes = dim / 4, inner = heads * dim;
+  const int64_t quad = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
+  const bool live = quad < static_cast<int64_t>(tokens) * heads * lanes;
+  const int64_t at = live ? quad * 4 : 0;
+  const int c = static_cast<int>(at % inner);
+  const T* row = proj + at / inner * ld + c;
+  const float4 kv = load4<T>(row + k_at), rv = load4<T>(row + r_at), vv = load4<T>(row + v_at), av = load4<T>(row + a_at);
+  const float4 z = *reinterpret_cast<const float4*>(lw + at), bias = *reinterpret_cast<const float4*>(w0 + c), a_shift = *reinterpret_cast<const float4*>(a_bias + c);
+  float ss = square_sum(kv, 0.f);
+  for (int step = lanes >> 1; step > 0; step >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, step);
+  if (!live) return;
+  const float4 u = scale_each(kv, 1.f / sqrtf(ss + 1e-6f));
+  *reinterpret_cast<float4*>(r_out + at) = rv;
+  *reinterpret_cast<float4*>(k_out + at) = kv;
+  *reinterpret_cast<float4*>(v_out + at) = vv;
+  *reinterpret_cast<float4*>(w_out + at) = make_float4(expf(-kDecayRate * sigmoid_f(z.x + bias.x)), expf(-kDecayRate * sigmoid_f(z.y + bias.y)),
+                                                       expf(-kDecayRate * sigmoid_f(z.z + bias.z)), expf(-kDecayRate * sigmoid_f(z.w + bias.w)));
+  *reinterpret_cast<float4*>(au_out + at) = make_float4(sigmoid_f(av.x + a_shift.x) * u.x, sigmoid_f(av.y + a_shift.y) * u.y, sigmoid_f(av.z + a_shift.z) * u.z,
+                                                        sigmoid_f(av.w + a_shift.w) * u.w);
+  *reinterpret_cast<float4*>(u_out + at) = u;
 }
 
 // A block owns `cols` columns of one head of one request; a column's dk rows are spread over
@@ -216,6 +247,20 @@ B200_API int b200_delta_general_prepare(const void* proj, int ld, int r_at, int 
   B200_REQUIRE(r_at >= 0 && k_at >= 0 && v_at >= 0 && a_at >= 0 && r_at + inner <= ld && k_at + inner <= ld && v_at + inner <= ld &&
                    a_at + inner <= ld,
                "delta_general_prepare: rows of %d numbers do not hold the projections", ld);
+  const int lanes = dim / 4, in_bytes = dtype == DTYPE_F32 ? 16 : 8;
+  const auto on = [](const void* p, int bytes) { return reinterpret_cast<uintptr_t>(p) % bytes == 0; };
+  if (dim % 4 == 0 && lanes <= 32 && (lanes & (lanes - 1)) == 0 && ld % 4 == 0 && r_at % 4 == 0 && k_at % 4 == 0 && v_at % 4 == 0 && a_at % 4 == 0 &&
+      on(proj, in_bytes) && on(lw, 16) && on(w0, 16) && on(a_bias, 16) && on(r_out, 16) && on(k_out, 16) && on(v_out, 16) && on(w_out, 16) && on(au_out, 16) &&
+      on(u_out, 16) && (dtype == DTYPE_F32 || dtype == DTYPE_BF16)) {
+    const dim3 quads(static_cast<unsigned>((static_cast<int64_t>(tokens) * heads * lanes + 255) / 256));
+    if (dtype == DTYPE_F32)
+      launch_kernel(delta_general_prepare_wide_kernel<float>, quads, dim3(256), 0, stream, static_cast<const float*>(proj), ld, r_at, k_at, v_at, a_at, lw, w0, a_bias,
+                    tokens, heads, dim, r_out, k_out, v_out, w_out, au_out, u_out);
+    else
+      launch_kernel(delta_general_prepare_wide_kernel<__nv_bfloat16>, quads, dim3(256), 0, stream, static_cast<const __nv_bfloat16*>(proj), ld, r_at, k_at, v_at, a_at,
+                    lw, w0, a_bias, tokens, heads, dim, r_out, k_out, v_out, w_out, au_out, u_out);
+    return b200_check_launch("delta_general_prepare");
+  }
   const int threads = 128;
   const dim3 grid(tokens, static_cast<unsigned>(min((heads + 3) / 4, 65535)));  // four warps, a head each
   if (dtype == DTYPE_F32) {

@@ -15,7 +15,10 @@
 // `conv_state_update` (one block per request: the slot's last inputs), `delta_recurrence` (the
 // columns of S are independent, so a thread group owns a column and walks the request's tokens),
 // `delta_output` (o / rms(o) * w * sigmoid(gate)).
+#include <type_traits>
+
 #include "common.cuh"
+#include "packs.cuh"
 
 namespace {
 
@@ -89,6 +92,107 @@ __global__ void delta_prepare_kernel(const T* proj, int ld, const T* decay_in, i
   }
 }
 
+// The same for prompt portions and four taps: four neighbouring tokens a block, four neighbouring channels a thread at a time, so a
+// row of inputs and a channel's taps are read once for the four tokens that want them, eight or sixteen bytes an access. One block a
+// token read two bytes at a time, every row four times: on a B200 2,048 tokens of 4,608 channels took 79 us with a decay per channel and
+// 46 with one per head (3,072 channels), now 58 and 30.
+constexpr int kWideTokens = 4, kWideTaps = 4;
+
+template <typename T>
+__global__ void __launch_bounds__(256)
+delta_prepare_wide_kernel(const T* proj, int ld, const T* decay_in, int decay_ld, const float* __restrict__ taps_w, const T* conv_state,
+                          const float* __restrict__ a_log, const float* __restrict__ dt_bias, const int* token_seq, const int* seq_q_start,
+                          const int* seq_slot, int tokens, int heads, int kv_heads, int dk, int dv, float* q_out, float* k_out, float* v_out, float* beta_out,
+                          float* decay_out, float* kq_out) {
+  extern __shared__ __align__(16) float y[];  // [kWideTokens][2 * kv_heads * dk]: q and k behind the convolution
+  __shared__ int start_of[kWideTokens], slot_of[kWideTokens];
+  wait_for_predecessor();
+  let_successor_start();
+  const int t0 = blockIdx.x * kWideTokens, tid = threadIdx.x, count = min(kWideTokens, tokens - t0);
+  const int qk = kv_heads * dk, vw = heads * dv, channels = 2 * qk + vw;
+  if (tid < count) {
+    const int seq = token_seq[t0 + tid];
+    start_of[tid] = seq_q_start[seq];
+    slot_of[tid] = seq_slot[seq];
+  }
+  __syncthreads();
+  for (int c = tid * 4; c < channels; c += blockDim.x * 4) {
+    float4 rows[kWideTokens + kWideTaps - 1];  // inputs of tokens t0 - 3 .. t0 + 3
+#pragma unroll
+    for (int i = 0; i < kWideTokens + kWideTaps - 1; ++i) {
+      const int t = t0 - (kWideTaps - 1) + i;
+      rows[i] = t >= 0 && t < tokens ? load4<T>(proj + static_cast<int64_t>(t) * ld + c) : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+    float4 taps[4];  // of channel c + x
+#pragma unroll
+    for (int x = 0; x < 4; ++x) taps[x] = *reinterpret_cast<const float4*>(taps_w + (c + x) * kWideTaps);
+#pragma unroll
+    for (int i = 0; i < kWideTokens; ++i) {
+      if (i >= count) break;
+      const int run = t0 + i - start_of[i];  // tokens of this request in front of t within the step
+      float4 in[kWideTaps];
+#pragma unroll
+      for (int j = 0; j < kWideTaps; ++j) {
+        in[j] = rows[i + j];
+        if (kWideTaps - 1 - j > run)  // from the request's slot
+          in[j] = load4<T>(conv_state + (static_cast<int64_t>(slot_of[i]) * (kWideTaps - 1) + run + j) * channels + c);
+      }
+      float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+      const float* w[4] = {&taps[0].x, &taps[1].x, &taps[2].x, &taps[3].x};
+#pragma unroll
+      for (int j = 0; j < kWideTaps; ++j) {
+        acc.x = fmaf(w[0][j], in[j].x, acc.x), acc.y = fmaf(w[1][j], in[j].y, acc.y);
+        acc.z = fmaf(w[2][j], in[j].z, acc.z), acc.w = fmaf(w[3][j], in[j].w, acc.w);
+      }
+      acc = make_float4(acc.x * sigmoid_f(acc.x), acc.y * sigmoid_f(acc.y), acc.z * sigmoid_f(acc.z), acc.w * sigmoid_f(acc.w));
+      if (c < 2 * qk) *reinterpret_cast<float4*>(y + i * 2 * qk + c) = acc;
+      else *reinterpret_cast<float4*>(v_out + static_cast<int64_t>(t0 + i) * vw + c - 2 * qk) = acc;
+    }
+  }
+  const bool per_head = kq_out != nullptr;
+  for (int idx = tid; idx < count * heads; idx += blockDim.x) {
+    const int64_t t = t0 + idx / heads;
+    const int h = idx % heads;
+    beta_out[t * heads + h] = sigmoid_f(to_f32<T>(proj[t * ld + channels + h]));
+    if (per_head) decay_out[t * heads + h] = -expf(a_log[h]) * softplus_f(to_f32<T>(decay_in[t * decay_ld + h]) + dt_bias[h]);
+  }
+  if (!per_head) {
+    for (int i = 0; i < count; ++i)
+      for (int c = tid * 4; c < heads * dk; c += blockDim.x * 4) {
+        const float4 z = load4<T>(decay_in + static_cast<int64_t>(t0 + i) * decay_ld + c), bias = *reinterpret_cast<const float4*>(dt_bias + c);
+        const float rate = -expf(a_log[c / dk]);
+        *reinterpret_cast<float4*>(decay_out + static_cast<int64_t>(t0 + i) * heads * dk + c) =
+            make_float4(expf(rate * softplus_f(z.x + bias.x)), expf(rate * softplus_f(z.y + bias.y)), expf(rate * softplus_f(z.z + bias.z)),
+                        expf(rate * softplus_f(z.w + bias.w)));
+      }
+  }
+  __syncthreads();
+  const int lane = tid & 31, warp = tid >> 5, warps = blockDim.x >> 5;
+  // unit vectors: one warp per (token, q/k head), q and k one after the other, and k . q
+  for (int item = warp; item < count * kv_heads; item += warps) {
+    const int64_t t = t0 + item / kv_heads;
+    const int head = item % kv_heads;
+    const float* q = y + item / kv_heads * 2 * qk + head * dk;
+    const float* k = q + qk;
+    float q_ss = 0.f, k_ss = 0.f, dot = 0.f;
+    for (int i = lane * 4; i < dk; i += 128) {
+      const float4 a = *reinterpret_cast<const float4*>(q + i), b = *reinterpret_cast<const float4*>(k + i);
+      q_ss = square_sum(a, q_ss), k_ss = square_sum(b, k_ss);
+      dot = fmaf(a.x, b.x, fmaf(a.y, b.y, fmaf(a.z, b.z, fmaf(a.w, b.w, dot))));
+    }
+    q_ss = warp_sum(q_ss), k_ss = warp_sum(k_ss);
+    const float q_factor = (1.f / sqrtf(q_ss + 1e-6f)) * (1.f / sqrtf(static_cast<float>(dk))), k_factor = 1.f / sqrtf(k_ss + 1e-6f);
+    for (int i = lane * 4; i < dk; i += 128) {
+      *reinterpret_cast<float4*>(q_out + t * qk + head * dk + i) = scale_each(*reinterpret_cast<const float4*>(q + i), q_factor);
+      *reinterpret_cast<float4*>(k_out + t * qk + head * dk + i) = scale_each(*reinterpret_cast<const float4*>(k + i), k_factor);
+    }
+    if (per_head) {
+      dot = warp_sum(dot);
+      if (lane == 0) kq_out[t * kv_heads + head] = dot * k_factor * q_factor;
+    }
+  }
+}
+
 // After a step the slot holds the last taps - 1 inputs of [old slot | the step's inputs].
 template <typename T>
 __global__ void conv_state_update_kernel(const T* proj, int ld, int channels, int taps, const int* seq_q_start,
@@ -99,7 +203,7 @@ __global__ void conv_state_update_kernel(const T* proj, int ld, int channels, in
   const int start = seq_q_start[seq], len = seq_q_len[seq];
   const int keep = taps - 1;
   T* state = conv_state + static_cast<int64_t>(seq_slot[seq]) * keep * channels;
-  for (int c = threadIdx.x; c < channels; c += blockDim.x) {
+  for (int c = blockIdx.y * blockDim.x + threadIdx.x; c < channels; c += gridDim.y * blockDim.x) {
     for (int r = 0; r < keep; ++r) {
       const int at = len + r;  // index into [old slot (keep) | inputs (len)]
       state[static_cast<int64_t>(r) * channels + c] =
@@ -262,6 +366,27 @@ __global__ void delta_output_kernel(const float* o, const float* __restrict__ we
   }
 }
 
+// The same with four numbers a thread: 2^n lanes hold one (token, head), dv = 4 x 2^n up to 128.
+template <typename T, bool SILU>
+__global__ void __launch_bounds__(256)
+delta_output_wide_kernel(const float* o, const float* __restrict__ weight, const T* gate, int gate_ld, int rows, int heads, int dv, float eps, T* out) {
+  wait_for_predecessor();
+  let_successor_start();
+  const int lanes = dv / 4;
+  const int64_t quad = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
+  const bool live = quad < static_cast<int64_t>(rows) * heads * lanes;
+  const int64_t item = live ? quad / lanes : 0;
+  const int i = static_cast<int>(quad % lanes) * 4, h = static_cast<int>(item % heads);
+  const float4 x = *reinterpret_cast<const float4*>(o + item * dv + i);
+  const float4 g = load4<T>(gate + item / heads * gate_ld + h * dv + i), w = *reinterpret_cast<const float4*>(weight + i);
+  float ss = square_sum(x, 0.f);
+  for (int step = lanes >> 1; step > 0; step >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, step);
+  const float inv = 1.f / sqrtf(ss / static_cast<float>(dv) + eps);
+  const auto gated = [](float z) { return SILU ? z * sigmoid_f(z) : sigmoid_f(z); };
+  if (live)
+    store4<T>(out + item * dv + i, make_float4(x.x * inv * w.x * gated(g.x), x.y * inv * w.y * gated(g.y), x.z * inv * w.z * gated(g.z), x.w * inv * w.w * gated(g.w)));
+}
+
 }  // namespace
 
 B200_API int b200_delta_prepare(const void* proj, int ld, const void* decay_in, int decay_ld, const float* taps_w, int taps,
@@ -276,6 +401,33 @@ B200_API int b200_delta_prepare(const void* proj, int ld, const void* decay_in, 
   const size_t smem = sizeof(float) * channels;
   B200_REQUIRE(smem <= 200 * 1024, "delta_prepare: %d convolved channels do not fit shared memory", channels);
   const int threads = 256;
+  const int update_blocks = (channels + threads - 1) / threads;  // a thread per channel: the slots' update is a tail of its own
+  // The wide form from a block an SM on, with rows, taps and results on 16-byte (bfloat16 rows: 8-byte) boundaries.
+  const size_t wide_smem = sizeof(float) * kWideTokens * 2 * kv_heads * dk;
+  const auto on = [](const void* p, int bytes) { return reinterpret_cast<uintptr_t>(p) % bytes == 0; };
+  const int in_bytes = dtype == DTYPE_F32 ? 16 : 8;
+  const bool wide = taps == kWideTaps && tokens >= kWideTokens * b200_sm_count_host() / 2 && ld % 4 == 0 && dk % 4 == 0 && dv % 4 == 0 && wide_smem <= 200 * 1024 &&
+                    on(proj, in_bytes) && on(conv_state, in_bytes) && on(taps_w, 16) && on(q_out, 16) && on(k_out, 16) && on(v_out, 16) &&
+                    (kq_out != nullptr || (decay_ld % 4 == 0 && on(decay_in, in_bytes) && on(dt_bias, 16) && on(decay_out, 16)));
+  auto launch_wide = [&](auto kernel, auto* typed) {
+    using T = typename std::remove_pointer<decltype(typed)>::type;
+    if (wide_smem > 40 * 1024) cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(wide_smem));
+    launch_kernel(kernel, dim3((tokens + kWideTokens - 1) / kWideTokens), dim3(threads), wide_smem, stream, typed, ld, static_cast<const T*>(decay_in), decay_ld,
+                  taps_w, static_cast<const T*>(conv_state), a_log, dt_bias, token_seq, seq_q_start, seq_slot, tokens, heads, kv_heads, dk, dv, q_out, k_out, v_out,
+                  beta_out, decay_out, kq_out);
+  };
+  if (wide && (dtype == DTYPE_F32 || dtype == DTYPE_BF16)) {
+    if (dtype == DTYPE_F32) launch_wide(delta_prepare_wide_kernel<float>, static_cast<const float*>(proj));
+    else launch_wide(delta_prepare_wide_kernel<__nv_bfloat16>, static_cast<const __nv_bfloat16*>(proj));
+    if (int status = b200_check_launch("delta_prepare")) return status;
+    if (dtype == DTYPE_F32)
+      launch_kernel(conv_state_update_kernel<float>, dim3(seqs, update_blocks), dim3(threads), 0, stream, static_cast<const float*>(proj), ld, channels, taps,
+                    seq_q_start, seq_q_len, seq_slot, static_cast<float*>(conv_state));
+    else
+      launch_kernel(conv_state_update_kernel<__nv_bfloat16>, dim3(seqs, update_blocks), dim3(threads), 0, stream, static_cast<const __nv_bfloat16*>(proj), ld,
+                    channels, taps, seq_q_start, seq_q_len, seq_slot, static_cast<__nv_bfloat16*>(conv_state));
+    return b200_check_launch("conv_state_update");
+  }
   if (dtype == DTYPE_F32) {
     if (smem > 48 * 1024)
       cudaFuncSetAttribute(delta_prepare_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
@@ -283,7 +435,7 @@ B200_API int b200_delta_prepare(const void* proj, int ld, const void* decay_in, 
                   static_cast<const float*>(decay_in), decay_ld, taps_w, taps, static_cast<const float*>(conv_state), a_log,
                   dt_bias, token_seq, seq_q_start, seq_slot, heads, kv_heads, dk, dv, q_out, k_out, v_out, beta_out, decay_out, kq_out);
     if (int status = b200_check_launch("delta_prepare")) return status;
-    launch_kernel(conv_state_update_kernel<float>, dim3(seqs), dim3(threads), 0, stream, static_cast<const float*>(proj), ld,
+    launch_kernel(conv_state_update_kernel<float>, dim3(seqs, update_blocks), dim3(threads), 0, stream, static_cast<const float*>(proj), ld,
                   channels, taps, seq_q_start, seq_q_len, seq_slot, static_cast<float*>(conv_state));
   } else if (dtype == DTYPE_BF16) {
     if (smem > 48 * 1024)
@@ -294,7 +446,7 @@ B200_API int b200_delta_prepare(const void* proj, int ld, const void* decay_in, 
                   taps, static_cast<const __nv_bfloat16*>(conv_state), a_log, dt_bias, token_seq, seq_q_start, seq_slot, heads,
                   kv_heads, dk, dv, q_out, k_out, v_out, beta_out, decay_out, kq_out);
     if (int status = b200_check_launch("delta_prepare")) return status;
-    launch_kernel(conv_state_update_kernel<__nv_bfloat16>, dim3(seqs), dim3(threads), 0, stream,
+    launch_kernel(conv_state_update_kernel<__nv_bfloat16>, dim3(seqs, update_blocks), dim3(threads), 0, stream,
                   static_cast<const __nv_bfloat16*>(proj), ld, channels, taps, seq_q_start, seq_q_len, seq_slot,
                   static_cast<__nv_bfloat16*>(conv_state));
   } else {
@@ -348,6 +500,19 @@ B200_API int b200_delta_output(const float* o, const float* weight, const void* 
   const int threads = 128;
   const int64_t items = static_cast<int64_t>(rows) * heads;
   const unsigned blocks = static_cast<unsigned>((items + 3) / 4);
+  const int lanes = dv / 4, in_bytes = dtype == DTYPE_F32 ? 16 : 8;
+  const auto on = [](const void* p, int bytes) { return reinterpret_cast<uintptr_t>(p) % bytes == 0; };
+  if (dv % 4 == 0 && lanes <= 32 && (lanes & (lanes - 1)) == 0 && gate_ld % 4 == 0 && on(o, 16) && on(weight, 16) && on(gate, in_bytes) && on(out, in_bytes) &&
+      (dtype == DTYPE_F32 || dtype == DTYPE_BF16)) {
+    const dim3 grid(static_cast<unsigned>((items * lanes + 255) / 256));
+    if (dtype == DTYPE_F32)
+      launch_kernel(silu ? delta_output_wide_kernel<float, true> : delta_output_wide_kernel<float, false>, grid, dim3(256), 0, stream, o, weight,
+                    static_cast<const float*>(gate), gate_ld, rows, heads, dv, eps, static_cast<float*>(out));
+    else
+      launch_kernel(silu ? delta_output_wide_kernel<__nv_bfloat16, true> : delta_output_wide_kernel<__nv_bfloat16, false>, grid, dim3(256), 0, stream, o, weight,
+                    static_cast<const __nv_bfloat16*>(gate), gate_ld, rows, heads, dv, eps, static_cast<__nv_bfloat16*>(out));
+    return b200_check_launch("delta_output");
+  }
   if (dtype == DTYPE_F32) {
     launch_kernel(silu ? delta_output_kernel<float, true> : delta_output_kernel<float, false>, dim3(blocks), dim3(threads), 0, stream, o, weight,
                   static_cast<const float*>(gate), gate_ld, rows, heads, dv, eps, static_cast<float*>(out));
