@@ -19,6 +19,14 @@
 // a weight by a sigmoid: no maximum, no sum, nothing the two softmax groups have to agree on. A
 // sink (the softmax forms) is one more term of a row's sum, added when the row is finished.
 //
+// LATENT: attention whose keys and values are expanded from one cached latent per token. For a prompt portion the expansion is one
+// library product over the request's latents in front of this kernel (rows of [keys 128 | values 128] per head, requests padded to
+// whole tiles of zeros), so a head's key is 128 numbers of that product and the 64 rotated numbers that all heads share (192 in all,
+// or 128 without a rotated part), against 576 and 512 in the latent space: 640 instead of 2,176 flops per query, key and head. Its key
+// tiles come as three boxes (two without the rotated part) from plain matrices; queries from the projections and the rotated rows.
+// Measured on a B200, 2,048 tokens of 12 heads, latent 512 + 64: 352 us in the latent space (mma.sync) and 18 in the two per-head
+// products around it -> 4 us gather, 9 expansion, 46 this kernel (350 TFLOP/s of the expanded flops).
+//
 // Every wait (mbarriers, and the shared-memory word the two softmax threads of a row pass the
 // turn with) is bounded; on a timeout the block records ERRBIT_TIMEOUT, skips its further waits,
 // runs out and frees its TMEM. Shapes the kernel does not take (other head sizes, pages under 16 rows,
@@ -69,6 +77,12 @@ struct PrefillParams {
   const float* bias;       // [q_heads][bias_reach + 1] by distance min(pos - key, bias_reach), added after the cap; null: none
   const float* bias_peak;  // [q_heads]: the largest entry of the head's row
   int bias_reach;
+  // The LATENT forms only (one key/value head per query head).
+  const __nv_bfloat16* q_rot;  // [rows][q_heads * 64]
+  const __nv_bfloat16* gate;   // logits [rows][q_heads], rows gate_ld apart, or null
+  int64_t q_ld, gate_ld;       // numbers from row to row of q and of gate
+  int q_head_ld;               // numbers from head to head of q
+  int latent_rank;             // column of the rotated numbers in a latent row
 };
 
 __device__ __forceinline__ uint32_t saddr(const void* p) { return static_cast<uint32_t>(__cvta_generic_to_shared(p)); }
@@ -218,15 +232,19 @@ __device__ __forceinline__ float capped_exponent(float raw, const PrefillParams&
 // in the second pass only, and only in tiles within reach.
 // KEPT and SIGMOID: see the top. Five instantiations: plain, CAPPED (cap and chunks), CAPPED with BIASED, KEPT, SIGMOID (which
 // is KEPT too).
-template <bool CAPPED, bool BIASED, bool KEPT = false, bool SIGMOID = false>
+// LATENT: 0, or the length of a key, 128 or 192 (see the top): two more. Then k_map covers the expanded rows and v_map the latent ones.
+template <bool CAPPED, bool BIASED, bool KEPT = false, bool SIGMOID = false, int LATENT = 0>
 __global__ void __launch_bounds__(kThreadsA, 1)
 flash_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap k_map, const __grid_constant__ CUtensorMap v_map,
                              const PrefillParams p) {
+  constexpr int kKeyDim = LATENT ? LATENT : kDim;             // numbers of a key
+  constexpr int kKeyTile = kKeyDim / 64 * kHalfBytes;         // bytes of a tile of queries or keys
+  constexpr int kSlotsK = kKeyDim > kDim ? 2 : kStagesK;      // longer keys: two tiles in flight are what fits
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   unsigned char* base = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   unsigned char* q_tile = base;                                   // 32 KB: two halves of [128 rows][64 dims]
-  unsigned char* k_ring = q_tile + kTileBytesA;                   // kStagesK x 32 KB
-  unsigned char* v_ring = k_ring + kStagesK * kTileBytesA;        // kStagesV x 32 KB
+  unsigned char* k_ring = q_tile + kKeyTile;                      // kStagesK x 32 KB (LATENT with rotated parts: 2 x 48 KB)
+  unsigned char* v_ring = k_ring + kSlotsK * kKeyTile;            // kStagesV x 32 KB
   int* pages = reinterpret_cast<int*>(v_ring + kStagesV * kTileBytesA);  // [kMaxChunks]
   __shared__ __align__(8) uint64_t k_full[kStagesK], k_empty[kStagesK], v_full[kStagesV], v_empty[kStagesV];
   // o_done[t & 3] completes when PV[t] has retired (and with it every earlier product). A ring of
@@ -272,7 +290,7 @@ flash_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap k_map, const __
   const int num_tiles = kept_tiles + tile_end - window_tile;
   auto start_of = [&](int it) { return (KEPT && it < kept_tiles ? it : window_tile + it - kept_tiles) * kKeys; };
   const int pieces_per_tile = kKeys / p.piece_rows;
-  if (num_tiles * pieces_per_tile > kMaxChunks) {
+  if (!LATENT && num_tiles * pieces_per_tile > kMaxChunks) {
     // The launcher sized the walk from the host's lengths; lengths on the device that exceed
     // them are an error of the caller, reported rather than walked.
     wait_for_predecessor();
@@ -306,7 +324,7 @@ flash_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap k_map, const __
   // part of the step's metadata, on the device before any kernel of the step ran, so all of
   // this may precede the wait for the kernel in front (which wrote the queries and the newest
   // keys).
-  for (int i = threadIdx.x; i < num_tiles * pieces_per_tile; i += kThreadsA) {
+  for (int i = threadIdx.x; !LATENT && i < num_tiles * pieces_per_tile; i += kThreadsA) {
     const int key = start_of(i / pieces_per_tile) + i % pieces_per_tile * p.piece_rows;
     // Pieces past the request's last key are read too (the table pads them with a page that
     // exists): their scores are masked, and their values only ever meet a probability of zero.
@@ -318,7 +336,7 @@ flash_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap k_map, const __
   }
   wait_for_predecessor();
   let_successor_start();
-  if (p.window > 0 || tile_end * kKeys > p.max_pages * p.page_size) {
+  if (!LATENT && (p.window > 0 || tile_end * kKeys > p.max_pages * p.page_size)) {
     // Pieces whose page the request no longer holds, or that lie past the block table, are
     // skipped by the loader; their rows must still hold finite numbers, since a masked
     // probability of zero times garbage may be NaN.
@@ -334,14 +352,19 @@ flash_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap k_map, const __
   // warp at a barrier of their own.
   constexpr int kFillThreads = 9 * 32;
   if (warp >= 1 && warp <= 9) {
-    for (int i = threadIdx.x - 32; i < kRows * 16; i += kFillThreads) {
-      const int r = i >> 4, c = i & 15;
+    constexpr int kChunks = kKeyDim / 8;  // 16-byte chunks of a row
+    for (int i = threadIdx.x - 32; i < kRows * kChunks; i += kFillThreads) {
+      const int r = i / kChunks, c = i % kChunks;
       const int row = row_base + r;
       uint4 value = make_uint4(0u, 0u, 0u, 0u);
       if (row < rows_total) {
         const int tok = row / p.group;
         const int head = kv_head * p.group + (row - tok * p.group);
-        value = *reinterpret_cast<const uint4*>(p.q + (static_cast<int64_t>(q_start + tok) * p.q_heads + head) * kDim + c * 8);
+        const int64_t at = q_start + tok;
+        if constexpr (LATENT != 0)
+          value = *reinterpret_cast<const uint4*>(c < 16 ? p.q + at * p.q_ld + head * p.q_head_ld + c * 8 : p.q_rot + (at * p.q_heads + head) * 64 + (c - 16) * 8);
+        else
+          value = *reinterpret_cast<const uint4*>(p.q + (at * p.q_heads + head) * kDim + c * 8);
       }
       *reinterpret_cast<uint4*>(q_tile + (c >> 3) * kHalfBytes + r * 128 + (((c & 7) ^ (r & 7)) << 4)) = value;
     }
@@ -361,17 +384,32 @@ flash_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap k_map, const __
     // (a converged warp with one elected lane issuing, as for the products below)
     const bool leader = elect_one();
     const bool keys = warp == 0;
-    const int stages = keys ? kStagesK : kStagesV;
+    const int stages = keys ? kSlotsK : kStagesV;
     uint64_t* full = keys ? k_full : v_full;
     uint64_t* empty = keys ? k_empty : v_empty;
     unsigned char* ring = keys ? k_ring : v_ring;
     const CUtensorMap* map = keys ? &k_map : &v_map;
     const int row_head = (keys || p.value_head < 0) ? kv_head : p.value_head;
+    int first_row = 0;  // LATENT: requests in front of this one, each padded to whole tiles
+    if constexpr (LATENT != 0)
+      for (int other = p.first_seq; other < seq; ++other) first_row += (p.seq_kv_len[other] + kKeys - 1) / kKeys * kKeys;
     for (int it = 0; it < num_tiles; ++it) {
       const int s = it % stages;
       if (it >= stages && !bar_wait(&empty[s], ((it / stages) - 1) & 1)) {
         if (leader) atomicOr(p.err, ERRBIT_TIMEOUT_A);
         break;
+      }
+      if constexpr (LATENT != 0) {
+        const int row = first_row + it * kKeys, column = kv_head * 2 * kDim + (keys ? 0 : kDim);
+        unsigned char* to = ring + s * (keys ? kKeyTile : kTileBytesA);
+        if (leader) {
+          bar_expect_tx(&full[s], keys ? kKeyTile : kTileBytesA);
+          tma_tile(to, &k_map, &full[s], column, row);
+          tma_tile(to + kHalfBytes, &k_map, &full[s], column + 64, row);
+          if (keys && kKeyDim > kDim) tma_tile(to + 2 * kHalfBytes, &v_map, &full[s], p.latent_rank, row);
+        }
+        __syncwarp();
+        continue;
       }
       uint32_t bytes = 0;
       for (int piece = 0; piece < pieces_per_tile; ++piece) {
@@ -413,15 +451,15 @@ flash_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap k_map, const __
     const uint64_t k_desc = desc_k_major(saddr(k_ring));
     const uint64_t v_desc = desc_mn_major(saddr(v_ring));
     auto scores = [&](int it) -> bool {  // S[it % 3] = Q K^T for tile `it`
-      const int s = it % kStagesK;
-      if (!bar_wait(&k_full[s], (it / kStagesK) & 1)) {
+      const int s = it % kSlotsK;
+      if (!bar_wait(&k_full[s], (it / kSlotsK) & 1)) {
         return false;
       }
       fence_after();
-      const uint64_t k_here = k_desc + static_cast<uint64_t>(s * (kTileBytesA >> 4));
+      const uint64_t k_here = k_desc + static_cast<uint64_t>(s * (kKeyTile >> 4));
       const uint32_t d = (tmem + (it % kScoreBuffers) * 128);
 #pragma unroll
-      for (int ks = 0; ks < kDim / 16; ++ks) {
+      for (int ks = 0; ks < kKeyDim / 16; ++ks) {
         constexpr int kHalf16 = kHalfBytes >> 4;
         const uint64_t off = static_cast<uint64_t>((ks >> 2) * kHalf16 + (ks & 3) * 2);  // 32 bytes per 16 dims
         if (leader) mma_ss(d, q_desc + off, k_here + off, id_s, ks > 0);
@@ -705,7 +743,10 @@ flash_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap k_map, const __
       const int token = min(row / p.group, q_len - 1);
       const int head = kv_head * p.group + (row - (row / p.group) * p.group);
       __nv_bfloat16* dst = p.out + (static_cast<int64_t>(q_start + token) * p.q_heads + head) * kDim;
-      const float inv = l > 0.f ? 1.f / l : 0.f;
+      float inv = l > 0.f ? 1.f / l : 0.f;
+      if constexpr (LATENT != 0) {
+        if (p.gate != nullptr) inv *= 1.f / (1.f + expf(-__bfloat162float(p.gate[(q_start + token) * p.gate_ld + head])));
+      }
 #pragma unroll 1
       for (int c0 = group * (kDim / 2); c0 < (group + 1) * (kDim / 2); c0 += 32) {
         uint32_t raw[32];
@@ -761,6 +802,52 @@ int arena_map(CUtensorMap* map, const void* arena, int64_t rows, int piece_rows)
              CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (status != CUDA_SUCCESS) return b200_fail("flash_prefill_tcgen05: cuTensorMapEncodeTiled failed (%d)", static_cast<int>(status));
   return 0;
+}
+
+// The latents of the requests from first_seq on, out of the cache's pages into rows of one matrix, each request padded to whole tiles
+// with zeros. One block per 16 rows of a request, 16 bytes a thread.
+constexpr int kGatherRows = 16;
+
+__global__ void __launch_bounds__(256)
+latent_gather_kernel(const __nv_bfloat16* rows, const int* __restrict__ block_table, const int* __restrict__ seq_kv_len, int first_seq, int max_pages, int num_pages,
+                     int page_size, int row_dim, __nv_bfloat16* out, int* err) {
+  wait_for_predecessor();
+  let_successor_start();
+  const int seq = first_seq + blockIdx.y, len = seq_kv_len[seq], padded = (len + kKeys - 1) / kKeys * kKeys, row0 = blockIdx.x * kGatherRows;
+  if (row0 >= padded) return;
+  int64_t first = row0;
+  for (int other = first_seq; other < seq; ++other) first += (seq_kv_len[other] + kKeys - 1) / kKeys * kKeys;
+  const int chunks = row_dim / 8;
+  for (int i = threadIdx.x; i < kGatherRows * chunks; i += blockDim.x) {
+    const int r = i / chunks, c = i % chunks * 8, key = row0 + r;
+    uint4 value = make_uint4(0u, 0u, 0u, 0u);
+    if (key < len) {
+      const int logical = key / page_size;
+      const int page = logical < max_pages ? block_table[static_cast<int64_t>(seq) * max_pages + logical] : -1;
+      if (page < 0 || page >= num_pages) atomicOr(err, ERRBIT_BAD_PAGE);
+      else value = *reinterpret_cast<const uint4*>(rows + (static_cast<int64_t>(page) * page_size + key % page_size) * row_dim + c);
+    }
+    *reinterpret_cast<uint4*>(out + (first + r) * row_dim + c) = value;
+  }
+}
+
+// A [rows][columns] bfloat16 matrix; boxes of 64 columns x 128 rows.
+int matrix_map(CUtensorMap* map, const void* matrix, int64_t rows, int64_t columns) {
+  EncodeTiledA encode = encode_tiled_a();
+  if (encode == nullptr) return b200_fail("latent_prefill_tcgen05: the driver does not provide cuTensorMapEncodeTiled");
+  const cuuint64_t dims[2] = {static_cast<cuuint64_t>(columns), static_cast<cuuint64_t>(rows)};
+  const cuuint64_t strides[1] = {static_cast<cuuint64_t>(columns) * 2};
+  const cuuint32_t box[2] = {64, kKeys};
+  const cuuint32_t elem[2] = {1, 1};
+  const CUresult status = encode(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(matrix), dims, strides, box, elem, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                                 CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  if (status != CUDA_SUCCESS) return b200_fail("latent_prefill_tcgen05: cuTensorMapEncodeTiled failed (%d)", static_cast<int>(status));
+  return 0;
+}
+
+template <int KEY_DIM>
+constexpr size_t latent_smem() {
+  return KEY_DIM / 64 * kHalfBytes * (1 + (KEY_DIM > kDim ? 2 : kStagesK)) + kStagesV * static_cast<size_t>(kTileBytesA) + kMaxChunks * sizeof(int) + 1024;
 }
 
 }  // namespace
@@ -858,5 +945,70 @@ B200_API int b200_flash_prefill_tcgen05(const void* q, const void* k_arena, cons
       : kept          ? launch_kernel(flash_prefill_tcgen05_kernel<false, false, true>, grid, dim3(kThreadsA), smem, stream, k_map, v_map, p)
                       : launch_kernel(flash_prefill_tcgen05_kernel<false, false>, grid, dim3(kThreadsA), smem, stream, k_map, v_map, p);
   if (status != cudaSuccess) return b200_fail("flash_prefill_tcgen05: %s", cudaGetErrorString(status));
+  return 0;
+}
+
+// Attention over latents of prompt portions with expanded keys and values: sizes the forms take.
+B200_API int b200_latent_prefill_supported(int heads, int dim, int rot_dim, int vdim, int rank, int page_size) {
+  return heads > 0 && heads <= 65535 && dim == kDim && vdim == kDim && (rot_dim == 0 || rot_dim == 64) && rank > 0 && rank % 8 == 0 && page_size > 0;
+}
+
+// Rows [requests' keys, each request padded to a multiple of 128][row_dim] out of the cache's pages [pages][page_size][row_dim].
+B200_API int b200_latent_gather(const void* rows, const int* block_table, const int* seq_kv_len, int first_seq, int num_seqs, int max_kv_len, int max_pages,
+                                int num_pages, int page_size, int row_dim, void* out, int* err, cudaStream_t stream) {
+  if (num_seqs <= 0) return 0;
+  B200_REQUIRE(num_seqs <= 65535 && max_kv_len > 0 && page_size > 0 && max_pages > 0 && row_dim > 0 && row_dim % 8 == 0, "latent_gather: bad sizes");
+  B200_REQUIRE(reinterpret_cast<uintptr_t>(rows) % 16 == 0 && reinterpret_cast<uintptr_t>(out) % 16 == 0, "latent_gather: operands must be aligned to 16 bytes");
+  const int padded = (max_kv_len + kKeys - 1) / kKeys * kKeys;
+  launch_kernel(latent_gather_kernel, dim3(padded / kGatherRows, num_seqs), dim3(256), 0, stream, static_cast<const __nv_bfloat16*>(rows), block_table, seq_kv_len,
+                first_seq, max_pages, num_pages, page_size, row_dim, static_cast<__nv_bfloat16*>(out), err);
+  return b200_check_launch("latent_gather");
+}
+
+// The portions' attention itself. `q`: plain query parts (128 numbers a head, heads q_head_ld and rows q_ld numbers apart), `q_rot` [rows][heads * 64] or
+// null; `expanded` [key_rows][heads * 256] and `latents` [key_rows][rank + rot_dim] as `b200_latent_gather` lays rows out; `out` [rows][heads * 128].
+B200_API int b200_latent_prefill_tcgen05(const void* q, int64_t q_ld, int q_head_ld, const void* q_rot, const void* expanded, const void* latents, int64_t key_rows,
+                                         int rank, int rot_dim, const int* seq_q_start, const int* seq_q_len, const int* seq_kv_len, int first_seq, int num_seqs,
+                                         int max_q_len, int heads, float scale, const float* sink, const void* gate, int64_t gate_ld, void* out, int* err,
+                                         cudaStream_t stream) {
+  if (num_seqs <= 0) return 0;
+  B200_REQUIRE(b200_latent_prefill_supported(heads, kDim, rot_dim, kDim, rank, 1) && (rot_dim == 0) == (q_rot == nullptr), "latent_prefill_tcgen05: shape not taken");
+  B200_REQUIRE(num_seqs <= 65535 && max_q_len > 0 && key_rows > 0 && key_rows % kKeys == 0 && q_ld % 8 == 0 && q_head_ld % 8 == 0, "latent_prefill_tcgen05: bad sizes");
+  const auto aligned = [](const void* a) { return reinterpret_cast<uintptr_t>(a) % 16 == 0; };
+  B200_REQUIRE(aligned(q) && aligned(q_rot) && aligned(expanded) && aligned(latents) && aligned(out), "latent_prefill_tcgen05: operands must be aligned to 16 bytes");
+  PrefillParams p = {};
+  p.q = static_cast<const __nv_bfloat16*>(q);
+  p.out = static_cast<__nv_bfloat16*>(out);
+  p.seq_q_start = seq_q_start;
+  p.seq_q_len = seq_q_len;
+  p.seq_kv_len = seq_kv_len;
+  p.err = err;
+  p.first_seq = first_seq;
+  p.q_heads = p.kv_heads = heads;
+  p.group = 1;
+  p.piece_rows = kKeys;
+  p.sink = sink;
+  p.value_head = -1;
+  p.scale = scale;
+  p.scale_log2 = scale * kLog2eA;
+  p.q_rot = static_cast<const __nv_bfloat16*>(q_rot);
+  p.gate = static_cast<const __nv_bfloat16*>(gate);
+  p.q_ld = q_ld;
+  p.gate_ld = gate_ld;
+  p.q_head_ld = q_head_ld;
+  p.latent_rank = rank;
+  CUtensorMap expanded_map, latent_map;
+  if (matrix_map(&expanded_map, expanded, key_rows, static_cast<int64_t>(heads) * 2 * kDim) != 0) return -1;
+  if (matrix_map(&latent_map, latents, key_rows, rank + rot_dim) != 0) return -1;
+  auto with_rot = flash_prefill_tcgen05_kernel<false, false, false, false, kDim + 64>;
+  auto plain = flash_prefill_tcgen05_kernel<false, false, false, false, kDim>;
+  static const bool raised =
+      cudaFuncSetAttribute(with_rot, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(latent_smem<kDim + 64>())) == cudaSuccess &&
+      cudaFuncSetAttribute(plain, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(latent_smem<kDim>())) == cudaSuccess;
+  B200_REQUIRE(raised, "latent_prefill_tcgen05: cannot size shared memory");
+  const dim3 grid((max_q_len + kRows - 1) / kRows, heads, num_seqs);
+  const cudaError_t status = rot_dim ? launch_kernel(with_rot, grid, dim3(kThreadsA), latent_smem<kDim + 64>(), stream, expanded_map, latent_map, p)
+                                     : launch_kernel(plain, grid, dim3(kThreadsA), latent_smem<kDim>(), stream, expanded_map, latent_map, p);
+  if (status != cudaSuccess) return b200_fail("latent_prefill_tcgen05: %s", cudaGetErrorString(status));
   return 0;
 }

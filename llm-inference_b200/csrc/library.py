@@ -64,6 +64,9 @@ _SIGNATURES: dict[str, list] = {
     "b200_paged_decode_attention_tma": [c_void_p] * 8 + [c_int] * 9 + [c_float, c_int, c_int] + [c_void_p] * 5,
     "b200_flash_prefill_tcgen05": [c_void_p] * 8 + [c_int] * 12 + [c_float, c_int, c_float, c_void_p, c_void_p, c_int, c_int, c_void_p, c_void_p,
                                    c_void_p, c_void_p],
+    "b200_latent_gather": [c_void_p] * 3 + [c_int] * 7 + [c_void_p] * 3,
+    "b200_latent_prefill_tcgen05": [c_void_p, c_int64, c_int] + [c_void_p] * 3 + [c_int64, c_int, c_int] + [c_void_p] * 3 + [c_int] * 4
+                                   + [c_float, c_void_p, c_void_p, c_int64] + [c_void_p] * 3,
     "b200_skinny_gemm": [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_void_p, c_int64, c_void_p, c_int, c_void_p],
     "b200_stream_gemm": [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_void_p, c_void_p],
     "b200_skinny_gemm_fold": [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_void_p, c_int64, c_void_p, c_int,
@@ -170,6 +173,8 @@ class KernelLibrary:
         self.lib.b200_latent_attention_mma_scratch.restype = c_int64
         self.lib.b200_portion_attention_f32_supported.argtypes = [c_int] * 3
         self.lib.b200_portion_attention_f32_supported.restype = c_int
+        self.lib.b200_latent_prefill_supported.argtypes = [c_int] * 6
+        self.lib.b200_latent_prefill_supported.restype = c_int
         self.lib.b200_state_chunks_supported.argtypes = [c_int] * 5
         self.lib.b200_state_chunks_supported.restype = c_int
         self.lib.b200_state_chunks_scratch.argtypes = [c_int] * 6

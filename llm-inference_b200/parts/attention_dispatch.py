@@ -158,6 +158,6 @@ def attend_latent(
         pieces = int(ctx.options.get("latent_pieces", 0)) or ops.latent_attention_pieces(decode_seqs, heads, ctx.max_kv_len, ops.sm_count(ctx))
         ops.latent_attention_mma(ctx, cache, q_lat, q_rot, sink, gate, out, heads, rank, rot_dim, scale,
                                  first_seq=0, num_seqs=decode_seqs, max_q_len=1, pieces=pieces)
-    if ctx.num_seqs > decode_seqs:
+    if ctx.num_seqs > decode_seqs and q_lat.shape[1] > decode_seqs:  # rows of the single tokens alone: the portions were expanded
         ops.latent_attention_mma(ctx, cache, q_lat, q_rot, sink, gate, out, heads, rank, rot_dim, scale,
                                  first_seq=decode_seqs, num_seqs=ctx.num_seqs - decode_seqs, max_q_len=ctx.max_q_len)

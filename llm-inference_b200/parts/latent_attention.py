@@ -31,6 +31,9 @@ class LatentAttention(Part):
     ``position`` None) positions do not enter at all: the cached row is the latent alone, and both latents' norms and the
     cache write are one kernel.
 
+    Prompt portions long enough (``ops.latent_expansion_rows``) take the other reading of the same formula: their keys and values are
+    expanded from the latents by one product, and attention runs head by head on those.
+
     The query (or its latent), latent and gate projections are one matrix product. Tensor names are
     ``prefix + q | dq | dq.norm | uq | dkv | dkv.norm | uk | uv | sink | g | o``."""
 
@@ -50,7 +53,7 @@ class LatentAttention(Part):
         self.has_sink, self.has_gate = bool(sink), bool(gate)
         self.position = build_part("position", position) if position is not None else None
         self.graph_safe = self.position.graph_safe if self.position is not None else True
-        self.w_in = self.w_uk_t = self.w_uv = self.w_o = self.sink = self.norm_weight = None
+        self.w_in = self.w_uk_t = self.w_uv = self.w_expand = self.w_o = self.sink = self.norm_weight = None
 
     def cache_spec(self) -> KVCacheSpec:
         return KVCacheSpec(1, self.rank + self.rot_dim, self.window, planes=1)
@@ -86,6 +89,9 @@ class LatentAttention(Part):
         # [heads, rank, dim]: the product that carries a query into the latent space reads W_uk[n]^T.
         self.w_uk_t = tensors[p + "uk"].to(device=device, dtype=dtype).view(self.heads, self.dim, self.rank).transpose(1, 2).contiguous()
         self.w_uv = tensors[p + "uv"].to(device=device, dtype=dtype).view(self.heads, self.vdim, self.rank).contiguous()
+        # [heads * (dim + vdim), rank]: a head's keys and values out of a latent, for prompt portions long enough to expand them.
+        uk = tensors[p + "uk"].to(device=device, dtype=dtype).view(self.heads, self.dim, self.rank)
+        self.w_expand = torch.cat([uk, self.w_uv], dim=1).reshape(-1, self.rank).contiguous()
         self.w_o = tensors[p + "o"].to(device=device, dtype=dtype).contiguous()
         self.norm_weight = tensors[p + "dkv.norm"].to(device=device, dtype=torch.float32).contiguous()
         self.sink = tensors[p + "sink"].to(device=device, dtype=torch.float32).contiguous() if self.has_sink else None
@@ -116,14 +122,20 @@ class LatentAttention(Part):
         else:
             queries, kv_offset = proj[:, :q_width], q_width
             self.position.apply_latent(ctx, cache, proj, 0, kv_offset, heads, self.dim, rank, self.norm_weight, self.eps, q_rot)
-        q_plain = queries.view(t, heads, self.dim + rot)[:, :, : self.dim].transpose(0, 1)
-        q_lat = ops.linear_per_head(ctx, q_plain, self.w_uk_t, ctx.buffer("latent_q", (heads, t, rank)))
         gate_at, gates = kv_offset + rank + rot, heads * (self.vdim if self.gate_per_element else 1)
         gate = proj[:, gate_at : gate_at + gates] if self.has_gate else None
-        mixed = ctx.buffer("latent_out", (heads, t, rank))
-        self.attend(ctx, cache, q_lat, q_rot, None if self.gate_per_element else gate, mixed)
+        head_gate = None if self.gate_per_element else gate
         attn = ctx.buffer("attn", (t, heads * self.vdim))
-        ops.linear_per_head(ctx, mixed, self.w_uv, attn.view(t, heads, self.vdim).transpose(0, 1))
+        key_rows = ops.latent_expansion_rows(ctx, cache, h.dtype, heads, self.dim, rot, self.vdim, rank)
+        if key_rows:
+            ops.latent_portions(ctx, cache, key_rows, queries, q_rot, self.w_expand, self.sink, head_gate, attn, heads, self.dim, rank, rot, self.scale)
+        absorbed = ctx.num_decode_seqs if key_rows else t  # rows that attend in the latent space (single tokens lead the batch)
+        if absorbed:
+            q_plain = queries[:absorbed].view(absorbed, heads, self.dim + rot)[:, :, : self.dim].transpose(0, 1)
+            q_lat = ops.linear_per_head(ctx, q_plain, self.w_uk_t, ctx.buffer("latent_q", (heads, absorbed, rank)))
+            mixed = ctx.buffer("latent_out", (heads, absorbed, rank))
+            self.attend(ctx, cache, q_lat, q_rot[:absorbed], None if head_gate is None else head_gate[:absorbed], mixed)
+            ops.linear_per_head(ctx, mixed, self.w_uv, attn[:absorbed].view(absorbed, heads, self.vdim).transpose(0, 1))
         if self.gate_per_element:
             attn = ops.sigmoid_mul(ctx, attn, gate, ctx.buffer("attn_gated", (t, heads * self.vdim)))
         return ops.linear(ctx, attn, self.w_o, ctx.buffer(self.out_name, (t, self.hidden_size)))

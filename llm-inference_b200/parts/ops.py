@@ -867,6 +867,55 @@ def latent_attention_mma(
     return out
 
 
+# Portions shorter than this on average attend in the latent space, where nothing is expanded: per key the expansion costs 2 x 256 x
+# rank flops a head, which a portion of a few dozen queries does not earn back.
+LATENT_EXPAND_FROM = 64
+LATENT_EXPAND_BYTES = 2 << 30  # at most this much scratch for expanded keys and values
+
+
+def latent_expansion_rows(ctx: StepContext, cache: CacheView, dtype: torch.dtype, heads: int, dim: int, rot_dim: int, vdim: int, rank: int) -> int:
+    """Key rows that the step's prompt portions would expand (every portion's keys padded to whole tiles of 128), or 0 where they attend
+    in the latent space: other sizes than the tcgen05 form takes, short portions, windows, ``options["attention"]`` other than
+    ``"auto"``, too much scratch."""
+    decode, seqs = ctx.num_decode_seqs, ctx.num_seqs - ctx.num_decode_seqs
+    if (
+        dtype != torch.bfloat16 or seqs <= 0 or cache.window or ctx.options.get("attention", "auto") != "auto"
+        or ctx.num_tokens - decode < LATENT_EXPAND_FROM * seqs
+        or not ctx.lib.lib.b200_latent_prefill_supported(heads, dim, rot_dim, vdim, rank, cache.page_size)
+    ):
+        return 0
+    rows = sum(-(-int(n) // 128) * 128 for n in ctx.host.seq_kv_len[decode:])
+    return rows if rows * heads * (dim + vdim) * 2 <= LATENT_EXPAND_BYTES else 0
+
+
+def latent_portions(
+    ctx: StepContext, cache: CacheView, key_rows: int, queries: torch.Tensor, q_rot: torch.Tensor, w_expand: torch.Tensor, sink: torch.Tensor | None,
+    gate: torch.Tensor | None, out: torch.Tensor, heads: int, dim: int, rank: int, rot_dim: int, scale: float,
+) -> torch.Tensor:
+    """Attention of the step's prompt portions with keys and values expanded from the cached latents: a gather of the portions' latents
+    out of their pages, one product with ``w_expand`` (``[heads * (dim + vdim), rank]``: a head's key matrix, then its value matrix),
+    the tcgen05 prefill kernel. ``queries``: rows of ``heads * (dim + rot_dim)`` numbers, rotated parts not yet rotated (they are in
+    ``q_rot``); rows of single tokens, which lead the batch, are left alone."""
+    first, row_dim = ctx.num_decode_seqs, rank + rot_dim
+    _need(queries.stride(1) == 1 and queries.dtype == torch.bfloat16 and queries.shape[1] == heads * (dim + rot_dim), "latent_portions: bad queries")
+    _need(tuple(out.shape) == (ctx.num_tokens, heads * dim) and out.is_contiguous() and out.dtype == torch.bfloat16, "latent_portions: bad output")
+    _need(gate is None or (gate.stride(1) == 1 and gate.dtype == torch.bfloat16), "latent_portions: bad gate")
+    _need(sink is None or (sink.dtype == torch.float32 and sink.numel() == heads), "latent_portions: the sink is float32 [heads]")
+    latents = ctx.buffer("latent_rows", (key_rows, row_dim), torch.bfloat16, per_token=False)
+    ctx.lib.call(
+        "b200_latent_gather", ptr(cache.keys), ptr(cache.block_table), ptr(ctx.seq_kv_len), c_int(first), c_int(ctx.num_seqs - first), c_int(ctx.max_kv_len),
+        c_int(cache.max_pages), c_int(cache.num_pages), c_int(cache.page_size), c_int(row_dim), ptr(latents), ptr(ctx.err), ctx.stream,
+    )
+    expanded = ctx.buffer("latent_expanded", (key_rows, w_expand.shape[0]), torch.bfloat16, per_token=False)
+    torch.mm(latents[:, :rank], w_expand.t(), out=expanded)
+    ctx.lib.call(
+        "b200_latent_prefill_tcgen05", ptr(queries), c_int64(queries.stride(0)), c_int(dim + rot_dim), ptr(q_rot if rot_dim else None), ptr(expanded), ptr(latents),
+        c_int64(key_rows), c_int(rank), c_int(rot_dim), ptr(ctx.seq_q_start), ptr(ctx.seq_q_len), ptr(ctx.seq_kv_len), c_int(first), c_int(ctx.num_seqs - first),
+        c_int(ctx.max_q_len), c_int(heads), c_float(scale), ptr(sink), ptr(gate), c_int64(gate.stride(0) if gate is not None else 0), ptr(out), ptr(ctx.err), ctx.stream,
+    )
+    return out
+
+
 # -- the gated delta rule -----------------------------------------------------------------------------------
 
 
