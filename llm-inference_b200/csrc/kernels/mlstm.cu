@@ -13,11 +13,17 @@
 // per token and moves m on. Only the differences of neighbouring m enter S and n, and they are formed from the m that are
 // kept, so the scan's order of additions cannot disturb them. `mlstm_recurrence`: the columns of S are independent, n is one
 // more column (its v is 1), so a group of lanes owns a column and walks the request's tokens. `mlstm_output` (a warp per
-// token and head): denominator, norm, gate. In a step of single tokens the recurrence and the output kernel work the gates
+// token and head): denominator, norm, gate. Longer portions run 32 tokens at a time in place of `mlstm_recurrence`, whose chain
+// of dependent tokens bounds it (state_chunks.cu; all kernels of this file for 512 tokens of 12 heads of 128 x 128 on a B200:
+// 107 -> 63 us, of 2,048 tokens 579 -> 219 us). In a step of single tokens the recurrence and the output kernel work the gates
 // out themselves (the output kernel, which runs last, moves m on) and `mlstm_gates` is not launched.
 #include <type_traits>
 
 #include "common.cuh"
+
+extern "C" int b200_memory_chunks(const float* q, const float* k, const float* v, int64_t ld, const float* keep, const float* put, float scale, const int* seq_q_start,
+                                  const int* seq_q_len, const int* seq_slot, int tokens, int seqs, int max_q_len, int heads, int dk, int dv, float* scratch,
+                                  int64_t scratch_floats, float* S, float* n, float* num, float* den, cudaStream_t stream);
 
 namespace {
 
@@ -319,11 +325,13 @@ __global__ void mlstm_output_kernel(const MemoryParams p, const float* __restric
 
 // The whole of the mixer between its two products. `proj` (float, rows `ld` apart) holds q, k (heads * dk each), v and the
 // gate logits (heads * dv each) and the two gates' logits (heads each) from the columns given. `single`: every request of the
-// step feeds one token (two launches instead of three). `norm`: [heads * dv]; `out`: [tokens][heads * dv].
+// step feeds one token (two launches instead of three). With `scratch` (b200_state_chunks_scratch, rule 3) portions run in
+// chunks. `norm`: [heads * dv]; `out`: [tokens][heads * dv].
 B200_API int b200_mlstm(const float* proj, int ld, int q_at, int k_at, int v_at, int g_at, int i_at, int f_at, const float* i_bias,
                         const float* f_bias, float cap, const int* seq_q_start, const int* seq_q_len, const int* seq_slot, int seqs,
                         int tokens, int single, int heads, int dk, int dv, float* S, float* n, float* m, float* keep, float* put,
-                        float* least, float* num, float* den, const float* norm, float eps, void* out, int dtype, cudaStream_t stream) {
+                        float* least, float* num, float* den, const float* norm, float eps, void* out, int dtype, int max_q_len, float* scratch,
+                        int64_t scratch_floats, cudaStream_t stream) {
   if (tokens == 0 || seqs == 0) return 0;
   B200_REQUIRE(tokens > 0 && seqs > 0 && heads > 0 && heads <= 65535 && dk > 0 && dv > 0 && cap > 0.f, "mlstm: bad sizes");
   B200_REQUIRE(dk <= 1024, "mlstm: %d key channels per head, at most 1024", dk);
@@ -334,6 +342,12 @@ B200_API int b200_mlstm(const float* proj, int ld, int q_at, int k_at, int v_at,
   if (!single) {
     launch_kernel(mlstm_gates_kernel, dim3(seqs, heads), dim3(kScanThreads), 0, stream, p);
     if (int status = b200_check_launch("mlstm_gates")) return status;
+  }
+  const bool chunks = !single && scratch != nullptr;
+  if (chunks) {
+    if (int status = b200_memory_chunks(proj + q_at, proj + k_at, proj + v_at, ld, keep, put, 1.f / sqrtf(static_cast<float>(dk)), seq_q_start, seq_q_len, seq_slot,
+                                        tokens, seqs, max_q_len, heads, dk, dv, scratch, scratch_floats, S, n, num, den, stream))
+      return status;
   }
   int lanes = 1;
   while ((dk + lanes - 1) / lanes > 8 && lanes < 32) lanes *= 2;
@@ -362,7 +376,7 @@ B200_API int b200_mlstm(const float* proj, int ld, int q_at, int k_at, int v_at,
     else launch(mlstm_recurrence_kernel<8, 1, kSingle>);
   };
   if (single) by_shape(std::true_type{});
-  else by_shape(std::false_type{});
+  else if (!chunks) by_shape(std::false_type{});
   if (int status = b200_check_launch("mlstm_recurrence")) return status;
   const int threads = 128;
   const unsigned blocks = static_cast<unsigned>((static_cast<int64_t>(tokens) * heads + 3) / 4);

@@ -1,5 +1,6 @@
 // Recurrent matrix states over prompt portions, 32 tokens at a time: the delta rule (one decay per head, or one per head and key
-// channel), the generalized delta rule, and the rule with a decay per channel and a bonus for the current token.
+// channel), the generalized delta rule, the rule with a decay per channel and a bonus for the current token, and the matrix memory's
+// (one decay and one weight per head and token, a normaliser beside the state).
 //
 // Token by token a portion costs tokens x the latency of one step, however few columns a head's state has. Over a chunk of tokens
 // the rule S <- g S; u = beta (v - S^T k); S <- S + k u^T; o = S^T q is a handful of small matrix products (the chunkwise form of
@@ -42,6 +43,8 @@ __host__ __device__ constexpr int padded_rows(int dk) { return dk <= 64 ? 64 : (
 __host__ __device__ constexpr int padded_columns(int dv) { return (dv + kColumns - 1) / kColumns * kColumns; }
 // A chunk's place among all chunks of the step: different for all (request, chunk), below tokens / C + requests + 1.
 __device__ __forceinline__ int64_t chunk_place(int start, int seq, int chunk) { return static_cast<int64_t>(start / C) + seq + chunk; }
+
+enum Rule { kDelta = 0, kGeneralDelta = 1, kLinear = 2, kMemory = 3 };
 
 template <int kBytes>
 __device__ __forceinline__ void stage_copy(float* smem, const float* gmem, bool valid) {
@@ -104,6 +107,7 @@ struct Scratch {
   float* a;   // [tokens][heads][C]: what reads out U
   float* av;  // [tokens][heads][C]: what reads out V
   float* e;   // [chunks][heads][rows]: e_last
+  float* n;   // [chunks][heads][rows]: the matrix memory's normaliser, likewise
   float* s;   // [chunks][heads][rows][columns]: what the values alone add, then the state in front of each chunk
 };
 
@@ -382,15 +386,18 @@ chunk_prepare_kernel(const float* q, const float* k, const float* v, const float
 
 // --- the same for rules in which the values enter as they are ---------------------------------------------------------------------------
 //
-// GENERAL: S <- w S + b (u^T S) + k v^T, o = S^T r, with b = -au. Otherwise S <- w S + k v^T, o = S^T r + bonus v read before the update.
+// GENERAL: S <- w S + b (u^T S) + k v^T, o = S^T r, with b = -au. kLinear: S <- w S + k v^T, o = S^T r + bonus v read before the update.
+// MEMORY: S <- keep S + put k v^T and n <- keep n + put k with two numbers per head and token, o = S^T r and n . r after the update, r
+// times `scale`: pairs are products of the raw rows, times the keeps between them.
 // One block per (chunk, head, request); the sums of the values (G_last K)^T V go where the chunk's state will be.
 constexpr int kValueTile = 64;
 constexpr int kLdV = kValueTile + 4;
 constexpr int kMaxLinearRows = 128;
 
 __host__ __device__ constexpr int linear_warp_sums(bool general) { return general ? 2 * inside_sums(2) : between_sums(1); }
-size_t linear_prepare_smem(int rows, bool general) {
-  return sizeof(float) * ((general ? 5 : 3) * C * (rows + 4) + C * kLdV + kGroups * rows + kWarps * linear_warp_sums(general) + (general ? 4 : 1) * C * (C + 1) +
+size_t linear_prepare_smem(int rows, int rule) {
+  const bool general = rule == kGeneralDelta;
+  return sizeof(float) * ((general ? 5 : (rule == kMemory ? 2 : 3)) * C * (rows + 4) + 3 * C + C * kLdV + kGroups * rows + kWarps * linear_warp_sums(general) + (general ? 4 : 1) * C * (C + 1) +
                           (general ? 2 : 0) * C * C);
 }
 
@@ -401,10 +408,14 @@ struct LinearRule {
   const float* w;
   const float* au;     // GENERAL
   const float* u;      // GENERAL
-  const float* bonus;  // otherwise: [tokens][heads]
+  const float* bonus;  // kLinear: [tokens][heads]
+  const float* put;    // MEMORY: [tokens][heads], as is w (the keeps)
+  float scale;         // MEMORY
+  int64_t ld;          // numbers from token to token of r, k, w, au and u (a head's numbers start at head * dk)
+  int64_t v_ld;        // of v (at head * dv)
 };
 
-template <int ROWS, int W, bool GENERAL>
+template <int ROWS, int W, int RULE>
 __global__ void __launch_bounds__(kThreads, 2)
 linear_chunk_prepare_kernel(LinearRule in, const int* __restrict__ seq_q_start, const int* __restrict__ seq_q_len, int heads, int dk, int dv, Scratch to) {
   extern __shared__ __align__(16) float chunk_smem[];
@@ -416,13 +427,14 @@ linear_chunk_prepare_kernel(LinearRule in, const int* __restrict__ seq_q_start, 
   const int64_t first = static_cast<int64_t>(start) + chunk * C, place = chunk_place(start, seq, chunk) * heads + head;
   constexpr int rows = ROWS, ld = ROWS + 4;
   const int columns = padded_columns(dv);
+  constexpr bool GENERAL = RULE == kGeneralDelta, MEMORY = RULE == kMemory;
   constexpr int kSums = linear_warp_sums(GENERAL);
   float* ls = chunk_smem;                                // GENERAL: [C][C]: -N
   float* ms = ls + (GENERAL ? C * C : 0);                // GENERAL: [C][C]: M
   float* rs = ms + (GENERAL ? C * C : 0);                // [C][ld]: r, then times the decays of its group in front of (GENERAL: up to) its token
   float* ks = rs + C * ld;                               // [C][ld]: k, then times the decays from the next token to its group's end
   float* gs = ks + C * ld;                               // [C][ld]
-  float* us = gs + C * ld;                               // GENERAL: [C][ld]: u, then times the decays of its group in front of its token
+  float* us = gs + (MEMORY ? 0 : C * ld);                // GENERAL: [C][ld]: u, then times the decays of its group in front of its token
   float* bb = us + (GENERAL ? C * ld : 0);               // GENERAL: [C][ld]: -au, then as k
   float* vs = bb + (GENERAL ? C * ld : 0);               // [C][kLdV]: a tile of the values
   float* whole = vs + C * kLdV;                          // [groups][rows]
@@ -431,19 +443,21 @@ linear_chunk_prepare_kernel(LinearRule in, const int* __restrict__ seq_q_start, 
   float* uk = rk + C * (C + 1);
   float* rb = uk + C * (C + 1);
   float* ub = rb + C * (C + 1);
+  float* es = MEMORY ? uk : ub + (GENERAL ? C * (C + 1) : 0);  // MEMORY: [C]: the keeps up to a token, multiplied, times scale
+  float* fs = es + C;                                           // MEMORY: [C]: the keeps behind a token times its put
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int64_t ld_in = static_cast<int64_t>(heads) * dk, at_in = static_cast<int64_t>(head) * dk;
+  const int64_t ld_in = in.ld, at_in = static_cast<int64_t>(head) * dk;
   auto stage_values = [&](int col0) {
     for (int r = warp; r < C; r += kWarps)
       for (int c = lane * W; c < kValueTile; c += 32 * W) {
         const bool valid = r < n && col0 + c < dv;
-        stage_copy<4 * W>(vs + r * kLdV + c, valid ? in.v + ((first + r) * heads + head) * dv + col0 + c : in.v, valid);
+        stage_copy<4 * W>(vs + r * kLdV + c, valid ? in.v + (first + r) * in.v_ld + static_cast<int64_t>(head) * dv + col0 + c : in.v, valid);
       }
   };
   wait_for_predecessor();
   stage_rows<W>(rs, ld, in.r, first, n, ld_in, at_in, dk, rows);
   stage_rows<W>(ks, ld, in.k, first, n, ld_in, at_in, dk, rows);
-  stage_rows<W>(gs, ld, in.w, first, n, ld_in, at_in, dk, rows);
+  if (!MEMORY) stage_rows<W>(gs, ld, in.w, first, n, ld_in, at_in, dk, rows);
   if (GENERAL) {
     stage_rows<W>(us, ld, in.u, first, n, ld_in, at_in, dk, rows);
     stage_rows<W>(bb, ld, in.au, first, n, ld_in, at_in, dk, rows);
@@ -457,7 +471,7 @@ linear_chunk_prepare_kernel(LinearRule in, const int* __restrict__ seq_q_start, 
     pairs_inside<ROWS, 2, true, true>(us, rs, ks, gs, mine);
     pairs_inside<ROWS, 2, true, true>(us, rs, bb, gs, mine + inside_sums(2));
   } else {
-    pairs_inside<ROWS, 1, true, true>(rs, nullptr, ks, gs, mine);
+    pairs_inside<ROWS, 1, !MEMORY, !MEMORY>(rs, nullptr, ks, gs, mine);
   }
   __syncthreads();
   if (GENERAL) {
@@ -466,7 +480,7 @@ linear_chunk_prepare_kernel(LinearRule in, const int* __restrict__ seq_q_start, 
   } else {
     add_up<1, true>(sums, kSums, rk, nullptr);
   }
-  for (int item = tid; item < kGroups * rows; item += kThreads) {  // a thread per (group, channel)
+  for (int item = tid; !MEMORY && item < kGroups * rows; item += kThreads) {  // a thread per (group, channel)
     const int c = item % rows, at = item / rows * kGroup * ld + c;
     float g[kGroup];
     float run = 1.f;
@@ -497,12 +511,44 @@ linear_chunk_prepare_kernel(LinearRule in, const int* __restrict__ seq_q_start, 
     __syncthreads();
     add_up<2, false>(sums, kSums, ub, rb);
   } else {
-    pairs_between<ROWS, 1, true>(rs, nullptr, ks, whole, mine);
+    pairs_between<ROWS, 1, !MEMORY>(rs, nullptr, ks, whole, mine);
     __syncthreads();
     add_up<1, false>(sums, kSums, rk, nullptr);
   }
   __syncthreads();
-  for (int i = warp; i < C; i += kWarps) {
+  if constexpr (MEMORY) {
+    // Column j = lane: the keeps of tokens j + 1 .. i multiplied, from one at i = j on.
+    const int64_t at = (first + lane) * heads + head;
+    const float keep = lane < n ? in.w[at] : 1.f, put = lane < n ? in.put[at] : 0.f;
+    float d = 1.f, prefix = 1.f, e = 1.f;
+    for (int i = 0; i < C; ++i) {
+      const float own = __shfl_sync(0xffffffffu, keep, i);
+      d = i > lane ? d * own : 1.f;
+      prefix *= own;
+      if (i == lane) e = prefix;
+      if ((i & 7) == warp && i < n) to.av[((first + i) * heads + head) * C + lane] = lane <= i ? d * put * rk[i * (C + 1) + lane] * in.scale : 0.f;
+    }
+    if (warp == 0) es[lane] = e, fs[lane] = d * put;
+    __syncthreads();
+    for (int c = tid; c < rows; c += kThreads) {
+      float* qt = to.qt + (first * heads + head) * rows + c;
+      float sum = 0.f;
+#pragma unroll 8
+      for (int i = 0; i < C; ++i) {
+        const float key = fs[i] * ks[i * ld + c];
+        ks[i * ld + c] = key;
+        sum += key;
+        if (i < n) *qt = es[i] * in.scale * rs[i * ld + c];
+        qt += static_cast<int64_t>(heads) * rows;
+      }
+      to.n[place * rows + c] = sum;
+      to.e[place * rows + c] = es[n - 1];
+#pragma unroll
+      for (int g = 0; g < kGroups; ++g) whole[g * rows + c] = 1.f;
+    }
+    __syncthreads();
+  }
+  for (int i = warp; !MEMORY && i < C; i += kWarps) {
     const int at = i * (C + 1) + lane;
     const int64_t row = ((first + i) * heads + head) * C + lane;
     if (GENERAL) {  // au came in with its own sign: b = -au
@@ -517,7 +563,7 @@ linear_chunk_prepare_kernel(LinearRule in, const int* __restrict__ seq_q_start, 
     }
   }
   // Scaled rows: r times all decays in front of (or up to) its token, b times all decays behind its token; a thread per (group, channel).
-  for (int item = tid; item < kGroups * rows; item += kThreads) {
+  for (int item = tid; !MEMORY && item < kGroups * rows; item += kThreads) {
     const int c = item % rows, group = item / rows;
     float before = 1.f, after = 1.f;
 #pragma unroll
@@ -538,7 +584,7 @@ linear_chunk_prepare_kernel(LinearRule in, const int* __restrict__ seq_q_start, 
       qt += step, kd += step;
     }
   }
-  for (int c = tid; c < rows; c += kThreads) to.e[place * rows + c] = whole[c] * whole[rows + c] * whole[2 * rows + c] * whole[3 * rows + c];
+  for (int c = tid; !MEMORY && c < rows; c += kThreads) to.e[place * rows + c] = whole[c] * whole[rows + c] * whole[2 * rows + c] * whole[3 * rows + c];
   if (GENERAL) __syncthreads();
   for (int col0 = 0; col0 < columns; col0 += kValueTile) {
     if (col0 > 0) {
@@ -627,13 +673,27 @@ linear_chunk_prepare_kernel(LinearRule in, const int* __restrict__ seq_q_start, 
 // Four neighbouring numbers of a head's state a thread, from chunk to chunk: eight chunks' sums are asked for at a time.
 __global__ void __launch_bounds__(kThreads)
 chunk_scan_kernel(const int* __restrict__ seq_q_start, const int* __restrict__ seq_q_len, const int* __restrict__ seq_slot, int heads, int dk, int dv, Scratch from,
-                  float* state) {
+                  float* state, float* normaliser) {
   let_successor_start();
   const int seq = blockIdx.z, head = blockIdx.y;
   const int start = seq_q_start[seq], len = seq_q_len[seq], chunks = (len + C - 1) / C;
   const int rows = padded_rows(dk), columns = padded_columns(dv);
   const int item = (blockIdx.x * kThreads + threadIdx.x) * 4;
-  if (item >= rows * columns) return;
+  if (item >= rows * columns) {  // the blocks behind the state's: a number of the normaliser a thread
+    const int c = blockIdx.x * kThreads + threadIdx.x - (rows * columns / 4 + kThreads - 1) / kThreads * kThreads;
+    if (normaliser == nullptr || c < 0 || c >= rows) return;
+    wait_for_predecessor();
+    float* own = normaliser + (static_cast<int64_t>(seq_slot[seq]) * heads + head) * dk + c;
+    float n = c < dk ? *own : 0.f;
+    const int64_t step = static_cast<int64_t>(heads) * rows, at = (chunk_place(start, seq, 0) * heads + head) * rows + c;
+    for (int chunk = 0; chunk < chunks; ++chunk) {
+      const float add = from.n[at + chunk * step];
+      from.n[at + chunk * step] = n;
+      n = fmaf(from.e[at + chunk * step], n, add);
+    }
+    if (c < dk && chunks > 0) *own = n;
+    return;
+  }
   const int row = item / columns, col = item % columns;
   float* base = state + (static_cast<int64_t>(seq_slot[seq]) * heads + head) * dk * dv + static_cast<int64_t>(row) * dv + col;
   float s[4];
@@ -865,7 +925,7 @@ constexpr size_t out_smem(int cols) { return sizeof(float) * 2 * (C * kLdSlab + 
 template <int COLS, bool WITH_U, bool WITH_V>
 __global__ void __launch_bounds__(COLS)
 chunk_out_kernel(const int* __restrict__ seq_q_start, const int* __restrict__ seq_q_len, int heads, int dv, int rows, int tiles, Scratch from, const float* v,
-                 int v_wide, float* out) {
+                 int64_t v_ld, int v_wide, float* out, float* den) {
   extern __shared__ __align__(16) float chunk_smem[];
   constexpr int kLdOut = COLS + 4, kStage = C * kLdSlab + C * kLdOut;
   let_successor_start();
@@ -902,12 +962,12 @@ chunk_out_kernel(const int* __restrict__ seq_q_start, const int* __restrict__ se
       for (int r = tid / (COLS / 4); r < C; r += 4) {
         const int c = tid % (COLS / 4) * 4;
         const bool valid = col0 + c < dv && r < n;
-        stage_copy<16>(right + r * kLdOut + c, valid ? v + ((first + r) * heads + head) * dv + col0 + c : v, valid);
+        stage_copy<16>(right + r * kLdOut + c, valid ? v + (first + r) * v_ld + static_cast<int64_t>(head) * dv + col0 + c : v, valid);
       }
     } else {
       for (int r = 0; r < C; ++r) {
         const bool valid = col0 + tid < dv && r < n;
-        stage_copy<4>(right + r * kLdOut + tid, valid ? v + ((first + r) * heads + head) * dv + col0 + tid : v, valid);
+        stage_copy<4>(right + r * kLdOut + tid, valid ? v + (first + r) * v_ld + static_cast<int64_t>(head) * dv + col0 + tid : v, valid);
       }
     }
     commit_copies();
@@ -917,6 +977,16 @@ chunk_out_kernel(const int* __restrict__ seq_q_start, const int* __restrict__ se
 #pragma unroll
   for (int i = 0; i < 8; ++i) acc[i][0] = acc[i][1] = acc[i][2] = acc[i][3] = 0.f;
   fetch(0);
+  if (den != nullptr && col0 == 0) {  // the normaliser read out as the state is: n . (e q) + the chunk's own pairs
+    const float* n0 = from.n + (chunk_place(start, seq, chunk) * heads + head) * rows;
+    for (int r = warp; r < n; r += COLS / 32) {
+      const int64_t row = (first + r) * heads + head;
+      float sum = from.av[row * C + lane];
+      for (int c = lane; c < rows; c += 32) sum = fmaf(from.qt[row * rows + c], n0[c], sum);
+      sum = warp_sum(sum);
+      if (lane == 0) den[row] = sum;
+    }
+  }
   for (int slab = 0; slab < slabs; ++slab) {
     if (slab + 1 < slabs) {
       fetch(slab + 1);
@@ -968,8 +1038,6 @@ chunk_out_kernel(const int* __restrict__ seq_q_start, const int* __restrict__ se
 
 // --- host ------------------------------------------------------------------------------------------------------------------------------
 
-enum Rule { kDelta = 0, kGeneralDelta = 1, kLinear = 2 };
-
 struct Sizes {
   int tokens, seqs, max_q_len, heads, dk, dv;
 };
@@ -980,12 +1048,12 @@ int64_t aligned_floats(int64_t n) { return (n + 3) / 4 * 4; }
 int64_t lay_out(int rule, const Sizes& z, float* base, Scratch* to) {
   const int64_t rows = padded_rows(z.dk), columns = padded_columns(z.dv), per_head = static_cast<int64_t>(z.tokens) * z.heads;
   const int64_t chunks = (static_cast<int64_t>(z.tokens) / C + z.seqs + 1) * z.heads;
-  const int64_t with_u = rule != kLinear ? 1 : 0, with_v = rule != kDelta ? 1 : 0;
-  const int64_t sizes[8] = {with_u * per_head * rows, with_u * per_head * rows, per_head * rows, with_u * per_head * columns,
-                            with_u * per_head * C, with_v * per_head * C, chunks * rows, chunks * rows * columns};
-  float** arrays[8] = {&to->y, &to->kd, &to->qt, &to->x, &to->a, &to->av, &to->e, &to->s};
+  const int64_t with_u = rule == kDelta || rule == kGeneralDelta ? 1 : 0, with_v = rule != kDelta ? 1 : 0, with_n = rule == kMemory ? 1 : 0;
+  const int64_t sizes[9] = {with_u * per_head * rows, with_u * per_head * rows, per_head * rows, with_u * per_head * columns,
+                            with_u * per_head * C, with_v * per_head * C, chunks * rows, with_n * chunks * rows, chunks * rows * columns};
+  float** arrays[9] = {&to->y, &to->kd, &to->qt, &to->x, &to->a, &to->av, &to->e, &to->n, &to->s};
   int64_t at = 0;
-  for (int i = 0; i < 8; ++i) {
+  for (int i = 0; i < 9; ++i) {
     *arrays[i] = base == nullptr ? nullptr : base + at;
     at += aligned_floats(sizes[i]);
   }
@@ -1004,9 +1072,10 @@ bool raise_prepares() {
             raise_smem(chunk_prepare_kernel<ROWS, 1, true>, delta) && raise_smem(chunk_prepare_kernel<ROWS, 4, true>, delta) &&
             raise_smem(chunk_walk_kernel<ROWS, false>, walk_smem(ROWS));
   if constexpr (ROWS <= kMaxLinearRows) {
-    const size_t general = linear_prepare_smem(ROWS, true), linear = linear_prepare_smem(ROWS, false);
-    ok = ok && raise_smem(linear_chunk_prepare_kernel<ROWS, 1, false>, linear) && raise_smem(linear_chunk_prepare_kernel<ROWS, 4, false>, linear) &&
-         raise_smem(linear_chunk_prepare_kernel<ROWS, 1, true>, general) && raise_smem(linear_chunk_prepare_kernel<ROWS, 4, true>, general) &&
+    const size_t general = linear_prepare_smem(ROWS, kGeneralDelta), linear = linear_prepare_smem(ROWS, kLinear), memory = linear_prepare_smem(ROWS, kMemory);
+    ok = ok && raise_smem(linear_chunk_prepare_kernel<ROWS, 1, kLinear>, linear) && raise_smem(linear_chunk_prepare_kernel<ROWS, 4, kLinear>, linear) &&
+         raise_smem(linear_chunk_prepare_kernel<ROWS, 1, kGeneralDelta>, general) && raise_smem(linear_chunk_prepare_kernel<ROWS, 4, kGeneralDelta>, general) &&
+         raise_smem(linear_chunk_prepare_kernel<ROWS, 1, kMemory>, memory) && raise_smem(linear_chunk_prepare_kernel<ROWS, 4, kMemory>, memory) &&
          raise_smem(chunk_walk_kernel<ROWS, true>, walk_smem(ROWS));
   }
   return ok;
@@ -1024,9 +1093,10 @@ auto delta_prepare_form(bool wide, bool per_head) {
 }
 
 template <int ROWS>
-auto linear_prepare_form(bool wide, bool general) {
-  return general ? (wide ? linear_chunk_prepare_kernel<ROWS, 4, true> : linear_chunk_prepare_kernel<ROWS, 1, true>)
-                 : (wide ? linear_chunk_prepare_kernel<ROWS, 4, false> : linear_chunk_prepare_kernel<ROWS, 1, false>);
+auto linear_prepare_form(bool wide, int rule) {
+  return rule == kGeneralDelta ? (wide ? linear_chunk_prepare_kernel<ROWS, 4, kGeneralDelta> : linear_chunk_prepare_kernel<ROWS, 1, kGeneralDelta>)
+         : rule == kMemory     ? (wide ? linear_chunk_prepare_kernel<ROWS, 4, kMemory> : linear_chunk_prepare_kernel<ROWS, 1, kMemory>)
+                               : (wide ? linear_chunk_prepare_kernel<ROWS, 4, kLinear> : linear_chunk_prepare_kernel<ROWS, 1, kLinear>);
 }
 
 bool aligned16(const void* p) { return reinterpret_cast<uintptr_t>(p) % 16 == 0; }
@@ -1048,19 +1118,33 @@ int launch_walk(const Sizes& z, const Requests& req, bool add, const Scratch& sc
 }
 
 template <bool WITH_U, bool WITH_V>
-int launch_out(const Sizes& z, const Requests& req, const Scratch& scratch, const float* v, float* out, cudaStream_t stream) {
+int launch_out(const Sizes& z, const Requests& req, const Scratch& scratch, const float* v, int64_t v_ld, float* out, float* den, cudaStream_t stream) {
   const int columns = padded_columns(z.dv), cols = columns <= 64 ? 64 : 128, tiles = (columns + cols - 1) / cols;
   launch_kernel(cols == 64 ? chunk_out_kernel<64, WITH_U, WITH_V> : chunk_out_kernel<128, WITH_U, WITH_V>, dim3((z.max_q_len + C - 1) / C, z.heads, z.seqs * tiles),
                 dim3(cols), out_smem(cols), stream, req.q_start, req.q_len, z.heads, z.dv, padded_rows(z.dk), tiles, scratch, v,
-                z.dv % 4 == 0 && aligned16(v) ? 1 : 0, out);
+                v_ld, z.dv % 4 == 0 && v_ld % 4 == 0 && aligned16(v) ? 1 : 0, out, den);
   return b200_check_launch("chunk_out");
+}
+
+int launch_linear_prepare(const Sizes& z, const Requests& req, int rule, bool wide, const LinearRule& in, const Scratch& scratch, cudaStream_t stream) {
+  const int rows = padded_rows(z.dk);
+  launch_kernel(rows == 64 ? linear_prepare_form<64>(wide, rule) : linear_prepare_form<128>(wide, rule), dim3((z.max_q_len + C - 1) / C, z.heads, z.seqs),
+                dim3(kThreads), linear_prepare_smem(rows, rule), stream, in, req.q_start, req.q_len, z.heads, z.dk, z.dv, scratch);
+  return b200_check_launch("linear_chunk_prepare");
+}
+
+int launch_scan(const Sizes& z, const Requests& req, const Scratch& scratch, float* state, float* normaliser, cudaStream_t stream) {
+  const int rows = padded_rows(z.dk), blocks = (rows * padded_columns(z.dv) / 4 + kThreads - 1) / kThreads;
+  launch_kernel(chunk_scan_kernel, dim3(blocks + (normaliser != nullptr ? (rows + kThreads - 1) / kThreads : 0), z.heads, z.seqs), dim3(kThreads), 0, stream, req.q_start,
+                req.q_len, req.slot, z.heads, z.dk, z.dv, scratch, state, normaliser);
+  return b200_check_launch("chunk_scan");
 }
 
 bool too_many_requests(const Sizes& z) { return static_cast<int64_t>(z.seqs) * ((padded_columns(z.dv) + 127) / 128) > 65535; }
 
 }  // namespace
 
-// Sizes the chunked form takes (`rule`: 0 the delta rule, 1 the generalized one, 2 the one without a removal); the caller walks token by
+// Sizes the chunked form takes (`rule`: 0 the delta rule, 1 the generalized one, 2 the one without a removal, 3 the matrix memory); the caller walks token by
 // token otherwise.
 B200_API int b200_state_chunks_supported(int rule, int heads, int kv_heads, int dk, int dv) {
   return heads > 0 && heads <= 65535 && kv_heads > 0 && heads % kv_heads == 0 && dk > 0 && dk <= (rule == kDelta ? kMaxRows : kMaxLinearRows) && dv > 0 &&
@@ -1093,7 +1177,7 @@ B200_API int b200_delta_chunks(const float* q, const float* k, const float* v, c
                 seq_q_len, heads, kv_heads, dk, dv, parts);
   if (int status = b200_check_launch("chunk_prepare")) return status;
   if (int status = launch_walk(z, req, false, parts, state, stream)) return status;
-  return launch_out<true, false>(z, req, parts, v, out, stream);
+  return launch_out<true, false>(z, req, parts, v, static_cast<int64_t>(heads) * dv, out, nullptr, stream);
 }
 
 // The rules in which the values enter as they are. With `u` the generalized delta rule S <- w S - au (u^T S) + k v^T, o = S^T r; with
@@ -1113,18 +1197,31 @@ B200_API int b200_linear_chunks(const float* r, const float* k, const float* v, 
   B200_REQUIRE(seqs <= 65535 && !too_many_requests(z), "linear_chunks: too many requests");
   B200_REQUIRE(raise_all(), "linear_chunks: cannot size shared memory");
   const bool wide = dk % 4 == 0 && dv % 4 == 0 && aligned16(r) && aligned16(k) && aligned16(v) && aligned16(w) && aligned16(au) && aligned16(u);
-  const bool general = rule == kGeneralDelta;
-  const int rows = padded_rows(dk), columns = padded_columns(dv);
-  auto prepare = rows == 64 ? linear_prepare_form<64>(wide, general) : linear_prepare_form<128>(wide, general);
-  launch_kernel(prepare, dim3((max_q_len + C - 1) / C, heads, seqs), dim3(kThreads), linear_prepare_smem(rows, general), stream, LinearRule{r, k, v, w, au, u, bonus},
-                seq_q_start, seq_q_len, heads, dk, dv, parts);
-  if (int status = b200_check_launch("linear_chunk_prepare")) return status;
-  if (general) {
+  const LinearRule in{r, k, v, w, au, u, bonus, nullptr, 1.f, static_cast<int64_t>(heads) * dk, static_cast<int64_t>(heads) * dv};
+  if (int status = launch_linear_prepare(z, req, rule, wide, in, parts, stream)) return status;
+  if (rule == kGeneralDelta) {
     if (int status = launch_walk(z, req, true, parts, state, stream)) return status;
-    return launch_out<true, true>(z, req, parts, v, out, stream);
+    return launch_out<true, true>(z, req, parts, v, in.v_ld, out, nullptr, stream);
   }
-  launch_kernel(chunk_scan_kernel, dim3((rows * columns / 4 + kThreads - 1) / kThreads, heads, seqs), dim3(kThreads), 0, stream, seq_q_start, seq_q_len, seq_slot, heads,
-                dk, dv, parts, state);
-  if (int status = b200_check_launch("chunk_scan")) return status;
-  return launch_out<false, true>(z, req, parts, v, out, stream);
+  if (int status = launch_scan(z, req, parts, state, nullptr, stream)) return status;
+  return launch_out<false, true>(z, req, parts, v, in.v_ld, out, nullptr, stream);
+}
+
+// The matrix memory: S <- keep S + put k v^T, n <- keep n + put k, num = scale S^T q, den = scale n . q after the update. q, k, v: rows ld numbers apart, a
+// head's numbers side by side; keep, put, den [tokens][heads]; num [tokens][heads][dv]. Called by b200_mlstm.
+extern "C" int b200_memory_chunks(const float* q, const float* k, const float* v, int64_t ld, const float* keep, const float* put, float scale, const int* seq_q_start,
+                                  const int* seq_q_len, const int* seq_slot, int tokens, int seqs, int max_q_len, int heads, int dk, int dv, float* scratch,
+                                  int64_t scratch_floats, float* S, float* n, float* num, float* den, cudaStream_t stream) {
+  B200_REQUIRE(tokens > 0 && seqs > 0 && max_q_len > 0 && b200_state_chunks_supported(kMemory, heads, heads, dk, dv), "memory_chunks: shape not taken");
+  const Sizes z = {tokens, seqs, max_q_len, heads, dk, dv};
+  const Requests req = {seq_q_start, seq_q_len, seq_slot};
+  Scratch parts;
+  B200_REQUIRE(aligned16(scratch) && lay_out(kMemory, z, scratch, &parts) <= scratch_floats, "memory_chunks: scratch too small or not aligned to 16 bytes");
+  B200_REQUIRE(seqs <= 65535 && !too_many_requests(z), "memory_chunks: too many requests");
+  B200_REQUIRE(raise_all(), "memory_chunks: cannot size shared memory");
+  const bool wide = dk % 4 == 0 && dv % 4 == 0 && ld % 4 == 0 && aligned16(q) && aligned16(k) && aligned16(v);
+  const LinearRule in{q, k, v, keep, nullptr, nullptr, nullptr, put, scale, ld, ld};
+  if (int status = launch_linear_prepare(z, req, kMemory, wide, in, parts, stream)) return status;
+  if (int status = launch_scan(z, req, parts, S, n, stream)) return status;
+  return launch_out<false, true>(z, req, parts, v, ld, num, den, stream);
 }

@@ -956,12 +956,20 @@ DELTA_CHUNK_FROM = 112
 # tokens, 61 and 62 at 200, 244 and 473 at 2,048.
 LINEAR_CHUNK_FROM = 80
 GENERAL_DELTA_CHUNK_FROM = 192
-_DELTA, _GENERAL_DELTA, _LINEAR = 0, 1, 2  # csrc/kernels/state_chunks.cu
+# The matrix memory, one request, 12 heads of 128 x 128, with its gates and its output: 54 us in chunks and 42 token by token at 128
+# tokens, 55 and 53 at 160, 56 and 54 at 200 (the chunked form's four launches bound it up to there), 63 and 107 at 512, 219 and 579 at
+# 2,048.
+MEMORY_CHUNK_FROM = 200
+# Scratch grows with the step's tokens (0.13 MB a token at 28 heads of 128 x 128): past this a step walks its portions token by token, as
+# if they were short, in the memory that takes.
+CHUNK_SCRATCH_BYTES = 2 << 30
+_DELTA, _GENERAL_DELTA, _LINEAR, _MEMORY = 0, 1, 2, 3  # csrc/kernels/state_chunks.cu
 
 
 def _chunk_scratch(ctx: StepContext, rule: int, longer_than: int, tokens: int, heads: int, kv_heads: int, dk: int, dv: int) -> torch.Tensor | None:
     """Scratch for a recurrence that runs chunk by chunk (csrc/kernels/state_chunks.cu), or None where it runs token by token:
-    portions of at most ``longer_than`` tokens and sizes the chunked form does not take. ``options["delta_portions"]``:
+    portions of at most ``longer_than`` tokens, sizes the chunked form does not take and steps whose scratch would pass
+    ``CHUNK_SCRATCH_BYTES``. ``options["delta_portions"]``:
     ``"chunks"`` or ``"tokens"`` forces one of the two."""
     choice = ctx.options.get("delta_portions", "auto")
     if choice == "tokens" or (choice == "auto" and not (
@@ -969,6 +977,8 @@ def _chunk_scratch(ctx: StepContext, rule: int, longer_than: int, tokens: int, h
     )):
         return None
     floats = int(ctx.lib.lib.b200_state_chunks_scratch(rule, tokens, ctx.num_seqs, heads, dk, dv))
+    if choice == "auto" and 4 * floats > CHUNK_SCRATCH_BYTES:
+        return None
     return ctx.buffer("state_chunks", (floats,), torch.float32, per_token=False)
 
 
@@ -1739,12 +1749,15 @@ def mlstm(ctx: StepContext, proj: torch.Tensor, columns: tuple[int, int, int, in
     single = ctx.num_tokens == ctx.num_seqs
     gates = [None] * 3 if single else [ctx.buffer("mlstm_" + name, (tokens, heads), f32) for name in ("keep", "put", "least")]
     num, den = ctx.buffer("mlstm_num", (tokens, heads * dv), f32), ctx.buffer("mlstm_den", (tokens, heads), f32)
+    scratch = None if single else _chunk_scratch(ctx, _MEMORY, MEMORY_CHUNK_FROM, tokens, heads, heads, dk, dv)
     ctx.lib.call(
         "b200_mlstm", ptr(proj), c_int(proj.shape[1]), *(c_int(c) for c in columns), ptr(i_bias), ptr(f_bias), c_float(cap), ptr(ctx.seq_q_start),
         ptr(ctx.seq_q_len), ptr(ctx.seq_slot), c_int(ctx.num_seqs), c_int(tokens), c_int(1 if single else 0), c_int(heads), c_int(dk), c_int(dv),
-        ptr(S), ptr(n), ptr(m), *(ptr(g) for g in gates), ptr(num), ptr(den), ptr(norm), c_float(eps), ptr(out), c_int(dtype_code(out.dtype)), ctx.stream,
+        ptr(S), ptr(n), ptr(m), *(ptr(g) for g in gates), ptr(num), ptr(den), ptr(norm), c_float(eps), ptr(out), c_int(dtype_code(out.dtype)), c_int(ctx.max_q_len),
+        ptr(scratch), c_int64(scratch.numel() if scratch is not None else 0), ctx.stream,
     )
-    ctx.lib.calls += 1 if single else 2  # the recurrence and the output kernel (and the gates') are launches of their own
+    # The recurrence and the output kernel (and the gates'; in chunks three in the recurrence's place) are launches of their own.
+    ctx.lib.calls += (1 if single else 2) + (2 if scratch is not None else 0)
     return out
 
 

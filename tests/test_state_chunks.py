@@ -146,3 +146,89 @@ def test_rules_in_which_the_values_enter_as_they_are(heads, dk, dv, runs, portio
         np.testing.assert_allclose(got, wanted, rtol=2e-5, atol=2e-6 * np.sqrt(np.mean(wanted**2)) * np.sqrt(dk) + 2e-5)
     others = [slot for slot in range(state.shape[0]) if slot not in slots]
     assert torch.equal(state[others], untouched[others])
+
+
+MEMORY_SIZES = [
+    (2, 128, 128, (97, 32, 1)),
+    (3, 33, 17, (31, 65)),
+    (1, 64, 70, (127,)),
+    (2, 16, 130, (96, 95, 98)),
+]
+
+
+@pytest.mark.parametrize("heads,dk,dv,runs", MEMORY_SIZES)
+@pytest.mark.parametrize("portions", ["chunks", "tokens"])
+def test_the_matrix_memory(heads, dk, dv, runs, portions):
+    """Given projections over portions that continue states: gates from nearly shut to wide open, the state, its normaliser and the
+    running maximum read back, the states of other requests untouched."""
+    from llm_inference_b200.parts import ops
+
+    n, cap, eps = sum(runs), 9.0, 1e-6
+    rng = np.random.default_rng(dk + dv)
+    widths = [heads * dk, heads * dk, heads * dv, heads * dv, heads, heads]
+    columns = tuple(int(c) for c in np.cumsum([0] + widths[:-1]))
+    proj = rng.normal(size=(n, sum(widths)))
+    proj[:, columns[4] : columns[5]] *= 6.0
+    proj[:, columns[5] :] = proj[:, columns[5] :] * 6.0 + 3.0
+    bias = rng.normal(size=(2, heads))
+    norm = 1.0 + rng.normal(0, 0.2, heads * dv)
+    start = [rng.normal(size=(len(runs), heads, dk, dv)), rng.normal(size=(len(runs), heads, dk)), rng.normal(size=(len(runs), heads))]
+    proj, bias, norm, *start = (a.astype(np.float32) for a in (proj, bias, norm, *start))
+    q, k, v, gate, i_log, f_log = (proj[:, c : c + w].astype(np.float64) for c, w in zip(columns, widths))
+    q, k, v = q.reshape(n, heads, dk) * dk**-0.5, k.reshape(n, heads, dk), v.reshape(n, heads, dv)
+    i_log = cap * np.tanh((i_log + bias[0]) / cap)
+    f_log = -np.logaddexp(0.0, -cap * np.tanh((f_log + bias[1]) / cap))
+    S, N, M = (a.astype(np.float64) for a in start)
+    want, weak, at = np.zeros((n, heads, dv)), np.zeros((n, heads)), 0
+    for s, run in enumerate(runs):
+        for t in range(at, at + run):
+            top = np.maximum(f_log[t] + M[s], i_log[t])
+            keep, put = np.exp(f_log[t] + M[s] - top), np.exp(i_log[t] - top)
+            M[s] = top
+            S[s] = keep[:, None, None] * S[s] + put[:, None, None] * k[t][..., None] * v[t][:, None]
+            N[s] = keep[:, None] * N[s] + put[:, None] * k[t]
+            want[t] = np.einsum("hkv,hk->hv", S[s], q[t])
+            # What a head's norm leaves of rounding: its read-out's size against the terms it was summed from.
+            weak[t] = np.linalg.norm(S[s], axis=(1, 2)) * np.linalg.norm(q[t], axis=-1) / np.linalg.norm(want[t], axis=-1)
+            want[t] /= np.maximum(np.abs((N[s] * q[t]).sum(-1)), np.exp(-top))[:, None]
+        at += run
+    want = want / np.sqrt((want**2).mean(-1, keepdims=True) + eps)
+    want = want * norm.reshape(heads, dv) / (1.0 + np.exp(-gate.reshape(n, heads, dv)))
+    slots = [4, 0, 2][: len(runs)]
+    runner, cache, ctx = device_context(runs, slots, ((heads, dk, dv), (heads, dk), (heads,)), {"delta_portions": portions})
+    state = cache.states[0]
+    untouched = [array.normal_().clone() for array in state]
+    for array, own in zip(state, start):
+        array[slots] = torch.from_numpy(own).cuda()
+    out = torch.full((n, heads * dv), float("nan"), device="cuda")
+    device = [torch.from_numpy(a).cuda() for a in (proj, bias, norm)]
+    ops.mlstm(ctx, device[0], columns, device[1][0], device[1][1], cap, state, heads, dk, dv, device[2], eps, out)
+    runner.check()
+    got = out.double().cpu().numpy().reshape(want.shape)
+    assert np.all(np.abs(got - want).max(-1) <= 2e-5 * (1.0 + weak) * (1.0 + np.abs(want).max(-1)))
+    for array, wanted in zip(state, (S, N, M)):
+        np.testing.assert_allclose(array[slots].double().cpu().numpy(), wanted, rtol=2e-5, atol=2e-5)
+    others = [slot for slot in range(state[0].shape[0]) if slot not in slots]
+    for array, before in zip(state, untouched):
+        assert torch.equal(array[others], before[others])
+
+
+def test_portions_whose_scratch_would_be_too_large_go_token_by_token(monkeypatch):
+    from llm_inference_b200.parts import ops
+
+    heads, dk, dv, n = 2, 64, 64, ops.LINEAR_CHUNK_FROM + 20
+    torch.manual_seed(3)
+    r, k, w, v, bonus = (torch.rand(n, heads * width, device="cuda") for width in (dk, dk, dk, dv, 1))
+
+    def run(choice):
+        runner, cache, ctx = device_context((n,), (1,), ((heads, dk, dv),), {"delta_portions": choice})
+        cache.states[0][0].zero_()
+        out = torch.empty(n, heads * dv, device="cuda")
+        ops.wkv_recurrence(ctx, r, k, v, bonus, w, cache.states[0][0], out, heads, dk, dv)
+        runner.check()
+        return out
+
+    tokens, chunks = run("tokens"), run("chunks")
+    assert torch.equal(run("auto"), chunks) and not torch.equal(chunks, tokens)
+    monkeypatch.setattr(ops, "CHUNK_SCRATCH_BYTES", 1 << 10)
+    assert torch.equal(run("auto"), tokens)
