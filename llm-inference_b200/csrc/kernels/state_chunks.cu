@@ -1144,15 +1144,16 @@ bool too_many_requests(const Sizes& z) { return static_cast<int64_t>(z.seqs) * (
 
 }  // namespace
 
-// Sizes the chunked form takes (`rule`: 0 the delta rule, 1 the generalized one, 2 the one without a removal, 3 the matrix memory); the caller walks token by
-// token otherwise.
-B200_API int b200_state_chunks_supported(int rule, int heads, int kv_heads, int dk, int dv) {
+// Sizes the chunked form takes (`rule`: 0 the delta rule, 1 the generalized one, 2 the one without a removal, 3 the matrix memory); the
+// caller walks token by token otherwise.
+static bool sizes_taken(int rule, int heads, int kv_heads, int dk, int dv) {
   return heads > 0 && heads <= 65535 && kv_heads > 0 && heads % kv_heads == 0 && dk > 0 && dk <= (rule == kDelta ? kMaxRows : kMaxLinearRows) && dv > 0 &&
          dv <= 65536;
 }
 
-// Numbers of scratch (32-bit, aligned to 16 bytes) that a call needs.
-B200_API int64_t b200_state_chunks_scratch(int rule, int tokens, int seqs, int heads, int dk, int dv) {
+// Numbers of scratch (32-bit, aligned to 16 bytes) that a call needs; 0: sizes the chunked form does not take.
+B200_API int64_t b200_state_chunks_scratch(int rule, int tokens, int seqs, int heads, int kv_heads, int dk, int dv) {
+  if (!sizes_taken(rule, heads, kv_heads, dk, dv)) return 0;
   Scratch scratch;
   return lay_out(rule, {tokens, seqs, 0, heads, dk, dv}, nullptr, &scratch);
 }
@@ -1163,7 +1164,7 @@ B200_API int b200_delta_chunks(const float* q, const float* k, const float* v, c
                                const int* seq_q_len, const int* seq_slot, int tokens, int seqs, int max_q_len, int heads, int kv_heads, int dk, int dv,
                                float* scratch, int64_t scratch_floats, float* state, float* out, cudaStream_t stream) {
   if (seqs == 0 || tokens == 0) return 0;
-  B200_REQUIRE(tokens > 0 && seqs > 0 && max_q_len > 0 && b200_state_chunks_supported(kDelta, heads, kv_heads, dk, dv), "delta_chunks: shape not taken");
+  B200_REQUIRE(tokens > 0 && seqs > 0 && max_q_len > 0 && sizes_taken(kDelta, heads, kv_heads, dk, dv), "delta_chunks: shape not taken");
   const Sizes z = {tokens, seqs, max_q_len, heads, dk, dv};
   const Requests req = {seq_q_start, seq_q_len, seq_slot};
   Scratch parts;
@@ -1189,7 +1190,7 @@ B200_API int b200_linear_chunks(const float* r, const float* k, const float* v, 
   if (seqs == 0 || tokens == 0) return 0;
   const int rule = u != nullptr ? kGeneralDelta : kLinear;
   B200_REQUIRE((u != nullptr) == (au != nullptr) && (u != nullptr) != (bonus != nullptr), "linear_chunks: either u and au or a bonus");
-  B200_REQUIRE(tokens > 0 && seqs > 0 && max_q_len > 0 && b200_state_chunks_supported(rule, heads, heads, dk, dv), "linear_chunks: shape not taken");
+  B200_REQUIRE(tokens > 0 && seqs > 0 && max_q_len > 0 && sizes_taken(rule, heads, heads, dk, dv), "linear_chunks: shape not taken");
   const Sizes z = {tokens, seqs, max_q_len, heads, dk, dv};
   const Requests req = {seq_q_start, seq_q_len, seq_slot};
   Scratch parts;
@@ -1212,7 +1213,7 @@ B200_API int b200_linear_chunks(const float* r, const float* k, const float* v, 
 extern "C" int b200_memory_chunks(const float* q, const float* k, const float* v, int64_t ld, const float* keep, const float* put, float scale, const int* seq_q_start,
                                   const int* seq_q_len, const int* seq_slot, int tokens, int seqs, int max_q_len, int heads, int dk, int dv, float* scratch,
                                   int64_t scratch_floats, float* S, float* n, float* num, float* den, cudaStream_t stream) {
-  B200_REQUIRE(tokens > 0 && seqs > 0 && max_q_len > 0 && b200_state_chunks_supported(kMemory, heads, heads, dk, dv), "memory_chunks: shape not taken");
+  B200_REQUIRE(tokens > 0 && seqs > 0 && max_q_len > 0 && sizes_taken(kMemory, heads, heads, dk, dv), "memory_chunks: shape not taken");
   const Sizes z = {tokens, seqs, max_q_len, heads, dk, dv};
   const Requests req = {seq_q_start, seq_q_len, seq_slot};
   Scratch parts;

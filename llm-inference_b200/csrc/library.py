@@ -175,9 +175,7 @@ class KernelLibrary:
         self.lib.b200_portion_attention_f32_supported.restype = c_int
         self.lib.b200_latent_prefill_supported.argtypes = [c_int] * 6
         self.lib.b200_latent_prefill_supported.restype = c_int
-        self.lib.b200_state_chunks_supported.argtypes = [c_int] * 5
-        self.lib.b200_state_chunks_supported.restype = c_int
-        self.lib.b200_state_chunks_scratch.argtypes = [c_int] * 6
+        self.lib.b200_state_chunks_scratch.argtypes = [c_int] * 7
         self.lib.b200_state_chunks_scratch.restype = c_int64
         self.lib.b200_delta_head_step_supported.argtypes = [c_int] * 4
         self.lib.b200_delta_head_step_supported.restype = c_int

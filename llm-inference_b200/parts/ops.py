@@ -946,20 +946,27 @@ def delta_prepare(
     ctx.lib.calls += 1  # the slot update is a launch of its own
 
 
-# Longest portion that is walked token by token. One request, 12 heads of 128 x 128 on a B200, chunks against tokens: 49 and 39 us at
-# 64 tokens, 53 and 52 us at 100, 64 and 87 us at 200, 252 and 731 us at 2,048 (one decay per head within 4 us of the same).
+# Longest portion that is walked token by token. The recurrences alone, one request, 12 heads of 128 x 128 on a B200, chunks against
+# tokens: 49 and 39 us at 64 tokens, 53 and 52 us at 100, 64 and 87 us at 200, 252 and 731 us at 2,048 (one decay per head within 4 us of
+# the same). A whole mixer called by itself, whose launches bound it at these sizes, with chunks and with tokens: one decay per channel 98
+# and 121 us at 116 tokens, one per head 81 and 75 at 116, 84 and 90 at 160.
 DELTA_CHUNK_FROM = 112
+HEAD_DELTA_CHUNK_FROM = 128
 
 
-# The same for the rules in which the values enter as they are, one request, 24 heads of 64 x 64. Without a removal: 39 us in chunks and
-# 33 token by token at 64 tokens, 38 and 43 at 100, 40 and 69 at 200, 101 and 564 at 2,048. Generalized delta rule: 51 and 39 us at 100
-# tokens, 61 and 62 at 200, 244 and 473 at 2,048.
+# The same for the rules in which the values enter as they are, one request, 24 heads of 64 x 64. Without a removal: 38 us in chunks and 43
+# token by token at 100 tokens, 40 and 69 at 200, 101 and 564 at 2,048; the whole mixer, which four launches instead of one bind: 120 and
+# 111 us at 128 tokens of 24 heads, 121 and 105 at 104 of 32, but 120 and 145 at 128 of 32, 120 and 169 at 144 of 24, 120 and 145 at 150
+# of 24 in two requests: the line lies at a number of (token, head) pairs, and for few heads where the chain alone is as long. Generalized delta rule: 61 and 62 us at 200 tokens, 244 and 473 at
+# 2,048; the whole mixer 104 and 91 at 200, 104 and 96 at 230.
 LINEAR_CHUNK_FROM = 80
-GENERAL_DELTA_CHUNK_FROM = 192
-# The matrix memory, one request, 12 heads of 128 x 128, with its gates and its output: 54 us in chunks and 42 token by token at 128
-# tokens, 55 and 53 at 160, 56 and 54 at 200 (the chunked form's four launches bound it up to there), 63 and 107 at 512, 219 and 579 at
-# 2,048.
-MEMORY_CHUNK_FROM = 200
+LINEAR_CHUNK_PAIRS = 3400
+LINEAR_CHUNK_ALWAYS_FROM = 141
+GENERAL_DELTA_CHUNK_FROM = 256
+# The matrix memory, one request, 12 heads of 128 x 128, with its gates and its output: 55 us in chunks and 53 token by token at 160
+# tokens, 56 and 54 at 200, 63 and 107 at 512, 219 and 579 at 2,048; the whole mixer 67 and 64 at 230 tokens of 12 heads, 79 and 84 at 300 in
+# two requests.
+MEMORY_CHUNK_FROM = 256
 # Scratch grows with the step's tokens (0.13 MB a token at 28 heads of 128 x 128): past this a step walks its portions token by token, as
 # if they were short, in the memory that takes.
 CHUNK_SCRATCH_BYTES = 2 << 30
@@ -972,12 +979,10 @@ def _chunk_scratch(ctx: StepContext, rule: int, longer_than: int, tokens: int, h
     ``CHUNK_SCRATCH_BYTES``. ``options["delta_portions"]``:
     ``"chunks"`` or ``"tokens"`` forces one of the two."""
     choice = ctx.options.get("delta_portions", "auto")
-    if choice == "tokens" or (choice == "auto" and not (
-        ctx.max_q_len > longer_than and ctx.lib.lib.b200_state_chunks_supported(rule, heads, kv_heads, dk, dv)
-    )):
+    if choice == "tokens" or (choice == "auto" and ctx.max_q_len <= longer_than):
         return None
-    floats = int(ctx.lib.lib.b200_state_chunks_scratch(rule, tokens, ctx.num_seqs, heads, dk, dv))
-    if choice == "auto" and 4 * floats > CHUNK_SCRATCH_BYTES:
+    floats = int(ctx.lib.lib.b200_state_chunks_scratch(rule, tokens, ctx.num_seqs, heads, kv_heads, dk, dv))
+    if choice == "auto" and not 0 < 4 * floats <= CHUNK_SCRATCH_BYTES:
         return None
     return ctx.buffer("state_chunks", (floats,), torch.float32, per_token=False)
 
@@ -987,7 +992,7 @@ def _delta_chunks(
     state: torch.Tensor, out: torch.Tensor, heads: int, kv_heads: int, dk: int, dv: int,
 ) -> bool:
     tokens = q.shape[0]
-    scratch = _chunk_scratch(ctx, _DELTA, DELTA_CHUNK_FROM, tokens, heads, kv_heads, dk, dv)
+    scratch = _chunk_scratch(ctx, _DELTA, HEAD_DELTA_CHUNK_FROM if per_head else DELTA_CHUNK_FROM, tokens, heads, kv_heads, dk, dv)
     if scratch is None:
         return False
     ctx.lib.call(
@@ -1004,7 +1009,9 @@ def _linear_chunks(
     bonus: torch.Tensor | None, state: torch.Tensor, out: torch.Tensor, heads: int, dk: int, dv: int,
 ) -> bool:
     tokens = r.shape[0]
-    rule, longer_than = (_LINEAR, LINEAR_CHUNK_FROM) if u is None else (_GENERAL_DELTA, GENERAL_DELTA_CHUNK_FROM)
+    rule, longer_than = _GENERAL_DELTA, GENERAL_DELTA_CHUNK_FROM
+    if u is None:
+        rule, longer_than = _LINEAR, LINEAR_CHUNK_FROM if tokens * heads > LINEAR_CHUNK_PAIRS else LINEAR_CHUNK_ALWAYS_FROM
     scratch = _chunk_scratch(ctx, rule, longer_than, tokens, heads, heads, dk, dv)
     if scratch is None:
         return False
@@ -1747,14 +1754,14 @@ def mlstm(ctx: StepContext, proj: torch.Tensor, columns: tuple[int, int, int, in
     _need(all(b.dtype == f32 and b.numel() == heads for b in (i_bias, f_bias)) and norm.dtype == f32 and norm.numel() == heads * dv, "mlstm: bad constants")
     _need(tuple(out.shape) == (tokens, heads * dv) and out.is_contiguous(), "mlstm: bad output")
     single = ctx.num_tokens == ctx.num_seqs
-    gates = [None] * 3 if single else [ctx.buffer("mlstm_" + name, (tokens, heads), f32) for name in ("keep", "put", "least")]
+    gates = None if single else ctx.buffer("mlstm_gates", (tokens, 3 * heads), f32).data_ptr()  # three arrays [tokens][heads]
     num, den = ctx.buffer("mlstm_num", (tokens, heads * dv), f32), ctx.buffer("mlstm_den", (tokens, heads), f32)
     scratch = None if single else _chunk_scratch(ctx, _MEMORY, MEMORY_CHUNK_FROM, tokens, heads, heads, dk, dv)
     ctx.lib.call(
         "b200_mlstm", ptr(proj), c_int(proj.shape[1]), *(c_int(c) for c in columns), ptr(i_bias), ptr(f_bias), c_float(cap), ptr(ctx.seq_q_start),
         ptr(ctx.seq_q_len), ptr(ctx.seq_slot), c_int(ctx.num_seqs), c_int(tokens), c_int(1 if single else 0), c_int(heads), c_int(dk), c_int(dv),
-        ptr(S), ptr(n), ptr(m), *(ptr(g) for g in gates), ptr(num), ptr(den), ptr(norm), c_float(eps), ptr(out), c_int(dtype_code(out.dtype)), c_int(ctx.max_q_len),
-        ptr(scratch), c_int64(scratch.numel() if scratch is not None else 0), ctx.stream,
+        ptr(S), ptr(n), ptr(m), *(gates and gates + 4 * i * tokens * heads for i in range(3)), ptr(num), ptr(den), ptr(norm), c_float(eps), ptr(out),
+        c_int(dtype_code(out.dtype)), c_int(ctx.max_q_len), ptr(scratch), c_int64(scratch.numel() if scratch is not None else 0), ctx.stream,
     )
     # The recurrence and the output kernel (and the gates'; in chunks three in the recurrence's place) are launches of their own.
     ctx.lib.calls += (1 if single else 2) + (2 if scratch is not None else 0)

@@ -216,7 +216,7 @@ def test_the_matrix_memory(heads, dk, dv, runs, portions):
 def test_portions_whose_scratch_would_be_too_large_go_token_by_token(monkeypatch):
     from llm_inference_b200.parts import ops
 
-    heads, dk, dv, n = 2, 64, 64, ops.LINEAR_CHUNK_FROM + 20
+    heads, dk, dv, n = 2, 64, 64, 160
     torch.manual_seed(3)
     r, k, w, v, bonus = (torch.rand(n, heads * width, device="cuda") for width in (dk, dk, dk, dv, 1))
 
