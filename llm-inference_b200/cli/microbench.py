@@ -28,6 +28,9 @@ class _Ctx(SimpleNamespace):
     def stream(self):
         return c_void_p(torch.cuda.current_stream().cuda_stream)
 
+    def portion_buffer(self, name, shape, dtype, limit):
+        return self.workspace.apart(name, shape, dtype, limit)
+
 
 def make_ctx(positions=None, token_seq=None, starts=None, runs=None, options=None):
     from ..csrc.library import kernels

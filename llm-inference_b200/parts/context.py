@@ -68,6 +68,7 @@ class Workspace:
     def __init__(self, device: torch.device, min_rows: int = 0) -> None:
         self.device = device
         self._flat: dict[str, torch.Tensor] = {}
+        self._apart: dict[str, torch.Tensor] = {}  # what no captured step uses, see `apart`
         # (name, dtype, shape) -> the view handed out last time; valid until a buffer moves.
         self._views: dict[tuple, torch.Tensor] = {}
         # Buffers whose first dimension counts tokens are sized for at least this many rows,
@@ -102,6 +103,23 @@ class Workspace:
         self._views[view_key] = view
         return view
 
+    def apart(self, name: str, shape: tuple[int, ...], dtype: torch.dtype, limit: int) -> torch.Tensor:
+        """A buffer that only steps use which are never captured: it may move without making captured addresses stale, so
+        ``generation`` stays. Its size goes with the lengths of requests, which grow from one portion of a prompt to the next:
+        it at least doubles (up to ``limit`` bytes, or what is asked for), and the old buffer is given up before the new one is
+        asked for. A view is good until the same name is asked for again."""
+        count = 1
+        for s in shape:
+            count *= int(s)
+        key = f"{name}:{dtype}"
+        flat = self._apart.get(key)
+        if flat is None or flat.numel() < count:
+            capacity = max(count, min(2 * flat.numel(), limit // dtype.itemsize) if flat is not None else 0, 1)
+            flat = None
+            self._apart.pop(key, None)
+            flat = self._apart[key] = torch.empty(capacity, dtype=dtype, device=self.device)
+        return flat[:count].view(shape)
+
     def zeros(self, name: str, count: int, dtype: torch.dtype) -> torch.Tensor:
         """A buffer that starts zeroed and whose users leave it zeroed (arrival counters)."""
         key = f"{name}:{dtype}:zeros"
@@ -113,7 +131,7 @@ class Workspace:
         return flat
 
     def bytes(self) -> int:
-        return sum(t.numel() * t.element_size() for t in self._flat.values())
+        return sum(t.numel() * t.element_size() for held in (self._flat, self._apart) for t in held.values())
 
 
 @dataclass
@@ -148,6 +166,13 @@ class StepContext:
         """Scratch for this step. ``per_token=False`` marks buffers whose row count is not
         the step's token count (logits of the wanted rows), which are sized as asked."""
         return self.workspace.get(name, shape, dtype or self.dtype, per_token=per_token)
+
+    def portion_buffer(self, name: str, shape: tuple[int, ...], dtype: torch.dtype, limit: int) -> torch.Tensor:
+        """Scratch of at most ``limit`` bytes that grows with prompt portions and the requests they belong to. Captured steps
+        reach it only where an option sends single tokens that way; theirs is a buffer of its own."""
+        if self.captured:
+            return self.buffer(name, shape, dtype, per_token=False)
+        return self.workspace.apart(name, shape, dtype, limit)
 
     @property
     def stream(self):

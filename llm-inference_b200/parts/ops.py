@@ -901,12 +901,12 @@ def latent_portions(
     _need(tuple(out.shape) == (ctx.num_tokens, heads * dim) and out.is_contiguous() and out.dtype == torch.bfloat16, "latent_portions: bad output")
     _need(gate is None or (gate.stride(1) == 1 and gate.dtype == torch.bfloat16), "latent_portions: bad gate")
     _need(sink is None or (sink.dtype == torch.float32 and sink.numel() == heads), "latent_portions: the sink is float32 [heads]")
-    latents = ctx.buffer("latent_rows", (key_rows, row_dim), torch.bfloat16, per_token=False)
+    latents = ctx.portion_buffer("latent_rows", (key_rows, row_dim), torch.bfloat16, LATENT_EXPAND_BYTES)
     ctx.lib.call(
         "b200_latent_gather", ptr(cache.keys), ptr(cache.block_table), ptr(ctx.seq_kv_len), c_int(first), c_int(ctx.num_seqs - first), c_int(ctx.max_kv_len),
         c_int(cache.max_pages), c_int(cache.num_pages), c_int(cache.page_size), c_int(row_dim), ptr(latents), ptr(ctx.err), ctx.stream,
     )
-    expanded = ctx.buffer("latent_expanded", (key_rows, w_expand.shape[0]), torch.bfloat16, per_token=False)
+    expanded = ctx.portion_buffer("latent_expanded", (key_rows, w_expand.shape[0]), torch.bfloat16, LATENT_EXPAND_BYTES)
     torch.mm(latents[:, :rank], w_expand.t(), out=expanded)
     ctx.lib.call(
         "b200_latent_prefill_tcgen05", ptr(queries), c_int64(queries.stride(0)), c_int(dim + rot_dim), ptr(q_rot if rot_dim else None), ptr(expanded), ptr(latents),
@@ -984,7 +984,7 @@ def _chunk_scratch(ctx: StepContext, rule: int, longer_than: int, tokens: int, h
     floats = int(ctx.lib.lib.b200_state_chunks_scratch(rule, tokens, ctx.num_seqs, heads, kv_heads, dk, dv))
     if choice == "auto" and not 0 < 4 * floats <= CHUNK_SCRATCH_BYTES:
         return None
-    return ctx.buffer("state_chunks", (floats,), torch.float32, per_token=False)
+    return ctx.portion_buffer("state_chunks", (floats,), torch.float32, CHUNK_SCRATCH_BYTES)
 
 
 def _delta_chunks(
