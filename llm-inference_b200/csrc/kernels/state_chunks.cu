@@ -29,6 +29,8 @@
 // by token -> 252 us (prepare 60, walk 130, out 60), 28 heads: 941 -> 449; one decay per head (before: outputs and triangular products
 // inside the walk): 305 -> 252 and 525 -> 450. 24 heads of 64 x 64: the generalized rule 473 -> 244 us (prepare 100, walk 90, out 35), the
 // rule without a removal 564 -> 101 us (prepare 51, scan 16, out 27).
+#include <type_traits>
+
 #include "common.cuh"
 
 namespace {
@@ -1000,22 +1002,31 @@ chunk_out_kernel(const int* __restrict__ seq_q_start, const int* __restrict__ se
     float sum[8][4];  // one slab's sum by itself: fewer roundings of the whole
 #pragma unroll
     for (int i = 0; i < 8; ++i) sum[i][0] = sum[i][1] = sum[i][2] = sum[i][3] = 0.f;
+    // Pairs of tokens form a triangle: a token leaves out those behind it (a value there that is not finite times a pair's zero is
+    // not zero). Tokens 4 i .. + 3 of a warp stand against tokens k .. k + 3, so only one group of four looks at its lanes.
+    auto multiply = [&](auto triangle) {
+      constexpr bool kTriangle = decltype(triangle)::value;
 #pragma unroll 2
-    for (int k = 0; k < C; k += 4) {
-      float4 b[4];
+      for (int k = 0; k < C; k += 4) {
+        float4 b[4];
 #pragma unroll
-      for (int x = 0; x < 4; ++x) b[x] = *reinterpret_cast<const float4*>(right + (k + x) * kLdOut);
+        for (int x = 0; x < 4; ++x) b[x] = *reinterpret_cast<const float4*>(right + (k + x) * kLdOut);
 #pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        const float4 a = *reinterpret_cast<const float4*>(left + i * 4 * kLdSlab + k);
-        const float f[4] = {a.x, a.y, a.z, a.w};
+        for (int i = 0; i < 8; ++i) {
+          if (kTriangle && k > 4 * i) continue;
+          const float4 a = *reinterpret_cast<const float4*>(left + i * 4 * kLdSlab + k);
+          const float f[4] = {a.x, a.y, a.z, a.w};
 #pragma unroll
-        for (int x = 0; x < 4; ++x) {
-          sum[i][0] = fmaf(f[x], b[x].x, sum[i][0]), sum[i][1] = fmaf(f[x], b[x].y, sum[i][1]);
-          sum[i][2] = fmaf(f[x], b[x].z, sum[i][2]), sum[i][3] = fmaf(f[x], b[x].w, sum[i][3]);
+          for (int x = 0; x < 4; ++x) {
+            if (kTriangle && k == 4 * i && x > it) continue;
+            sum[i][0] = fmaf(f[x], b[x].x, sum[i][0]), sum[i][1] = fmaf(f[x], b[x].y, sum[i][1]);
+            sum[i][2] = fmaf(f[x], b[x].z, sum[i][2]), sum[i][3] = fmaf(f[x], b[x].w, sum[i][3]);
+          }
         }
       }
-    }
+    };
+    if (slab < state_slabs) multiply(std::false_type{});
+    else multiply(std::true_type{});
 #pragma unroll
     for (int i = 0; i < 8; ++i) acc[i][0] += sum[i][0], acc[i][1] += sum[i][1], acc[i][2] += sum[i][2], acc[i][3] += sum[i][3];
     __syncthreads();
