@@ -237,10 +237,12 @@ B200_API int b200_portion_attention_f32(const float* q, const float* k_arena, co
                         first_seq, max_pages, num_pages, q_heads, kv_heads, head_dim, page_size, window, scale};
   const bool narrow = head_dim <= 64;
   auto kernel = narrow ? portion_attention_f32_kernel<64> : portion_attention_f32_kernel<128>;
-  static const bool raised =
-      cudaFuncSetAttribute(portion_attention_f32_kernel<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(portion_smem(64))) == cudaSuccess &&
-      cudaFuncSetAttribute(portion_attention_f32_kernel<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(portion_smem(128))) == cudaSuccess;
-  B200_REQUIRE(raised, "portion_attention_f32: cannot size shared memory");
+  static OncePerDevice raised;
+  const auto raise = [] {
+    return cudaFuncSetAttribute(portion_attention_f32_kernel<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(portion_smem(64))) == cudaSuccess &&
+           cudaFuncSetAttribute(portion_attention_f32_kernel<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(portion_smem(128))) == cudaSuccess;
+  };
+  B200_REQUIRE(raised(raise), "portion_attention_f32: cannot size shared memory");
   const int64_t rows = static_cast<int64_t>(max_q_len) * (q_heads / kv_heads);
   const dim3 grid(static_cast<unsigned>((rows + kRows - 1) / kRows), kv_heads, num_seqs);
   kernel<<<grid, kThreads, portion_smem(narrow ? 64 : 128), stream>>>(p);

@@ -1002,10 +1002,12 @@ B200_API int b200_latent_prefill_tcgen05(const void* q, int64_t q_ld, int q_head
   if (matrix_map(&latent_map, latents, key_rows, rank + rot_dim) != 0) return -1;
   auto with_rot = flash_prefill_tcgen05_kernel<false, false, false, false, kDim + 64>;
   auto plain = flash_prefill_tcgen05_kernel<false, false, false, false, kDim>;
-  static const bool raised =
-      cudaFuncSetAttribute(with_rot, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(latent_smem<kDim + 64>())) == cudaSuccess &&
-      cudaFuncSetAttribute(plain, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(latent_smem<kDim>())) == cudaSuccess;
-  B200_REQUIRE(raised, "latent_prefill_tcgen05: cannot size shared memory");
+  static OncePerDevice raised;
+  const auto raise = [&] {
+    return cudaFuncSetAttribute(with_rot, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(latent_smem<kDim + 64>())) == cudaSuccess &&
+           cudaFuncSetAttribute(plain, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(latent_smem<kDim>())) == cudaSuccess;
+  };
+  B200_REQUIRE(raised(raise), "latent_prefill_tcgen05: cannot size shared memory");
   const dim3 grid((max_q_len + kRows - 1) / kRows, heads, num_seqs);
   const cudaError_t status = rot_dim ? launch_kernel(with_rot, grid, dim3(kThreadsA), latent_smem<kDim + 64>(), stream, expanded_map, latent_map, p)
                                      : launch_kernel(plain, grid, dim3(kThreadsA), latent_smem<kDim>(), stream, expanded_map, latent_map, p);

@@ -9,6 +9,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <atomic>
 #include <cstdarg>
 #include <cstdio>
 
@@ -130,6 +131,31 @@ __device__ __forceinline__ float fold_rstd(const NormFold& fold, int m) {
   for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
   return rsqrtf(sum / static_cast<float>(fold.width) + fold.eps);
 }
+
+// What a device has to be told once (a kernel's limit of dynamic shared memory belongs to the device that is current when it is
+// raised): `action` runs until it has succeeded on the current device, and is not run there again. A failure is not kept.
+constexpr int kMaxDevices = 64;
+class OncePerDevice {
+ public:
+  template <typename Action>
+  bool operator()(Action action) {
+    int device = 0;
+    if (cudaGetDevice(&device) != cudaSuccess || device < 0 || device >= kMaxDevices) {
+      cudaGetLastError();
+      return false;
+    }
+    if (done_[device].load(std::memory_order_acquire)) return true;
+    if (!action()) {
+      cudaGetLastError();
+      return false;
+    }
+    done_[device].store(true, std::memory_order_release);
+    return true;
+  }
+
+ private:
+  std::atomic<bool> done_[kMaxDevices] = {};
+};
 
 bool b200_overlap_enabled();
 int b200_sm_count_host();  // SMs of the current device (cached)

@@ -122,10 +122,12 @@ struct Product {
 template <int BM, int BN, int TM, int TN>
 int launch_tiles(const Product& p, bool wide, cudaStream_t stream) {
   constexpr size_t smem = tile_smem<BM, BN>();
-  static const bool raised =
-      cudaFuncSetAttribute(gemm_f32_kernel<BM, BN, TM, TN, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)) == cudaSuccess &&
-      cudaFuncSetAttribute(gemm_f32_kernel<BM, BN, TM, TN, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)) == cudaSuccess;
-  if (!raised) return b200_fail("gemm_f32: cannot size shared memory");
+  static OncePerDevice raised;
+  if (!raised([] {
+        return cudaFuncSetAttribute(gemm_f32_kernel<BM, BN, TM, TN, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)) == cudaSuccess &&
+               cudaFuncSetAttribute(gemm_f32_kernel<BM, BN, TM, TN, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)) == cudaSuccess;
+      }))
+    return b200_fail("gemm_f32: cannot size shared memory");
   const dim3 grid((p.N + BN - 1) / BN, (p.M + BM - 1) / BM, p.batch);
   B200_REQUIRE(grid.y <= 65535, "gemm_f32: too many rows (%d)", p.M);
   auto kernel = wide ? gemm_f32_kernel<BM, BN, TM, TN, 4> : gemm_f32_kernel<BM, BN, TM, TN, 1>;

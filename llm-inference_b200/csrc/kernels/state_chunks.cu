@@ -1093,8 +1093,8 @@ bool raise_prepares() {
 }
 
 bool raise_all() {
-  static const bool raised = raise_prepares<64>() && raise_prepares<128>() && raise_prepares<256>();
-  return raised;
+  static OncePerDevice raised;
+  return raised([] { return raise_prepares<64>() && raise_prepares<128>() && raise_prepares<256>(); });
 }
 
 template <int ROWS>

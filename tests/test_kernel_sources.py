@@ -76,3 +76,37 @@ def test_the_rule_reads_a_kernel_as_intended():
     assert name == "demo_kernel" and "wait_for_predecessor" in body
     restricted = [p.split()[-1] for p in params.split(",") if "__restrict__" in p]
     assert restricted == ["weight", "x"] and "x" not in BEFORE_THE_CHAIN
+
+
+def test_limits_of_shared_memory_are_raised_on_every_device():
+    """A flag that a process sets once leaves its second device with the first limit, and keeps a failure for good."""
+    for path in sorted(KERNELS.glob("*.cu")):
+        text = re.sub(r"//[^\n]*", "", path.read_text())
+        assert not re.search(r"static\s+const\s+bool\s+\w+\s*=", text), path.name
+
+
+def test_what_is_done_once_per_device(tmp_path):
+    """The class behind those limits, against a device number and an action that the test sets."""
+    import shutil
+    import subprocess
+
+    import pytest
+
+    compiler = shutil.which("g++")
+    if compiler is None:
+        pytest.skip("no C++ compiler")
+    found = re.search(r"constexpr int kMaxDevices = \d+;\nclass OncePerDevice \{.*?\n\};", (KERNELS / "common.cuh").read_text(), re.S)
+    (tmp_path / "once.cpp").write_text(
+        "#include <atomic>\n#include <cassert>\n"
+        "enum { cudaSuccess = 0 };\nstatic int current = 0, refused = 0;\n"
+        "static int cudaGetDevice(int* d) { *d = current; return refused; }\nstatic int cudaGetLastError() { return 0; }\n"
+        + found.group(0) + "\n"
+        "int main() {\n  OncePerDevice once;\n  int runs = 0, works = 0;\n  auto action = [&] { ++runs; return works != 0; };\n"
+        "  assert(!once(action) && !once(action) && runs == 2);  // a failure is not kept\n"
+        "  works = 1;\n  assert(once(action) && once(action) && runs == 3);\n"
+        "  current = 1;\n  assert(once(action) && once(action) && runs == 4);\n"
+        "  current = kMaxDevices;\n  assert(!once(action) && runs == 4);\n"
+        "  current = 0, refused = 1;\n  assert(!once(action) && runs == 4);\n  return 0;\n}\n"
+    )
+    subprocess.run([compiler, "-std=c++17", "-o", str(tmp_path / "once"), str(tmp_path / "once.cpp")], check=True)
+    subprocess.run([str(tmp_path / "once")], check=True)
