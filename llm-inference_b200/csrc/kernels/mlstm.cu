@@ -325,11 +325,11 @@ __global__ void mlstm_output_kernel(const MemoryParams p, const float* __restric
 
 // The whole of the mixer between its two products. `proj` (float, rows `ld` apart) holds q, k (heads * dk each), v and the
 // gate logits (heads * dv each) and the two gates' logits (heads each) from the columns given. `single`: every request of the
-// step feeds one token (two launches instead of three). With `scratch` (b200_state_chunks_scratch, rule 3) portions run in
-// chunks. `norm`: [heads * dv]; `out`: [tokens][heads * dv].
+// step feeds one token (two launches instead of three). With `scratch` (b200_state_chunks_scratch, rule 3) the requests behind the first
+// `walked` ones run in chunks; without, `walked` is all of them. `norm`: [heads * dv]; `out`: [tokens][heads * dv].
 B200_API int b200_mlstm(const float* proj, int ld, int q_at, int k_at, int v_at, int g_at, int i_at, int f_at, const float* i_bias,
                         const float* f_bias, float cap, const int* seq_q_start, const int* seq_q_len, const int* seq_slot, int seqs,
-                        int tokens, int single, int heads, int dk, int dv, float* S, float* n, float* m, float* keep, float* put,
+                        int walked, int tokens, int single, int heads, int dk, int dv, float* S, float* n, float* m, float* keep, float* put,
                         float* least, float* num, float* den, const float* norm, float eps, void* out, int dtype, int max_q_len, float* scratch,
                         int64_t scratch_floats, cudaStream_t stream) {
   if (tokens == 0 || seqs == 0) return 0;
@@ -343,10 +343,10 @@ B200_API int b200_mlstm(const float* proj, int ld, int q_at, int k_at, int v_at,
     launch_kernel(mlstm_gates_kernel, dim3(seqs, heads), dim3(kScanThreads), 0, stream, p);
     if (int status = b200_check_launch("mlstm_gates")) return status;
   }
-  const bool chunks = !single && scratch != nullptr;
-  if (chunks) {
-    if (int status = b200_memory_chunks(proj + q_at, proj + k_at, proj + v_at, ld, keep, put, 1.f / sqrtf(static_cast<float>(dk)), seq_q_start, seq_q_len, seq_slot,
-                                        tokens, seqs, max_q_len, heads, dk, dv, scratch, scratch_floats, S, n, num, den, stream))
+  B200_REQUIRE(walked >= 0 && walked <= seqs && (single || scratch != nullptr || walked == seqs), "mlstm: %d of %d requests walked", walked, seqs);
+  if (walked < seqs && !single) {
+    if (int status = b200_memory_chunks(proj + q_at, proj + k_at, proj + v_at, ld, keep, put, 1.f / sqrtf(static_cast<float>(dk)), seq_q_start + walked, seq_q_len + walked,
+                                        seq_slot + walked, tokens, seqs - walked, max_q_len, heads, dk, dv, scratch, scratch_floats, S, n, num, den, stream))
       return status;
   }
   int lanes = 1;
@@ -354,7 +354,7 @@ B200_API int b200_mlstm(const float* proj, int ld, int q_at, int k_at, int v_at,
   const int rows = (dk + lanes - 1) / lanes;
   const int per = rows <= 8 ? 8 : (rows <= 16 ? 16 : 32);
   const int cols = kRecurrenceThreads / lanes;
-  const dim3 grid(seqs, heads, (dv + 1 + cols - 1) / cols);
+  const dim3 grid(single ? seqs : walked, heads, (dv + 1 + cols - 1) / cols);
   B200_REQUIRE(grid.z <= 65535, "mlstm: too many columns");
   const size_t smem = single ? 0 : sizeof(float) * 2 * (kStage * (2 * per * lanes + cols) + 2 * kStage);
   B200_REQUIRE(smem <= 200 * 1024, "mlstm: the staged tokens do not fit shared memory");
@@ -376,7 +376,7 @@ B200_API int b200_mlstm(const float* proj, int ld, int q_at, int k_at, int v_at,
     else launch(mlstm_recurrence_kernel<8, 1, kSingle>);
   };
   if (single) by_shape(std::true_type{});
-  else if (!chunks) by_shape(std::false_type{});
+  else if (walked > 0) by_shape(std::false_type{});
   if (int status = b200_check_launch("mlstm_recurrence")) return status;
   const int threads = 128;
   const unsigned blocks = static_cast<unsigned>((static_cast<int64_t>(tokens) * heads + 3) / 4);

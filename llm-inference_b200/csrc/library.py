@@ -121,7 +121,7 @@ _SIGNATURES: dict[str, list] = {
     "b200_sandwich_norm": [c_void_p] * 3 + [c_float, c_float, c_void_p, c_void_p, c_float, c_float, c_void_p, c_float, c_void_p, c_int, c_int,
                            c_void_p, c_int] + [c_void_p] * 7 + [c_int, c_void_p],
     "b200_shift_norm": [c_void_p] * 10 + [c_int, c_int, c_void_p, c_int, c_void_p],
-    "b200_mlstm": [c_void_p] + [c_int] * 7 + [c_void_p, c_void_p, c_float] + [c_void_p] * 3 + [c_int] * 6 + [c_void_p] * 9
+    "b200_mlstm": [c_void_p] + [c_int] * 7 + [c_void_p, c_void_p, c_float] + [c_void_p] * 3 + [c_int] * 7 + [c_void_p] * 9
                   + [c_float, c_void_p, c_int, c_int, c_void_p, c_int64, c_void_p],
     "b200_clamped_glu": [c_void_p, c_int, c_int, c_float, c_void_p, c_int, c_void_p],
     "b200_mingru": [c_void_p, c_int] + [c_void_p] * 4 + [c_int] * 4 + [c_void_p] * 3 + [c_int, c_void_p],

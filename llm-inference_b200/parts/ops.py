@@ -949,7 +949,10 @@ def delta_prepare(
 # Longest portion that is walked token by token. The recurrences alone, one request, 12 heads of 128 x 128 on a B200, chunks against
 # tokens: 49 and 39 us at 64 tokens, 53 and 52 us at 100, 64 and 87 us at 200, 252 and 731 us at 2,048 (one decay per head within 4 us of
 # the same). A whole mixer called by itself, whose launches bound it at these sizes, with chunks and with tokens: one decay per channel 98
-# and 121 us at 116 tokens, one per head 81 and 75 at 116, 84 and 90 at 160.
+# and 121 us at 116 tokens, one per head 81 and 75 at 116, 84 and 90 at 160. Beside decoded tokens, which are walked either way, the lines
+# lie at the same lengths: with 63 of them chunks and tokens take 161 and 158 us at 100 tokens and 162 and 174 at 128 (one decay per
+# channel), 147 and 152 at 128 and 157 and 167 at 160 (one per head). Decoded tokens inside the chunks' grids cost more than the
+# portion: 200 of them beside 512 tokens 732 us a layer, walked in front of the chunks 370, all token by token 543.
 DELTA_CHUNK_FROM = 112
 HEAD_DELTA_CHUNK_FROM = 128
 
@@ -973,70 +976,80 @@ CHUNK_SCRATCH_BYTES = 2 << 30
 _DELTA, _GENERAL_DELTA, _LINEAR, _MEMORY = 0, 1, 2, 3  # csrc/kernels/state_chunks.cu
 
 
-def _chunk_scratch(ctx: StepContext, rule: int, longer_than: int, tokens: int, heads: int, kv_heads: int, dk: int, dv: int) -> torch.Tensor | None:
+def _chunk_scratch(ctx: StepContext, rule: int, longer_than: int, tokens: int, heads: int, kv_heads: int, dk: int, dv: int) -> tuple[torch.Tensor | None, int]:
     """Scratch for a recurrence that runs chunk by chunk (csrc/kernels/state_chunks.cu), or None where it runs token by token:
     portions of at most ``longer_than`` tokens, sizes the chunked form does not take and steps whose scratch would pass
     ``CHUNK_SCRATCH_BYTES``. ``options["delta_portions"]``:
-    ``"chunks"`` or ``"tokens"`` forces one of the two."""
+    ``"chunks"`` or ``"tokens"`` forces one of the two for prompt portions. And the number of requests that are walked token by token:
+    with chunks the single tokens that lead the batch (a step of single tokens only goes the forced way as a whole)."""
     choice = ctx.options.get("delta_portions", "auto")
     if choice == "tokens" or (choice == "auto" and ctx.max_q_len <= longer_than):
-        return None
-    floats = int(ctx.lib.lib.b200_state_chunks_scratch(rule, tokens, ctx.num_seqs, heads, kv_heads, dk, dv))
+        return None, ctx.num_seqs
+    walked = ctx.num_decode_seqs if ctx.num_decode_seqs < ctx.num_seqs else 0
+    floats = int(ctx.lib.lib.b200_state_chunks_scratch(rule, tokens, ctx.num_seqs - walked, heads, kv_heads, dk, dv))
     if choice == "auto" and not 0 < 4 * floats <= CHUNK_SCRATCH_BYTES:
-        return None
-    return ctx.portion_buffer("state_chunks", (floats,), torch.float32, CHUNK_SCRATCH_BYTES)
+        return None, ctx.num_seqs
+    return ctx.portion_buffer("state_chunks", (floats,), torch.float32, CHUNK_SCRATCH_BYTES), walked
+
+
+def _portion_arguments(ctx: StepContext, walked: int) -> tuple:
+    """The metadata of the requests behind the first ``walked`` ones, as the chunked entry points take it."""
+    return tuple(_offset(array, 4 * walked) for array in (ctx.seq_q_start, ctx.seq_q_len, ctx.seq_slot))
 
 
 def _delta_chunks(
     ctx: StepContext, q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, beta: torch.Tensor, decay: torch.Tensor, per_head: bool,
     state: torch.Tensor, out: torch.Tensor, heads: int, kv_heads: int, dk: int, dv: int,
-) -> bool:
+) -> int:
+    """Runs the step's portions in chunks where that is the way; returns how many leading requests are left to be walked token by token."""
     tokens = q.shape[0]
-    scratch = _chunk_scratch(ctx, _DELTA, HEAD_DELTA_CHUNK_FROM if per_head else DELTA_CHUNK_FROM, tokens, heads, kv_heads, dk, dv)
+    scratch, walked = _chunk_scratch(ctx, _DELTA, HEAD_DELTA_CHUNK_FROM if per_head else DELTA_CHUNK_FROM, tokens, heads, kv_heads, dk, dv)
     if scratch is None:
-        return False
+        return walked
     ctx.lib.call(
-        "b200_delta_chunks", ptr(q), ptr(k), ptr(v), ptr(beta), ptr(decay), c_int(1 if per_head else 0), ptr(ctx.seq_q_start), ptr(ctx.seq_q_len),
-        ptr(ctx.seq_slot), c_int(tokens), c_int(ctx.num_seqs), c_int(ctx.max_q_len), c_int(heads), c_int(kv_heads), c_int(dk), c_int(dv),
+        "b200_delta_chunks", ptr(q), ptr(k), ptr(v), ptr(beta), ptr(decay), c_int(1 if per_head else 0), *_portion_arguments(ctx, walked),
+        c_int(tokens), c_int(ctx.num_seqs - walked), c_int(ctx.max_q_len), c_int(heads), c_int(kv_heads), c_int(dk), c_int(dv),
         ptr(scratch), c_int64(scratch.numel()), ptr(state), ptr(out), ctx.stream,
     )
     ctx.lib.calls += 2  # further kernels of the call
-    return True
+    return walked
 
 
 def _linear_chunks(
     ctx: StepContext, r: torch.Tensor, k: torch.Tensor, v: torch.Tensor, w: torch.Tensor, au: torch.Tensor | None, u: torch.Tensor | None,
     bonus: torch.Tensor | None, state: torch.Tensor, out: torch.Tensor, heads: int, dk: int, dv: int,
-) -> bool:
+) -> int:
+    """As :func:`_delta_chunks`, for the rules in which the values enter as they are."""
     tokens = r.shape[0]
     rule, longer_than = _GENERAL_DELTA, GENERAL_DELTA_CHUNK_FROM
     if u is None:
         rule, longer_than = _LINEAR, LINEAR_CHUNK_FROM if tokens * heads > LINEAR_CHUNK_PAIRS else LINEAR_CHUNK_ALWAYS_FROM
-    scratch = _chunk_scratch(ctx, rule, longer_than, tokens, heads, heads, dk, dv)
+    scratch, walked = _chunk_scratch(ctx, rule, longer_than, tokens, heads, heads, dk, dv)
     if scratch is None:
-        return False
+        return walked
     ctx.lib.call(
-        "b200_linear_chunks", ptr(r), ptr(k), ptr(v), ptr(w), ptr(au), ptr(u), ptr(bonus), ptr(ctx.seq_q_start), ptr(ctx.seq_q_len),
-        ptr(ctx.seq_slot), c_int(tokens), c_int(ctx.num_seqs), c_int(ctx.max_q_len), c_int(heads), c_int(dk), c_int(dv),
+        "b200_linear_chunks", ptr(r), ptr(k), ptr(v), ptr(w), ptr(au), ptr(u), ptr(bonus), *_portion_arguments(ctx, walked),
+        c_int(tokens), c_int(ctx.num_seqs - walked), c_int(ctx.max_q_len), c_int(heads), c_int(dk), c_int(dv),
         ptr(scratch), c_int64(scratch.numel()), ptr(state), ptr(out), ctx.stream,
     )
     ctx.lib.calls += 3 if u is None else 2  # further kernels of the call
-    return True
+    return walked
 
 
 def delta_recurrence(
     ctx: StepContext, q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, beta: torch.Tensor, decay: torch.Tensor,
     state: torch.Tensor, out: torch.Tensor, heads: int, kv_heads: int, dk: int, dv: int,
 ) -> torch.Tensor:
-    """The delta rule with a decay per head and key channel over every request's new tokens: chunk by chunk or token by token
-    (see ``_chunk_scratch``)."""
+    """The delta rule with a decay per head and key channel over every request's new tokens: portions chunk by chunk or token by
+    token (see ``_chunk_scratch``), single tokens in front of them always the latter."""
     _need(state.dtype == torch.float32 and tuple(state.shape[1:]) == (heads, dk, dv) and state.is_contiguous(), "delta_recurrence: the state is float32 [slots, heads, dk, dv]")
     _need(out.dtype == torch.float32 and tuple(out.shape) == (q.shape[0], heads * dv) and out.is_contiguous(), "delta_recurrence: bad output")
-    if _delta_chunks(ctx, q, k, v, beta, decay, False, state, out, heads, kv_heads, dk, dv):
+    walked = _delta_chunks(ctx, q, k, v, beta, decay, False, state, out, heads, kv_heads, dk, dv)
+    if not walked:
         return out
     ctx.lib.call(
         "b200_delta_recurrence", ptr(q), ptr(k), ptr(v), ptr(beta), ptr(decay), ptr(ctx.seq_q_start), ptr(ctx.seq_q_len),
-        ptr(ctx.seq_slot), c_int(ctx.num_seqs), c_int(heads), c_int(kv_heads), c_int(dk), c_int(dv), ptr(state), ptr(out),
+        ptr(ctx.seq_slot), c_int(walked), c_int(heads), c_int(kv_heads), c_int(dk), c_int(dv), ptr(state), ptr(out),
         ctx.stream,
     )
     return out
@@ -1068,11 +1081,12 @@ def delta_head_recurrence(
     _need(state.dtype == torch.float32 and tuple(state.shape[1:]) == (heads, dk, dv) and state.is_contiguous(), "delta_head_recurrence: the state is float32 [slots, heads, dk, dv]")
     for tensor, width in ((q, kv_heads * dk), (k, kv_heads * dk), (v, heads * dv), (beta, heads), (log_decay, heads), (kq, kv_heads), (out, heads * dv)):
         _need(tensor.dtype == torch.float32 and tuple(tensor.shape) == (tokens, width) and tensor.is_contiguous(), "delta_head_recurrence: bad operands")
-    if _delta_chunks(ctx, q, k, v, beta, log_decay, True, state, out, heads, kv_heads, dk, dv):
+    walked = _delta_chunks(ctx, q, k, v, beta, log_decay, True, state, out, heads, kv_heads, dk, dv)
+    if not walked:
         return out
     ctx.lib.call(
         "b200_delta_head_recurrence", ptr(q), ptr(k), ptr(v), ptr(beta), ptr(log_decay), ptr(kq), ptr(ctx.seq_q_start), ptr(ctx.seq_q_len),
-        ptr(ctx.seq_slot), c_int(ctx.num_seqs), c_int(ctx.max_q_len), c_int(heads), c_int(kv_heads), c_int(dk), c_int(dv), ptr(state), ptr(out), ctx.stream,
+        ptr(ctx.seq_slot), c_int(walked), c_int(ctx.max_q_len if walked == ctx.num_seqs else 1), c_int(heads), c_int(kv_heads), c_int(dk), c_int(dv), ptr(state), ptr(out), ctx.stream,
     )
     return out
 
@@ -1213,11 +1227,12 @@ def wkv_recurrence(
 ) -> torch.Tensor:
     _need(state.dtype == torch.float32 and tuple(state.shape[1:]) == (heads, dk, dv) and state.is_contiguous(), "wkv_recurrence: the state is float32 [slots, heads, dk, dv]")
     _need(out.dtype == torch.float32 and tuple(out.shape) == (r.shape[0], heads * dv) and out.is_contiguous(), "wkv_recurrence: bad output")
-    if _linear_chunks(ctx, r, k, v, decay, None, None, bonus, state, out, heads, dk, dv):
+    walked = _linear_chunks(ctx, r, k, v, decay, None, None, bonus, state, out, heads, dk, dv)
+    if not walked:
         return out
     ctx.lib.call(
         "b200_wkv_recurrence", ptr(r), ptr(k), ptr(v), ptr(bonus), ptr(decay), ptr(ctx.seq_q_start), ptr(ctx.seq_q_len), ptr(ctx.seq_slot),
-        c_int(ctx.num_seqs), c_int(heads), c_int(dk), c_int(dv), ptr(state), ptr(out), ctx.stream,
+        c_int(walked), c_int(heads), c_int(dk), c_int(dv), ptr(state), ptr(out), ctx.stream,
     )
     return out
 
@@ -1473,11 +1488,12 @@ def delta_general_recurrence(
     """``S <- diag(w) S - au (u^T S) + k v^T``, ``o = S^T r`` per head and token, each request from its slot of ``state``."""
     _need(state.dtype == torch.float32 and tuple(state.shape[1:]) == (heads, dk, dv) and state.is_contiguous(), "delta_general_recurrence: the state is float32 [slots, heads, dk, dv]")
     _need(out.dtype == torch.float32 and tuple(out.shape) == (r.shape[0], heads * dv) and out.is_contiguous(), "delta_general_recurrence: bad output")
-    if _linear_chunks(ctx, r, k, v, w, au, u, None, state, out, heads, dk, dv):
+    walked = _linear_chunks(ctx, r, k, v, w, au, u, None, state, out, heads, dk, dv)
+    if not walked:
         return out
     ctx.lib.call(
         "b200_delta_general_recurrence", ptr(r), ptr(k), ptr(v), ptr(w), ptr(au), ptr(u), ptr(ctx.seq_q_start), ptr(ctx.seq_q_len),
-        ptr(ctx.seq_slot), c_int(ctx.num_seqs), c_int(max(ctx.max_q_len, 1)), c_int(heads), c_int(dk), c_int(dv), ptr(state), ptr(out), ctx.stream,
+        ptr(ctx.seq_slot), c_int(walked), c_int(max(ctx.max_q_len, 1) if walked == ctx.num_seqs else 1), c_int(heads), c_int(dk), c_int(dv), ptr(state), ptr(out), ctx.stream,
     )
     return out
 
@@ -1756,15 +1772,15 @@ def mlstm(ctx: StepContext, proj: torch.Tensor, columns: tuple[int, int, int, in
     single = ctx.num_tokens == ctx.num_seqs
     gates = None if single else ctx.buffer("mlstm_gates", (tokens, 3 * heads), f32).data_ptr()  # three arrays [tokens][heads]
     num, den = ctx.buffer("mlstm_num", (tokens, heads * dv), f32), ctx.buffer("mlstm_den", (tokens, heads), f32)
-    scratch = None if single else _chunk_scratch(ctx, _MEMORY, MEMORY_CHUNK_FROM, tokens, heads, heads, dk, dv)
+    scratch, walked = (None, ctx.num_seqs) if single else _chunk_scratch(ctx, _MEMORY, MEMORY_CHUNK_FROM, tokens, heads, heads, dk, dv)
     ctx.lib.call(
         "b200_mlstm", ptr(proj), c_int(proj.shape[1]), *(c_int(c) for c in columns), ptr(i_bias), ptr(f_bias), c_float(cap), ptr(ctx.seq_q_start),
-        ptr(ctx.seq_q_len), ptr(ctx.seq_slot), c_int(ctx.num_seqs), c_int(tokens), c_int(1 if single else 0), c_int(heads), c_int(dk), c_int(dv),
+        ptr(ctx.seq_q_len), ptr(ctx.seq_slot), c_int(ctx.num_seqs), c_int(walked), c_int(tokens), c_int(1 if single else 0), c_int(heads), c_int(dk), c_int(dv),
         ptr(S), ptr(n), ptr(m), *(gates and gates + 4 * i * tokens * heads for i in range(3)), ptr(num), ptr(den), ptr(norm), c_float(eps), ptr(out),
         c_int(dtype_code(out.dtype)), c_int(ctx.max_q_len), ptr(scratch), c_int64(scratch.numel() if scratch is not None else 0), ctx.stream,
     )
-    # The recurrence and the output kernel (and the gates'; in chunks three in the recurrence's place) are launches of their own.
-    ctx.lib.calls += (1 if single else 2) + (2 if scratch is not None else 0)
+    # The output kernel, the recurrence where it runs, the gates' and the three kernels of chunks are launches of their own.
+    ctx.lib.calls += (0 if single else 1) + (1 if walked else 0) + (3 if scratch is not None else 0)
     return out
 
 
