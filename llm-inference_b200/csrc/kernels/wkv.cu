@@ -381,8 +381,8 @@ B200_API int b200_wkv_prepare(const void* r, const void* k, const void* v, const
 }
 
 B200_API int b200_wkv_recurrence(const float* r, const float* k, const float* v, const float* bonus, const float* decay,
-                                 const int* seq_q_start, const int* seq_q_len, const int* seq_slot, int seqs, int heads, int dk, int dv,
-                                 float* state, float* out, cudaStream_t stream) {
+                                 const int* seq_q_start, const int* seq_q_len, const int* seq_slot, int seqs, int max_q_len,
+                                 int heads, int dk, int dv, float* state, float* out, cudaStream_t stream) {
   if (seqs == 0) return 0;
   B200_REQUIRE(seqs > 0 && heads > 0 && heads <= 65535 && dk > 0 && dv > 0, "wkv_recurrence: bad sizes");
   B200_REQUIRE(dk <= 1024, "wkv_recurrence: %d key channels per head, at most 1024", dk);
@@ -399,9 +399,12 @@ B200_API int b200_wkv_recurrence(const float* r, const float* k, const float* v,
   const auto aligned = [](const void* p) { return reinterpret_cast<uintptr_t>(p) % 16 == 0; };
   const int vec = dk % 4 == 0 && dv % 4 == 0 && aligned(r) && aligned(k) && aligned(v) && aligned(decay) ? 1 : 0;
   B200_REQUIRE(smem <= 200 * 1024, "wkv_recurrence: the staged tokens do not fit shared memory");
+  // A step with prompt portions launches the ordinary way: made resident early, the few blocks are packed several to an SM
+  // onto the SMs that the predecessor's last wave leaves free and walk their tokens there to the end.
+  const bool ordered = max_q_len > kStage;
   auto launch = [&](auto kernel) {
     if (smem > 48 * 1024) cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
-    launch_kernel(kernel, grid, dim3(kRecurrenceThreads), smem, stream, r, k, v, bonus, decay, seq_q_start, seq_q_len, seq_slot, heads,
+    launch_kernel_as(ordered, kernel, grid, dim3(kRecurrenceThreads), smem, stream, r, k, v, bonus, decay, seq_q_start, seq_q_len, seq_slot, heads,
                   dk, dv, vec, state, out);
   };
   if (per == 32) launch(wkv_recurrence_kernel<32, 32>);

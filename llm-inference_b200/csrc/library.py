@@ -105,7 +105,7 @@ _SIGNATURES: dict[str, list] = {
     "b200_wkv_shift_mix": [c_void_p] * 7 + [c_int] * 4 + [c_void_p, c_int, c_void_p],
     "b200_tanh_rows": [c_void_p, c_int64, c_int, c_void_p],
     "b200_wkv_prepare": [c_void_p] * 6 + [c_int] * 3 + [c_void_p] * 5 + [c_int, c_void_p],
-    "b200_wkv_recurrence": [c_void_p] * 8 + [c_int] * 4 + [c_void_p] * 3,
+    "b200_wkv_recurrence": [c_void_p] * 8 + [c_int] * 5 + [c_void_p] * 3,
     "b200_wkv_output": [c_void_p] * 3 + [c_int, c_int, c_int, c_int, c_float, c_int, c_void_p, c_int, c_void_p],
     "b200_norm_kv_write": [c_void_p, c_int] + [c_void_p] * 4 + [c_int, c_int] + [c_void_p] * 5 + [c_int] * 9 + [c_float, c_int, c_int,
                            c_void_p, c_void_p],

@@ -1232,7 +1232,7 @@ def wkv_recurrence(
         return out
     ctx.lib.call(
         "b200_wkv_recurrence", ptr(r), ptr(k), ptr(v), ptr(bonus), ptr(decay), ptr(ctx.seq_q_start), ptr(ctx.seq_q_len), ptr(ctx.seq_slot),
-        c_int(walked), c_int(heads), c_int(dk), c_int(dv), ptr(state), ptr(out), ctx.stream,
+        c_int(walked), c_int(ctx.max_q_len if walked == ctx.num_seqs else 1), c_int(heads), c_int(dk), c_int(dv), ptr(state), ptr(out), ctx.stream,
     )
     return out
 
