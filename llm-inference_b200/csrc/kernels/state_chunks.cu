@@ -102,6 +102,7 @@ __device__ __forceinline__ quad_t load_quad(const float* p) {
 // What `chunk_prepare` hands on, and the walk's result. Rows of `padded_rows(dk)` and `padded_columns(dv)` numbers, so all copies
 // are whole 16-byte steps whatever the sizes.
 struct Scratch {
+  int head0, heads;  // the heads that a pass takes: all, or as many as the scratch holds
   float* y;   // [tokens][heads][rows]
   float* kd;  // [tokens][heads][rows]: G_last,j k_j
   float* qt;  // [tokens][heads][rows]: e_i q_i
@@ -261,7 +262,7 @@ chunk_prepare_kernel(const float* q, const float* k, const float* v, const float
                      const int* __restrict__ seq_q_len, int heads, int kv_heads, int dk, int dv, Scratch to) {
   extern __shared__ __align__(16) float chunk_smem[];
   let_successor_start();
-  const int seq = blockIdx.z, head = blockIdx.y, chunk = blockIdx.x;
+  const int seq = blockIdx.z, own_head = blockIdx.y, head = to.head0 + own_head, chunk = blockIdx.x;
   const int n = min(C, seq_q_len[seq] - chunk * C);
   if (n <= 0) return;
   const int start = seq_q_start[seq], kvh = head / (heads / kv_heads);
@@ -322,7 +323,7 @@ chunk_prepare_kernel(const float* q, const float* k, const float* v, const float
   {
     float own = 0.f, d = 0.f, prefix = 0.f, e = 0.f;
     if (PER_HEAD) own = lane < n ? decay[(first + lane) * heads + head] : 0.f;
-    float* a = to.a + (first * heads + head) * C + lane;
+    float* a = to.a + (first * to.heads + own_head) * C + lane;
     for (int i = 0; i < C; ++i) {
       if (PER_HEAD) {  // D_ij of column j = lane, the sum of the logarithms from token j + 1 on, grows with i from zero at i = j
         const float gi = __shfl_sync(0xffffffffu, own, i);
@@ -333,7 +334,7 @@ chunk_prepare_kernel(const float* q, const float* k, const float* v, const float
       if ((i & 7) == warp) {
         const float between = PER_HEAD ? expf(d) : 1.f;
         ls[i * C + lane] = lane < i ? bs[i] * between * kk[i * (C + 1) + lane] : 0.f;
-        if (i < n) a[static_cast<int64_t>(i) * heads * C] = lane <= i ? between * qk[i * (C + 1) + lane] : 0.f;
+        if (i < n) a[static_cast<int64_t>(i) * to.heads * C] = lane <= i ? between * qk[i * (C + 1) + lane] : 0.f;
       }
     }
     if (PER_HEAD && warp == 0) es[lane] = expf(e), fs[lane] = expf(d);  // d is now D_last,j: tokens past n added nothing
@@ -342,9 +343,9 @@ chunk_prepare_kernel(const float* q, const float* k, const float* v, const float
   for (int column = tid; column < rows + columns; column += kThreads) {
     float x[C];
     float* to_x;
-    const int64_t stride = static_cast<int64_t>(heads) * (column < rows ? rows : columns);
+    const int64_t stride = static_cast<int64_t>(to.heads) * (column < rows ? rows : columns);
     if (column < rows) {
-      const int64_t at = (first * heads + head) * rows + column;
+      const int64_t at = (first * to.heads + own_head) * rows + column;
       float* qt = to.qt + at;
       float* kd = to.kd + at;
       to_x = to.y + at;
@@ -366,12 +367,12 @@ chunk_prepare_kernel(const float* q, const float* k, const float* v, const float
         qt += stride, kd += stride;
         x[i] = -bs[i] * e * key;
       }
-      to.e[(chunk_place(start, seq, chunk) * heads + head) * rows + column] =
+      to.e[(chunk_place(start, seq, chunk) * to.heads + own_head) * rows + column] =
           PER_HEAD ? es[n - 1] : before[kGroups - 1] * whole[(kGroups - 1) * rows + column];
     } else {
       const int c = column - rows;
       const float* value = v + (first * heads + head) * dv + c;
-      to_x = to.x + (first * heads + head) * columns + c;
+      to_x = to.x + (first * to.heads + own_head) * columns + c;
 #pragma unroll
       for (int i = 0; i < C; ++i) x[i] = i < n && c < dv ? value[static_cast<int64_t>(i) * heads * dv] : 0.f;
 #pragma unroll
@@ -422,11 +423,11 @@ __global__ void __launch_bounds__(kThreads, 2)
 linear_chunk_prepare_kernel(LinearRule in, const int* __restrict__ seq_q_start, const int* __restrict__ seq_q_len, int heads, int dk, int dv, Scratch to) {
   extern __shared__ __align__(16) float chunk_smem[];
   let_successor_start();
-  const int seq = blockIdx.z, head = blockIdx.y, chunk = blockIdx.x;
+  const int seq = blockIdx.z, own_head = blockIdx.y, head = to.head0 + own_head, chunk = blockIdx.x;
   const int n = min(C, seq_q_len[seq] - chunk * C);
   if (n <= 0) return;
   const int start = seq_q_start[seq];
-  const int64_t first = static_cast<int64_t>(start) + chunk * C, place = chunk_place(start, seq, chunk) * heads + head;
+  const int64_t first = static_cast<int64_t>(start) + chunk * C, place = chunk_place(start, seq, chunk) * to.heads + own_head;
   constexpr int rows = ROWS, ld = ROWS + 4;
   const int columns = padded_columns(dv);
   constexpr bool GENERAL = RULE == kGeneralDelta, MEMORY = RULE == kMemory;
@@ -528,12 +529,12 @@ linear_chunk_prepare_kernel(LinearRule in, const int* __restrict__ seq_q_start, 
       d = i > lane ? d * own : 1.f;
       prefix *= own;
       if (i == lane) e = prefix;
-      if ((i & 7) == warp && i < n) to.av[((first + i) * heads + head) * C + lane] = lane <= i ? d * put * rk[i * (C + 1) + lane] * in.scale : 0.f;
+      if ((i & 7) == warp && i < n) to.av[((first + i) * to.heads + own_head) * C + lane] = lane <= i ? d * put * rk[i * (C + 1) + lane] * in.scale : 0.f;
     }
     if (warp == 0) es[lane] = e, fs[lane] = d * put;
     __syncthreads();
     for (int c = tid; c < rows; c += kThreads) {
-      float* qt = to.qt + (first * heads + head) * rows + c;
+      float* qt = to.qt + (first * to.heads + own_head) * rows + c;
       float sum = 0.f;
 #pragma unroll 8
       for (int i = 0; i < C; ++i) {
@@ -541,7 +542,7 @@ linear_chunk_prepare_kernel(LinearRule in, const int* __restrict__ seq_q_start, 
         ks[i * ld + c] = key;
         sum += key;
         if (i < n) *qt = es[i] * in.scale * rs[i * ld + c];
-        qt += static_cast<int64_t>(heads) * rows;
+        qt += static_cast<int64_t>(to.heads) * rows;
       }
       to.n[place * rows + c] = sum;
       to.e[place * rows + c] = es[n - 1];
@@ -552,7 +553,7 @@ linear_chunk_prepare_kernel(LinearRule in, const int* __restrict__ seq_q_start, 
   }
   for (int i = warp; !MEMORY && i < C; i += kWarps) {
     const int at = i * (C + 1) + lane;
-    const int64_t row = ((first + i) * heads + head) * C + lane;
+    const int64_t row = ((first + i) * to.heads + own_head) * C + lane;
     if (GENERAL) {  // au came in with its own sign: b = -au
       ls[i * C + lane] = lane < i ? ub[at] : 0.f;
       ms[i * C + lane] = lane < i ? uk[at] : 0.f;
@@ -573,7 +574,7 @@ linear_chunk_prepare_kernel(LinearRule in, const int* __restrict__ seq_q_start, 
       before *= g < group ? whole[g * rows + c] : 1.f;
       after *= g + 1 > group ? whole[(g + 1) * rows + c] : 1.f;
     }
-    const int64_t at = ((first + group * kGroup) * heads + head) * rows + c, step = static_cast<int64_t>(heads) * rows;
+    const int64_t at = ((first + group * kGroup) * to.heads + own_head) * rows + c, step = static_cast<int64_t>(to.heads) * rows;
     float* qt = to.qt + at;
     float* kd = to.kd + at;
 #pragma unroll
@@ -618,8 +619,8 @@ linear_chunk_prepare_kernel(LinearRule in, const int* __restrict__ seq_q_start, 
           }
           x[i] = sum0 + sum1;
         }
-        stride = static_cast<int64_t>(heads) * columns;
-        to_x = to.x + (first * heads + head) * columns + col0 + c;
+        stride = static_cast<int64_t>(to.heads) * columns;
+        to_x = to.x + (first * to.heads + own_head) * columns + col0 + c;
       } else {
         const int channel = c - kValueTile;
         float before = 1.f;
@@ -628,8 +629,8 @@ linear_chunk_prepare_kernel(LinearRule in, const int* __restrict__ seq_q_start, 
           if (i > 0 && i % kGroup == 0) before *= whole[(i / kGroup - 1) * rows + channel];
           x[i] = before * us[i * ld + channel];
         }
-        stride = static_cast<int64_t>(heads) * rows;
-        to_x = to.y + (first * heads + head) * rows + channel;
+        stride = static_cast<int64_t>(to.heads) * rows;
+        to_x = to.y + (first * to.heads + own_head) * rows + channel;
       }
       substitute(ls, x);
       if (tid >= kValueTile || col0 + c < columns) {
@@ -677,7 +678,7 @@ __global__ void __launch_bounds__(kThreads)
 chunk_scan_kernel(const int* __restrict__ seq_q_start, const int* __restrict__ seq_q_len, const int* __restrict__ seq_slot, int heads, int dk, int dv, Scratch from,
                   float* state, float* normaliser) {
   let_successor_start();
-  const int seq = blockIdx.z, head = blockIdx.y;
+  const int seq = blockIdx.z, own_head = blockIdx.y, head = from.head0 + own_head;
   const int start = seq_q_start[seq], len = seq_q_len[seq], chunks = (len + C - 1) / C;
   const int rows = padded_rows(dk), columns = padded_columns(dv);
   const int item = (blockIdx.x * kThreads + threadIdx.x) * 4;
@@ -687,7 +688,7 @@ chunk_scan_kernel(const int* __restrict__ seq_q_start, const int* __restrict__ s
     wait_for_predecessor();
     float* own = normaliser + (static_cast<int64_t>(seq_slot[seq]) * heads + head) * dk + c;
     float n = c < dk ? *own : 0.f;
-    const int64_t step = static_cast<int64_t>(heads) * rows, at = (chunk_place(start, seq, 0) * heads + head) * rows + c;
+    const int64_t step = static_cast<int64_t>(from.heads) * rows, at = (chunk_place(start, seq, 0) * from.heads + own_head) * rows + c;
     for (int chunk = 0; chunk < chunks; ++chunk) {
       const float add = from.n[at + chunk * step];
       from.n[at + chunk * step] = n;
@@ -702,10 +703,10 @@ chunk_scan_kernel(const int* __restrict__ seq_q_start, const int* __restrict__ s
   wait_for_predecessor();
 #pragma unroll
   for (int x = 0; x < 4; ++x) s[x] = row < dk && col + x < dv ? base[x] : 0.f;
-  const int64_t place = chunk_place(start, seq, 0) * heads + head;
+  const int64_t place = chunk_place(start, seq, 0) * from.heads + own_head;
   const float* e = from.e + place * rows + row;
   float* sums = from.s + place * rows * columns + item;
-  const int64_t step_e = static_cast<int64_t>(heads) * rows, step = step_e * columns;
+  const int64_t step_e = static_cast<int64_t>(from.heads) * rows, step = step_e * columns;
   constexpr int kAhead = 8;
   for (int chunk = 0; chunk < chunks; chunk += kAhead) {
     float4 add[kAhead];
@@ -752,7 +753,7 @@ chunk_walk_kernel(const int* __restrict__ seq_q_start, const int* __restrict__ s
   constexpr int kLdS = ROWS + 8;                  // 8 banks from column to column
   constexpr int kRowX = kSplit == 4 ? 24 : 16;    // the rows that lanes read side by side in different banks
   let_successor_start();
-  const int col0 = blockIdx.x * kColumns, head = blockIdx.y, seq = blockIdx.z;
+  const int col0 = blockIdx.x * kColumns, own_head = blockIdx.y, head = from.head0 + own_head, seq = blockIdx.z;
   const int start = seq_q_start[seq], len = seq_q_len[seq];
   const int columns = padded_columns(dv);
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -769,16 +770,16 @@ chunk_walk_kernel(const int* __restrict__ seq_q_start, const int* __restrict__ s
 #pragma unroll
     for (int idx = tid; idx < C * ROWS / 4; idx += kThreads) {
       const int r = idx / (ROWS / 4), c = idx % (ROWS / 4) * 4;
-      const int64_t at = r < n ? ((first + r) * heads + head) * ROWS + c : 0;
+      const int64_t at = r < n ? ((first + r) * from.heads + own_head) * ROWS + c : 0;
       stage_copy<16>(ys + r * kLd + c, from.y + at, r < n);
       stage_copy<16>(kds + r * kLd + c, from.kd + at, r < n);
     }
     if (tid < C * kColumns / 4) {
       const int r = tid / 4, c = tid % 4 * 4;
-      stage_copy<16>(ws + r * kColumns + c, from.x + (r < n ? ((first + r) * heads + head) * columns + col0 + c : 0), r < n);
+      stage_copy<16>(ws + r * kColumns + c, from.x + (r < n ? ((first + r) * from.heads + own_head) * columns + col0 + c : 0), r < n);
     } else if (tid < C * kColumns / 4 + ROWS / 4) {
       const int c = (tid - C * kColumns / 4) * 4;
-      stage_copy<16>(es + c, from.e + (chunk_place(start, seq, chunk) * heads + head) * ROWS + c, true);
+      stage_copy<16>(es + c, from.e + (chunk_place(start, seq, chunk) * from.heads + own_head) * ROWS + c, true);
     }
     commit_copies();
   };
@@ -797,7 +798,7 @@ chunk_walk_kernel(const int* __restrict__ seq_q_start, const int* __restrict__ s
   for (int chunk = 0; chunk < chunks; ++chunk) {
     const int n = min(C, len - chunk * C);
     const int64_t first = static_cast<int64_t>(start) + chunk * C;
-    float* s_out = from.s + ((chunk_place(start, seq, chunk) * heads + head) * ROWS + row0) * columns + col0 + cg * 4;
+    float* s_out = from.s + ((chunk_place(start, seq, chunk) * from.heads + own_head) * ROWS + row0) * columns + col0 + cg * 4;
     float4 own[kPer];
     if (ADD) {
 #pragma unroll
@@ -858,7 +859,7 @@ chunk_walk_kernel(const int* __restrict__ seq_q_start, const int* __restrict__ s
       const float u1 = from_pair(b4 ? row[1] : row[3], b4 ? row[3] : row[1], 16) + ws[i * kColumns + c + 4];
       xs[i * kRowX + c] = u0, xs[i * kRowX + c + 4] = u1;
       if (i < n) {
-        float* to = from.x + ((first + i) * heads + head) * columns + col0 + c;
+        float* to = from.x + ((first + i) * from.heads + own_head) * columns + col0 + c;
         to[0] = u0, to[4] = u1;
       }
     }
@@ -931,13 +932,13 @@ chunk_out_kernel(const int* __restrict__ seq_q_start, const int* __restrict__ se
   extern __shared__ __align__(16) float chunk_smem[];
   constexpr int kLdOut = COLS + 4, kStage = C * kLdSlab + C * kLdOut;
   let_successor_start();
-  const int seq = blockIdx.z / tiles, col0 = blockIdx.z % tiles * COLS, head = blockIdx.y, chunk = blockIdx.x;
+  const int seq = blockIdx.z / tiles, col0 = blockIdx.z % tiles * COLS, own_head = blockIdx.y, head = from.head0 + own_head, chunk = blockIdx.x;
   const int start = seq_q_start[seq], n = min(C, seq_q_len[seq] - chunk * C);
   if (n <= 0) return;
   const int64_t first = static_cast<int64_t>(start) + chunk * C;
   const int columns = padded_columns(dv), width = min(COLS, columns - col0);
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const float* states = from.s + (chunk_place(start, seq, chunk) * heads + head) * rows * columns + col0;
+  const float* states = from.s + (chunk_place(start, seq, chunk) * from.heads + own_head) * rows * columns + col0;
   const int state_slabs = rows / C, slabs = state_slabs + (WITH_U ? 1 : 0) + (WITH_V ? 1 : 0);
   wait_for_predecessor();
   auto fetch = [&](int slab) {
@@ -948,7 +949,7 @@ chunk_out_kernel(const int* __restrict__ seq_q_start, const int* __restrict__ se
 #pragma unroll
     for (int r = tid >> 3; r < C; r += COLS / 8) {
       const int c = (tid & 7) * 4;
-      const int64_t row = (first + r) * heads + head;
+      const int64_t row = (first + r) * from.heads + own_head;
       stage_copy<16>(left + r * kLdSlab + c, r < n ? (in_state ? from.qt + row * rows + slab * C + c : pairs + row * C + c) : from.qt, r < n);
     }
     if (in_state || is_u) {
@@ -956,7 +957,7 @@ chunk_out_kernel(const int* __restrict__ seq_q_start, const int* __restrict__ se
       for (int r = tid / (COLS / 4); r < C; r += 4) {
         const int c = tid % (COLS / 4) * 4;
         const bool valid = c < width && (in_state || r < n);
-        const float* at = in_state ? states + static_cast<int64_t>(slab * C + r) * columns + c : from.x + ((first + r) * heads + head) * columns + col0 + c;
+        const float* at = in_state ? states + static_cast<int64_t>(slab * C + r) * columns + c : from.x + ((first + r) * from.heads + own_head) * columns + col0 + c;
         stage_copy<16>(right + r * kLdOut + c, valid ? at : from.qt, valid);
       }
     } else if (v_wide) {
@@ -980,13 +981,13 @@ chunk_out_kernel(const int* __restrict__ seq_q_start, const int* __restrict__ se
   for (int i = 0; i < 8; ++i) acc[i][0] = acc[i][1] = acc[i][2] = acc[i][3] = 0.f;
   fetch(0);
   if (den != nullptr && col0 == 0) {  // the normaliser read out as the state is: n . (e q) + the chunk's own pairs
-    const float* n0 = from.n + (chunk_place(start, seq, chunk) * heads + head) * rows;
+    const float* n0 = from.n + (chunk_place(start, seq, chunk) * from.heads + own_head) * rows;
     for (int r = warp; r < n; r += COLS / 32) {
-      const int64_t row = (first + r) * heads + head;
+      const int64_t row = (first + r) * from.heads + own_head;
       float sum = from.av[row * C + lane];
       for (int c = lane; c < rows; c += 32) sum = fmaf(from.qt[row * rows + c], n0[c], sum);
       sum = warp_sum(sum);
-      if (lane == 0) den[row] = sum;
+      if (lane == 0) den[(first + r) * heads + head] = sum;
     }
   }
   for (int slab = 0; slab < slabs; ++slab) {
@@ -1055,14 +1056,15 @@ struct Sizes {
 
 int64_t aligned_floats(int64_t n) { return (n + 3) / 4 * 4; }
 
-// The scratch's arrays one after another in `base` (null pointers with a null base); returns the numbers they need.
-int64_t lay_out(int rule, const Sizes& z, float* base, Scratch* to) {
-  const int64_t rows = padded_rows(z.dk), columns = padded_columns(z.dv), per_head = static_cast<int64_t>(z.tokens) * z.heads;
-  const int64_t chunks = (static_cast<int64_t>(z.tokens) / C + z.seqs + 1) * z.heads;
+// The scratch's arrays for so many heads one after another in `base` (null pointers with a null base); returns the numbers they need.
+int64_t lay_out(int rule, const Sizes& z, int heads, float* base, Scratch* to) {
+  const int64_t rows = padded_rows(z.dk), columns = padded_columns(z.dv), per_head = static_cast<int64_t>(z.tokens) * heads;
+  const int64_t chunks = (static_cast<int64_t>(z.tokens) / C + z.seqs + 1) * heads;
   const int64_t with_u = rule == kDelta || rule == kGeneralDelta ? 1 : 0, with_v = rule != kDelta ? 1 : 0, with_n = rule == kMemory ? 1 : 0;
   const int64_t sizes[9] = {with_u * per_head * rows, with_u * per_head * rows, per_head * rows, with_u * per_head * columns,
                             with_u * per_head * C, with_v * per_head * C, chunks * rows, with_n * chunks * rows, chunks * rows * columns};
   float** arrays[9] = {&to->y, &to->kd, &to->qt, &to->x, &to->a, &to->av, &to->e, &to->n, &to->s};
+  to->head0 = 0, to->heads = heads;
   int64_t at = 0;
   for (int i = 0; i < 9; ++i) {
     *arrays[i] = base == nullptr ? nullptr : base + at;
@@ -1112,6 +1114,25 @@ auto linear_prepare_form(bool wide, int rule) {
 
 bool aligned16(const void* p) { return reinterpret_cast<uintptr_t>(p) % 16 == 0; }
 
+// Heads know nothing of one another, so a scratch that does not hold all of them takes them in as few equal parts as fit, one after the
+// other through the same scratch. Each part costs another walk of the same length with fewer blocks: 2,048 tokens of 28 heads of 128 x 128
+// with one decay per head take 418 us in one part, 481 in two, 627 in three, 786 in four (token by token 810), 24 heads of 64 x 64 under the
+// generalized rule 236, 335, 417 and 544 (465).
+template <typename Pass>
+int part_by_part(const char* name, int rule, const Sizes& z, float* base, int64_t floats, Pass pass) {
+  Scratch scratch;
+  int heads = z.heads;
+  for (int parts = 2; heads > 1 && lay_out(rule, z, heads, nullptr, &scratch) > floats; ++parts) heads = (z.heads + parts - 1) / parts;
+  B200_REQUIRE(aligned16(base) && lay_out(rule, z, heads, base, &scratch) <= floats, "%s: scratch too small or not aligned to 16 bytes", name);
+  B200_REQUIRE(z.seqs <= 65535 && static_cast<int64_t>(z.seqs) * ((padded_columns(z.dv) + 127) / 128) <= 65535, "%s: too many requests", name);
+  B200_REQUIRE(raise_all(), "%s: cannot size shared memory", name);
+  for (int head = 0; head < z.heads; head += heads) {
+    scratch.head0 = head, scratch.heads = min(heads, z.heads - head);
+    if (int status = pass(scratch)) return status;
+  }
+  return 0;
+}
+
 struct Requests {
   const int* q_start;
   const int* q_len;
@@ -1123,7 +1144,7 @@ int launch_walk(const Sizes& z, const Requests& req, bool add, const Scratch& sc
   auto walk = add ? (rows == 64 ? chunk_walk_kernel<64, true> : chunk_walk_kernel<128, true>)
                   : (rows == 64 ? chunk_walk_kernel<64, false> : (rows == 128 ? chunk_walk_kernel<128, false> : chunk_walk_kernel<256, false>));
   // The ordinary way, not early: the few long-lived blocks should spread over all SMs, not over those the kernel in front leaves first.
-  launch_kernel_as(true, walk, dim3(padded_columns(z.dv) / kColumns, z.heads, z.seqs), dim3(kThreads), walk_smem(rows), stream, req.q_start, req.q_len, req.slot,
+  launch_kernel_as(true, walk, dim3(padded_columns(z.dv) / kColumns, scratch.heads, z.seqs), dim3(kThreads), walk_smem(rows), stream, req.q_start, req.q_len, req.slot,
                    z.heads, z.dk, z.dv, scratch, state);
   return b200_check_launch("chunk_walk");
 }
@@ -1131,7 +1152,7 @@ int launch_walk(const Sizes& z, const Requests& req, bool add, const Scratch& sc
 template <bool WITH_U, bool WITH_V>
 int launch_out(const Sizes& z, const Requests& req, const Scratch& scratch, const float* v, int64_t v_ld, float* out, float* den, cudaStream_t stream) {
   const int columns = padded_columns(z.dv), cols = columns <= 64 ? 64 : 128, tiles = (columns + cols - 1) / cols;
-  launch_kernel(cols == 64 ? chunk_out_kernel<64, WITH_U, WITH_V> : chunk_out_kernel<128, WITH_U, WITH_V>, dim3((z.max_q_len + C - 1) / C, z.heads, z.seqs * tiles),
+  launch_kernel(cols == 64 ? chunk_out_kernel<64, WITH_U, WITH_V> : chunk_out_kernel<128, WITH_U, WITH_V>, dim3((z.max_q_len + C - 1) / C, scratch.heads, z.seqs * tiles),
                 dim3(cols), out_smem(cols), stream, req.q_start, req.q_len, z.heads, z.dv, padded_rows(z.dk), tiles, scratch, v,
                 v_ld, z.dv % 4 == 0 && v_ld % 4 == 0 && aligned16(v) ? 1 : 0, out, den);
   return b200_check_launch("chunk_out");
@@ -1139,19 +1160,17 @@ int launch_out(const Sizes& z, const Requests& req, const Scratch& scratch, cons
 
 int launch_linear_prepare(const Sizes& z, const Requests& req, int rule, bool wide, const LinearRule& in, const Scratch& scratch, cudaStream_t stream) {
   const int rows = padded_rows(z.dk);
-  launch_kernel(rows == 64 ? linear_prepare_form<64>(wide, rule) : linear_prepare_form<128>(wide, rule), dim3((z.max_q_len + C - 1) / C, z.heads, z.seqs),
+  launch_kernel(rows == 64 ? linear_prepare_form<64>(wide, rule) : linear_prepare_form<128>(wide, rule), dim3((z.max_q_len + C - 1) / C, scratch.heads, z.seqs),
                 dim3(kThreads), linear_prepare_smem(rows, rule), stream, in, req.q_start, req.q_len, z.heads, z.dk, z.dv, scratch);
   return b200_check_launch("linear_chunk_prepare");
 }
 
 int launch_scan(const Sizes& z, const Requests& req, const Scratch& scratch, float* state, float* normaliser, cudaStream_t stream) {
   const int rows = padded_rows(z.dk), blocks = (rows * padded_columns(z.dv) / 4 + kThreads - 1) / kThreads;
-  launch_kernel(chunk_scan_kernel, dim3(blocks + (normaliser != nullptr ? (rows + kThreads - 1) / kThreads : 0), z.heads, z.seqs), dim3(kThreads), 0, stream, req.q_start,
+  launch_kernel(chunk_scan_kernel, dim3(blocks + (normaliser != nullptr ? (rows + kThreads - 1) / kThreads : 0), scratch.heads, z.seqs), dim3(kThreads), 0, stream, req.q_start,
                 req.q_len, req.slot, z.heads, z.dk, z.dv, scratch, state, normaliser);
   return b200_check_launch("chunk_scan");
 }
-
-bool too_many_requests(const Sizes& z) { return static_cast<int64_t>(z.seqs) * ((padded_columns(z.dv) + 127) / 128) > 65535; }
 
 }  // namespace
 
@@ -1162,11 +1181,12 @@ static bool sizes_taken(int rule, int heads, int kv_heads, int dk, int dv) {
          dv <= 65536;
 }
 
-// Numbers of scratch (32-bit, aligned to 16 bytes) that a call needs; 0: sizes the chunked form does not take.
+// Numbers of scratch (32-bit, aligned to 16 bytes) that a call needs to take all heads at once; 0: sizes the chunked form does not take. A
+// call takes any scratch that holds at least one head.
 B200_API int64_t b200_state_chunks_scratch(int rule, int tokens, int seqs, int heads, int kv_heads, int dk, int dv) {
   if (!sizes_taken(rule, heads, kv_heads, dk, dv)) return 0;
   Scratch scratch;
-  return lay_out(rule, {tokens, seqs, 0, heads, dk, dv}, nullptr, &scratch);
+  return lay_out(rule, {tokens, seqs, 0, heads, dk, dv}, heads, nullptr, &scratch);
 }
 
 // The delta rule over every request's new tokens; operands as `delta_prepare` leaves them. per_head = 0: `decay` [tokens][heads][dk]
@@ -1178,18 +1198,16 @@ B200_API int b200_delta_chunks(const float* q, const float* k, const float* v, c
   B200_REQUIRE(tokens > 0 && seqs > 0 && max_q_len > 0 && sizes_taken(kDelta, heads, kv_heads, dk, dv), "delta_chunks: shape not taken");
   const Sizes z = {tokens, seqs, max_q_len, heads, dk, dv};
   const Requests req = {seq_q_start, seq_q_len, seq_slot};
-  Scratch parts;
-  B200_REQUIRE(aligned16(scratch) && lay_out(kDelta, z, scratch, &parts) <= scratch_floats, "delta_chunks: scratch too small or not aligned to 16 bytes");
-  B200_REQUIRE(seqs <= 65535 && !too_many_requests(z), "delta_chunks: too many requests");
-  B200_REQUIRE(raise_all(), "delta_chunks: cannot size shared memory");
   const bool wide = dk % 4 == 0 && aligned16(q) && aligned16(k) && (per_head || aligned16(decay));
   const int rows = padded_rows(dk);
   auto prepare = rows == 64 ? delta_prepare_form<64>(wide, per_head) : (rows == 128 ? delta_prepare_form<128>(wide, per_head) : delta_prepare_form<256>(wide, per_head));
-  launch_kernel(prepare, dim3((max_q_len + C - 1) / C, heads, seqs), dim3(kThreads), prepare_smem(rows), stream, q, k, v, beta, decay, seq_q_start,
-                seq_q_len, heads, kv_heads, dk, dv, parts);
-  if (int status = b200_check_launch("chunk_prepare")) return status;
-  if (int status = launch_walk(z, req, false, parts, state, stream)) return status;
-  return launch_out<true, false>(z, req, parts, v, static_cast<int64_t>(heads) * dv, out, nullptr, stream);
+  return part_by_part("delta_chunks", kDelta, z, scratch, scratch_floats, [&](const Scratch& parts) -> int {
+    launch_kernel(prepare, dim3((max_q_len + C - 1) / C, parts.heads, seqs), dim3(kThreads), prepare_smem(rows), stream, q, k, v, beta, decay, seq_q_start,
+                  seq_q_len, heads, kv_heads, dk, dv, parts);
+    if (int status = b200_check_launch("chunk_prepare")) return status;
+    if (int status = launch_walk(z, req, false, parts, state, stream)) return status;
+    return launch_out<true, false>(z, req, parts, v, static_cast<int64_t>(heads) * dv, out, nullptr, stream);
+  });
 }
 
 // The rules in which the values enter as they are. With `u` the generalized delta rule S <- w S - au (u^T S) + k v^T, o = S^T r; with
@@ -1204,19 +1222,17 @@ B200_API int b200_linear_chunks(const float* r, const float* k, const float* v, 
   B200_REQUIRE(tokens > 0 && seqs > 0 && max_q_len > 0 && sizes_taken(rule, heads, heads, dk, dv), "linear_chunks: shape not taken");
   const Sizes z = {tokens, seqs, max_q_len, heads, dk, dv};
   const Requests req = {seq_q_start, seq_q_len, seq_slot};
-  Scratch parts;
-  B200_REQUIRE(aligned16(scratch) && lay_out(rule, z, scratch, &parts) <= scratch_floats, "linear_chunks: scratch too small or not aligned to 16 bytes");
-  B200_REQUIRE(seqs <= 65535 && !too_many_requests(z), "linear_chunks: too many requests");
-  B200_REQUIRE(raise_all(), "linear_chunks: cannot size shared memory");
   const bool wide = dk % 4 == 0 && dv % 4 == 0 && aligned16(r) && aligned16(k) && aligned16(v) && aligned16(w) && aligned16(au) && aligned16(u);
   const LinearRule in{r, k, v, w, au, u, bonus, nullptr, 1.f, static_cast<int64_t>(heads) * dk, static_cast<int64_t>(heads) * dv};
-  if (int status = launch_linear_prepare(z, req, rule, wide, in, parts, stream)) return status;
-  if (rule == kGeneralDelta) {
-    if (int status = launch_walk(z, req, true, parts, state, stream)) return status;
-    return launch_out<true, true>(z, req, parts, v, in.v_ld, out, nullptr, stream);
-  }
-  if (int status = launch_scan(z, req, parts, state, nullptr, stream)) return status;
-  return launch_out<false, true>(z, req, parts, v, in.v_ld, out, nullptr, stream);
+  return part_by_part("linear_chunks", rule, z, scratch, scratch_floats, [&](const Scratch& parts) -> int {
+    if (int status = launch_linear_prepare(z, req, rule, wide, in, parts, stream)) return status;
+    if (rule == kGeneralDelta) {
+      if (int status = launch_walk(z, req, true, parts, state, stream)) return status;
+      return launch_out<true, true>(z, req, parts, v, in.v_ld, out, nullptr, stream);
+    }
+    if (int status = launch_scan(z, req, parts, state, nullptr, stream)) return status;
+    return launch_out<false, true>(z, req, parts, v, in.v_ld, out, nullptr, stream);
+  });
 }
 
 // The matrix memory: S <- keep S + put k v^T, n <- keep n + put k, num = scale S^T q, den = scale n . q after the update. q, k, v: rows ld numbers apart, a
@@ -1227,13 +1243,11 @@ extern "C" int b200_memory_chunks(const float* q, const float* k, const float* v
   B200_REQUIRE(tokens > 0 && seqs > 0 && max_q_len > 0 && sizes_taken(kMemory, heads, heads, dk, dv), "memory_chunks: shape not taken");
   const Sizes z = {tokens, seqs, max_q_len, heads, dk, dv};
   const Requests req = {seq_q_start, seq_q_len, seq_slot};
-  Scratch parts;
-  B200_REQUIRE(aligned16(scratch) && lay_out(kMemory, z, scratch, &parts) <= scratch_floats, "memory_chunks: scratch too small or not aligned to 16 bytes");
-  B200_REQUIRE(seqs <= 65535 && !too_many_requests(z), "memory_chunks: too many requests");
-  B200_REQUIRE(raise_all(), "memory_chunks: cannot size shared memory");
   const bool wide = dk % 4 == 0 && dv % 4 == 0 && ld % 4 == 0 && aligned16(q) && aligned16(k) && aligned16(v);
   const LinearRule in{q, k, v, keep, nullptr, nullptr, nullptr, put, scale, ld, ld};
-  if (int status = launch_linear_prepare(z, req, kMemory, wide, in, parts, stream)) return status;
-  if (int status = launch_scan(z, req, parts, S, n, stream)) return status;
-  return launch_out<false, true>(z, req, parts, v, ld, num, den, stream);
+  return part_by_part("memory_chunks", kMemory, z, scratch, scratch_floats, [&](const Scratch& parts) -> int {
+    if (int status = launch_linear_prepare(z, req, kMemory, wide, in, parts, stream)) return status;
+    if (int status = launch_scan(z, req, parts, S, n, stream)) return status;
+    return launch_out<false, true>(z, req, parts, v, ld, num, den, stream);
+  });
 }

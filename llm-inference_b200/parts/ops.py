@@ -970,25 +970,36 @@ GENERAL_DELTA_CHUNK_FROM = 256
 # tokens, 56 and 54 at 200, 63 and 107 at 512, 219 and 579 at 2,048; the whole mixer 67 and 64 at 230 tokens of 12 heads, 79 and 84 at 300 in
 # two requests.
 MEMORY_CHUNK_FROM = 256
-# Scratch grows with the step's tokens (0.13 MB a token at 28 heads of 128 x 128): past this a step walks its portions token by token, as
-# if they were short, in the memory that takes.
+# Scratch grows with the step's tokens (0.13 MB a token at 28 heads of 128 x 128): past this a step takes its heads in parts, and past so
+# many parts it walks its portions token by token, as if they were short, in the memory that takes.
 CHUNK_SCRATCH_BYTES = 2 << 30
+CHUNK_PARTS = 3  # where chunks in parts stop being faster: state_chunks.cu has the figures
 _DELTA, _GENERAL_DELTA, _LINEAR, _MEMORY = 0, 1, 2, 3  # csrc/kernels/state_chunks.cu
 
 
-def _chunk_scratch(ctx: StepContext, rule: int, longer_than: int, tokens: int, heads: int, kv_heads: int, dk: int, dv: int) -> tuple[torch.Tensor | None, int]:
+def _chunk_scratch(
+    ctx: StepContext, rule: int, longer_than: int, tokens: int, heads: int, kv_heads: int, dk: int, dv: int,
+) -> tuple[torch.Tensor | None, int]:
     """Scratch for a recurrence that runs chunk by chunk (csrc/kernels/state_chunks.cu), or None where it runs token by token:
     portions of at most ``longer_than`` tokens, sizes the chunked form does not take and steps whose scratch would pass
-    ``CHUNK_SCRATCH_BYTES``. ``options["delta_portions"]``:
+    ``CHUNK_SCRATCH_BYTES`` even for a ``CHUNK_PARTS``-th of the heads. ``options["delta_portions"]``:
     ``"chunks"`` or ``"tokens"`` forces one of the two for prompt portions. And the number of requests that are walked token by token:
-    with chunks the single tokens that lead the batch (a step of single tokens only goes the forced way as a whole)."""
+    with chunks the single tokens that lead the batch (a step of single tokens only goes the forced way as a whole). Counts the
+    three launches of every part but one."""
     choice = ctx.options.get("delta_portions", "auto")
     if choice == "tokens" or (choice == "auto" and ctx.max_q_len <= longer_than):
         return None, ctx.num_seqs
     walked = ctx.num_decode_seqs if ctx.num_decode_seqs < ctx.num_seqs else 0
-    floats = int(ctx.lib.lib.b200_state_chunks_scratch(rule, tokens, ctx.num_seqs - walked, heads, kv_heads, dk, dv))
-    if choice == "auto" and not 0 < 4 * floats <= CHUNK_SCRATCH_BYTES:
-        return None, ctx.num_seqs
+    size = ctx.lib.lib.b200_state_chunks_scratch
+    floats, parts = int(size(rule, tokens, ctx.num_seqs - walked, heads, kv_heads, dk, dv)), 1
+    if choice == "auto":
+        while 4 * floats > CHUNK_SCRATCH_BYTES and parts < min(CHUNK_PARTS, heads):
+            parts += 1
+            some = -(-heads // parts)
+            floats = int(size(rule, tokens, ctx.num_seqs - walked, some, some, dk, dv))
+        if not 0 < 4 * floats <= CHUNK_SCRATCH_BYTES:
+            return None, ctx.num_seqs
+    ctx.lib.calls += 3 * parts - 1
     return ctx.portion_buffer("state_chunks", (floats,), torch.float32, CHUNK_SCRATCH_BYTES), walked
 
 
@@ -1011,7 +1022,6 @@ def _delta_chunks(
         c_int(tokens), c_int(ctx.num_seqs - walked), c_int(ctx.max_q_len), c_int(heads), c_int(kv_heads), c_int(dk), c_int(dv),
         ptr(scratch), c_int64(scratch.numel()), ptr(state), ptr(out), ctx.stream,
     )
-    ctx.lib.calls += 2  # further kernels of the call
     return walked
 
 
@@ -1032,7 +1042,6 @@ def _linear_chunks(
         c_int(tokens), c_int(ctx.num_seqs - walked), c_int(ctx.max_q_len), c_int(heads), c_int(dk), c_int(dv),
         ptr(scratch), c_int64(scratch.numel()), ptr(state), ptr(out), ctx.stream,
     )
-    ctx.lib.calls += 3 if u is None else 2  # further kernels of the call
     return walked
 
 
@@ -1779,8 +1788,8 @@ def mlstm(ctx: StepContext, proj: torch.Tensor, columns: tuple[int, int, int, in
         ptr(S), ptr(n), ptr(m), *(gates and gates + 4 * i * tokens * heads for i in range(3)), ptr(num), ptr(den), ptr(norm), c_float(eps), ptr(out),
         c_int(dtype_code(out.dtype)), c_int(ctx.max_q_len), ptr(scratch), c_int64(scratch.numel() if scratch is not None else 0), ctx.stream,
     )
-    # The output kernel, the recurrence where it runs, the gates' and the three kernels of chunks are launches of their own.
-    ctx.lib.calls += (0 if single else 1) + (1 if walked else 0) + (3 if scratch is not None else 0)
+    # The output kernel, the recurrence where it runs and the gates' are launches of their own; the chunks' have been counted but for one.
+    ctx.lib.calls += (0 if single else 1) + (1 if walked else 0) + (1 if scratch is not None else 0)
     return out
 
 
