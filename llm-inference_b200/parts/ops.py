@@ -957,14 +957,13 @@ DELTA_CHUNK_FROM = 112
 HEAD_DELTA_CHUNK_FROM = 128
 
 
-# The same for the rules in which the values enter as they are, one request, 24 heads of 64 x 64. Without a removal: 38 us in chunks and 43
-# token by token at 100 tokens, 40 and 69 at 200, 101 and 564 at 2,048; the whole mixer, which four launches instead of one bind: 120 and
-# 111 us at 128 tokens of 24 heads, 121 and 105 at 104 of 32, but 120 and 145 at 128 of 32, 120 and 169 at 144 of 24, 120 and 145 at 150
-# of 24 in two requests: the line lies at a number of (token, head) pairs, and for few heads where the chain alone is as long. Generalized delta rule: 61 and 62 us at 200 tokens, 244 and 473 at
-# 2,048; the whole mixer 104 and 91 at 200, 104 and 96 at 230.
-LINEAR_CHUNK_FROM = 80
-LINEAR_CHUNK_PAIRS = 3400
-LINEAR_CHUNK_ALWAYS_FROM = 141
+# The same for the rules in which the values enter as they are, one request, 24 heads of 64 x 64. Without a removal the whole mixer, tokens
+# and chunks: on the device 52 and 48 us at 64 tokens, 64 and 55 at 100, 69 and 56 at 120, 88 and 59 at 180; called by itself, when the host's
+# four launches instead of one bind it, 122 and 140 at 64, 135 and 143 at 100, 139 and 141 at 120, 145 and 140 at 141 (32 heads: 134 and 141
+# at 100, 140 and 141 at 120, 145 and 142 at 141). The line lies where a call by itself breaks even; a step of a whole model that waits for
+# the host (one prompt of up to 400 tokens in a model of 1B) pays each layer in chunks with two further launches, 10 us. Generalized delta rule: 61 and 62 us at
+# 200 tokens in chunks and token by token, 244 and 473 at 2,048; the whole mixer 104 and 91 at 200, 104 and 96 at 230.
+LINEAR_CHUNK_FROM = 120
 GENERAL_DELTA_CHUNK_FROM = 256
 # The matrix memory, one request, 12 heads of 128 x 128, with its gates and its output: 55 us in chunks and 53 token by token at 160
 # tokens, 56 and 54 at 200, 63 and 107 at 512, 219 and 579 at 2,048; the whole mixer 67 and 64 at 230 tokens of 12 heads, 79 and 84 at 300 in
@@ -1031,9 +1030,7 @@ def _linear_chunks(
 ) -> int:
     """As :func:`_delta_chunks`, for the rules in which the values enter as they are."""
     tokens = r.shape[0]
-    rule, longer_than = _GENERAL_DELTA, GENERAL_DELTA_CHUNK_FROM
-    if u is None:
-        rule, longer_than = _LINEAR, LINEAR_CHUNK_FROM if tokens * heads > LINEAR_CHUNK_PAIRS else LINEAR_CHUNK_ALWAYS_FROM
+    rule, longer_than = (_LINEAR, LINEAR_CHUNK_FROM) if u is None else (_GENERAL_DELTA, GENERAL_DELTA_CHUNK_FROM)
     scratch, walked = _chunk_scratch(ctx, rule, longer_than, tokens, heads, heads, dk, dv)
     if scratch is None:
         return walked
