@@ -69,6 +69,7 @@ class Workspace:
         self.device = device
         self._flat: dict[str, torch.Tensor] = {}
         self._apart: dict[str, torch.Tensor] = {}  # what no captured step uses, see `apart`
+        self._apart_views: dict[str, torch.Tensor] = {}
         # (name, dtype, shape) -> the view handed out last time; valid until a buffer moves.
         self._views: dict[tuple, torch.Tensor] = {}
         # Buffers whose first dimension counts tokens are sized for at least this many rows,
@@ -108,17 +109,22 @@ class Workspace:
         ``generation`` stays. Its size goes with the lengths of requests, which grow from one portion of a prompt to the next:
         it at least doubles (up to ``limit`` bytes, or what is asked for), and the old buffer is given up before the new one is
         asked for. A view is good until the same name is asked for again."""
+        key = f"{name}:{dtype}"
+        view = self._apart_views.get(key)
+        if view is not None and view.shape == shape:  # every layer of a step asks for the same
+            return view
         count = 1
         for s in shape:
             count *= int(s)
-        key = f"{name}:{dtype}"
         flat = self._apart.get(key)
         if flat is None or flat.numel() < count:
             capacity = max(count, min(2 * flat.numel(), limit // dtype.itemsize) if flat is not None else 0, 1)
-            flat = None
+            flat = view = None
             self._apart.pop(key, None)
+            self._apart_views.pop(key, None)
             flat = self._apart[key] = torch.empty(capacity, dtype=dtype, device=self.device)
-        return flat[:count].view(shape)
+        view = self._apart_views[key] = flat[:count].view(shape)
+        return view
 
     def zeros(self, name: str, count: int, dtype: torch.dtype) -> torch.Tensor:
         """A buffer that starts zeroed and whose users leave it zeroed (arrival counters)."""
