@@ -83,6 +83,7 @@ struct PrefillParams {
   int64_t q_ld, gate_ld;       // numbers from row to row of q and of gate
   int q_head_ld;               // numbers from head to head of q
   int latent_rank;             // column of the rotated numbers in a latent row
+  int min_q_len;               // requests of fewer new tokens are left out, and their keys are not among the rows
 };
 
 __device__ __forceinline__ uint32_t saddr(const void* p) { return static_cast<uint32_t>(__cvta_generic_to_shared(p)); }
@@ -271,7 +272,7 @@ flash_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap k_map, const __
   // A block with nothing to do still waits for the kernel in front before it ends: the kernel
   // behind may pass its own wait once every block of this grid has ended, and must not do so
   // while this kernel's predecessor still runs.
-  if (row_base >= rows_total) {
+  if (row_base >= rows_total || (LATENT && q_len < p.min_q_len)) {
     wait_for_predecessor();
     let_successor_start();
     return;
@@ -392,7 +393,8 @@ flash_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap k_map, const __
     const int row_head = (keys || p.value_head < 0) ? kv_head : p.value_head;
     int first_row = 0;  // LATENT: requests in front of this one, each padded to whole tiles
     if constexpr (LATENT != 0)
-      for (int other = p.first_seq; other < seq; ++other) first_row += (p.seq_kv_len[other] + kKeys - 1) / kKeys * kKeys;
+      for (int other = p.first_seq; other < seq; ++other)
+        if (p.seq_q_len[other] >= p.min_q_len) first_row += (p.seq_kv_len[other] + kKeys - 1) / kKeys * kKeys;
     for (int it = 0; it < num_tiles; ++it) {
       const int s = it % stages;
       if (it >= stages && !bar_wait(&empty[s], ((it / stages) - 1) & 1)) {
@@ -804,19 +806,20 @@ int arena_map(CUtensorMap* map, const void* arena, int64_t rows, int piece_rows)
   return 0;
 }
 
-// The latents of the requests from first_seq on, out of the cache's pages into rows of one matrix, each request padded to whole tiles
-// with zeros. One block per 16 rows of a request, 16 bytes a thread.
+// The latents of the requests from first_seq on that have min_q_len new tokens and more, out of the cache's pages into rows of one matrix,
+// each request padded to whole tiles with zeros. One block per 16 rows of a request, 16 bytes a thread.
 constexpr int kGatherRows = 16;
 
 __global__ void __launch_bounds__(256)
-latent_gather_kernel(const __nv_bfloat16* rows, const int* __restrict__ block_table, const int* __restrict__ seq_kv_len, int first_seq, int max_pages, int num_pages,
-                     int page_size, int row_dim, __nv_bfloat16* out, int* err) {
+latent_gather_kernel(const __nv_bfloat16* rows, const int* __restrict__ block_table, const int* __restrict__ seq_q_len, const int* __restrict__ seq_kv_len, int first_seq,
+                     int min_q_len, int max_pages, int num_pages, int page_size, int row_dim, __nv_bfloat16* out, int* err) {
   wait_for_predecessor();
   let_successor_start();
   const int seq = first_seq + blockIdx.y, len = seq_kv_len[seq], padded = (len + kKeys - 1) / kKeys * kKeys, row0 = blockIdx.x * kGatherRows;
-  if (row0 >= padded) return;
+  if (row0 >= padded || seq_q_len[seq] < min_q_len) return;
   int64_t first = row0;
-  for (int other = first_seq; other < seq; ++other) first += (seq_kv_len[other] + kKeys - 1) / kKeys * kKeys;
+  for (int other = first_seq; other < seq; ++other)
+    if (seq_q_len[other] >= min_q_len) first += (seq_kv_len[other] + kKeys - 1) / kKeys * kKeys;
   const int chunks = row_dim / 8;
   for (int i = threadIdx.x; i < kGatherRows * chunks; i += blockDim.x) {
     const int r = i / chunks, c = i % chunks * 8, key = row0 + r;
@@ -953,23 +956,25 @@ B200_API int b200_latent_prefill_supported(int heads, int dim, int rot_dim, int 
   return heads > 0 && heads <= 65535 && dim == kDim && vdim == kDim && (rot_dim == 0 || rot_dim == 64) && rank > 0 && rank % 8 == 0 && page_size > 0;
 }
 
-// Rows [requests' keys, each request padded to a multiple of 128][row_dim] out of the cache's pages [pages][page_size][row_dim].
-B200_API int b200_latent_gather(const void* rows, const int* block_table, const int* seq_kv_len, int first_seq, int num_seqs, int max_kv_len, int max_pages,
-                                int num_pages, int page_size, int row_dim, void* out, int* err, cudaStream_t stream) {
+// Rows [requests' keys, each request padded to a multiple of 128][row_dim] out of the cache's pages [pages][page_size][row_dim]; requests of
+// fewer than min_q_len new tokens are left out.
+B200_API int b200_latent_gather(const void* rows, const int* block_table, const int* seq_q_len, const int* seq_kv_len, int first_seq, int num_seqs, int min_q_len,
+                                int max_kv_len, int max_pages, int num_pages, int page_size, int row_dim, void* out, int* err, cudaStream_t stream) {
   if (num_seqs <= 0) return 0;
   B200_REQUIRE(num_seqs <= 65535 && max_kv_len > 0 && page_size > 0 && max_pages > 0 && row_dim > 0 && row_dim % 8 == 0, "latent_gather: bad sizes");
   B200_REQUIRE(reinterpret_cast<uintptr_t>(rows) % 16 == 0 && reinterpret_cast<uintptr_t>(out) % 16 == 0, "latent_gather: operands must be aligned to 16 bytes");
   const int padded = (max_kv_len + kKeys - 1) / kKeys * kKeys;
-  launch_kernel(latent_gather_kernel, dim3(padded / kGatherRows, num_seqs), dim3(256), 0, stream, static_cast<const __nv_bfloat16*>(rows), block_table, seq_kv_len,
-                first_seq, max_pages, num_pages, page_size, row_dim, static_cast<__nv_bfloat16*>(out), err);
+  launch_kernel(latent_gather_kernel, dim3(padded / kGatherRows, num_seqs), dim3(256), 0, stream, static_cast<const __nv_bfloat16*>(rows), block_table, seq_q_len,
+                seq_kv_len, first_seq, min_q_len, max_pages, num_pages, page_size, row_dim, static_cast<__nv_bfloat16*>(out), err);
   return b200_check_launch("latent_gather");
 }
 
 // The portions' attention itself. `q`: plain query parts (128 numbers a head, heads q_head_ld and rows q_ld numbers apart), `q_rot` [rows][heads * 64] or
-// null; `expanded` [key_rows][heads * 256] and `latents` [key_rows][rank + rot_dim] as `b200_latent_gather` lays rows out; `out` [rows][heads * 128].
+// null; `expanded` [key_rows][heads * 256] and `latents` [key_rows][rank + rot_dim] as `b200_latent_gather` lays rows out, with the same min_q_len;
+// `out` [rows][heads * 128].
 B200_API int b200_latent_prefill_tcgen05(const void* q, int64_t q_ld, int q_head_ld, const void* q_rot, const void* expanded, const void* latents, int64_t key_rows,
                                          int rank, int rot_dim, const int* seq_q_start, const int* seq_q_len, const int* seq_kv_len, int first_seq, int num_seqs,
-                                         int max_q_len, int heads, float scale, const float* sink, const void* gate, int64_t gate_ld, void* out, int* err,
+                                         int min_q_len, int max_q_len, int heads, float scale, const float* sink, const void* gate, int64_t gate_ld, void* out, int* err,
                                          cudaStream_t stream) {
   if (num_seqs <= 0) return 0;
   B200_REQUIRE(b200_latent_prefill_supported(heads, kDim, rot_dim, kDim, rank, 1) && (rot_dim == 0) == (q_rot == nullptr), "latent_prefill_tcgen05: shape not taken");
@@ -997,6 +1002,7 @@ B200_API int b200_latent_prefill_tcgen05(const void* q, int64_t q_ld, int q_head
   p.gate_ld = gate_ld;
   p.q_head_ld = q_head_ld;
   p.latent_rank = rank;
+  p.min_q_len = min_q_len;
   CUtensorMap expanded_map, latent_map;
   if (matrix_map(&expanded_map, expanded, key_rows, static_cast<int64_t>(heads) * 2 * kDim) != 0) return -1;
   if (matrix_map(&latent_map, latents, key_rows, rank + rot_dim) != 0) return -1;

@@ -45,7 +45,7 @@ struct LatentParams {
   __nv_bfloat16* out;           // [token][head][rank] through the two strides
   int64_t out_token, out_head;
   float* partial;               // [seq][row][piece][2 + rank] when the keys are cut
-  int rows_cap;                 // rows per request in `partial`
+  int rows_cap;                 // rows per request in `partial`; requests with more rows are left out
   int heads, rank, rot_dim;
   float scale_log2;
   int stages;                   // K tiles in flight: 3 where shared memory allows, else 2
@@ -129,6 +129,7 @@ __global__ void __launch_bounds__(64 * RW, 1) latent_attention_mma_kernel(const 
   const int q_start = p.seq_q_start[seq], q_len = p.seq_q_len[seq], kv_len = p.seq_kv_len[seq];
   wait_for_predecessor();
   const int rows_total = q_len * p.heads;
+  if (rows_total > p.rows_cap) return;
   const int blocks = (rows_total + BM - 1) / BM;
   if (static_cast<int>(blockIdx.x) >= blocks) return;
   const int block = blocks - 1 - blockIdx.x;  // the rows with the most keys first
@@ -398,7 +399,8 @@ B200_API int64_t b200_latent_attention_mma_scratch(int num_seqs, int max_q_len, 
   return pieces > 1 ? static_cast<int64_t>(num_seqs) * max_q_len * heads * pieces * (rank + 2) : 0;
 }
 
-// Requests first_seq .. first_seq + num_seqs of the step, each with up to max_q_len new tokens.
+// Requests first_seq .. first_seq + num_seqs of the step that have at most max_q_len new tokens (the others' outputs are left alone; with
+// pieces > 1 all have to).
 B200_API int b200_latent_attention_mma(const void* q_lat, int64_t q_lat_token, int64_t q_lat_head, const void* q_rot,
                                        const void* arena, const int* block_table, int max_pages, int num_pages, int page_size,
                                        const int* seq_q_start, const int* seq_q_len, const int* seq_kv_len, int first_seq,

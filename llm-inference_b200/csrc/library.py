@@ -64,8 +64,8 @@ _SIGNATURES: dict[str, list] = {
     "b200_paged_decode_attention_tma": [c_void_p] * 8 + [c_int] * 9 + [c_float, c_int, c_int] + [c_void_p] * 5,
     "b200_flash_prefill_tcgen05": [c_void_p] * 8 + [c_int] * 12 + [c_float, c_int, c_float, c_void_p, c_void_p, c_int, c_int, c_void_p, c_void_p,
                                    c_void_p, c_void_p],
-    "b200_latent_gather": [c_void_p] * 3 + [c_int] * 7 + [c_void_p] * 3,
-    "b200_latent_prefill_tcgen05": [c_void_p, c_int64, c_int] + [c_void_p] * 3 + [c_int64, c_int, c_int] + [c_void_p] * 3 + [c_int] * 4
+    "b200_latent_gather": [c_void_p] * 4 + [c_int] * 8 + [c_void_p] * 3,
+    "b200_latent_prefill_tcgen05": [c_void_p, c_int64, c_int] + [c_void_p] * 3 + [c_int64, c_int, c_int] + [c_void_p] * 3 + [c_int] * 5
                                    + [c_float, c_void_p, c_void_p, c_int64] + [c_void_p] * 3,
     "b200_skinny_gemm": [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_void_p, c_int64, c_void_p, c_int, c_void_p],
     "b200_stream_gemm": [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_void_p, c_void_p],

@@ -135,6 +135,8 @@ def attend_latent(
     rank: int,
     rot_dim: int,
     scale: float,
+    *,
+    most_tokens: int | None = None,
 ) -> None:
     """Attention over cached latents (parts/latent_attention.py). bfloat16 with a shape the
     tensor-core kernel takes: the step's single-token requests (which lead the batch) in one
@@ -142,7 +144,8 @@ def attend_latent(
     prompt portions in another, one block per 64 (token, head) rows. float32 and every other
     shape: the plain kernel. ``options["attention"]``: ``"plain"`` forces the plain kernel,
     ``"flash"`` refuses what the tensor-core kernel does not take; ``options["latent_pieces"]``
-    forces the number of pieces."""
+    forces the number of pieces. ``most_tokens``: the operands reach up to the last request of at most so many new tokens, longer ones
+    attend elsewhere and what their rows of ``out`` hold afterwards is not defined."""
     choice = ctx.options.get("attention", "auto")
     tuned = (
         choice != "plain" and q_lat.dtype == torch.bfloat16 and not cache.window
@@ -158,6 +161,6 @@ def attend_latent(
         pieces = int(ctx.options.get("latent_pieces", 0)) or ops.latent_attention_pieces(decode_seqs, heads, ctx.max_kv_len, ops.sm_count(ctx))
         ops.latent_attention_mma(ctx, cache, q_lat, q_rot, sink, gate, out, heads, rank, rot_dim, scale,
                                  first_seq=0, num_seqs=decode_seqs, max_q_len=1, pieces=pieces)
-    if ctx.num_seqs > decode_seqs and q_lat.shape[1] > decode_seqs:  # rows of the single tokens alone: the portions were expanded
+    if ctx.num_seqs > decode_seqs and q_lat.shape[1] > decode_seqs:
         ops.latent_attention_mma(ctx, cache, q_lat, q_rot, sink, gate, out, heads, rank, rot_dim, scale,
-                                 first_seq=decode_seqs, num_seqs=ctx.num_seqs - decode_seqs, max_q_len=ctx.max_q_len)
+                                 first_seq=decode_seqs, num_seqs=ctx.num_seqs - decode_seqs, max_q_len=ctx.max_q_len if most_tokens is None else most_tokens)

@@ -31,7 +31,7 @@ class LatentAttention(Part):
     ``position`` None) positions do not enter at all: the cached row is the latent alone, and both latents' norms and the
     cache write are one kernel.
 
-    Prompt portions long enough (``ops.latent_expansion_rows``) take the other reading of the same formula: their keys and values are
+    Requests whose prompt portion is long enough (``ops.latent_expansion``) take the other reading of the same formula: their keys and values are
     expanded from the latents by one product, and attention runs head by head on those.
 
     The query (or its latent), latent and gate projections are one matrix product. Tensor names are
@@ -126,24 +126,26 @@ class LatentAttention(Part):
         gate = proj[:, gate_at : gate_at + gates] if self.has_gate else None
         head_gate = None if self.gate_per_element else gate
         attn = ctx.buffer("attn", (t, heads * self.vdim))
-        key_rows = ops.latent_expansion_rows(ctx, cache, h.dtype, heads, self.dim, rot, self.vdim, rank)
-        if key_rows:
-            ops.latent_portions(ctx, cache, key_rows, queries, q_rot, self.w_expand, self.sink, head_gate, attn, heads, self.dim, rank, rot, self.scale)
-        absorbed = ctx.num_decode_seqs if key_rows else t  # rows that attend in the latent space (single tokens lead the batch)
+        # Rows of longer requests among the absorbed ones are computed for nothing and written over below.
+        fewest, key_rows, absorbed = ops.latent_expansion(ctx, cache, h.dtype, heads, self.dim, rot, self.vdim, rank)
         if absorbed:
             q_plain = queries[:absorbed].view(absorbed, heads, self.dim + rot)[:, :, : self.dim].transpose(0, 1)
             q_lat = ops.linear_per_head(ctx, q_plain, self.w_uk_t, ctx.buffer("latent_q", (heads, absorbed, rank)))
             mixed = ctx.buffer("latent_out", (heads, absorbed, rank))
-            self.attend(ctx, cache, q_lat, q_rot[:absorbed], None if head_gate is None else head_gate[:absorbed], mixed)
+            self.attend(ctx, cache, q_lat, q_rot[:absorbed], None if head_gate is None else head_gate[:absorbed], mixed,
+                        most_tokens=fewest - 1 if key_rows else None)
             ops.linear_per_head(ctx, mixed, self.w_uv, attn[:absorbed].view(absorbed, heads, self.vdim).transpose(0, 1))
+        if key_rows:
+            ops.latent_portions(ctx, cache, fewest, key_rows, queries, q_rot, self.w_expand, self.sink, head_gate, attn, heads, self.dim, rank, rot, self.scale)
         if self.gate_per_element:
             attn = ops.sigmoid_mul(ctx, attn, gate, ctx.buffer("attn_gated", (t, heads * self.vdim)))
         return ops.linear(ctx, attn, self.w_o, ctx.buffer(self.out_name, (t, self.hidden_size)))
 
-    def attend(self, ctx: StepContext, cache: CacheView, q_lat, q_rot, gate, out) -> None:
+    def attend(self, ctx: StepContext, cache: CacheView, q_lat, q_rot, gate, out, *, most_tokens: int | None = None) -> None:
         from . import attention_dispatch
 
-        attention_dispatch.attend_latent(ctx, cache, q_lat, q_rot, self.sink, gate, out, self.heads, self.rank, self.rot_dim, self.scale)
+        attention_dispatch.attend_latent(ctx, cache, q_lat, q_rot, self.sink, gate, out, self.heads, self.rank, self.rot_dim, self.scale,
+                                         most_tokens=most_tokens)
 
 
 register_part("mixer", "latent_attention", LatentAttention)

@@ -12,6 +12,7 @@ from ctypes import c_float, c_int, c_int64
 from dataclasses import dataclass
 from typing import Any
 
+import numpy as np
 import torch
 
 from ..csrc.library import KernelError, dtype_code, ptr
@@ -867,35 +868,62 @@ def latent_attention_mma(
     return out
 
 
-# Portions shorter than this on average attend in the latent space, where nothing is expanded: per key the expansion costs 2 x 256 x
-# rank flops a head, which a portion of a few dozen queries does not earn back.
-LATENT_EXPAND_FROM = 64
+# Portions of at least so many tokens expand their keys and values: per key the expansion costs the same whatever the portion, and the
+# latent space a walk for every 64 (token, head) rows, so keys and heads cancel out as soon as there is work for every SM. Whole layers
+# of 12 heads on a B200, expanded against the latent space: 60 requests of 16 tokens behind 500 keys 236 and 174 us, of 48 tokens 273
+# and 352, of 100 tokens 332 and 698; behind 4,000 keys 1,125 and 930, 1,177 and 1,834, 1,261 and 3,659.
+LATENT_EXPAND_FROM = 48
+# Shorter portions leave SMs idle in the latent space, where one block walks 64 rows' keys one tile after another, so a few of them
+# expand all the same: where the keys to expand, at 0.4 ns a key and head (its bytes), cost less than the longest walk at 107 ns a key,
+# with a margin for the gather and the product as launches of their own. One request of 48 tokens behind 16,000 keys takes 317 us
+# expanded and 1,736 in the latent space; 20 of two tokens behind 500, 4,000 and 16,000 keys 86 and 82, 389 and 426, 1,516 and 1,582 us,
+# 60 of them behind 500 and 4,000 188 and 85, 1,090 and 449.
+LATENT_EXPAND_NS, LATENT_WALK_NS, LATENT_MARGIN_NS = 0.4, 107.0, 10_000.0
 LATENT_EXPAND_BYTES = 2 << 30  # at most this much scratch for expanded keys and values
 
 
-def latent_expansion_rows(ctx: StepContext, cache: CacheView, dtype: torch.dtype, heads: int, dim: int, rot_dim: int, vdim: int, rank: int) -> int:
-    """Key rows that the step's prompt portions would expand (every portion's keys padded to whole tiles of 128), or 0 where they attend
-    in the latent space: other sizes than the tcgen05 form takes, short portions, windows, ``options["attention"]`` other than
-    ``"auto"``, too much scratch."""
-    decode, seqs = ctx.num_decode_seqs, ctx.num_seqs - ctx.num_decode_seqs
+def latent_expand_from(new: np.ndarray, keys: np.ndarray, heads: int, sms: int) -> int:
+    """The fewest new tokens with which a request of the step expands: two where all portions do (``new`` tokens behind and among
+    ``keys``, one entry a portion), otherwise ``LATENT_EXPAND_FROM``."""
+    short = new < LATENT_EXPAND_FROM
+    if not short.any():
+        return LATENT_EXPAND_FROM
+    new, keys = new[short].astype(np.int64), keys[short].astype(np.int64)
+    blocks = -(-new * heads // 64)
+    walk = max(int(keys.max()), -(-int(blocks.sum()) // sms) * float((blocks * keys).sum()) / float(blocks.sum()))
+    expansion = float((-(-keys // 128) * 128).sum()) * heads * LATENT_EXPAND_NS
+    return 2 if expansion + LATENT_MARGIN_NS < walk * LATENT_WALK_NS else LATENT_EXPAND_FROM
+
+
+def latent_expansion(ctx: StepContext, cache: CacheView, dtype: torch.dtype, heads: int, dim: int, rot_dim: int, vdim: int, rank: int) -> tuple[int, int, int]:
+    """(fewest new tokens with which a request of the step expands its keys and values; the key rows of those requests, each padded to
+    whole tiles of 128; the step's rows up to the last request that attends in the latent space). No key rows where none expands: other
+    sizes than the tcgen05 form takes, windows, ``options["attention"]`` other than ``"auto"``, too much scratch."""
+    decode = ctx.num_decode_seqs
     if (
-        dtype != torch.bfloat16 or seqs <= 0 or cache.window or ctx.options.get("attention", "auto") != "auto"
-        or ctx.num_tokens - decode < LATENT_EXPAND_FROM * seqs
+        dtype != torch.bfloat16 or decode == ctx.num_seqs or cache.window or ctx.options.get("attention", "auto") != "auto"
         or not ctx.lib.lib.b200_latent_prefill_supported(heads, dim, rot_dim, vdim, rank, cache.page_size)
     ):
-        return 0
-    rows = sum(-(-int(n) // 128) * 128 for n in ctx.host.seq_kv_len[decode:])
-    return rows if rows * heads * (dim + vdim) * 2 <= LATENT_EXPAND_BYTES else 0
+        return 0, 0, ctx.num_tokens
+    new, keys = ctx.host.seq_q_len[decode:], ctx.host.seq_kv_len[decode:]
+    padded = -(-keys.astype(np.int64) // 128) * 128
+    for fewest in {latent_expand_from(new, keys, heads, sm_count(ctx)): None, LATENT_EXPAND_FROM: None}:
+        rows = int(padded[new >= fewest].sum())
+        if 0 < rows * heads * (dim + vdim) * 2 <= LATENT_EXPAND_BYTES:
+            absorbed = decode + np.flatnonzero(new < fewest)
+            last = int(absorbed[-1]) if absorbed.size else decode - 1
+            return fewest, rows, int(ctx.host.seq_q_start[last] + ctx.host.seq_q_len[last]) if last >= 0 else 0
+    return 0, 0, ctx.num_tokens
 
 
 def latent_portions(
-    ctx: StepContext, cache: CacheView, key_rows: int, queries: torch.Tensor, q_rot: torch.Tensor, w_expand: torch.Tensor, sink: torch.Tensor | None,
+    ctx: StepContext, cache: CacheView, fewest: int, key_rows: int, queries: torch.Tensor, q_rot: torch.Tensor, w_expand: torch.Tensor, sink: torch.Tensor | None,
     gate: torch.Tensor | None, out: torch.Tensor, heads: int, dim: int, rank: int, rot_dim: int, scale: float,
 ) -> torch.Tensor:
-    """Attention of the step's prompt portions with keys and values expanded from the cached latents: a gather of the portions' latents
-    out of their pages, one product with ``w_expand`` (``[heads * (dim + vdim), rank]``: a head's key matrix, then its value matrix),
+    """Attention of the step's prompt portions of ``fewest`` tokens and more with keys and values expanded from the cached
+    latents: a gather of the portions' latents out of their pages, one product with ``w_expand`` (``[heads * (dim + vdim), rank]``: a head's key matrix, then its value matrix),
     the tcgen05 prefill kernel. ``queries``: rows of ``heads * (dim + rot_dim)`` numbers, rotated parts not yet rotated (they are in
-    ``q_rot``); rows of single tokens, which lead the batch, are left alone."""
+    ``q_rot``); the other requests' rows of ``out`` are left alone."""
     first, row_dim = ctx.num_decode_seqs, rank + rot_dim
     _need(queries.stride(1) == 1 and queries.dtype == torch.bfloat16 and queries.shape[1] == heads * (dim + rot_dim), "latent_portions: bad queries")
     _need(tuple(out.shape) == (ctx.num_tokens, heads * dim) and out.is_contiguous() and out.dtype == torch.bfloat16, "latent_portions: bad output")
@@ -903,15 +931,15 @@ def latent_portions(
     _need(sink is None or (sink.dtype == torch.float32 and sink.numel() == heads), "latent_portions: the sink is float32 [heads]")
     latents = ctx.portion_buffer("latent_rows", (key_rows, row_dim), torch.bfloat16, LATENT_EXPAND_BYTES)
     ctx.lib.call(
-        "b200_latent_gather", ptr(cache.keys), ptr(cache.block_table), ptr(ctx.seq_kv_len), c_int(first), c_int(ctx.num_seqs - first), c_int(ctx.max_kv_len),
-        c_int(cache.max_pages), c_int(cache.num_pages), c_int(cache.page_size), c_int(row_dim), ptr(latents), ptr(ctx.err), ctx.stream,
+        "b200_latent_gather", ptr(cache.keys), ptr(cache.block_table), ptr(ctx.seq_q_len), ptr(ctx.seq_kv_len), c_int(first), c_int(ctx.num_seqs - first), c_int(fewest),
+        c_int(ctx.max_kv_len), c_int(cache.max_pages), c_int(cache.num_pages), c_int(cache.page_size), c_int(row_dim), ptr(latents), ptr(ctx.err), ctx.stream,
     )
     expanded = ctx.portion_buffer("latent_expanded", (key_rows, w_expand.shape[0]), torch.bfloat16, LATENT_EXPAND_BYTES)
     torch.mm(latents[:, :rank], w_expand.t(), out=expanded)
     ctx.lib.call(
         "b200_latent_prefill_tcgen05", ptr(queries), c_int64(queries.stride(0)), c_int(dim + rot_dim), ptr(q_rot if rot_dim else None), ptr(expanded), ptr(latents),
         c_int64(key_rows), c_int(rank), c_int(rot_dim), ptr(ctx.seq_q_start), ptr(ctx.seq_q_len), ptr(ctx.seq_kv_len), c_int(first), c_int(ctx.num_seqs - first),
-        c_int(ctx.max_q_len), c_int(heads), c_float(scale), ptr(sink), ptr(gate), c_int64(gate.stride(0) if gate is not None else 0), ptr(out), ptr(ctx.err), ctx.stream,
+        c_int(fewest), c_int(ctx.max_q_len), c_int(heads), c_float(scale), ptr(sink), ptr(gate), c_int64(gate.stride(0) if gate is not None else 0), ptr(out), ptr(ctx.err), ctx.stream,
     )
     return out
 
