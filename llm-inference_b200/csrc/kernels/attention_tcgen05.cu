@@ -952,8 +952,8 @@ B200_API int b200_flash_prefill_tcgen05(const void* q, const void* k_arena, cons
 }
 
 // Attention over latents of prompt portions with expanded keys and values: sizes the forms take.
-B200_API int b200_latent_prefill_supported(int heads, int dim, int rot_dim, int vdim, int rank, int page_size) {
-  return heads > 0 && heads <= 65535 && dim == kDim && vdim == kDim && (rot_dim == 0 || rot_dim == 64) && rank > 0 && rank % 8 == 0 && page_size > 0;
+B200_API int b200_latent_prefill_supported(int heads, int dim, int rot_dim, int vdim, int rank) {
+  return heads > 0 && heads <= 65535 && dim == kDim && vdim == kDim && (rot_dim == 0 || rot_dim == 64) && rank > 0 && rank % 8 == 0;
 }
 
 // Rows [requests' keys, each request padded to a multiple of 128][row_dim] out of the cache's pages [pages][page_size][row_dim]; requests of
@@ -977,7 +977,7 @@ B200_API int b200_latent_prefill_tcgen05(const void* q, int64_t q_ld, int q_head
                                          int min_q_len, int max_q_len, int heads, float scale, const float* sink, const void* gate, int64_t gate_ld, void* out, int* err,
                                          cudaStream_t stream) {
   if (num_seqs <= 0) return 0;
-  B200_REQUIRE(b200_latent_prefill_supported(heads, kDim, rot_dim, kDim, rank, 1) && (rot_dim == 0) == (q_rot == nullptr), "latent_prefill_tcgen05: shape not taken");
+  B200_REQUIRE(b200_latent_prefill_supported(heads, kDim, rot_dim, kDim, rank) && (rot_dim == 0) == (q_rot == nullptr), "latent_prefill_tcgen05: shape not taken");
   B200_REQUIRE(num_seqs <= 65535 && max_q_len > 0 && key_rows > 0 && key_rows % kKeys == 0 && q_ld % 8 == 0 && q_head_ld % 8 == 0, "latent_prefill_tcgen05: bad sizes");
   const auto aligned = [](const void* a) { return reinterpret_cast<uintptr_t>(a) % 16 == 0; };
   B200_REQUIRE(aligned(q) && aligned(q_rot) && aligned(expanded) && aligned(latents) && aligned(out), "latent_prefill_tcgen05: operands must be aligned to 16 bytes");

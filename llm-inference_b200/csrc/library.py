@@ -173,7 +173,7 @@ class KernelLibrary:
         self.lib.b200_latent_attention_mma_scratch.restype = c_int64
         self.lib.b200_portion_attention_f32_supported.argtypes = [c_int] * 3
         self.lib.b200_portion_attention_f32_supported.restype = c_int
-        self.lib.b200_latent_prefill_supported.argtypes = [c_int] * 6
+        self.lib.b200_latent_prefill_supported.argtypes = [c_int] * 5
         self.lib.b200_latent_prefill_supported.restype = c_int
         self.lib.b200_state_chunks_scratch.argtypes = [c_int] * 7
         self.lib.b200_state_chunks_scratch.restype = c_int64

@@ -4,6 +4,7 @@ from __future__ import annotations
 
 import torch
 
+from ..csrc.library import kernels
 from ..weights.loader import TensorSpec
 from . import ops
 from .base import KVCacheSpec, Part, PartSpec, build_part, register_part, whole_steps
@@ -89,9 +90,12 @@ class LatentAttention(Part):
         # [heads, rank, dim]: the product that carries a query into the latent space reads W_uk[n]^T.
         self.w_uk_t = tensors[p + "uk"].to(device=device, dtype=dtype).view(self.heads, self.dim, self.rank).transpose(1, 2).contiguous()
         self.w_uv = tensors[p + "uv"].to(device=device, dtype=dtype).view(self.heads, self.vdim, self.rank).contiguous()
-        # [heads * (dim + vdim), rank]: a head's keys and values out of a latent, for prompt portions long enough to expand them.
-        uk = tensors[p + "uk"].to(device=device, dtype=dtype).view(self.heads, self.dim, self.rank)
-        self.w_expand = torch.cat([uk, self.w_uv], dim=1).reshape(-1, self.rank).contiguous()
+        # [heads * (dim + vdim), rank]: a head's keys and values out of a latent, for prompt portions long enough to expand them, where the
+        # kernel for it takes the layer (a copy of both matrices, which steps of single tokens do not read).
+        self.w_expand = None
+        if dtype == torch.bfloat16 and device.type == "cuda" and not self.window and ops.latent_expansion_supported(kernels(), self.heads, self.dim, self.rot_dim, self.vdim, self.rank):
+            uk = tensors[p + "uk"].to(device=device, dtype=dtype).view(self.heads, self.dim, self.rank)
+            self.w_expand = torch.cat([uk, self.w_uv], dim=1).reshape(-1, self.rank).contiguous()
         self.w_o = tensors[p + "o"].to(device=device, dtype=dtype).contiguous()
         self.norm_weight = tensors[p + "dkv.norm"].to(device=device, dtype=torch.float32).contiguous()
         self.sink = tensors[p + "sink"].to(device=device, dtype=torch.float32).contiguous() if self.has_sink else None

@@ -895,6 +895,10 @@ def latent_expand_from(new: np.ndarray, keys: np.ndarray, heads: int, sms: int) 
     return 2 if expansion + LATENT_MARGIN_NS < walk * LATENT_WALK_NS else LATENT_EXPAND_FROM
 
 
+def latent_expansion_supported(lib, heads: int, dim: int, rot_dim: int, vdim: int, rank: int) -> bool:
+    return bool(lib.lib.b200_latent_prefill_supported(heads, dim, rot_dim, vdim, rank))
+
+
 def latent_expansion(ctx: StepContext, cache: CacheView, dtype: torch.dtype, heads: int, dim: int, rot_dim: int, vdim: int, rank: int) -> tuple[int, int, int]:
     """(fewest new tokens with which a request of the step expands its keys and values; the key rows of those requests, each padded to
     whole tiles of 128; the step's rows up to the last request that attends in the latent space). No key rows where none expands: other
@@ -902,7 +906,7 @@ def latent_expansion(ctx: StepContext, cache: CacheView, dtype: torch.dtype, hea
     decode = ctx.num_decode_seqs
     if (
         dtype != torch.bfloat16 or decode == ctx.num_seqs or cache.window or ctx.options.get("attention", "auto") != "auto"
-        or not ctx.lib.lib.b200_latent_prefill_supported(heads, dim, rot_dim, vdim, rank, cache.page_size)
+        or not latent_expansion_supported(ctx.lib, heads, dim, rot_dim, vdim, rank)
     ):
         return 0, 0, ctx.num_tokens
     new, keys = ctx.host.seq_q_len[decode:], ctx.host.seq_kv_len[decode:]

@@ -106,3 +106,16 @@ def test_neighbours_change_no_bits_of_a_long_portion(form):
     beside, _ = forward(part, (100, 50), (0, 10), rows)
     split, _ = forward(part, (100, 25, 25), (0, 10, 0), rows)  # the 50 become two short requests
     assert torch.equal(beside[:100], split[:100])
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("change,dtype,kept", [({}, torch.bfloat16, True), ({}, torch.float32, False), ({"window": 40}, torch.bfloat16, False),
+                                               ({"dim": 96}, torch.bfloat16, False), ({"rank": 68}, torch.bfloat16, False)])
+def test_the_expanding_matrix_is_held_only_where_it_can_be_used(change, dtype, kept):
+    from llm_inference_b200.parts import PartSpec, build_part
+    from llm_inference_b200.weights import random_weights
+
+    sizes = dict(dict(prefix="", hidden_size=64, heads=2, dim=128, rot_dim=0, vdim=128, rank=64, scale=0.1, eps=1e-5), **change)
+    part = build_part("mixer", PartSpec("latent_attention", sizes))
+    part.load(random_weights(part.tensor_specs(), seed=3, std=0.2), dtype, torch.device("cuda:0"))
+    assert (part.w_expand is not None) == kept
