@@ -1355,12 +1355,13 @@ def moe_route(ctx: StepContext, logits: torch.Tensor, groups: int, keep: int, to
     )
 
 
-# Where tall tiles on tcgen05 beat short ones on mma.sync before an expert fills two of them: its tile of 128 places has to be a quarter
-# full, and the whole work large enough to pay for the gather pass and the longer pipeline. Both products on a B200, mma.sync and tcgen05
-# in us: 32 experts of 1,120 x 1,536, four a token: 256 tokens 137 and 134, 512 tokens 186 and 138, 1,777 tokens 413 and 190; of 2,368 x
-# 3,584: 192 tokens 352 and 378, 256 tokens 391 and 385, 1,024 tokens 999 and 463; 16 experts of 512 x 2,048, two a token: 512 tokens 83
-# and 98, 1,024 tokens 116 and 106; of 256 x 512: 2,048 tokens 63 and 79. Both form the same sums in the same order, to the bit.
-MOE_TALL_SLOTS = 32
+# Where tall tiles on tcgen05 beat short ones on mma.sync before an expert fills two of them: its tile of 128 places has to be about a
+# third full, and the whole work large enough to pay for the gather pass and the longer pipeline. Sorting and both products on a B200,
+# mma.sync and tcgen05 in us. By slots an expert: 16 experts of 2,368 x 3,584: 32 slots 189 and 219, 38 slots 213 and 221; 128 of 768 x
+# 2,048: 32 slots 293 and 316, 40 slots 360 and 324; 32 of 1,120 x 1,536: 32 slots 102 and 94, 40 slots 129 and 97, 48 slots 132 and 98; 32 of
+# 704 x 2,048: 36 slots 104 and 96, 40 slots 106 and 97. By the work: 16 experts of 512 x 2,048 at 1.48e9 65 and 71, 1.61e9 80 and 72, 1.88e9 87
+# and 75; 64 of 512 x 1,024 at 1.21e9 79 and 88, 1.61e9 91 and 91, 2.01e9 102 and 95. Both form the same sums in the same order, to the bit.
+MOE_TALL_SLOTS = 40
 MOE_TALL_PRODUCTS = 1_750_000_000  # slots x width x inner width
 
 
