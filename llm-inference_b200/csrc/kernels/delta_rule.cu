@@ -402,7 +402,7 @@ B200_API int b200_delta_prepare(const void* proj, int ld, const void* decay_in, 
   B200_REQUIRE(smem <= 200 * 1024, "delta_prepare: %d convolved channels do not fit shared memory", channels);
   const int threads = 256;
   const int update_blocks = (channels + threads - 1) / threads;  // a thread per channel: the slots' update is a tail of its own
-  // The wide form from a block an SM on, with rows, taps and results on 16-byte (bfloat16 rows: 8-byte) boundaries.
+  // The wide form from half a block an SM on, with rows, taps and results on 16-byte (bfloat16 rows: 8-byte) boundaries.
   const size_t wide_smem = sizeof(float) * kWideTokens * 2 * kv_heads * dk;
   const auto on = [](const void* p, int bytes) { return reinterpret_cast<uintptr_t>(p) % bytes == 0; };
   const int in_bytes = dtype == DTYPE_F32 ? 16 : 8;

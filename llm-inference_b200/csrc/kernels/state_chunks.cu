@@ -446,7 +446,7 @@ linear_chunk_prepare_kernel(LinearRule in, const int* __restrict__ seq_q_start, 
   float* uk = rk + C * (C + 1);
   float* rb = uk + C * (C + 1);
   float* ub = rb + C * (C + 1);
-  float* es = MEMORY ? uk : ub + (GENERAL ? C * (C + 1) : 0);  // MEMORY: [C]: the keeps up to a token, multiplied, times scale
+  float* es = MEMORY ? uk : ub + (GENERAL ? C * (C + 1) : 0);  // MEMORY: [C]: the keeps up to a token, multiplied
   float* fs = es + C;                                           // MEMORY: [C]: the keeps behind a token times its put
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int64_t ld_in = in.ld, at_in = static_cast<int64_t>(head) * dk;

@@ -36,7 +36,7 @@ FORMS = {
 @pytest.mark.parametrize("form", FORMS)
 @pytest.mark.parametrize("runs,starts", [((128,), (0,)), ((1, 1, 129, 66), (77, 0, 3, 127)), ((200, 64), (0, 192))])
 def test_expanded_portions_agree_with_the_latent_space(form, runs, starts):
-    from llm_inference_b200.parts import PartSpec, build_part
+    from llm_inference_b200.parts import PartSpec, build_part, ops
     from llm_inference_b200.weights import random_weights
 
     sizes = dict(FORMS[form])
@@ -56,6 +56,8 @@ def test_expanded_portions_agree_with_the_latent_space(form, runs, starts):
         view.keys.normal_(0.0, 0.7)
         ctx.options = {"attention": choice}
         results[choice] = part.forward(ctx, view, h).double().clone()
+        rows = ops.latent_expansion(ctx, view, h.dtype, heads, 128, rot, 128, sizes["rank"])[1]
+        assert (rows > 0) == (choice == "auto")  # the tcgen05 form is what is compared with the two others
         runner.check()
     scale = results["plain"].abs().max()
     off = {name: ((results[name] - results["plain"]).norm() / results["plain"].norm()).item() for name in ("auto", "flash")}
