@@ -12,7 +12,6 @@ from ctypes import c_float, c_int, c_int64
 from dataclasses import dataclass
 from typing import Any
 
-import numpy as np
 import torch
 
 from ..csrc.library import KernelError, dtype_code, ptr
@@ -882,17 +881,24 @@ LATENT_EXPAND_NS, LATENT_WALK_NS, LATENT_MARGIN_NS = 0.4, 107.0, 10_000.0
 LATENT_EXPAND_BYTES = 2 << 30  # at most this much scratch for expanded keys and values
 
 
-def latent_expand_from(new: np.ndarray, keys: np.ndarray, heads: int, sms: int) -> int:
+def latent_expand_from(new: list[int], keys: list[int], heads: int, sms: int) -> int:
     """The fewest new tokens with which a request of the step expands: two where all portions do (``new`` tokens behind and among
     ``keys``, one entry a portion), otherwise ``LATENT_EXPAND_FROM``."""
-    short = new < LATENT_EXPAND_FROM
-    if not short.any():
+    short = [(n, k) for n, k in zip(new, keys) if n < LATENT_EXPAND_FROM]
+    if not short:
         return LATENT_EXPAND_FROM
-    new, keys = new[short].astype(np.int64), keys[short].astype(np.int64)
-    blocks = -(-new * heads // 64)
-    walk = max(int(keys.max()), -(-int(blocks.sum()) // sms) * float((blocks * keys).sum()) / float(blocks.sum()))
-    expansion = float((-(-keys // 128) * 128).sum()) * heads * LATENT_EXPAND_NS
-    return 2 if expansion + LATENT_MARGIN_NS < walk * LATENT_WALK_NS else LATENT_EXPAND_FROM
+    most, longest = max(short)[0], max(keys)
+    if sum(k for _, k in short) * heads * LATENT_EXPAND_NS + LATENT_MARGIN_NS >= longest * -(-len(short) * -(-most * heads // 64) // sms) * LATENT_WALK_NS:
+        return LATENT_EXPAND_FROM  # not even if all were as long as the longest
+    blocks = pairs = longest = padded = 0
+    for n, k in short:
+        b = -(-n * heads // 64)
+        blocks += b
+        pairs += b * k
+        longest = max(longest, k)
+        padded += -(-k // 128) * 128
+    walk = max(longest, -(-blocks // sms) * pairs / blocks)
+    return 2 if padded * heads * LATENT_EXPAND_NS + LATENT_MARGIN_NS < walk * LATENT_WALK_NS else LATENT_EXPAND_FROM
 
 
 def latent_expansion_supported(lib, heads: int, dim: int, rot_dim: int, vdim: int, rank: int) -> bool:
@@ -909,15 +915,21 @@ def latent_expansion(ctx: StepContext, cache: CacheView, dtype: torch.dtype, hea
         or not latent_expansion_supported(ctx.lib, heads, dim, rot_dim, vdim, rank)
     ):
         return 0, 0, ctx.num_tokens
-    new, keys = ctx.host.seq_q_len[decode:], ctx.host.seq_kv_len[decode:]
-    padded = -(-keys.astype(np.int64) // 128) * 128
-    for fewest in {latent_expand_from(new, keys, heads, sm_count(ctx)): None, LATENT_EXPAND_FROM: None}:
-        rows = int(padded[new >= fewest].sum())
+    new, keys = ctx.host.seq_q_len[decode:].tolist(), ctx.host.seq_kv_len[decode:].tolist()
+    fewest = latent_expand_from(new, keys, heads, sm_count(ctx))
+    while max(new) >= fewest:
+        rows = sum(-(-k // 128) for n, k in zip(new, keys) if n >= fewest) * 128
         if 0 < rows * heads * (dim + vdim) * 2 <= LATENT_EXPAND_BYTES:
-            absorbed = decode + np.flatnonzero(new < fewest)
-            last = int(absorbed[-1]) if absorbed.size else decode - 1
-            return fewest, rows, int(ctx.host.seq_q_start[last] + ctx.host.seq_q_len[last]) if last >= 0 else 0
-    return 0, 0, ctx.num_tokens
+            break
+        if fewest == LATENT_EXPAND_FROM:
+            return 0, 0, ctx.num_tokens
+        fewest = LATENT_EXPAND_FROM
+    else:
+        return 0, 0, ctx.num_tokens
+    last = len(new)
+    while last and new[last - 1] >= fewest:
+        last -= 1
+    return fewest, rows, decode + sum(new[:last])  # single tokens lead the batch
 
 
 def latent_portions(

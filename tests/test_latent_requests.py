@@ -3,7 +3,6 @@ ones where that takes less than their walks in the latent space, in whatever ord
 
 from __future__ import annotations
 
-import numpy as np
 import pytest
 import torch
 
@@ -17,12 +16,12 @@ from test_latent_portions import FORMS, step_of
 def test_short_portions_expand_where_that_was_measured_to_take_less(requests, new, keys, heads, expand):
     from llm_inference_b200.parts import ops
 
-    lengths = np.full(requests, new, dtype=np.int32), np.full(requests, keys + new, dtype=np.int32)
+    lengths = [new] * requests, [keys + new] * requests
     assert (ops.latent_expand_from(*lengths, heads, 148) == 2) == expand
     # Long portions beside them change nothing; without short ones there is nothing to decide.
-    beside = np.append(lengths[0], 2000).astype(np.int32), np.append(lengths[1], 2000).astype(np.int32)
+    beside = lengths[0] + [2000], lengths[1] + [2000]
     assert ops.latent_expand_from(*beside, heads, 148) == ops.latent_expand_from(*lengths, heads, 148)
-    assert ops.latent_expand_from(np.array([48, 2000]), np.array([48, 2000]), heads, 148) == ops.LATENT_EXPAND_FROM
+    assert ops.latent_expand_from([48, 2000], [48, 2000], heads, 148) == ops.LATENT_EXPAND_FROM
 
 
 def built(form):
