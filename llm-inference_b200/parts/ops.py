@@ -1013,11 +1013,20 @@ GENERAL_DELTA_CHUNK_FROM = 256
 # tokens, 56 and 54 at 200, 63 and 107 at 512, 219 and 579 at 2,048; the whole mixer 67 and 64 at 230 tokens of 12 heads, 79 and 84 at 300 in
 # two requests.
 MEMORY_CHUNK_FROM = 256
+# Both of these rules' steps token by token are short, so where enough (request, head) chains stand side by side to fill the SMs, chunks come
+# level only in longer portions. Whole mixers, tokens and chunks: generalized rule, 24 heads, requests of 300 tokens: 4 of them 189 and 198 us,
+# 8 318 and 340, 13 479 and 517; of 512: 4 of them 301 and 294, 8 530 and 532; one of 300 with 80 heads 245 and 241. Matrix memory, 12 heads, of
+# 300: 4 of them 200 and 158, 8 287 and 308, 13 422 and 488; 8 of 512 471 and 470; of 300 with 40 heads: one 213 and 197, 8 1,135 and 1,232.
+MANY_CHAINS, MANY_CHAINS_CHUNK_FROM = 96, 512
 # Scratch grows with the step's tokens (0.13 MB a token at 28 heads of 128 x 128): past this a step takes its heads in parts, and past so
 # many parts it walks its portions token by token, as if they were short, in the memory that takes.
 CHUNK_SCRATCH_BYTES = 2 << 30
 CHUNK_PARTS = 3  # where chunks in parts stop being faster: state_chunks.cu has the figures
 _DELTA, _GENERAL_DELTA, _LINEAR, _MEMORY = 0, 1, 2, 3  # csrc/kernels/state_chunks.cu
+
+
+def _chunk_from(ctx: StepContext, line: int, heads: int) -> int:
+    return MANY_CHAINS_CHUNK_FROM if (ctx.num_seqs - ctx.num_decode_seqs) * heads >= MANY_CHAINS else line
 
 
 def _chunk_scratch(
@@ -1074,7 +1083,7 @@ def _linear_chunks(
 ) -> int:
     """As :func:`_delta_chunks`, for the rules in which the values enter as they are."""
     tokens = r.shape[0]
-    rule, longer_than = (_LINEAR, LINEAR_CHUNK_FROM) if u is None else (_GENERAL_DELTA, GENERAL_DELTA_CHUNK_FROM)
+    rule, longer_than = (_LINEAR, LINEAR_CHUNK_FROM) if u is None else (_GENERAL_DELTA, _chunk_from(ctx, GENERAL_DELTA_CHUNK_FROM, heads))
     scratch, walked = _chunk_scratch(ctx, rule, longer_than, tokens, heads, heads, dk, dv)
     if scratch is None:
         return walked
@@ -1823,7 +1832,7 @@ def mlstm(ctx: StepContext, proj: torch.Tensor, columns: tuple[int, int, int, in
     single = ctx.num_tokens == ctx.num_seqs
     gates = None if single else ctx.buffer("mlstm_gates", (tokens, 3 * heads), f32).data_ptr()  # three arrays [tokens][heads]
     num, den = ctx.buffer("mlstm_num", (tokens, heads * dv), f32), ctx.buffer("mlstm_den", (tokens, heads), f32)
-    scratch, walked = (None, ctx.num_seqs) if single else _chunk_scratch(ctx, _MEMORY, MEMORY_CHUNK_FROM, tokens, heads, heads, dk, dv)
+    scratch, walked = (None, ctx.num_seqs) if single else _chunk_scratch(ctx, _MEMORY, _chunk_from(ctx, MEMORY_CHUNK_FROM, heads), tokens, heads, heads, dk, dv)
     ctx.lib.call(
         "b200_mlstm", ptr(proj), c_int(proj.shape[1]), *(c_int(c) for c in columns), ptr(i_bias), ptr(f_bias), c_float(cap), ptr(ctx.seq_q_start),
         ptr(ctx.seq_q_len), ptr(ctx.seq_slot), c_int(ctx.num_seqs), c_int(walked), c_int(tokens), c_int(1 if single else 0), c_int(heads), c_int(dk), c_int(dv),
