@@ -130,8 +130,16 @@ class LatentAttention(Part):
         gate = proj[:, gate_at : gate_at + gates] if self.has_gate else None
         head_gate = None if self.gate_per_element else gate
         attn = ctx.buffer("attn", (t, heads * self.vdim))
-        # Rows of longer requests among the absorbed ones are computed for nothing and written over below.
         fewest, key_rows, absorbed = ops.latent_expansion(ctx, cache, h.dtype, heads, self.dim, rot, self.vdim, rank)
+
+        def expand() -> None:
+            ops.latent_portions(ctx, cache, fewest, key_rows, queries, q_rot, self.w_expand, self.sink, head_gate, attn, heads, self.dim, rank, rot, self.scale)
+
+        # Rows of longer requests among the absorbed ones are computed for nothing and then written over. Where there are none the long
+        # portions go first: the host launches the short kernels while they run.
+        written_over = absorbed > ctx.num_decode_seqs
+        if key_rows and not written_over:
+            expand()
         if absorbed:
             q_plain = queries[:absorbed].view(absorbed, heads, self.dim + rot)[:, :, : self.dim].transpose(0, 1)
             q_lat = ops.linear_per_head(ctx, q_plain, self.w_uk_t, ctx.buffer("latent_q", (heads, absorbed, rank)))
@@ -139,8 +147,8 @@ class LatentAttention(Part):
             self.attend(ctx, cache, q_lat, q_rot[:absorbed], None if head_gate is None else head_gate[:absorbed], mixed,
                         most_tokens=fewest - 1 if key_rows else None)
             ops.linear_per_head(ctx, mixed, self.w_uv, attn[:absorbed].view(absorbed, heads, self.vdim).transpose(0, 1))
-        if key_rows:
-            ops.latent_portions(ctx, cache, fewest, key_rows, queries, q_rot, self.w_expand, self.sink, head_gate, attn, heads, self.dim, rank, rot, self.scale)
+        if key_rows and written_over:
+            expand()
         if self.gate_per_element:
             attn = ops.sigmoid_mul(ctx, attn, gate, ctx.buffer("attn_gated", (t, heads * self.vdim)))
         return ops.linear(ctx, attn, self.w_o, ctx.buffer(self.out_name, (t, self.hidden_size)))
