@@ -19,16 +19,15 @@
 //   chunk_walk       a head's chunks one after another, a tile of 16 columns of S per block: U = W + Y S, S <- e S + (G_last K)^T U;
 //   chunk_scan       the same without U: S <- e S + the chunk's own sum, element by element;
 //   chunk_out        all chunks side by side again: O = (e Q) S + A U, from the states left at each chunk's start.
-// Only what the next chunk waits for is in the walk. Everything is 32-bit FMAs (no reduced-precision tensor-core mode): state,
-// decays and gates stay what they are token by token, up to the order of sums. Decays enter as products (or sums of their logarithms)
-// from token j on, never as quotients of products from the chunk's start, so strong decays in front of a pair cost it no digits.
+// Only what the next chunk waits for is in the walk. All numbers stay 32-bit: sums are FMAs where pairs of tokens are made and triangles
+// solved, and products on the tensor cores of numbers taken apart into three bfloat16 ones where a chunk meets the state (`mma_split`).
+// Against 64 bits, outputs and states are as far off as with FMAs throughout (2,048 tokens, 2-norm: a decay per channel 1.76e-7 and 1.53e-7,
+// before 1.92e-7 and 1.61e-7; generalized rule 1.77e-7 and 1.71e-7, before 1.96e-7 and 1.68e-7). Decays enter as products (or sums of their
+// logarithms) from token j on, never as quotients of products from the chunk's start, so strong decays in front of a pair cost it no digits.
 //
-// What bounds it: the walk, a chain of chunks in which a block does 2 x 32 x dk x 16 FMAs per chunk (1,024 cycles of an SM's FMA pipe
-// at dk = 128) and takes about twice as many cycles' worth of operands out of shared memory, between two block-wide barriers.
-// Measured on a B200 (one request of 2,048 tokens, heads of 128 x 128; all three kernels): a decay per channel, 12 heads: 731 us token
-// by token -> 252 us (prepare 60, walk 130, out 60), 28 heads: 941 -> 449; one decay per head (before: outputs and triangular products
-// inside the walk): 305 -> 252 and 525 -> 450. 24 heads of 64 x 64: the generalized rule 473 -> 244 us (prepare 100, walk 90, out 35), the
-// rule without a removal 564 -> 101 us (prepare 51, scan 16, out 27).
+// Measured on a B200 (one request of 2,048 tokens, all three kernels; walk and outputs with FMAs, on the tensor cores): heads of 128 x 128, a
+// decay per channel, 12 of them 230 -> 172 us (prepare 60, walk 135 -> 80, out 35 -> 30), 28 of them 430 -> 319; 24 heads of 64 x 64 under the
+// generalized rule 229 -> 181 us (prepare 97, walk 91 -> 55, out 35 -> 27).
 #include <type_traits>
 
 #include "common.cuh"
@@ -49,10 +48,11 @@ __device__ __forceinline__ int64_t chunk_place(int start, int seq, int chunk) { 
 enum Rule { kDelta = 0, kGeneralDelta = 1, kLinear = 2, kMemory = 3 };
 
 template <int kBytes>
-__device__ __forceinline__ void stage_copy(float* smem, const float* gmem, bool valid) {
+__device__ __forceinline__ void stage_copy(float* smem, const void* gmem, bool valid = true) {
   const uint32_t s = static_cast<uint32_t>(__cvta_generic_to_shared(smem));
   const int bytes = valid ? kBytes : 0;
-  asm volatile("cp.async.ca.shared.global [%0], [%1], %2, %3;" ::"r"(s), "l"(gmem), "n"(kBytes), "r"(bytes) : "memory");
+  if (kBytes == 16) asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(s), "l"(gmem), "r"(bytes) : "memory");
+  else asm volatile("cp.async.ca.shared.global [%0], [%1], %2, %3;" ::"r"(s), "l"(gmem), "n"(kBytes), "r"(bytes) : "memory");
 }
 __device__ __forceinline__ void commit_copies() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 template <int LEFT>
@@ -99,20 +99,85 @@ __device__ __forceinline__ quad_t load_quad(const float* p) {
   return {v.x, v.y};
 }
 
-// What `chunk_prepare` hands on, and the walk's result. Rows of `padded_rows(dk)` and `padded_columns(dv)` numbers, so all copies
-// are whole 16-byte steps whatever the sizes.
+// What the preparing kernels hand on, and the walk's result, by (chunk's place, head): rows of `padded_rows(dk)` and `padded_columns(dv)`
+// numbers, whole chunks of C tokens (those past a request's end are zeros in y, kd and x). Each array runs along what its reader multiplies
+// over, four neighbouring numbers for the lane that wants them; y, kd and s lie as the lanes of a warp want them side by side (`y_place`,
+// `kd_place`, `s_place`).
 struct Scratch {
   int head0, heads;  // the heads that a pass takes: all, or as many as the scratch holds
-  float* y;   // [tokens][heads][rows]
-  float* kd;  // [tokens][heads][rows]: G_last,j k_j
-  float* qt;  // [tokens][heads][rows]: e_i q_i
-  float* x;   // [tokens][heads][columns]: W, then U
-  float* a;   // [tokens][heads][C]: what reads out U
-  float* av;  // [tokens][heads][C]: what reads out V
+  float* y;   // [chunks][heads][rows x C]
+  float* kd;  // [chunks][heads][rows x C]: G_last,j k_j
+  float* qt;  // [chunks][heads][C][rows]: e_i q_i
+  float* x;   // [chunks][heads][columns][C]: W, then U
+  float* a;   // [chunks][heads][C][C]: what reads out U
+  float* av;  // [chunks][heads][C][C]: what reads out V
   float* e;   // [chunks][heads][rows]: e_last
   float* n;   // [chunks][heads][rows]: the matrix memory's normaliser, likewise
-  float* s;   // [chunks][heads][rows][columns]: what the values alone add, then the state in front of each chunk
+  float* s;   // [chunks][heads][columns x rows]: what the values alone add, then the state in front of each chunk
 };
+
+// Of column g = lane / 4 of an operand B, the token (or row) of sixteen that stands there in tile t (of two): D's layout, in which lane q
+// has columns 2 q and 2 q + 1 of either tile, then gives it four neighbours, 4 q .. + 3.
+__device__ __forceinline__ int in_sixteen(int t, int g) { return 4 * (g >> 1) + 2 * t + (g & 1); }
+// Rows of sixteen are a warp's of the walk. y: by (sixteen rows, sixteen tokens, tile) the lanes' four rows of a token each.
+__device__ __forceinline__ int y_place(int token, int row) {
+  const int g = (token & 12) / 2 + (token & 1), tile = token / 16 * 2 + (token >> 1 & 1);
+  return row / 16 * (16 * C) + tile * 128 + g * 16 + (row & 15);
+}
+// kd: by (sixteen rows, tile, sixteen tokens) the lanes' four tokens of a row each.
+__device__ __forceinline__ int kd_place(int token, int row) {
+  const int g = (row & 12) / 2 + (row & 1), tile = row >> 1 & 1;
+  return row / 16 * (16 * C) + (tile * 2 + token / 16) * 128 + g * 16 + (token & 15);
+}
+// s: by (sixteen columns, sixteen rows, eight of the columns) the lanes' four rows of a column each.
+__device__ __forceinline__ int s_place(int col, int row, int rows) {
+  return col / 16 * (16 * rows) + row / 16 * 256 + (col >> 3 & 1) * 128 + (col & 7) * 16 + (row & 15);
+}
+
+// --- products of 32-bit numbers on the tensor cores ----------------------------------------------------------------------------------
+//
+// A number is the sum of three bfloat16 ones, to its last bit: the nearest, the nearest to what is left, and the rest (8 + 8 + 8 bits). Of the
+// nine products of two such sums the six largest are taken; the others are below 2^-26 of the whole. Products of 8-bit numbers are exact in
+// 32 bits. The tensor core's own sums drop bits below the last, so few are chained: the five small products of a step of 16 first, the large
+// one last, and what is summed beyond one step is added with ordinary rounding. What is not finite becomes NaN.
+struct Split {  // two neighbouring numbers, packed
+  uint32_t part[3];
+};
+__device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
+  uint32_t d;
+  asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(d) : "f"(hi), "f"(lo));
+  return d;
+}
+__device__ __forceinline__ Split split_pair(float x, float y) {
+  Split out;
+#pragma unroll
+  for (int i = 0; i < 3; ++i) {
+    out.part[i] = pack_bf16(x, y);
+    if (i < 2) x -= __uint_as_float(out.part[i] << 16), y -= __uint_as_float(out.part[i] & 0xffff0000u);
+  }
+  return out;
+}
+// D[16][8] += A[16][16] B[16][8]. Of a lane (g = lane / 4, q = lane % 4), over the step's numbers along which is summed, in an order of
+// this file's own: it holds 4 q .. + 3 of them. A: row g 4q, + 1; row g + 8 likewise; row g 4q + 2, + 3; row g + 8 likewise. B: column g
+// 4q, + 1; 4q + 2, + 3. D: row g columns 2q, + 1; row g + 8 likewise.
+__device__ __forceinline__ void mma_bf16(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+  asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
+      : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
+      : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+struct SplitA {  // a lane's share of A
+  uint32_t part[3][4];
+  __device__ __forceinline__ void set(int at, const Split& s) { part[0][at] = s.part[0], part[1][at] = s.part[1], part[2][at] = s.part[2]; }
+};
+struct SplitB {  // of B
+  Split lo, hi;
+  __device__ __forceinline__ explicit SplitB(float4 v) : lo(split_pair(v.x, v.y)), hi(split_pair(v.z, v.w)) {}
+};
+__device__ __forceinline__ void mma_split(float (&d)[4], const SplitA& a, const SplitB& b) {
+  constexpr int order[6][2] = {{2, 0}, {0, 2}, {1, 1}, {1, 0}, {0, 1}, {0, 0}};
+#pragma unroll
+  for (int i = 0; i < 6; ++i) mma_bf16(d, a.part[order[i][0]], b.lo.part[order[i][1]], b.hi.part[order[i][1]]);
+}
 
 // Solves (I + l) x = rhs in place, row after row: x_i = rhs_i - sum_{j < i} l[i][j] x_j.
 __device__ __forceinline__ void substitute(const float* l, float (&x)[C]) {
@@ -129,6 +194,18 @@ __device__ __forceinline__ void substitute(const float* l, float (&x)[C]) {
     }
     x[i] = sum0 + sum1;
   }
+}
+
+// What a thread holds of a column for the chunk's tokens, as `y` lies or side by side; zeros past the request's end.
+__device__ __forceinline__ void store_y(float* to, int row, const float (&x)[C], int n) {
+  to += y_place(0, row);
+#pragma unroll
+  for (int i = 0; i < C; ++i) to[y_place(i, 0)] = i < n ? x[i] : 0.f;
+}
+__device__ __forceinline__ void store_column(float* to, const float (&x)[C], int n) {
+#pragma unroll
+  for (int i = 0; i < C; i += 4)
+    *reinterpret_cast<float4*>(to + i) = make_float4(i < n ? x[i] : 0.f, i + 1 < n ? x[i + 1] : 0.f, i + 2 < n ? x[i + 2] : 0.f, i + 3 < n ? x[i + 3] : 0.f);
 }
 
 // --- what does not depend on the state -------------------------------------------------------------------------------------------
@@ -266,7 +343,7 @@ chunk_prepare_kernel(const float* q, const float* k, const float* v, const float
   const int n = min(C, seq_q_len[seq] - chunk * C);
   if (n <= 0) return;
   const int start = seq_q_start[seq], kvh = head / (heads / kv_heads);
-  const int64_t first = static_cast<int64_t>(start) + chunk * C;
+  const int64_t first = static_cast<int64_t>(start) + chunk * C, place = chunk_place(start, seq, chunk) * to.heads + own_head;
   constexpr int rows = ROWS, ld = ROWS + 4;
   const int columns = padded_columns(dv);
   float* ks = chunk_smem;                     // [C][ld]: keys, then times the decays of their group up to their own token
@@ -323,7 +400,7 @@ chunk_prepare_kernel(const float* q, const float* k, const float* v, const float
   {
     float own = 0.f, d = 0.f, prefix = 0.f, e = 0.f;
     if (PER_HEAD) own = lane < n ? decay[(first + lane) * heads + head] : 0.f;
-    float* a = to.a + (first * to.heads + own_head) * C + lane;
+    float* a = to.a + place * C * C + lane;
     for (int i = 0; i < C; ++i) {
       if (PER_HEAD) {  // D_ij of column j = lane, the sum of the logarithms from token j + 1 on, grows with i from zero at i = j
         const float gi = __shfl_sync(0xffffffffu, own, i);
@@ -334,7 +411,7 @@ chunk_prepare_kernel(const float* q, const float* k, const float* v, const float
       if ((i & 7) == warp) {
         const float between = PER_HEAD ? expf(d) : 1.f;
         ls[i * C + lane] = lane < i ? bs[i] * between * kk[i * (C + 1) + lane] : 0.f;
-        if (i < n) a[static_cast<int64_t>(i) * to.heads * C] = lane <= i ? between * qk[i * (C + 1) + lane] : 0.f;
+        a[i * C] = lane <= i ? between * qk[i * (C + 1) + lane] : 0.f;
       }
     }
     if (PER_HEAD && warp == 0) es[lane] = expf(e), fs[lane] = expf(d);  // d is now D_last,j: tokens past n added nothing
@@ -342,13 +419,9 @@ chunk_prepare_kernel(const float* q, const float* k, const float* v, const float
   __syncthreads();
   for (int column = tid; column < rows + columns; column += kThreads) {
     float x[C];
-    float* to_x;
-    const int64_t stride = static_cast<int64_t>(to.heads) * (column < rows ? rows : columns);
     if (column < rows) {
-      const int64_t at = (first * to.heads + own_head) * rows + column;
-      float* qt = to.qt + at;
-      float* kd = to.kd + at;
-      to_x = to.y + at;
+      float* qt = to.qt + place * C * rows + column;
+      float* kd = to.kd + place * rows * C + kd_place(0, column);
       float before[kGroups], after[kGroups];  // whole groups in front of and behind a token's own
       if (!PER_HEAD) {
         before[0] = after[kGroups - 1] = 1.f;
@@ -358,32 +431,30 @@ chunk_prepare_kernel(const float* q, const float* k, const float* v, const float
         for (int g = kGroups - 2; g >= 0; --g) after[g] = after[g + 1] * whole[(g + 1) * rows + column];
       }
 #pragma unroll
-      for (int i = 0; i < C; ++i) {
-        const float key = ks[i * ld + column], e = PER_HEAD ? es[i] : before[i / kGroup];
-        if (i < n) {
-          *qt = e * qs[i * ld + column];
-          *kd = PER_HEAD ? fs[i] * key : after[i / kGroup] * gs[i * ld + column];
+      for (int i0 = 0; i0 < C; i0 += 4) {
+        float decayed[4];
+#pragma unroll
+        for (int y = 0; y < 4; ++y) {
+          const int i = i0 + y;
+          const float key = ks[i * ld + column], e = PER_HEAD ? es[i] : before[i / kGroup];
+          qt[i * rows] = e * qs[i * ld + column];
+          decayed[y] = i < n ? (PER_HEAD ? fs[i] * key : after[i / kGroup] * gs[i * ld + column]) : 0.f;
+          x[i] = -bs[i] * e * key;
         }
-        qt += stride, kd += stride;
-        x[i] = -bs[i] * e * key;
+        *reinterpret_cast<float4*>(kd + kd_place(i0, 0)) = make_float4(decayed[0], decayed[1], decayed[2], decayed[3]);
       }
-      to.e[(chunk_place(start, seq, chunk) * to.heads + own_head) * rows + column] =
-          PER_HEAD ? es[n - 1] : before[kGroups - 1] * whole[(kGroups - 1) * rows + column];
+      to.e[place * rows + column] = PER_HEAD ? es[n - 1] : before[kGroups - 1] * whole[(kGroups - 1) * rows + column];
     } else {
       const int c = column - rows;
       const float* value = v + (first * heads + head) * dv + c;
-      to_x = to.x + (first * to.heads + own_head) * columns + c;
 #pragma unroll
       for (int i = 0; i < C; ++i) x[i] = i < n && c < dv ? value[static_cast<int64_t>(i) * heads * dv] : 0.f;
 #pragma unroll
       for (int i = 0; i < C; ++i) x[i] *= bs[i];
     }
     substitute(ls, x);
-#pragma unroll
-    for (int i = 0; i < C; ++i) {
-      if (i < n) *to_x = x[i];
-      to_x += stride;
-    }
+    if (column < rows) store_y(to.y + place * C * rows, column, x, n);
+    else store_column(to.x + (place * columns + column - rows) * C, x, n);
   }
 }
 
@@ -529,20 +600,19 @@ linear_chunk_prepare_kernel(LinearRule in, const int* __restrict__ seq_q_start, 
       d = i > lane ? d * own : 1.f;
       prefix *= own;
       if (i == lane) e = prefix;
-      if ((i & 7) == warp && i < n) to.av[((first + i) * to.heads + own_head) * C + lane] = lane <= i ? d * put * rk[i * (C + 1) + lane] * in.scale : 0.f;
+      if ((i & 7) == warp) to.av[(place * C + i) * C + lane] = lane <= i ? d * put * rk[i * (C + 1) + lane] * in.scale : 0.f;
     }
     if (warp == 0) es[lane] = e, fs[lane] = d * put;
     __syncthreads();
     for (int c = tid; c < rows; c += kThreads) {
-      float* qt = to.qt + (first * to.heads + own_head) * rows + c;
+      float* qt = to.qt + place * C * rows + c;
       float sum = 0.f;
 #pragma unroll 8
       for (int i = 0; i < C; ++i) {
         const float key = fs[i] * ks[i * ld + c];
         ks[i * ld + c] = key;
         sum += key;
-        if (i < n) *qt = es[i] * in.scale * rs[i * ld + c];
-        qt += static_cast<int64_t>(to.heads) * rows;
+        qt[i * rows] = es[i] * in.scale * rs[i * ld + c];
       }
       to.n[place * rows + c] = sum;
       to.e[place * rows + c] = es[n - 1];
@@ -553,16 +623,14 @@ linear_chunk_prepare_kernel(LinearRule in, const int* __restrict__ seq_q_start, 
   }
   for (int i = warp; !MEMORY && i < C; i += kWarps) {
     const int at = i * (C + 1) + lane;
-    const int64_t row = ((first + i) * to.heads + own_head) * C + lane;
+    const int64_t row = (place * C + i) * C + lane;
     if (GENERAL) {  // au came in with its own sign: b = -au
       ls[i * C + lane] = lane < i ? ub[at] : 0.f;
       ms[i * C + lane] = lane < i ? uk[at] : 0.f;
-      if (i < n) {
-        to.a[row] = lane <= i ? -rb[at] : 0.f;
-        to.av[row] = lane <= i ? rk[at] : 0.f;
-      }
-    } else if (i < n) {
-      to.av[row] = lane < i ? rk[at] : (lane == i ? in.bonus[(first + i) * heads + head] : 0.f);
+      to.a[row] = lane <= i ? -rb[at] : 0.f;
+      to.av[row] = lane <= i ? rk[at] : 0.f;
+    } else {
+      to.av[row] = lane < i ? rk[at] : (lane == i && i < n ? in.bonus[(first + i) * heads + head] : 0.f);
     }
   }
   // Scaled rows: r times all decays in front of (or up to) its token, b times all decays behind its token; a thread per (group, channel).
@@ -574,17 +642,16 @@ linear_chunk_prepare_kernel(LinearRule in, const int* __restrict__ seq_q_start, 
       before *= g < group ? whole[g * rows + c] : 1.f;
       after *= g + 1 > group ? whole[(g + 1) * rows + c] : 1.f;
     }
-    const int64_t at = ((first + group * kGroup) * to.heads + own_head) * rows + c, step = static_cast<int64_t>(to.heads) * rows;
-    float* qt = to.qt + at;
-    float* kd = to.kd + at;
+    float* qt = to.qt + (place * C + group * kGroup) * rows + c;
 #pragma unroll
-    for (int r = 0; r < kGroup; ++r) {
-      const int from = (group * kGroup + r) * ld + c;
-      if (group * kGroup + r < n) {
-        *qt = before * rs[from];
-        if (GENERAL) *kd = -after * bb[from];
-      }
-      qt += step, kd += step;
+    for (int r = 0; r < kGroup; ++r) qt[r * rows] = before * rs[(group * kGroup + r) * ld + c];
+    if (GENERAL) {
+      float decayed[kGroup];
+#pragma unroll
+      for (int r = 0; r < kGroup; ++r) decayed[r] = group * kGroup + r < n ? -after * bb[(group * kGroup + r) * ld + c] : 0.f;
+      float* kd = to.kd + place * rows * C + kd_place(group * kGroup, c);
+      *reinterpret_cast<float4*>(kd) = make_float4(decayed[0], decayed[1], decayed[2], decayed[3]);
+      *reinterpret_cast<float4*>(kd + 4) = make_float4(decayed[4], decayed[5], decayed[6], decayed[7]);
     }
   }
   for (int c = tid; !MEMORY && c < rows; c += kThreads) to.e[place * rows + c] = whole[c] * whole[rows + c] * whole[2 * rows + c] * whole[3 * rows + c];
@@ -599,8 +666,6 @@ linear_chunk_prepare_kernel(LinearRule in, const int* __restrict__ seq_q_start, 
     }
     if (GENERAL && tid < kValueTile + (col0 == 0 ? rows : 0)) {  // a thread per column of [M V | e U]
       float x[C];
-      float* to_x;
-      int64_t stride;
       const int c = tid;
       if (tid < kValueTile) {
         float value[C];
@@ -619,8 +684,6 @@ linear_chunk_prepare_kernel(LinearRule in, const int* __restrict__ seq_q_start, 
           }
           x[i] = sum0 + sum1;
         }
-        stride = static_cast<int64_t>(to.heads) * columns;
-        to_x = to.x + (first * to.heads + own_head) * columns + col0 + c;
       } else {
         const int channel = c - kValueTile;
         float before = 1.f;
@@ -629,17 +692,10 @@ linear_chunk_prepare_kernel(LinearRule in, const int* __restrict__ seq_q_start, 
           if (i > 0 && i % kGroup == 0) before *= whole[(i / kGroup - 1) * rows + channel];
           x[i] = before * us[i * ld + channel];
         }
-        stride = static_cast<int64_t>(to.heads) * rows;
-        to_x = to.y + (first * to.heads + own_head) * rows + channel;
       }
       substitute(ls, x);
-      if (tid >= kValueTile || col0 + c < columns) {
-#pragma unroll
-        for (int i = 0; i < C; ++i) {
-          if (i < n) *to_x = x[i];
-          to_x += stride;
-        }
-      }
+      if (tid >= kValueTile) store_y(to.y + place * C * rows, c - kValueTile, x, n);
+      else if (col0 + c < columns) store_column(to.x + (place * columns + col0 + c) * C, x, n);
     }
     // (G_last K)^T V over the tile: four rows by four columns a thread, group after group of tokens.
     const int rt = (tid & 15) * 4, ct = (tid >> 4) * 4;
@@ -666,24 +722,26 @@ linear_chunk_prepare_kernel(LinearRule in, const int* __restrict__ seq_q_start, 
       }
       if (col0 + ct < columns) {
 #pragma unroll
-        for (int r = 0; r < 4; ++r)
-          *reinterpret_cast<float4*>(to.s + (place * rows + row + r) * columns + col0 + ct) = make_float4(acc[r][0], acc[r][1], acc[r][2], acc[r][3]);
+        for (int c = 0; c < 4; ++c)
+          *reinterpret_cast<float4*>(to.s + place * columns * rows + s_place(col0 + ct + c, row, rows)) = make_float4(acc[0][c], acc[1][c], acc[2][c], acc[3][c]);
       }
     }
   }
 }
 
-// Four neighbouring numbers of a head's state a thread, from chunk to chunk: eight chunks' sums are asked for at a time.
-__global__ void __launch_bounds__(kThreads)
+// Four neighbouring rows of a column of a head's state a thread, from chunk to chunk: eight chunks' sums are asked for at a time. A warp
+// has eight columns of sixteen rows, so that the state, whose rows run the other way, is read and written in whole sectors too.
+constexpr int kScanThreads = 64;  // small blocks: 24 heads of 64 x 64 are 384 of them, one for every warp scheduler of the chip
+__global__ void __launch_bounds__(kScanThreads, 1)
 chunk_scan_kernel(const int* __restrict__ seq_q_start, const int* __restrict__ seq_q_len, const int* __restrict__ seq_slot, int heads, int dk, int dv, Scratch from,
                   float* state, float* normaliser) {
   let_successor_start();
   const int seq = blockIdx.z, own_head = blockIdx.y, head = from.head0 + own_head;
   const int start = seq_q_start[seq], len = seq_q_len[seq], chunks = (len + C - 1) / C;
   const int rows = padded_rows(dk), columns = padded_columns(dv);
-  const int item = (blockIdx.x * kThreads + threadIdx.x) * 4;
-  if (item >= rows * columns) {  // the blocks behind the state's: a number of the normaliser a thread
-    const int c = blockIdx.x * kThreads + threadIdx.x - (rows * columns / 4 + kThreads - 1) / kThreads * kThreads;
+  const int idx = blockIdx.x * kScanThreads + threadIdx.x;
+  if (idx * 4 >= rows * columns) {  // the blocks behind the state's: a number of the normaliser a thread
+    const int c = idx - (rows * columns / 4 + kScanThreads - 1) / kScanThreads * kScanThreads;
     if (normaliser == nullptr || c < 0 || c >= rows) return;
     wait_for_predecessor();
     float* own = normaliser + (static_cast<int64_t>(seq_slot[seq]) * heads + head) * dk + c;
@@ -697,355 +755,340 @@ chunk_scan_kernel(const int* __restrict__ seq_q_start, const int* __restrict__ s
     if (c < dk && chunks > 0) *own = n;
     return;
   }
-  const int row = item / columns, col = item % columns;
+  const int tile = idx / 32, lane = threadIdx.x & 31;  // `s_place` from thread to thread
+  const int row = tile / 2 % (rows / 16) * 16 + (lane & 3) * 4, col = tile / 2 / (rows / 16) * 16 + (tile & 1) * 8 + lane / 4;
   float* base = state + (static_cast<int64_t>(seq_slot[seq]) * heads + head) * dk * dv + static_cast<int64_t>(row) * dv + col;
   float s[4];
   wait_for_predecessor();
 #pragma unroll
-  for (int x = 0; x < 4; ++x) s[x] = row < dk && col + x < dv ? base[x] : 0.f;
+  for (int x = 0; x < 4; ++x) s[x] = row + x < dk && col < dv ? base[static_cast<int64_t>(x) * dv] : 0.f;
   const int64_t place = chunk_place(start, seq, 0) * from.heads + own_head;
   const float* e = from.e + place * rows + row;
-  float* sums = from.s + place * rows * columns + item;
+  float* sums = from.s + place * columns * rows + idx * 4;
   const int64_t step_e = static_cast<int64_t>(from.heads) * rows, step = step_e * columns;
   constexpr int kAhead = 8;
   for (int chunk = 0; chunk < chunks; chunk += kAhead) {
-    float4 add[kAhead];
-    float keep[kAhead];
+    float4 add[kAhead], keep[kAhead];
 #pragma unroll
     for (int i = 0; i < kAhead; ++i)
-      if (chunk + i < chunks) add[i] = *reinterpret_cast<const float4*>(sums + (chunk + i) * step), keep[i] = e[(chunk + i) * step_e];
+      if (chunk + i < chunks) add[i] = *reinterpret_cast<const float4*>(sums + (chunk + i) * step), keep[i] = *reinterpret_cast<const float4*>(e + (chunk + i) * step_e);
 #pragma unroll
     for (int i = 0; i < kAhead; ++i)
       if (chunk + i < chunks) {
         *reinterpret_cast<float4*>(sums + (chunk + i) * step) = make_float4(s[0], s[1], s[2], s[3]);
-        s[0] = fmaf(keep[i], s[0], add[i].x), s[1] = fmaf(keep[i], s[1], add[i].y);
-        s[2] = fmaf(keep[i], s[2], add[i].z), s[3] = fmaf(keep[i], s[3], add[i].w);
+        s[0] = fmaf(keep[i].x, s[0], add[i].x), s[1] = fmaf(keep[i].y, s[1], add[i].y);
+        s[2] = fmaf(keep[i].z, s[2], add[i].z), s[3] = fmaf(keep[i].w, s[3], add[i].w);
       }
   }
   if (chunks > 0) {
 #pragma unroll
     for (int x = 0; x < 4; ++x)
-      if (row < dk && col + x < dv) base[x] = s[x];
+      if (row + x < dk && col < dv) base[static_cast<int64_t>(x) * dv] = s[x];
   }
 }
 
 // --- the walk ------------------------------------------------------------------------------------------------------------------------
 //
-// One block per (16 columns of the state, head, request). U = W + Y S: a warp has four tokens, its lanes four groups of columns times
-// eight parts of the rows, whose sums meet by shuffles. S <- e S + Kd^T U: a warp has an eighth of the rows, a lane four rows by four
-// columns over every kSplit-th token; after the shuffles it keeps its kPer rows of S in registers, with a transposed copy in shared
-// memory for the next chunk's first product.
-__host__ __device__ constexpr int walk_stage(int rows) { return 2 * C * (rows + 4) + C * kColumns + rows; }
-__host__ __device__ constexpr int walk_tile(int rows) { return kColumns * (rows + 8); }
-constexpr int kMaxRowX = 24;
-constexpr size_t walk_smem(int rows) { return sizeof(float) * (2 * walk_stage(rows) + walk_tile(rows) + C * kMaxRowX); }
-
-__device__ __forceinline__ float from_pair(float give, float keep, int with) { return keep + __shfl_xor_sync(0xffffffffu, give, with); }
+// One block per (16 columns of the state, head, request), a warp per 16 rows, which it keeps in registers, transposed, as the tensor core
+// leaves them (D: 16 columns x 2 times 8 rows): D's layout is A's, so the state goes into the next chunk's first product without leaving
+// its lanes. That product, U^T = W^T + S^T Y^T, is summed over the warps through shared memory, each warp adding up its share of the sums; S^T <-
+// e S^T + U^T Kd then wants nothing of the other warps. A lane's share of the operands comes by its own asynchronous copies, two chunks ahead,
+// so that nobody waits for anybody's (loads into registers a chunk ahead did: 101 us where this takes 80, a third of it spent
+// waiting for memory; copies that also go into L1 112).
+// What bounds it: the chain product, sum over warps, product, in turn and once a chunk: 2,400 cycles, of which the tensor core works 830 (heads
+// of 128 x 128). Tried: operands in parts in memory, made where they are prepared, half as many bytes again: 76 us, but 5 us more there;
+// taking them apart while the warps wait for one another: 95 us.
+constexpr int kSumPairs = 8;  // pairs of U^T's numbers that a lane holds: (half of the chunk, pair of four tokens, column g or g + 8)
+__host__ __device__ constexpr int walk_stages(int rows) { return rows <= 128 ? 3 : 2; }  // two blocks fit an SM up to 128 rows
+__host__ __device__ constexpr int own_pairs(int rows) { return rows < 16 * kSumPairs ? 16 * kSumPairs / rows : 1; }  // that a warp adds up
+// Bytes of a stage: per lane four pieces of y, four of kd, two of what the values add and its pairs of W; and e.
+__host__ __device__ constexpr int walk_stage(int rows, bool add) { return 2 * rows * (16 * (add ? 10 : 8) + 8 * own_pairs(rows)) + 4 * rows; }
+constexpr size_t walk_smem(int rows, bool add) { return walk_stages(rows) * walk_stage(rows, add); }
 
 template <int ROWS, bool ADD>  // ADD: what the values alone add to S stands where the chunk's state goes
-__global__ void __launch_bounds__(kThreads, ROWS <= 128 ? 2 : 1)
+__global__ void __launch_bounds__(2 * ROWS, ROWS <= 128 ? 2 : 1)
 chunk_walk_kernel(const int* __restrict__ seq_q_start, const int* __restrict__ seq_q_len, const int* __restrict__ seq_slot, int heads, int dk, int dv,
                   Scratch from, float* state) {
   extern __shared__ __align__(16) float chunk_smem[];
-  constexpr int kSplit = kThreads / ROWS;         // lanes that share a tile of S: 4, 2 or 1
-  constexpr int kPer = 4 / kSplit;                // rows of S that a lane keeps
-  constexpr int kLd = ROWS + 4;
-  constexpr int kLdS = ROWS + 8;                  // 8 banks from column to column
-  constexpr int kRowX = kSplit == 4 ? 24 : 16;    // the rows that lanes read side by side in different banks
+  constexpr int kParts = ROWS / 16, kOwn = own_pairs(ROWS), kLanes = 2 * ROWS, kStages = walk_stages(ROWS);
+  constexpr int kPairsAt = (ADD ? 10 : 8) * kLanes * 4, kDecaysAt = kPairsAt + kOwn * kLanes * 2;  // in a stage
+  __shared__ uint4 us[2][3][32];  // U^T in parts, as the lanes of every warp want it
   let_successor_start();
   const int col0 = blockIdx.x * kColumns, own_head = blockIdx.y, head = from.head0 + own_head, seq = blockIdx.z;
   const int start = seq_q_start[seq], len = seq_q_len[seq];
-  const int columns = padded_columns(dv);
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  float* tile = chunk_smem + 2 * walk_stage(ROWS);  // [16 columns][kLdS]: S, transposed
-  float* xs = tile + walk_tile(ROWS);               // [C][kRowX]: U
-  const int chunks = (len + C - 1) / C;
-  auto fetch = [&](int chunk) {
-    float* ys = chunk_smem + (chunk & 1) * walk_stage(ROWS);
-    float* kds = ys + C * kLd;
-    float* ws = kds + C * kLd;
-    float* es = ws + C * kColumns;
-    const int n = min(C, len - chunk * C);
-    const int64_t first = static_cast<int64_t>(start) + chunk * C;
+  const int columns = padded_columns(dv), chunks = (len + C - 1) / C;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, q = lane & 3;
+  const int row0 = warp * 16 + 4 * q;  // the four rows that the lane keeps, of columns g and g + 8
+  const bool adds_up = kParts <= kSumPairs || warp < kSumPairs;
+  const int64_t place = chunk_place(start, seq, 0) * from.heads + own_head;
+  const float* y = from.y + place * ROWS * C + warp * 16 * C + lane * 4;
+  const float* kd = from.kd + place * ROWS * C + warp * 16 * C + lane * 4;
+  const float* e = from.e + place * ROWS + row0;
+  float* s_out = from.s + place * columns * ROWS + col0 * ROWS + warp * 256 + lane * 4;
+  int64_t x_at[kOwn];
 #pragma unroll
-    for (int idx = tid; idx < C * ROWS / 4; idx += kThreads) {
-      const int r = idx / (ROWS / 4), c = idx % (ROWS / 4) * 4;
-      const int64_t at = r < n ? ((first + r) * from.heads + own_head) * ROWS + c : 0;
-      stage_copy<16>(ys + r * kLd + c, from.y + at, r < n);
-      stage_copy<16>(kds + r * kLd + c, from.kd + at, r < n);
-    }
-    if (tid < C * kColumns / 4) {
-      const int r = tid / 4, c = tid % 4 * 4;
-      stage_copy<16>(ws + r * kColumns + c, from.x + (r < n ? ((first + r) * from.heads + own_head) * columns + col0 + c : 0), r < n);
-    } else if (tid < C * kColumns / 4 + ROWS / 4) {
-      const int c = (tid - C * kColumns / 4) * 4;
-      stage_copy<16>(es + c, from.e + (chunk_place(start, seq, chunk) * from.heads + own_head) * ROWS + c, true);
+  for (int o = 0; o < kOwn; ++o) {
+    const int pair = warp + o * kParts;
+    x_at[o] = (place * columns + col0 + g + 8 * (pair & 1)) * C + 16 * (pair >> 2) + 4 * q + (pair & 2);
+  }
+  const int64_t step = from.heads, step_y = step * C * ROWS, step_s = step * columns * ROWS, step_x = step * columns * C;
+  auto stage_of = [&](int chunk) { return chunk_smem + chunk % kStages * (walk_stage(ROWS, ADD) / 4); };
+  auto fetch = [&](int chunk) {
+    if (chunk < chunks) {
+      float* stage = stage_of(chunk) + tid * 4;
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        stage_copy<16>(stage + i * kLanes * 4, y + chunk * step_y + i * 128, true);
+        stage_copy<16>(stage + (4 + i) * kLanes * 4, kd + chunk * step_y + i * 128, true);
+      }
+      if (ADD) {
+        stage_copy<16>(stage + 8 * kLanes * 4, s_out + chunk * step_s, true);
+        stage_copy<16>(stage + 9 * kLanes * 4, s_out + chunk * step_s + 128, true);
+      }
+      if (lane < 4) stage_copy<16>(stage_of(chunk) + kDecaysAt + row0, e + chunk * step * ROWS, true);
+#pragma unroll
+      for (int o = 0; o < kOwn; ++o)
+        if (adds_up) stage_copy<8>(stage_of(chunk) + kPairsAt + (o * kLanes + tid) * 2, from.x + x_at[o] + chunk * step_x, true);
     }
     commit_copies();
   };
-  const int jp = lane % kSplit, cg = lane / kSplit % 4;
-  const int quad = warp * (ROWS / kWarps) + lane / (4 * kSplit) * 4;  // the lane's tile: rows quad .. + 3, columns 4 cg .. + 3
-  const int row0 = quad + jp * kPer;                                  // the rows it keeps
+  auto staged = [&](int chunk, int piece) { return *reinterpret_cast<const float4*>(stage_of(chunk) + (piece * kLanes + tid) * 4); };
   float* s_base = state + (static_cast<int64_t>(seq_slot[seq]) * heads + head) * dk * dv + col0;
-  float s[kPer][4];
+  auto in_state = [&](int t, int i) -> float* {  // where s[t][i] comes from and goes to
+    const int row = row0 + 2 * t + (i & 1), col = g + 8 * (i >> 1);
+    return row < dk && col0 + col < dv ? s_base + static_cast<int64_t>(row) * dv + col : nullptr;
+  };
+  float s[2][4];  // rows row0 + 2 t, + 1 of column g, the same of column g + 8
   wait_for_predecessor();
-  if (chunks > 0) fetch(0);
+  if (chunks == 0) return;
 #pragma unroll
-  for (int r = 0; r < kPer; ++r)
+  for (int chunk = 0; chunk < kStages - 1; ++chunk) fetch(chunk);
 #pragma unroll
-    for (int c = 0; c < 4; ++c)
-      s[r][c] = row0 + r < dk && col0 + cg * 4 + c < dv ? s_base[static_cast<int64_t>(row0 + r) * dv + cg * 4 + c] : 0.f;
+  for (int t = 0; t < 2; ++t)
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const float* at = in_state(t, i);
+      s[t][i] = at != nullptr ? *at : 0.f;
+    }
   for (int chunk = 0; chunk < chunks; ++chunk) {
-    const int n = min(C, len - chunk * C);
-    const int64_t first = static_cast<int64_t>(start) + chunk * C;
-    float* s_out = from.s + ((chunk_place(start, seq, chunk) * from.heads + own_head) * ROWS + row0) * columns + col0 + cg * 4;
-    float4 own[kPer];
-    if (ADD) {
-#pragma unroll
-      for (int r = 0; r < kPer; ++r) own[r] = *reinterpret_cast<const float4*>(s_out + static_cast<int64_t>(r) * columns);
-    }
-#pragma unroll
-    for (int c = 0; c < 4; ++c) {
-      float* to = tile + (cg * 4 + c) * kLdS + row0;
-      if (kPer == 4) *reinterpret_cast<float4*>(to) = make_float4(s[0][c], s[kPer / 4][c], s[kPer / 2][c], s[kPer - 1][c]);
-      else if (kPer == 2) *reinterpret_cast<float2*>(to) = make_float2(s[0][c], s[kPer - 1][c]);
-      else *to = s[0][c];
-    }
-    wait_copies<0>();
-    __syncthreads();  // S and the chunk's operands are there, and nobody reads the other stage any more
-    if (chunk + 1 < chunks) fetch(chunk + 1);
-    const float* ys = chunk_smem + (chunk & 1) * walk_stage(ROWS);
-    const float* kds = ys + C * kLd;
-    const float* ws = kds + C * kLd;
-    const float* es = ws + C * kColumns;
+    __syncwarp();  // four lanes copy the warp's decays
+    fetch(chunk + kStages - 1);
+    wait_copies<kStages - 1>();
+    float* own_sums = stage_of(chunk) + warp * 128 + lane * 2;  // a warp's sums go where its share of Y was
     {
-      // Tokens 4 warp .. + 3, columns ct, ct + 4, .., every eighth group of four rows; sums over even and odd rows side by side.
-      const int ct = lane & 3, part = lane >> 2;
-      const float* y = ys + warp * 4 * kLd + part * 4;
-      const float* t = tile + ct * kLdS + part * 4;
-      pair_t acc[4][4];
+      SplitA left;
 #pragma unroll
-      for (int i = 0; i < 4; ++i)
+      for (int t = 0; t < 2; ++t) left.set(2 * t, split_pair(s[t][0], s[t][1])), left.set(2 * t + 1, split_pair(s[t][2], s[t][3]));
+      float acc[4][4];
 #pragma unroll
-        for (int c = 0; c < 4; ++c) acc[i][c] = 0;
-#pragma unroll
-      for (int k = 0; k < ROWS; k += 32) {
-        quad_t a[4], b[4];
-#pragma unroll
-        for (int x = 0; x < 4; ++x) {
-          a[x] = load_quad(y + x * kLd + k);
-          b[x] = load_quad(t + x * 4 * kLdS + k);
-        }
-#pragma unroll
-        for (int i = 0; i < 4; ++i)
-#pragma unroll
-          for (int c = 0; c < 4; ++c) acc[i][c] = fma_pair(a[i].hi, b[c].hi, fma_pair(a[i].lo, b[c].lo, acc[i][c]));
+      for (int t = 0; t < 4; ++t) {
+        acc[t][0] = acc[t][1] = acc[t][2] = acc[t][3] = 0.f;
+        mma_split(acc[t], left, SplitB(staged(chunk, t)));
       }
-      // The eight parts meet: a lane ends with two columns of one token.
-      const bool b2 = lane & 4, b3 = lane & 8, b4 = lane & 16;
-      float sum[4][4], two[2][4], row[4];
+      __syncwarp();
 #pragma unroll
-      for (int i = 0; i < 4; ++i)
+      for (int t = 0; t < 4; ++t)
 #pragma unroll
-        for (int c = 0; c < 4; ++c) sum[i][c] = sum_pair(acc[i][c]);
-#pragma unroll
-      for (int i = 0; i < 2; ++i)
-#pragma unroll
-        for (int c = 0; c < 4; ++c) two[i][c] = from_pair(b2 ? sum[i][c] : sum[i + 2][c], b2 ? sum[i + 2][c] : sum[i][c], 4);
-#pragma unroll
-      for (int c = 0; c < 4; ++c) row[c] = from_pair(b3 ? two[0][c] : two[1][c], b3 ? two[1][c] : two[0][c], 8);
-      const int i = warp * 4 + (b2 ? 2 : 0) + (b3 ? 1 : 0), c = ct + (b4 ? 8 : 0);
-      const float u0 = from_pair(b4 ? row[0] : row[2], b4 ? row[2] : row[0], 16) + ws[i * kColumns + c];
-      const float u1 = from_pair(b4 ? row[1] : row[3], b4 ? row[3] : row[1], 16) + ws[i * kColumns + c + 4];
-      xs[i * kRowX + c] = u0, xs[i * kRowX + c + 4] = u1;
-      if (i < n) {
-        float* to = from.x + ((first + i) * from.heads + own_head) * columns + col0 + c;
-        to[0] = u0, to[4] = u1;
-      }
+        for (int h = 0; h < 2; ++h) *reinterpret_cast<float2*>(own_sums + t * kLanes * 4 + h * 64) = make_float2(acc[t][2 * h], acc[t][2 * h + 1]);
     }
     // The state in front of the chunk, for `chunk_out`.
-#pragma unroll
-    for (int r = 0; r < kPer; ++r) *reinterpret_cast<float4*>(s_out + static_cast<int64_t>(r) * columns) = make_float4(s[r][0], s[r][1], s[r][2], s[r][3]);
+    *reinterpret_cast<float4*>(s_out + chunk * step_s) = make_float4(s[0][0], s[0][1], s[1][0], s[1][1]);
+    *reinterpret_cast<float4*>(s_out + chunk * step_s + 128) = make_float4(s[0][2], s[0][3], s[1][2], s[1][3]);
     __syncthreads();
-    {
-      float add[4][4];  // summed apart from the state, which is rounded once a chunk
+    if (adds_up) {
 #pragma unroll
-      for (int r = 0; r < 4; ++r) add[r][0] = add[r][1] = add[r][2] = add[r][3] = 0.f;
-      const float* kd = kds + jp * kLd + quad;
-      const float* x = xs + jp * kRowX + cg * 4;
-#pragma unroll 4
-      for (int j = 0; j < C; j += kSplit) {
-        const float4 u = *reinterpret_cast<const float4*>(x + j * kRowX);
-        const float4 kj = *reinterpret_cast<const float4*>(kd + j * kLd);
-        const float f[4] = {kj.x, kj.y, kj.z, kj.w};
+      for (int o = 0; o < kOwn; ++o) {
+        const int pair = warp + o * kParts;
+        float2 part[kParts];
 #pragma unroll
-        for (int r = 0; r < 4; ++r) {
-          add[r][0] = fmaf(f[r], u.x, add[r][0]), add[r][1] = fmaf(f[r], u.y, add[r][1]);
-          add[r][2] = fmaf(f[r], u.z, add[r][2]), add[r][3] = fmaf(f[r], u.w, add[r][3]);
-        }
-      }
-      // The lanes of a tile meet, each keeping kPer rows.
-      if (kSplit == 4) {
-        const bool high = jp & 2;
+        for (int w = 0; w < kParts; ++w) part[w] = *reinterpret_cast<const float2*>(stage_of(chunk) + (pair >> 1) * kLanes * 4 + w * 128 + (pair & 1) * 64 + lane * 2);
+        const float2 w = *reinterpret_cast<const float2*>(stage_of(chunk) + kPairsAt + (o * kLanes + tid) * 2);
 #pragma unroll
-        for (int r = 0; r < 2; ++r)
+        for (int half = kParts / 2; half > 0; half /= 2)
 #pragma unroll
-          for (int c = 0; c < 4; ++c) add[r][c] = from_pair(high ? add[r][c] : add[r + 2][c], high ? add[r + 2][c] : add[r][c], 2);
-      }
-      if (kSplit >= 2) {
-        const bool high = jp & 1;
+          for (int i = 0; i < half; ++i) part[i].x += part[i + half].x, part[i].y += part[i + half].y;
+        const float2 u = make_float2(part[0].x + w.x, part[0].y + w.y);
+        const Split parts = split_pair(u.x, u.y);
 #pragma unroll
-        for (int r = 0; r < kPer; ++r)
-#pragma unroll
-          for (int c = 0; c < 4; ++c) add[r][c] = from_pair(high ? add[r][c] : add[r + kPer][c], high ? add[r + kPer][c] : add[r][c], 1);
-      }
-#pragma unroll
-      for (int r = 0; r < kPer; ++r) {
-        const float e = es[row0 + r];
-        if (ADD) add[r][0] += own[r].x, add[r][1] += own[r].y, add[r][2] += own[r].z, add[r][3] += own[r].w;
-#pragma unroll
-        for (int c = 0; c < 4; ++c) s[r][c] = fmaf(e, s[r][c], add[r][c]);
+        for (int p = 0; p < 3; ++p) reinterpret_cast<uint32_t*>(&us[pair >> 2][p][lane])[pair & 3] = parts.part[p];
+        *reinterpret_cast<float2*>(from.x + x_at[o] + chunk * step_x) = u;
       }
     }
-  }
-  if (chunks > 0) {
+    __syncthreads();
+    float sum[2][2][4];  // apart from the state, which is rounded once a chunk
 #pragma unroll
-    for (int r = 0; r < kPer; ++r)
+    for (int h = 0; h < 2; ++h) {
+      SplitA left;
 #pragma unroll
-      for (int c = 0; c < 4; ++c)
-        if (row0 + r < dk && col0 + cg * 4 + c < dv) s_base[static_cast<int64_t>(row0 + r) * dv + cg * 4 + c] = s[r][c];
+      for (int p = 0; p < 3; ++p) {
+        const uint4 word = us[h][p][lane];
+        left.part[p][0] = word.x, left.part[p][1] = word.y, left.part[p][2] = word.z, left.part[p][3] = word.w;
+      }
+#pragma unroll
+      for (int t = 0; t < 2; ++t) {
+        sum[t][h][0] = sum[t][h][1] = sum[t][h][2] = sum[t][h][3] = 0.f;
+        mma_split(sum[t][h], left, SplitB(staged(chunk, 4 + 2 * t + h)));
+      }
+    }
+    const float4 ef = *reinterpret_cast<const float4*>(stage_of(chunk) + kDecaysAt + row0);
+    const float decays[4] = {ef.x, ef.y, ef.z, ef.w};
+    float values[2][4] = {};
+    if (ADD) {
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const float4 add = staged(chunk, 8 + h);
+        values[h][0] = add.x, values[h][1] = add.y, values[h][2] = add.z, values[h][3] = add.w;
+      }
+    }
+#pragma unroll
+    for (int t = 0; t < 2; ++t)
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        float more = sum[t][0][i] + sum[t][1][i];
+        if (ADD) more += values[i >> 1][2 * t + (i & 1)];
+        s[t][i] = fmaf(decays[2 * t + (i & 1)], s[t][i], more);
+      }
   }
+#pragma unroll
+  for (int t = 0; t < 2; ++t)
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      float* at = in_state(t, i);
+      if (at != nullptr) *at = s[t][i];
+    }
 }
 
 // --- outputs ---------------------------------------------------------------------------------------------------------------------------
 //
-// One block per (chunk, head, request and COLS columns): O = Qt S (+ A U) (+ Av V) as one product over rows + 32 (+ 32) numbers, 32 of
-// them at a time by cp.async in two stages. A thread has eight tokens and four neighbouring columns: 12 numbers read for 32 FMAs, since
-// what an SM takes out of shared memory (32 numbers a cycle, however many lanes want the same one) bounds this kernel.
-constexpr int kLdSlab = C + 4;
-constexpr size_t out_smem(int cols) { return sizeof(float) * 2 * (C * kLdSlab + C * (cols + 4)); }
-
+// One block per (chunk, head, request and COLS columns), 32 columns a warp: O = Qt S (+ A U) (+ Av V) as one product over rows + 32 (+ 32)
+// numbers, 16 at a time, each lane's share of the operands straight from memory one step ahead. Pairs of tokens form a triangle: a token
+// leaves out those behind it. What is not finite there times a pair's zero would not be zero, so it goes into the product as a zero, and the
+// tokens that it does reach are set to NaN behind it.
 template <int COLS, bool WITH_U, bool WITH_V>
-__global__ void __launch_bounds__(COLS)
+__global__ void __launch_bounds__(COLS, 384 / COLS)
 chunk_out_kernel(const int* __restrict__ seq_q_start, const int* __restrict__ seq_q_len, int heads, int dv, int rows, int tiles, Scratch from, const float* v,
-                 int64_t v_ld, int v_wide, float* out, float* den) {
-  extern __shared__ __align__(16) float chunk_smem[];
-  constexpr int kLdOut = COLS + 4, kStage = C * kLdSlab + C * kLdOut;
+                 int64_t v_ld, float* out, float* den) {
   let_successor_start();
-  const int seq = blockIdx.z / tiles, col0 = blockIdx.z % tiles * COLS, own_head = blockIdx.y, head = from.head0 + own_head, chunk = blockIdx.x;
+  const int seq = blockIdx.z / tiles, own_head = blockIdx.y, head = from.head0 + own_head, chunk = blockIdx.x;
   const int start = seq_q_start[seq], n = min(C, seq_q_len[seq] - chunk * C);
   if (n <= 0) return;
-  const int64_t first = static_cast<int64_t>(start) + chunk * C;
-  const int columns = padded_columns(dv), width = min(COLS, columns - col0);
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const float* states = from.s + (chunk_place(start, seq, chunk) * from.heads + own_head) * rows * columns + col0;
-  const int state_slabs = rows / C, slabs = state_slabs + (WITH_U ? 1 : 0) + (WITH_V ? 1 : 0);
+  const int64_t first = static_cast<int64_t>(start) + chunk * C, place = chunk_place(start, seq, chunk) * from.heads + own_head;
+  const int columns = padded_columns(dv);
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, q = lane & 3;
+  const int col0 = blockIdx.z % tiles * COLS + warp * 32;  // columns col0 + 8 t + g in B, col0 + 8 t + 2 q, + 1 in D
+  const int state_steps = rows / 16, steps = state_steps + (WITH_U ? 2 : 0) + (WITH_V ? 2 : 0);
   wait_for_predecessor();
-  auto fetch = [&](int slab) {
-    float* left = chunk_smem + (slab & 1) * kStage;
-    float* right = left + C * kLdSlab;
-    const bool in_state = slab < state_slabs, is_u = WITH_U && slab == state_slabs;
-    const float* pairs = is_u ? from.a : from.av;
-#pragma unroll
-    for (int r = tid >> 3; r < C; r += COLS / 8) {
-      const int c = (tid & 7) * 4;
-      const int64_t row = (first + r) * from.heads + own_head;
-      stage_copy<16>(left + r * kLdSlab + c, r < n ? (in_state ? from.qt + row * rows + slab * C + c : pairs + row * C + c) : from.qt, r < n);
-    }
-    if (in_state || is_u) {
-#pragma unroll
-      for (int r = tid / (COLS / 4); r < C; r += 4) {
-        const int c = tid % (COLS / 4) * 4;
-        const bool valid = c < width && (in_state || r < n);
-        const float* at = in_state ? states + static_cast<int64_t>(slab * C + r) * columns + c : from.x + ((first + r) * from.heads + own_head) * columns + col0 + c;
-        stage_copy<16>(right + r * kLdOut + c, valid ? at : from.qt, valid);
-      }
-    } else if (v_wide) {
-#pragma unroll
-      for (int r = tid / (COLS / 4); r < C; r += 4) {
-        const int c = tid % (COLS / 4) * 4;
-        const bool valid = col0 + c < dv && r < n;
-        stage_copy<16>(right + r * kLdOut + c, valid ? v + (first + r) * v_ld + static_cast<int64_t>(head) * dv + col0 + c : v, valid);
-      }
-    } else {
-      for (int r = 0; r < C; ++r) {
-        const bool valid = col0 + tid < dv && r < n;
-        stage_copy<4>(right + r * kLdOut + tid, valid ? v + (first + r) * v_ld + static_cast<int64_t>(head) * dv + col0 + tid : v, valid);
-      }
-    }
-    commit_copies();
-  };
-  const int ct = (lane & 7) + 8 * warp, it = lane >> 3;  // columns 4 ct .. + 3, tokens it, it + 4, ..
-  float acc[8][4];
-#pragma unroll
-  for (int i = 0; i < 8; ++i) acc[i][0] = acc[i][1] = acc[i][2] = acc[i][3] = 0.f;
-  fetch(0);
-  if (den != nullptr && col0 == 0) {  // the normaliser read out as the state is: n . (e q) + the chunk's own pairs
-    const float* n0 = from.n + (chunk_place(start, seq, chunk) * from.heads + own_head) * rows;
+  if (den != nullptr && blockIdx.z % tiles == 0) {  // the normaliser read out as the state is: n . (e q) + the chunk's own pairs
+    const float* n0 = from.n + place * rows;
     for (int r = warp; r < n; r += COLS / 32) {
-      const int64_t row = (first + r) * from.heads + own_head;
-      float sum = from.av[row * C + lane];
-      for (int c = lane; c < rows; c += 32) sum = fmaf(from.qt[row * rows + c], n0[c], sum);
+      float sum = from.av[(place * C + r) * C + lane];
+      for (int c = lane; c < rows; c += 32) sum = fmaf(from.qt[(place * C + r) * rows + c], n0[c], sum);
       sum = warp_sum(sum);
       if (lane == 0) den[(first + r) * heads + head] = sum;
     }
   }
-  for (int slab = 0; slab < slabs; ++slab) {
-    if (slab + 1 < slabs) {
-      fetch(slab + 1);
-      wait_copies<1>();
-    } else {
-      wait_copies<0>();
+  if (col0 >= columns) return;
+  float4 left[4], right[4];
+  auto fetch = [&](int step) {
+    const bool in_state = step < state_steps, is_u = WITH_U && step < state_steps + 2;
+    const int half = (step - state_steps) & 1;  // of the chunk's tokens, behind the state
+    const float* from_left = in_state ? from.qt + place * C * rows + step * 16 : (is_u ? from.a : from.av) + place * C * C + half * 16;
+    const int ld = in_state ? rows : C;
+#pragma unroll
+    for (int r = 0; r < 4; ++r) left[r] = *reinterpret_cast<const float4*>(from_left + (8 * r + g) * ld + 4 * q);
+#pragma unroll
+    for (int t = 0; t < 4; ++t) {
+      const int col = col0 + 8 * t + g;
+      if (in_state || is_u) {
+        const float* at = in_state ? from.s + place * columns * rows + s_place(col, step * 16 + 4 * q, rows) : from.x + (place * columns + col) * C + half * 16 + 4 * q;
+        right[t] = col < columns ? *reinterpret_cast<const float4*>(at) : make_float4(0.f, 0.f, 0.f, 0.f);
+      } else {
+        const int token = half * 16 + 4 * q;
+        const float* at = v + (first + token) * v_ld + static_cast<int64_t>(head) * dv + col;
+        const bool valid = col < dv;
+        right[t] = make_float4(valid && token < n ? at[0] : 0.f, valid && token + 1 < n ? at[v_ld] : 0.f, valid && token + 2 < n ? at[2 * v_ld] : 0.f,
+                               valid && token + 3 < n ? at[3 * v_ld] : 0.f);
+      }
     }
-    __syncthreads();
-    const float* left = chunk_smem + (slab & 1) * kStage + it * kLdSlab;
-    const float* right = chunk_smem + (slab & 1) * kStage + C * kLdSlab + ct * 4;
-    float sum[8][4];  // one slab's sum by itself: fewer roundings of the whole
+  };
+  float acc[2][4][4];  // tokens 16 m + g (+ 8) of columns 2 q, + 1 of tile t
 #pragma unroll
-    for (int i = 0; i < 8; ++i) sum[i][0] = sum[i][1] = sum[i][2] = sum[i][3] = 0.f;
-    // Pairs of tokens form a triangle: a token leaves out those behind it (a value there that is not finite times a pair's zero is
-    // not zero). Tokens 4 i .. + 3 of a warp stand against tokens k .. k + 3, so only one group of four looks at its lanes.
-    auto multiply = [&](auto triangle) {
-      constexpr bool kTriangle = decltype(triangle)::value;
-#pragma unroll 2
-      for (int k = 0; k < C; k += 4) {
-        float4 b[4];
+  for (int m = 0; m < 2; ++m)
 #pragma unroll
-        for (int x = 0; x < 4; ++x) b[x] = *reinterpret_cast<const float4*>(right + (k + x) * kLdOut);
+    for (int t = 0; t < 4; ++t) acc[m][t][0] = acc[m][t][1] = acc[m][t][2] = acc[m][t][3] = 0.f;
+  int spoilt[4] = {C, C, C, C};  // the first token of a column whose U or V is not finite
+  bool any_spoilt = false;
+  fetch(0);
+  for (int step = 0; step < steps; ++step) {
+    const bool pairs = step >= state_steps;
+    const int half = (step - state_steps) & 1;
+    if (pairs) {
+      bool found = false;
 #pragma unroll
-        for (int i = 0; i < 8; ++i) {
-          if (kTriangle && k > 4 * i) continue;
-          const float4 a = *reinterpret_cast<const float4*>(left + i * 4 * kLdSlab + k);
-          const float f[4] = {a.x, a.y, a.z, a.w};
+      for (int t = 0; t < 4; ++t) {
+        float* numbers[4] = {&right[t].x, &right[t].y, &right[t].z, &right[t].w};
 #pragma unroll
-          for (int x = 0; x < 4; ++x) {
-            if (kTriangle && k == 4 * i && x > it) continue;
-            sum[i][0] = fmaf(f[x], b[x].x, sum[i][0]), sum[i][1] = fmaf(f[x], b[x].y, sum[i][1]);
-            sum[i][2] = fmaf(f[x], b[x].z, sum[i][2]), sum[i][3] = fmaf(f[x], b[x].w, sum[i][3]);
-          }
+        for (int i = 3; i >= 0; --i)
+          if (!isfinite(*numbers[i])) *numbers[i] = 0.f, spoilt[t] = min(spoilt[t], half * 16 + 4 * q + i), found = true;
+      }
+      any_spoilt |= __any_sync(0xffffffffu, found);
+    }
+    SplitA a[2];
+#pragma unroll
+    for (int r = 0; r < 4; ++r) a[r >> 1].set(r & 1, split_pair(left[r].x, left[r].y)), a[r >> 1].set((r & 1) + 2, split_pair(left[r].z, left[r].w));
+    SplitB b[4] = {SplitB(right[0]), SplitB(right[1]), SplitB(right[2]), SplitB(right[3])};
+    if (step + 1 < steps) fetch(step + 1);
+#pragma unroll
+    for (int m = 0; m < 2; ++m) {
+      if ((m == 0 && pairs && half == 1) || 16 * m >= n) continue;  // tokens behind, or none
+      float sum[4][4];
+#pragma unroll
+      for (int t = 0; t < 4; ++t) {
+        sum[t][0] = sum[t][1] = sum[t][2] = sum[t][3] = 0.f;
+        mma_split(sum[t], a[m], b[t]);
+      }
+#pragma unroll
+      for (int t = 0; t < 4; ++t)
+#pragma unroll
+        for (int i = 0; i < 4; ++i) acc[m][t][i] += sum[t][i];
+    }
+  }
+  if (any_spoilt) {
+#pragma unroll
+    for (int t = 0; t < 4; ++t) {
+      int token = spoilt[t];  // of column g: the least of its four lanes
+      token = min(token, __shfl_xor_sync(0xffffffffu, token, 1));
+      token = min(token, __shfl_xor_sync(0xffffffffu, token, 2));
+#pragma unroll
+      for (int c = 0; c < 2; ++c) {
+        const int from_token = __shfl_sync(0xffffffffu, token, (2 * q + c) * 4);
+#pragma unroll
+        for (int m = 0; m < 2; ++m) {
+          if (16 * m + g >= from_token) acc[m][t][c] = NAN;
+          if (16 * m + g + 8 >= from_token) acc[m][t][2 + c] = NAN;
         }
       }
-    };
-    if (slab < state_slabs) multiply(std::false_type{});
-    else multiply(std::true_type{});
-#pragma unroll
-    for (int i = 0; i < 8; ++i) acc[i][0] += sum[i][0], acc[i][1] += sum[i][1], acc[i][2] += sum[i][2], acc[i][3] += sum[i][3];
-    __syncthreads();
-  }
-  const int c = col0 + ct * 4;
-#pragma unroll
-  for (int i = 0; i < 8; ++i) {
-    const int row = it + 4 * i;
-    if (row >= n) continue;
-    float* to = out + ((first + row) * heads + head) * dv + c;
-    if (dv % 4 == 0 && (reinterpret_cast<uintptr_t>(out) & 15) == 0) {
-      if (c < dv) *reinterpret_cast<float4*>(to) = make_float4(acc[i][0], acc[i][1], acc[i][2], acc[i][3]);
-    } else {
-#pragma unroll
-      for (int x = 0; x < 4; ++x)
-        if (c + x < dv) to[x] = acc[i][x];
     }
   }
+  const bool wide = dv % 2 == 0 && (reinterpret_cast<uintptr_t>(out) & 7) == 0;
+#pragma unroll
+  for (int m = 0; m < 2; ++m)
+#pragma unroll
+    for (int r = 0; r < 2; ++r) {
+      const int token = 16 * m + 8 * r + g;
+      if (token >= n) continue;
+#pragma unroll
+      for (int t = 0; t < 4; ++t) {
+        const int col = col0 + 8 * t + 2 * q;
+        float* to = out + ((first + token) * heads + head) * dv + col;
+        if (wide) {
+          if (col < dv) *reinterpret_cast<float2*>(to) = make_float2(acc[m][t][2 * r], acc[m][t][2 * r + 1]);
+        } else {
+          if (col < dv) to[0] = acc[m][t][2 * r];
+          if (col + 1 < dv) to[1] = acc[m][t][2 * r + 1];
+        }
+      }
+    }
 }
 
 // --- host ------------------------------------------------------------------------------------------------------------------------------
@@ -1058,8 +1101,8 @@ int64_t aligned_floats(int64_t n) { return (n + 3) / 4 * 4; }
 
 // The scratch's arrays for so many heads one after another in `base` (null pointers with a null base); returns the numbers they need.
 int64_t lay_out(int rule, const Sizes& z, int heads, float* base, Scratch* to) {
-  const int64_t rows = padded_rows(z.dk), columns = padded_columns(z.dv), per_head = static_cast<int64_t>(z.tokens) * heads;
-  const int64_t chunks = (static_cast<int64_t>(z.tokens) / C + z.seqs + 1) * heads;
+  const int64_t rows = padded_rows(z.dk), columns = padded_columns(z.dv);
+  const int64_t chunks = (static_cast<int64_t>(z.tokens) / C + z.seqs + 1) * heads, per_head = chunks * C;
   const int64_t with_u = rule == kDelta || rule == kGeneralDelta ? 1 : 0, with_v = rule != kDelta ? 1 : 0, with_n = rule == kMemory ? 1 : 0;
   const int64_t sizes[9] = {with_u * per_head * rows, with_u * per_head * rows, per_head * rows, with_u * per_head * columns,
                             with_u * per_head * C, with_v * per_head * C, chunks * rows, with_n * chunks * rows, chunks * rows * columns};
@@ -1083,13 +1126,13 @@ bool raise_prepares() {
   const size_t delta = prepare_smem(ROWS);
   bool ok = raise_smem(chunk_prepare_kernel<ROWS, 1, false>, delta) && raise_smem(chunk_prepare_kernel<ROWS, 4, false>, delta) &&
             raise_smem(chunk_prepare_kernel<ROWS, 1, true>, delta) && raise_smem(chunk_prepare_kernel<ROWS, 4, true>, delta) &&
-            raise_smem(chunk_walk_kernel<ROWS, false>, walk_smem(ROWS));
+            raise_smem(chunk_walk_kernel<ROWS, false>, walk_smem(ROWS, false));
   if constexpr (ROWS <= kMaxLinearRows) {
     const size_t general = linear_prepare_smem(ROWS, kGeneralDelta), linear = linear_prepare_smem(ROWS, kLinear), memory = linear_prepare_smem(ROWS, kMemory);
     ok = ok && raise_smem(linear_chunk_prepare_kernel<ROWS, 1, kLinear>, linear) && raise_smem(linear_chunk_prepare_kernel<ROWS, 4, kLinear>, linear) &&
          raise_smem(linear_chunk_prepare_kernel<ROWS, 1, kGeneralDelta>, general) && raise_smem(linear_chunk_prepare_kernel<ROWS, 4, kGeneralDelta>, general) &&
          raise_smem(linear_chunk_prepare_kernel<ROWS, 1, kMemory>, memory) && raise_smem(linear_chunk_prepare_kernel<ROWS, 4, kMemory>, memory) &&
-         raise_smem(chunk_walk_kernel<ROWS, true>, walk_smem(ROWS));
+         raise_smem(chunk_walk_kernel<ROWS, true>, walk_smem(ROWS, true));
   }
   return ok;
 }
@@ -1144,7 +1187,7 @@ int launch_walk(const Sizes& z, const Requests& req, bool add, const Scratch& sc
   auto walk = add ? (rows == 64 ? chunk_walk_kernel<64, true> : chunk_walk_kernel<128, true>)
                   : (rows == 64 ? chunk_walk_kernel<64, false> : (rows == 128 ? chunk_walk_kernel<128, false> : chunk_walk_kernel<256, false>));
   // The ordinary way, not early: the few long-lived blocks should spread over all SMs, not over those the kernel in front leaves first.
-  launch_kernel_as(true, walk, dim3(padded_columns(z.dv) / kColumns, scratch.heads, z.seqs), dim3(kThreads), walk_smem(rows), stream, req.q_start, req.q_len, req.slot,
+  launch_kernel_as(true, walk, dim3(padded_columns(z.dv) / kColumns, scratch.heads, z.seqs), dim3(2 * rows), walk_smem(rows, add), stream, req.q_start, req.q_len, req.slot,
                    z.heads, z.dk, z.dv, scratch, state);
   return b200_check_launch("chunk_walk");
 }
@@ -1153,8 +1196,7 @@ template <bool WITH_U, bool WITH_V>
 int launch_out(const Sizes& z, const Requests& req, const Scratch& scratch, const float* v, int64_t v_ld, float* out, float* den, cudaStream_t stream) {
   const int columns = padded_columns(z.dv), cols = columns <= 64 ? 64 : 128, tiles = (columns + cols - 1) / cols;
   launch_kernel(cols == 64 ? chunk_out_kernel<64, WITH_U, WITH_V> : chunk_out_kernel<128, WITH_U, WITH_V>, dim3((z.max_q_len + C - 1) / C, scratch.heads, z.seqs * tiles),
-                dim3(cols), out_smem(cols), stream, req.q_start, req.q_len, z.heads, z.dv, padded_rows(z.dk), tiles, scratch, v,
-                v_ld, z.dv % 4 == 0 && v_ld % 4 == 0 && aligned16(v) ? 1 : 0, out, den);
+                dim3(cols), 0, stream, req.q_start, req.q_len, z.heads, z.dv, padded_rows(z.dk), tiles, scratch, v, v_ld, out, den);
   return b200_check_launch("chunk_out");
 }
 
@@ -1166,8 +1208,8 @@ int launch_linear_prepare(const Sizes& z, const Requests& req, int rule, bool wi
 }
 
 int launch_scan(const Sizes& z, const Requests& req, const Scratch& scratch, float* state, float* normaliser, cudaStream_t stream) {
-  const int rows = padded_rows(z.dk), blocks = (rows * padded_columns(z.dv) / 4 + kThreads - 1) / kThreads;
-  launch_kernel(chunk_scan_kernel, dim3(blocks + (normaliser != nullptr ? (rows + kThreads - 1) / kThreads : 0), scratch.heads, z.seqs), dim3(kThreads), 0, stream, req.q_start,
+  const int rows = padded_rows(z.dk), blocks = (rows * padded_columns(z.dv) / 4 + kScanThreads - 1) / kScanThreads;
+  launch_kernel(chunk_scan_kernel, dim3(blocks + (normaliser != nullptr ? (rows + kScanThreads - 1) / kScanThreads : 0), scratch.heads, z.seqs), dim3(kScanThreads), 0, stream, req.q_start,
                 req.q_len, req.slot, z.heads, z.dk, z.dv, scratch, state, normaliser);
   return b200_check_launch("chunk_scan");
 }
