@@ -74,10 +74,10 @@ delta_general_prepare_wide_kernel(const T* proj, int ld, int r_at, int k_at, int
   *reinterpret_cast<float4*>(r_out + at) = rv;
   *reinterpret_cast<float4*>(k_out + at) = kv;
   *reinterpret_cast<float4*>(v_out + at) = vv;
-  *reinterpret_cast<float4*>(w_out + at) = make_float4(expf(-kDecayRate * sigmoid_f(z.x + bias.x)), expf(-kDecayRate * sigmoid_f(z.y + bias.y)),
-                                                       expf(-kDecayRate * sigmoid_f(z.z + bias.z)), expf(-kDecayRate * sigmoid_f(z.w + bias.w)));
-  *reinterpret_cast<float4*>(au_out + at) = make_float4(sigmoid_f(av.x + a_shift.x) * u.x, sigmoid_f(av.y + a_shift.y) * u.y, sigmoid_f(av.z + a_shift.z) * u.z,
-                                                        sigmoid_f(av.w + a_shift.w) * u.w);
+  *reinterpret_cast<float4*>(w_out + at) = make_float4(expf(-kDecayRate * sigmoid_quick(z.x + bias.x)), expf(-kDecayRate * sigmoid_quick(z.y + bias.y)),
+                                                       expf(-kDecayRate * sigmoid_quick(z.z + bias.z)), expf(-kDecayRate * sigmoid_quick(z.w + bias.w)));
+  *reinterpret_cast<float4*>(au_out + at) = make_float4(sigmoid_quick(av.x + a_shift.x) * u.x, sigmoid_quick(av.y + a_shift.y) * u.y, sigmoid_quick(av.z + a_shift.z) * u.z,
+                                                        sigmoid_quick(av.w + a_shift.w) * u.w);
   *reinterpret_cast<float4*>(u_out + at) = u;
 }
 

@@ -23,6 +23,7 @@
 namespace {
 
 __device__ __forceinline__ float sigmoid_f(float x) { return 1.f / (1.f + expf(-x)); }
+__device__ __forceinline__ float silu_f(float x) { return x * sigmoid_quick(x); }
 __device__ __forceinline__ float softplus_f(float x) { return x > 20.f ? x : log1pf(expf(x)); }
 
 // `proj` rows: [q (kv_heads*dk) | k (kv_heads*dk) | v (heads*dv) | b (heads)]; the first
@@ -92,104 +93,162 @@ __global__ void delta_prepare_kernel(const T* proj, int ld, const T* decay_in, i
   }
 }
 
-// The same for prompt portions and four taps: four neighbouring tokens a block, four neighbouring channels a thread at a time, so a
-// row of inputs and a channel's taps are read once for the four tokens that want them, eight or sixteen bytes an access. One block a
-// token read two bytes at a time, every row four times: on a B200 2,048 tokens of 4,608 channels took 79 us with a decay per channel and
-// 46 with one per head (3,072 channels), now 58 and 30.
-constexpr int kWideTokens = 4, kWideTaps = 4;
+// The same for prompt portions and four taps. A warp takes four neighbouring tokens and up to 128 channels: a q and a k head, or a piece of
+// the values or of the decays, four neighbouring channels a lane, so that nothing passes through shared memory, rows and taps
+// are read once for the four tokens that want them, and a lane's seven rows are asked for together. Only tokens next to a request's
+// start look into its slot.
+// What bounds it: instructions (exponentials, logarithms, quotients). One block for four tokens of all channels held 128 registers a thread, so
+// two blocks an SM, and went through a token's rows with a look at its request for every tap: on a B200 2,048 tokens of 4,608 channels took
+// 58 us with a decay per channel and 30 with one per head (3,072 channels), now 29 and 16
+// (with divisions 52 and 26: their code, in line sixteen times, did not fit what an SM holds of it).
+constexpr int kWideTokens = 4, kWideTaps = 4, kWideChannels = 128;
 
+struct WidePrepare {
+  int ld, decay_ld, tokens, heads, kv_heads, dk, dv;
+  const float* taps_w;
+  const float* a_log;
+  const float* dt_bias;
+  const int* token_seq;
+  const int* seq_q_start;
+  const int* seq_slot;
+  float* q_out;
+  float* k_out;
+  float* v_out;
+  float* beta_out;
+  float* decay_out;
+  float* kq_out;
+  int v_pieces, decay_pieces;
+};
+
+// Channels c .. + 3 of tokens t0 .. + 3 behind the convolution and silu. `inside`: all of them at least three tokens into one request.
 template <typename T>
-__global__ void __launch_bounds__(256)
-delta_prepare_wide_kernel(const T* proj, int ld, const T* decay_in, int decay_ld, const float* __restrict__ taps_w, const T* conv_state,
-                          const float* __restrict__ a_log, const float* __restrict__ dt_bias, const int* token_seq, const int* seq_q_start,
-                          const int* seq_slot, int tokens, int heads, int kv_heads, int dk, int dv, float* q_out, float* k_out, float* v_out, float* beta_out,
-                          float* decay_out, float* kq_out) {
-  extern __shared__ __align__(16) float y[];  // [kWideTokens][2 * kv_heads * dk]: q and k behind the convolution
-  __shared__ int start_of[kWideTokens], slot_of[kWideTokens];
+__device__ __forceinline__ void convolve_wide(float4 (&y)[kWideTokens], const WidePrepare& p, const T* proj, const T* conv_state, int t0, int count, bool inside, int c) {
+  float4 rows[kWideTokens + kWideTaps - 1];  // inputs of tokens t0 - 3 .. t0 + 3
+#pragma unroll
+  for (int i = 0; i < kWideTokens + kWideTaps - 1; ++i) {
+    const int t = t0 - (kWideTaps - 1) + i;
+    rows[i] = t >= 0 && t < p.tokens ? load4<T>(proj + static_cast<int64_t>(t) * p.ld + c) : make_float4(0.f, 0.f, 0.f, 0.f);
+  }
+  float4 taps[4];  // of channel c + x
+#pragma unroll
+  for (int x = 0; x < 4; ++x) taps[x] = *reinterpret_cast<const float4*>(p.taps_w + (c + x) * kWideTaps);
+  const float* w[4] = {&taps[0].x, &taps[1].x, &taps[2].x, &taps[3].x};
+#pragma unroll
+  for (int i = 0; i < kWideTokens; ++i) {
+    float4 in[kWideTaps];
+#pragma unroll
+    for (int j = 0; j < kWideTaps; ++j) in[j] = rows[i + j];
+    if (!inside && i < count) {
+      const int seq = p.token_seq[t0 + i], run = t0 + i - p.seq_q_start[seq];  // tokens of this request in front of t within the step
+      const int64_t slot = static_cast<int64_t>(p.seq_slot[seq]) * (kWideTaps - 1);
+#pragma unroll
+      for (int j = 0; j < kWideTaps - 1; ++j)
+        if (kWideTaps - 1 - j > run) in[j] = load4<T>(conv_state + (slot + run + j) * (2 * p.kv_heads * p.dk + p.heads * p.dv) + c);
+    }
+    float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+    for (int j = 0; j < kWideTaps; ++j) {
+      acc.x = fmaf(w[0][j], in[j].x, acc.x), acc.y = fmaf(w[1][j], in[j].y, acc.y);
+      acc.z = fmaf(w[2][j], in[j].z, acc.z), acc.w = fmaf(w[3][j], in[j].w, acc.w);
+    }
+    y[i] = make_float4(silu_f(acc.x), silu_f(acc.y), silu_f(acc.z), silu_f(acc.w));
+  }
+}
+
+template <typename T, int QUADS>  // QUADS: a q or k head has up to 128 QUADS channels
+__global__ void __launch_bounds__(128, QUADS == 1 ? 6 : 4)
+delta_prepare_wide_kernel(const WidePrepare p, const T* proj, const T* decay_in, const T* conv_state) {
+  const int items = p.kv_heads + p.v_pieces + p.decay_pieces + 1;
+  const int64_t warp = static_cast<int64_t>(blockIdx.x) * 4 + (threadIdx.x >> 5);
+  // Tokens run fastest: what an SM works on at a time is then of one kind, whose code it holds.
+  const int groups = (p.tokens + kWideTokens - 1) / kWideTokens;
+  const int t0 = static_cast<int>(warp % groups) * kWideTokens, lane = threadIdx.x & 31;
+  int item = static_cast<int>(warp / groups);
+  if (item >= items) return;
+  const int count = min(kWideTokens, p.tokens - t0);
+  const int qk = p.kv_heads * p.dk, vw = p.heads * p.dv;
+  const int seq = p.token_seq[t0];
+  const bool inside = p.token_seq[t0 + count - 1] == seq && t0 - p.seq_q_start[seq] >= kWideTaps - 1;
   wait_for_predecessor();
   let_successor_start();
-  const int t0 = blockIdx.x * kWideTokens, tid = threadIdx.x, count = min(kWideTokens, tokens - t0);
-  const int qk = kv_heads * dk, vw = heads * dv, channels = 2 * qk + vw;
-  if (tid < count) {
-    const int seq = token_seq[t0 + tid];
-    start_of[tid] = seq_q_start[seq];
-    slot_of[tid] = seq_slot[seq];
-  }
-  __syncthreads();
-  for (int c = tid * 4; c < channels; c += blockDim.x * 4) {
-    float4 rows[kWideTokens + kWideTaps - 1];  // inputs of tokens t0 - 3 .. t0 + 3
+  if (item < p.kv_heads) {  // unit vectors, and k . q
+    float q_factor[kWideTokens], k_factor[kWideTokens], dot[kWideTokens];
+    float4 q[QUADS][kWideTokens], k[QUADS][kWideTokens];
 #pragma unroll
-    for (int i = 0; i < kWideTokens + kWideTaps - 1; ++i) {
-      const int t = t0 - (kWideTaps - 1) + i;
-      rows[i] = t >= 0 && t < tokens ? load4<T>(proj + static_cast<int64_t>(t) * ld + c) : make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int x = 0; x < QUADS; ++x) {
+      const int c = x * kWideChannels + lane * 4;
+      if (c < p.dk) {
+        convolve_wide<T>(q[x], p, proj, conv_state, t0, count, inside, item * p.dk + c);
+        convolve_wide<T>(k[x], p, proj, conv_state, t0, count, inside, qk + item * p.dk + c);
+      } else {
+#pragma unroll
+        for (int i = 0; i < kWideTokens; ++i) q[x][i] = k[x][i] = make_float4(0.f, 0.f, 0.f, 0.f);
+      }
     }
-    float4 taps[4];  // of channel c + x
 #pragma unroll
-    for (int x = 0; x < 4; ++x) taps[x] = *reinterpret_cast<const float4*>(taps_w + (c + x) * kWideTaps);
+    for (int i = 0; i < kWideTokens; ++i) {
+      float q_ss = 0.f, k_ss = 0.f;
+      dot[i] = 0.f;
+#pragma unroll
+      for (int x = 0; x < QUADS; ++x) {
+        const float4 a = q[x][i], b = k[x][i];
+        q_ss = square_sum(a, q_ss), k_ss = square_sum(b, k_ss);
+        dot[i] = fmaf(a.x, b.x, fmaf(a.y, b.y, fmaf(a.z, b.z, fmaf(a.w, b.w, dot[i]))));
+      }
+      q_ss = warp_sum(q_ss), k_ss = warp_sum(k_ss);
+      q_factor[i] = (1.f / sqrtf(q_ss + 1e-6f)) * (1.f / sqrtf(static_cast<float>(p.dk))), k_factor[i] = 1.f / sqrtf(k_ss + 1e-6f);
+    }
 #pragma unroll
     for (int i = 0; i < kWideTokens; ++i) {
       if (i >= count) break;
-      const int run = t0 + i - start_of[i];  // tokens of this request in front of t within the step
-      float4 in[kWideTaps];
+      const int64_t t = t0 + i;
 #pragma unroll
-      for (int j = 0; j < kWideTaps; ++j) {
-        in[j] = rows[i + j];
-        if (kWideTaps - 1 - j > run)  // from the request's slot
-          in[j] = load4<T>(conv_state + (static_cast<int64_t>(slot_of[i]) * (kWideTaps - 1) + run + j) * channels + c);
+      for (int x = 0; x < QUADS; ++x) {
+        const int c = x * kWideChannels + lane * 4;
+        if (c >= p.dk) break;
+        *reinterpret_cast<float4*>(p.q_out + t * qk + item * p.dk + c) = scale_each(q[x][i], q_factor[i]);
+        *reinterpret_cast<float4*>(p.k_out + t * qk + item * p.dk + c) = scale_each(k[x][i], k_factor[i]);
       }
-      float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
-      const float* w[4] = {&taps[0].x, &taps[1].x, &taps[2].x, &taps[3].x};
+      if (p.kq_out != nullptr) {
+        const float whole = warp_sum(dot[i]);
+        if (lane == 0) p.kq_out[t * p.kv_heads + item] = whole * k_factor[i] * q_factor[i];
+      }
+    }
+    return;
+  }
+  item -= p.kv_heads;
+  if (item < p.v_pieces) {
+    const int c = item * kWideChannels + lane * 4;
+    if (c >= vw) return;
+    float4 y[kWideTokens];
+    convolve_wide<T>(y, p, proj, conv_state, t0, count, inside, 2 * qk + c);
 #pragma unroll
-      for (int j = 0; j < kWideTaps; ++j) {
-        acc.x = fmaf(w[0][j], in[j].x, acc.x), acc.y = fmaf(w[1][j], in[j].y, acc.y);
-        acc.z = fmaf(w[2][j], in[j].z, acc.z), acc.w = fmaf(w[3][j], in[j].w, acc.w);
-      }
-      acc = make_float4(acc.x * sigmoid_f(acc.x), acc.y * sigmoid_f(acc.y), acc.z * sigmoid_f(acc.z), acc.w * sigmoid_f(acc.w));
-      if (c < 2 * qk) *reinterpret_cast<float4*>(y + i * 2 * qk + c) = acc;
-      else *reinterpret_cast<float4*>(v_out + static_cast<int64_t>(t0 + i) * vw + c - 2 * qk) = acc;
-    }
+    for (int i = 0; i < kWideTokens; ++i)
+      if (i < count) *reinterpret_cast<float4*>(p.v_out + static_cast<int64_t>(t0 + i) * vw + c) = y[i];
+    return;
   }
-  const bool per_head = kq_out != nullptr;
-  for (int idx = tid; idx < count * heads; idx += blockDim.x) {
-    const int64_t t = t0 + idx / heads;
-    const int h = idx % heads;
-    beta_out[t * heads + h] = sigmoid_f(to_f32<T>(proj[t * ld + channels + h]));
-    if (per_head) decay_out[t * heads + h] = -expf(a_log[h]) * softplus_f(to_f32<T>(decay_in[t * decay_ld + h]) + dt_bias[h]);
+  item -= p.v_pieces;
+  if (item < p.decay_pieces) {  // one per head and key channel
+    const int c = item * kWideChannels + lane * 4;
+    if (c >= p.heads * p.dk) return;
+    const float rate = -expf(p.a_log[c / p.dk]);
+    const float4 bias = *reinterpret_cast<const float4*>(p.dt_bias + c);
+    float4 next = load4<T>(decay_in + static_cast<int64_t>(t0) * p.decay_ld + c);
+#pragma unroll 1
+    for (int i = 0; i < count; ++i) {
+      const float4 z = next;
+      if (i + 1 < count) next = load4<T>(decay_in + static_cast<int64_t>(t0 + i + 1) * p.decay_ld + c);
+      *reinterpret_cast<float4*>(p.decay_out + static_cast<int64_t>(t0 + i) * p.heads * p.dk + c) =
+          make_float4(expf(rate * softplus_f(z.x + bias.x)), expf(rate * softplus_f(z.y + bias.y)), expf(rate * softplus_f(z.z + bias.z)),
+                      expf(rate * softplus_f(z.w + bias.w)));
+    }
+    return;
   }
-  if (!per_head) {
-    for (int i = 0; i < count; ++i)
-      for (int c = tid * 4; c < heads * dk; c += blockDim.x * 4) {
-        const float4 z = load4<T>(decay_in + static_cast<int64_t>(t0 + i) * decay_ld + c), bias = *reinterpret_cast<const float4*>(dt_bias + c);
-        const float rate = -expf(a_log[c / dk]);
-        *reinterpret_cast<float4*>(decay_out + static_cast<int64_t>(t0 + i) * heads * dk + c) =
-            make_float4(expf(rate * softplus_f(z.x + bias.x)), expf(rate * softplus_f(z.y + bias.y)), expf(rate * softplus_f(z.z + bias.z)),
-                        expf(rate * softplus_f(z.w + bias.w)));
-      }
-  }
-  __syncthreads();
-  const int lane = tid & 31, warp = tid >> 5, warps = blockDim.x >> 5;
-  // unit vectors: one warp per (token, q/k head), q and k one after the other, and k . q
-  for (int item = warp; item < count * kv_heads; item += warps) {
-    const int64_t t = t0 + item / kv_heads;
-    const int head = item % kv_heads;
-    const float* q = y + item / kv_heads * 2 * qk + head * dk;
-    const float* k = q + qk;
-    float q_ss = 0.f, k_ss = 0.f, dot = 0.f;
-    for (int i = lane * 4; i < dk; i += 128) {
-      const float4 a = *reinterpret_cast<const float4*>(q + i), b = *reinterpret_cast<const float4*>(k + i);
-      q_ss = square_sum(a, q_ss), k_ss = square_sum(b, k_ss);
-      dot = fmaf(a.x, b.x, fmaf(a.y, b.y, fmaf(a.z, b.z, fmaf(a.w, b.w, dot))));
-    }
-    q_ss = warp_sum(q_ss), k_ss = warp_sum(k_ss);
-    const float q_factor = (1.f / sqrtf(q_ss + 1e-6f)) * (1.f / sqrtf(static_cast<float>(dk))), k_factor = 1.f / sqrtf(k_ss + 1e-6f);
-    for (int i = lane * 4; i < dk; i += 128) {
-      *reinterpret_cast<float4*>(q_out + t * qk + head * dk + i) = scale_each(*reinterpret_cast<const float4*>(q + i), q_factor);
-      *reinterpret_cast<float4*>(k_out + t * qk + head * dk + i) = scale_each(*reinterpret_cast<const float4*>(k + i), k_factor);
-    }
-    if (per_head) {
-      dot = warp_sum(dot);
-      if (lane == 0) kq_out[t * kv_heads + head] = dot * k_factor * q_factor;
-    }
+  for (int idx = lane; idx < count * p.heads; idx += 32) {
+    const int64_t t = t0 + idx / p.heads;
+    const int h = idx % p.heads;
+    p.beta_out[t * p.heads + h] = sigmoid_f(to_f32<T>(proj[t * p.ld + 2 * qk + vw + h]));
+    if (p.kq_out != nullptr) p.decay_out[t * p.heads + h] = -expf(p.a_log[h]) * softplus_f(to_f32<T>(decay_in[t * p.decay_ld + h]) + p.dt_bias[h]);
   }
 }
 
@@ -382,7 +441,7 @@ delta_output_wide_kernel(const float* o, const float* __restrict__ weight, const
   float ss = square_sum(x, 0.f);
   for (int step = lanes >> 1; step > 0; step >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, step);
   const float inv = 1.f / sqrtf(ss / static_cast<float>(dv) + eps);
-  const auto gated = [](float z) { return SILU ? z * sigmoid_f(z) : sigmoid_f(z); };
+  const auto gated = [](float z) { return SILU ? silu_f(z) : sigmoid_quick(z); };
   if (live)
     store4<T>(out + item * dv + i, make_float4(x.x * inv * w.x * gated(g.x), x.y * inv * w.y * gated(g.y), x.z * inv * w.z * gated(g.z), x.w * inv * w.w * gated(g.w)));
 }
@@ -403,22 +462,23 @@ B200_API int b200_delta_prepare(const void* proj, int ld, const void* decay_in, 
   const int threads = 256;
   const int update_blocks = (channels + threads - 1) / threads;  // a thread per channel: the slots' update is a tail of its own
   // The wide form from half a block an SM on, with rows, taps and results on 16-byte (bfloat16 rows: 8-byte) boundaries.
-  const size_t wide_smem = sizeof(float) * kWideTokens * 2 * kv_heads * dk;
   const auto on = [](const void* p, int bytes) { return reinterpret_cast<uintptr_t>(p) % bytes == 0; };
   const int in_bytes = dtype == DTYPE_F32 ? 16 : 8;
-  const bool wide = taps == kWideTaps && tokens >= kWideTokens * b200_sm_count_host() / 2 && ld % 4 == 0 && dk % 4 == 0 && dv % 4 == 0 && wide_smem <= 200 * 1024 &&
+  const bool wide = taps == kWideTaps && tokens >= kWideTokens * b200_sm_count_host() / 2 && ld % 4 == 0 && dk % 4 == 0 && dv % 4 == 0 && dk <= 2 * kWideChannels &&
                     on(proj, in_bytes) && on(conv_state, in_bytes) && on(taps_w, 16) && on(q_out, 16) && on(k_out, 16) && on(v_out, 16) &&
                     (kq_out != nullptr || (decay_ld % 4 == 0 && on(decay_in, in_bytes) && on(dt_bias, 16) && on(decay_out, 16)));
   auto launch_wide = [&](auto kernel, auto* typed) {
     using T = typename std::remove_pointer<decltype(typed)>::type;
-    if (wide_smem > 40 * 1024) cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(wide_smem));
-    launch_kernel(kernel, dim3((tokens + kWideTokens - 1) / kWideTokens), dim3(threads), wide_smem, stream, typed, ld, static_cast<const T*>(decay_in), decay_ld,
-                  taps_w, static_cast<const T*>(conv_state), a_log, dt_bias, token_seq, seq_q_start, seq_slot, tokens, heads, kv_heads, dk, dv, q_out, k_out, v_out,
-                  beta_out, decay_out, kq_out);
+    const auto pieces = [](int64_t n) { return static_cast<int>((n + kWideChannels - 1) / kWideChannels); };
+    const WidePrepare p = {ld, decay_ld, tokens, heads, kv_heads, dk, dv, taps_w, a_log, dt_bias, token_seq, seq_q_start, seq_slot, q_out, k_out, v_out, beta_out,
+                           decay_out, kq_out, pieces(static_cast<int64_t>(heads) * dv), kq_out != nullptr ? 0 : pieces(static_cast<int64_t>(heads) * dk)};
+    const int64_t warps = static_cast<int64_t>((tokens + kWideTokens - 1) / kWideTokens) * (kv_heads + p.v_pieces + p.decay_pieces + 1);
+    launch_kernel(kernel, dim3(static_cast<unsigned>((warps + 3) / 4)), dim3(128), 0, stream, p, typed, static_cast<const T*>(decay_in), static_cast<const T*>(conv_state));
   };
   if (wide && (dtype == DTYPE_F32 || dtype == DTYPE_BF16)) {
-    if (dtype == DTYPE_F32) launch_wide(delta_prepare_wide_kernel<float>, static_cast<const float*>(proj));
-    else launch_wide(delta_prepare_wide_kernel<__nv_bfloat16>, static_cast<const __nv_bfloat16*>(proj));
+    const bool one = dk <= kWideChannels;
+    if (dtype == DTYPE_F32) launch_wide(one ? delta_prepare_wide_kernel<float, 1> : delta_prepare_wide_kernel<float, 2>, static_cast<const float*>(proj));
+    else launch_wide(one ? delta_prepare_wide_kernel<__nv_bfloat16, 1> : delta_prepare_wide_kernel<__nv_bfloat16, 2>, static_cast<const __nv_bfloat16*>(proj));
     if (int status = b200_check_launch("delta_prepare")) return status;
     if (dtype == DTYPE_F32)
       launch_kernel(conv_state_update_kernel<float>, dim3(seqs, update_blocks), dim3(threads), 0, stream, static_cast<const float*>(proj), ld, channels, taps,

@@ -280,7 +280,7 @@ wkv_output_wide_kernel(const float* o, const float* __restrict__ weight, const T
   float ss = square_sum(x, 0.f);
   for (int step = lanes >> 1; step > 0; step >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, step);
   const float inv = 1.f / sqrtf(ss / static_cast<float>(dv) + eps);
-  const auto gated = [&](float z) { return sigmoid_gate ? sigmoid_f(z) : z * sigmoid_f(z); };
+  const auto gated = [&](float z) { return sigmoid_gate ? sigmoid_quick(z) : z * sigmoid_quick(z); };
   if (live)
     store4<T>(out + at, make_float4(x.x * inv * w.x * gated(g.x), x.y * inv * w.y * gated(g.y), x.z * inv * w.z * gated(g.z), x.w * inv * w.w * gated(g.w)));
 }
