@@ -1,4 +1,5 @@
-// True 32-bit matrix product for the float32 path:  C[M,N] = A[M,K] * W[N,K]^T (+ bias[N]).
+// True 32-bit matrix product for the float32 path:  C[M,N] = A[M,K] * W[N,K]^T (+ bias[N]); matrices that `b200_gemm_f32_split_takes`
+// names go to the kernel in gemm_f32_split.cu instead.
 //
 // Plain FMA on CUDA cores: no tensor cores, no TF32, no split accumulation. Each output
 // element is one chain of FMAs over k = 0..K-1 in order, so a row's result does not depend on

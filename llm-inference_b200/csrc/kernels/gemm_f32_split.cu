@@ -1,0 +1,311 @@
+// True 32-bit matrix product on the fifth-generation tensor cores:  C[M,N] = A[M,K] * W[N,K]^T (+ bias[N]), 32-bit operands and result.
+//
+// A number is the sum of three bfloat16 ones to its last bit: the nearest, the nearest to what is left, and the rest (8 + 8 + 8 bits). Of the nine
+// products of two such sums the six largest are taken; the others are below 2^-26 of the whole. Products of 8-bit numbers are exact in 32
+// bits. `tcgen05.mma` drops bits below the last when it adds, so its chains are short: over 64 numbers the twenty small products first, the
+// four large ones last, into an accumulator of their own, which is then added to 32-bit registers with ordinary rounding. Against 64
+// bits results are nearer than those of the FMA kernel (gemm_f32.cu), whose chains are K long: figures at `b200_gemm_f32_split_takes`.
+//
+// A block computes 128 rows of W by TOKENS rows of A (D[row of W][token]: W is the MMA's 128-row side). Eight warps fetch 32-bit rows, 64
+// numbers a stage, take them apart and store the parts K-major with 128-byte swizzle; one elected thread issues the 24 products of a
+// stage; four warps add up the accumulators, two of which take turns in TMEM. An output's sums are the same whatever the tile, so a row's result
+// does not depend on how many rows are in the call. Operands that are not finite make their row or column NaN.
+//
+// What bounds it: shared memory. Per stage at 128 x 128 the parts are 96 KB written and 192 KB read by the products, 2,300 cycles of an SM where
+// the tensor core needs 1,540; measured 3,290 (2,570 at 128 x 64). Two stages ahead in registers instead of one changed nothing.
+// Every wait is bounded; a block that gives up sets the timeout bit, frees its TMEM and leaves.
+#include "common.cuh"
+
+namespace {
+
+constexpr int kRows = 128;      // rows of W a block: MMA M
+constexpr int kBlockK = 64;     // numbers a stage: 128 bytes of a part, one swizzle row
+constexpr int kMmaK = 16;
+constexpr int kParts = 3;
+constexpr int kFetchWarps = 8;  // warps 0-7 fetch, 8 issues (9-11 only give their registers away), 12-15 add up
+constexpr int kAddWarp = 12;
+constexpr int kFetchThreads = kFetchWarps * 32;
+constexpr int kThreads = 512;
+// Registers a thread of the three kinds of warps, out of 512 x 128 at launch.
+constexpr int kFetchRegisters = 120, kIssueRegisters = 56, kAddRegisters = 208;
+static_assert(2 * kFetchRegisters + kIssueRegisters + kAddRegisters <= 4 * 128, "more registers than the block was launched with");
+constexpr long long kWaitCycles = 4000000000LL;  // about two seconds
+constexpr int ERRBIT_TIMEOUT = 8;
+
+__host__ __device__ constexpr int split_stages(int tokens) { return tokens <= 64 ? 3 : 2; }
+__host__ __device__ constexpr uint32_t part_bytes(int rows) { return static_cast<uint32_t>(rows) * kBlockK * 2; }
+__host__ __device__ constexpr uint32_t stage_bytes(int tokens) { return kParts * part_bytes(kRows + tokens); }
+constexpr size_t split_smem(int tokens) { return static_cast<size_t>(split_stages(tokens)) * stage_bytes(tokens) + 1024; }
+
+__device__ __forceinline__ uint32_t smem_addr(const void* p) { return static_cast<uint32_t>(__cvta_generic_to_shared(p)); }
+__device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count) {
+  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_addr(bar)), "r"(count) : "memory");
+}
+__device__ __forceinline__ void mbar_arrive(uint64_t* bar) { asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_addr(bar)) : "memory"); }
+// Bounded wait for the phase with the given parity to complete.
+__device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity) {
+  const uint32_t addr = smem_addr(bar);
+  const long long start = clock64();
+  while (true) {
+    uint32_t done;
+    asm volatile(
+        "{\n"
+        ".reg .pred p;\n"
+        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n"
+        "selp.u32 %0, 1, 0, p;\n"
+        "}\n"
+        : "=r"(done)
+        : "r"(addr), "r"(parity)
+        : "memory");
+    if (done) return true;
+    if (clock64() - start > kWaitCycles) return false;
+  }
+}
+// Shared-memory matrix descriptor of a K-major tile with 128-byte rows and 128-byte swizzle: groups of 8 rows are 1024 bytes apart.
+__device__ __forceinline__ uint64_t umma_smem_desc(uint32_t addr) {
+  uint64_t desc = 0;
+  desc |= static_cast<uint64_t>((addr & 0x3FFFFu) >> 4);
+  desc |= static_cast<uint64_t>(1) << 16;
+  desc |= static_cast<uint64_t>(1024 >> 4) << 32;
+  desc |= static_cast<uint64_t>(1) << 46;  // descriptor version (sm_100)
+  desc |= static_cast<uint64_t>(2) << 61;  // SWIZZLE_128B
+  return desc;
+}
+__device__ __forceinline__ void umma_bf16(uint32_t tmem_d, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, bool accumulate) {
+  asm volatile(
+      "{\n"
+      ".reg .pred p;\n"
+      "setp.ne.b32 p, %4, 0;\n"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n"
+      "}\n" ::"r"(tmem_d), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate ? 1u : 0u)
+      : "memory");
+}
+__device__ __forceinline__ void umma_commit(uint64_t* bar) {
+  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_addr(bar)) : "memory");
+}
+__device__ __forceinline__ void tmem_load_16(uint32_t taddr, float (&v)[16]) {
+  uint32_t r[16];
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
+        "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+      : "r"(taddr)
+      : "memory");
+  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+  for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(r[i]);
+}
+
+__device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
+  uint32_t d;
+  asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(d) : "f"(hi), "f"(lo));
+  return d;
+}
+// Eight neighbouring numbers of a row, in parts, to piece `piece` of the row in the three tiles of parts.
+__device__ __forceinline__ void store_parts(unsigned char* tile, uint32_t bytes, int row, int piece, float4 a, float4 b) {
+  float v[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+  unsigned char* to = tile + row * 128 + ((piece ^ (row & 7)) << 4);
+#pragma unroll
+  for (int p = 0; p < kParts; ++p) {
+    uint32_t word[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      word[i] = pack_bf16(v[2 * i], v[2 * i + 1]);
+      if (p + 1 < kParts) v[2 * i] -= __uint_as_float(word[i] << 16), v[2 * i + 1] -= __uint_as_float(word[i] & 0xffff0000u);
+    }
+    *reinterpret_cast<uint4*>(to + p * bytes) = make_uint4(word[0], word[1], word[2], word[3]);
+  }
+}
+
+struct SplitProduct {
+  const float* A;
+  const float* W;
+  const float* bias;
+  float* C;
+  int M, N, K, lda, ldw, ldc;
+  int* err;
+};
+
+template <int TOKENS>
+__global__ void __launch_bounds__(kThreads, 1)
+gemm_f32_split_kernel(const SplitProduct p) {
+  extern __shared__ __align__(1024) unsigned char smem_raw[];
+  constexpr int kStages = split_stages(TOKENS);
+  constexpr uint32_t kColumns = 2 * TOKENS < 32 ? 32 : 2 * TOKENS;  // of TMEM: two accumulators; a power of two
+  constexpr int kWItems = kRows * 8 / kFetchThreads, kAItems = TOKENS * 8 >= kFetchThreads ? TOKENS * 8 / kFetchThreads : 1;
+  unsigned char* tiles = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  __shared__ __align__(8) uint64_t full_bar[kStages], empty_bar[kStages], sum_full[2], sum_empty[2];
+  __shared__ uint32_t tmem_base_shared;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int n0 = blockIdx.x * kRows, m0 = blockIdx.y * TOKENS;
+  const int steps = (p.K + kBlockK - 1) / kBlockK;
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < kStages; ++s) mbar_init(&full_bar[s], kFetchWarps), mbar_init(&empty_bar[s], 1);
+    for (int b = 0; b < 2; ++b) mbar_init(&sum_full[b], 1), mbar_init(&sum_empty[b], 4);
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  if (warp == kFetchWarps) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_addr(&tmem_base_shared)), "r"(kColumns) : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  const uint32_t tmem_base = tmem_base_shared;
+  wait_for_predecessor();
+  let_successor_start();
+
+  if (warp < kFetchWarps) {
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kFetchRegisters));
+    // ---- fetch: eight lanes a row, eight numbers a lane; a stage's numbers are on the way while the one before is taken apart ----
+    const int piece = threadIdx.x & 7, row0 = threadIdx.x >> 3;  // rows row0, row0 + 32, ..
+    const bool takes_a = TOKENS * 8 >= kFetchThreads || row0 < TOKENS;
+    float4 w[kWItems][2], a[kAItems][2];
+    auto fetch = [&](float4 (&to)[2], const float* from, int64_t ld, int row, bool valid, int step) {
+      const int k = step * kBlockK + piece * 8;
+#pragma unroll
+      for (int h = 0; h < 2; ++h)
+        to[h] = valid && k + 4 * h < p.K ? *reinterpret_cast<const float4*>(from + row * ld + k + 4 * h) : make_float4(0.f, 0.f, 0.f, 0.f);
+    };
+    auto fetch_stage = [&](int step) {
+#pragma unroll
+      for (int i = 0; i < kWItems; ++i) fetch(w[i], p.W, p.ldw, n0 + row0 + 32 * i, n0 + row0 + 32 * i < p.N, step);
+#pragma unroll
+      for (int i = 0; i < kAItems; ++i) fetch(a[i], p.A, p.lda, m0 + row0 + 32 * i, takes_a && m0 + row0 + 32 * i < p.M, step);
+    };
+    fetch_stage(0);
+    for (int step = 0; step < steps; ++step) {
+      const int s = step % kStages;
+      if (step >= kStages && !mbar_wait(&empty_bar[s], (step / kStages - 1) & 1)) {
+        if (lane == 0) atomicOr(p.err, ERRBIT_TIMEOUT);
+        break;
+      }
+      unsigned char* stage = tiles + static_cast<size_t>(s) * stage_bytes(TOKENS);
+#pragma unroll
+      for (int i = 0; i < kWItems; ++i) store_parts(stage, part_bytes(kRows), row0 + 32 * i, piece, w[i][0], w[i][1]);
+      if (takes_a) {
+#pragma unroll
+        for (int i = 0; i < kAItems; ++i) store_parts(stage + kParts * part_bytes(kRows), part_bytes(TOKENS), row0 + 32 * i, piece, a[i][0], a[i][1]);
+      }
+      if (step + 1 < steps) fetch_stage(step + 1);
+      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&full_bar[s]);
+    }
+  } else if (warp < kAddWarp) {
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kIssueRegisters));
+    if (warp == kFetchWarps) {
+      // ---- issue: the whole warp walks the loop, one elected lane issues ----
+      uint32_t chosen;
+      asm volatile("{\n.reg .pred p;\nelect.sync _|p, 0xffffffff;\nselp.u32 %0, 1, 0, p;\n}\n" : "=r"(chosen));
+      const bool leader = chosen != 0;
+      const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | (static_cast<uint32_t>(TOKENS >> 3) << 17) | (static_cast<uint32_t>(kRows >> 4) << 24);
+      const uint64_t w_first = umma_smem_desc(smem_addr(tiles)), a_first = umma_smem_desc(smem_addr(tiles) + kParts * part_bytes(kRows));
+      for (int step = 0; step < steps; ++step) {
+        const int s = step % kStages, b = step & 1;
+        if (!mbar_wait(&full_bar[s], (step / kStages) & 1) || (step >= 2 && !mbar_wait(&sum_empty[b], (step / 2 - 1) & 1))) {
+          if (leader) atomicOr(p.err, ERRBIT_TIMEOUT);
+          break;
+        }
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        if (leader) {
+          constexpr int order[6][2] = {{2, 0}, {0, 2}, {1, 1}, {1, 0}, {0, 1}, {0, 0}};
+          const uint64_t stage_units = static_cast<uint64_t>(s) * (stage_bytes(TOKENS) >> 4);
+#pragma unroll
+          for (int x = 0; x < 6; ++x)
+#pragma unroll
+            for (int k = 0; k < kBlockK / kMmaK; ++k) {
+              const uint64_t at = stage_units + static_cast<uint64_t>(k * (kMmaK * 2 >> 4));
+              umma_bf16(tmem_base + b * TOKENS, w_first + at + order[x][0] * (part_bytes(kRows) >> 4), a_first + at + order[x][1] * (part_bytes(TOKENS) >> 4), idesc,
+                        x > 0 || k > 0);
+            }
+          umma_commit(&empty_bar[s]);
+          umma_commit(&sum_full[b]);
+        }
+        __syncwarp();
+      }
+    }
+  } else {
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kAddRegisters));
+    // ---- add up: TMEM lanes 32 * quarter .. + 31 are rows of W, columns are tokens ----
+    const int quarter = warp & 3;  // a warp reads the lanes of its place among four
+    const int n = n0 + quarter * 32 + lane;
+    float sum[TOKENS];
+#pragma unroll
+    for (int i = 0; i < TOKENS; ++i) sum[i] = 0.f;
+    bool have = true;
+    for (int step = 0; step < steps; ++step) {
+      const int b = step & 1;
+      if (!mbar_wait(&sum_full[b], (step / 2) & 1)) {
+        if (lane == 0) atomicOr(p.err, ERRBIT_TIMEOUT);
+        have = false;
+        break;
+      }
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+#pragma unroll
+      for (int c = 0; c < TOKENS; c += 16) {
+        float part[16];
+        tmem_load_16(tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + b * TOKENS + c, part);
+#pragma unroll
+        for (int i = 0; i < 16; ++i) sum[c + i] += part[i];
+      }
+      asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&sum_empty[b]);
+    }
+    if (have && n < p.N) {
+      const float more = p.bias != nullptr ? p.bias[n] : 0.f;
+#pragma unroll
+      for (int i = 0; i < TOKENS; ++i)
+        if (m0 + i < p.M) p.C[static_cast<int64_t>(m0 + i) * p.ldc + n] = sum[i] + more;
+    }
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  if (warp == kFetchWarps) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(kColumns) : "memory");
+}
+
+template <int TOKENS>
+int launch_tokens(const SplitProduct& p, cudaStream_t stream) {
+  static OncePerDevice raised;
+  if (!raised([] { return cudaFuncSetAttribute(gemm_f32_split_kernel<TOKENS>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(split_smem(TOKENS))) == cudaSuccess; }))
+    return b200_fail("gemm_f32_split: cannot size shared memory");
+  const dim3 grid((p.N + kRows - 1) / kRows, (p.M + TOKENS - 1) / TOKENS);
+  B200_REQUIRE(grid.y <= 65535, "gemm_f32_split: too many rows (%d)", p.M);
+  launch_kernel(gemm_f32_split_kernel<TOKENS>, grid, dim3(kThreads), split_smem(TOKENS), stream, p);
+  return b200_check_launch("gemm_f32_split");
+}
+
+}  // namespace
+
+// Whether this kernel takes a product, by its matrix alone, so that all calls with one matrix sum alike. Measured on a B200 (N x K, rows; us;
+// FMA kernel and this one; error against 64 bits): 2,048 x 1,536: 1 row 41 and 22, 100 rows 68 and 24, 500 rows 108 and 34, 2,048 rows 313 and 85 (7.0e-7 and
+// 1.2e-7); 17,920 x 1,536: 16 rows 60 and 33, 500 rows 701 and 179, 2,048 rows 2,634 and 716; 1,536 x 8,960: 1 row 220 and 110, 500 rows 601
+// and 178 (1.7e-6 and 2.3e-7). Level, at what a launch takes, for 128 x 256 up to 500 rows (2,048 rows 15 and 11); 4,096 x 64 at
+// 2,048 rows 34 and 35.
+B200_API int b200_gemm_f32_split_takes(int N, int K) { return N >= 128 && K >= 256 && K % 4 == 0 ? 1 : 0; }
+
+// `tokens`: 16, 32, 64 or 128 rows of A a block; 0: by the sizes.
+B200_API int b200_gemm_f32_split(const float* A, const float* W, const float* bias, float* C, int M, int N, int K, int lda, int ldw, int ldc, int tokens, int* err,
+                                 cudaStream_t stream) {
+  if (M == 0 || N == 0) return 0;
+  B200_REQUIRE(M > 0 && N > 0 && K > 0 && K % 4 == 0 && lda % 4 == 0 && ldw % 4 == 0, "gemm_f32_split: bad sizes %d x %d x %d", M, N, K);
+  B200_REQUIRE(lda >= K && ldw >= K && ldc >= N, "gemm_f32_split: leading dimensions too small");
+  B200_REQUIRE(reinterpret_cast<uintptr_t>(A) % 16 == 0 && reinterpret_cast<uintptr_t>(W) % 16 == 0, "gemm_f32_split: operands must be 16-byte aligned");
+  const SplitProduct p = {A, W, bias, C, M, N, K, lda, ldw, ldc, err};
+  if (tokens == 0) {
+    // The tile that is done first: as many waves of blocks as the SMs need, a wave as long as one tile takes (2,048 x 1,536).
+    constexpr int tiles[4] = {16, 32, 64, 128}, times[4] = {23, 26, 33, 41};
+    int64_t best = 0;
+    for (int i = 0; i < 4; ++i) {
+      const int64_t blocks = static_cast<int64_t>((N + kRows - 1) / kRows) * ((M + tiles[i] - 1) / tiles[i]), sms = b200_sm_count_host();
+      const int64_t time = (blocks + sms - 1) / sms * times[i];
+      if (i == 0 || time < best) best = time, tokens = tiles[i];
+    }
+  }
+  if (tokens == 16) return launch_tokens<16>(p, stream);
+  if (tokens == 32) return launch_tokens<32>(p, stream);
+  if (tokens == 64) return launch_tokens<64>(p, stream);
+  B200_REQUIRE(tokens == 128, "gemm_f32_split: tiles of 16, 32, 64 or 128 rows");
+  return launch_tokens<128>(p, stream);
+}

@@ -59,6 +59,7 @@ _SIGNATURES: dict[str, list] = {
     + [c_float, c_int, c_float, c_void_p, c_int, c_int, c_void_p, c_void_p, c_int, c_void_p, c_void_p],
     "b200_portion_attention_f32": [c_void_p] * 4 + [c_int] * 2 + [c_void_p] * 3 + [c_int] * 3 + [c_void_p] * 2 + [c_int] * 5 + [c_float, c_void_p, c_void_p],
     "b200_gemm_f32": [c_void_p] * 4 + [c_int] * 6 + [c_void_p],
+    "b200_gemm_f32_split": [c_void_p] * 4 + [c_int] * 7 + [c_void_p] * 2,
     "b200_paged_flash_attention": [c_void_p] * 8 + [c_int] * 12 + [c_float, c_int, c_int, c_int, c_float, c_void_p, c_int, c_int, c_void_p,
                                    c_void_p, c_void_p, c_void_p, c_void_p],
     "b200_paged_decode_attention_tma": [c_void_p] * 8 + [c_int] * 9 + [c_float, c_int, c_int] + [c_void_p] * 5,
@@ -154,6 +155,8 @@ class KernelLibrary:
         self.lib.b200_decode_attention_tma_supported.restype = c_int
         self.lib.b200_flash_prefill_tcgen05_supported.argtypes = [c_int] * 5
         self.lib.b200_flash_prefill_tcgen05_supported.restype = c_int
+        self.lib.b200_gemm_f32_split_takes.argtypes = [c_int] * 2
+        self.lib.b200_gemm_f32_split_takes.restype = c_int
         self.lib.b200_skinny_gemm_supported.argtypes = [c_int] * 4
         self.lib.b200_skinny_gemm_supported.restype = c_int
         self.lib.b200_skinny_gemm_scratch.argtypes = [c_int, c_int, c_int, ctypes.POINTER(c_int64), ctypes.POINTER(c_int)]

@@ -3,7 +3,8 @@
 Each function checks shapes and strides, then launches on the current CUDA stream. Matrix
 products in bfloat16 go to the vendor library through ``torch.mm``, as the reference sends
 its linear layers to cuBLASLt (cuda/execution_context.cu:95-110); in float32 they use this
-engine's own FMA kernel so that nothing runs in a reduced-precision matrix mode.
+engine's own kernels so that nothing runs in a reduced-precision matrix mode: FMAs, or exact parts of
+32-bit numbers on the tensor cores (csrc/kernels/gemm_f32_split.cu).
 """
 
 from __future__ import annotations
@@ -115,10 +116,11 @@ def linear(
     if x.dtype == torch.float32:
         _need(weight.dtype == torch.float32 and out.dtype == torch.float32, "linear: float32 path needs float32 operands")
         _need(bias is None or bias.dtype == torch.float32, "linear: bias must be float32")
-        ctx.lib.call(
-            "b200_gemm_f32", ptr(x), ptr(weight), ptr(bias), ptr(out), c_int(m), c_int(n), c_int(k),
-            c_int(k), c_int(k), c_int(n), ctx.stream,
-        )
+        sizes = (c_int(m), c_int(n), c_int(k), c_int(k), c_int(k), c_int(n))
+        if ctx.lib.lib.b200_gemm_f32_split_takes(n, k) and x.data_ptr() % 16 == 0 and weight.data_ptr() % 16 == 0:
+            ctx.lib.call("b200_gemm_f32_split", ptr(x), ptr(weight), ptr(bias), ptr(out), *sizes, c_int(0), ptr(ctx.err), ctx.stream)
+        else:
+            ctx.lib.call("b200_gemm_f32", ptr(x), ptr(weight), ptr(bias), ptr(out), *sizes, ctx.stream)
         return out
     _need(x.dtype == torch.bfloat16 and weight.dtype == torch.bfloat16, "linear: bfloat16 path needs bfloat16 operands")
     if bias is None:

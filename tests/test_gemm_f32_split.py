@@ -1,0 +1,68 @@
+"""The true 32-bit product on the tensor cores: against 64 bits at the ends of its tiles and stages, nearer than chains of FMAs, the same bits for
+a row whatever tile computes it, numbers of very different sizes, operands that are not finite."""
+
+from __future__ import annotations
+
+from ctypes import c_int
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def product(a, w, bias=None, tokens=0):
+    from llm_inference_b200.cli.microbench import make_ctx
+    from llm_inference_b200.csrc.library import ptr
+
+    ctx = make_ctx(positions=[0] * a.shape[0])
+    (m, k), n = a.shape, w.shape[0]
+    out = torch.full((m, n), float("nan"), device="cuda")
+    ctx.lib.call("b200_gemm_f32_split", ptr(a), ptr(w), ptr(bias), ptr(out), *(c_int(v) for v in (m, n, k, k, k, n, tokens)), ptr(ctx.err), ctx.stream)
+    assert int(ctx.err.item()) == 0
+    return out
+
+
+# Rounding alone: a part is exact, what is left out of a product below 2^-26 of it, a stage of 64 numbers ends in a handful of roundings (2^-23
+# each, towards zero inside the tensor core), and K / 64 stages add up with ordinary rounding: 2^-22 of the whole at these K, with room.
+CLOSE = 5e-7
+
+
+@pytest.mark.parametrize("m,n,k", [(1, 128, 256), (17, 129, 260), (65, 300, 516), (130, 1000, 1028), (500, 256, 2052)])
+@pytest.mark.parametrize("tokens", [16, 32, 64, 128])
+def test_against_64_bits(m, n, k, tokens):
+    torch.manual_seed(m + n)
+    a, w, bias = torch.randn(m, k, device="cuda"), torch.randn(n, k, device="cuda"), torch.randn(n, device="cuda")
+    want = a.double() @ w.double().T + bias.double()
+    got = product(a, w, bias, tokens)
+    assert ((got.double() - want).norm() / want.norm()).item() < CLOSE
+    assert torch.equal(got, product(a, w, bias))
+
+
+@pytest.mark.parametrize("n,k", [(2080, 260), (151, 1024)])
+def test_rows_and_the_call_they_are_in(n, k):
+    from llm_inference_b200.cli.microbench import make_ctx
+    from llm_inference_b200.parts import ops
+
+    torch.manual_seed(n)
+    a, w = torch.randn(700, k, device="cuda"), torch.randn(n, k, device="cuda")
+    linear = lambda x: ops.linear(make_ctx(positions=[0] * x.shape[0]), x, w, torch.empty(x.shape[0], n, device="cuda"))
+    whole = linear(a)
+    for rows in (1, 16, 17, 33, 64, 200):
+        assert torch.equal(linear(a[:rows].contiguous()), whole[:rows]), rows
+
+
+def test_sizes_far_apart_and_what_is_not_finite():
+    torch.manual_seed(0)
+    a = torch.randn(40, 512, device="cuda") * 10.0 ** torch.randint(-18, 18, (40, 1), device="cuda")
+    w = torch.randn(200, 512, device="cuda") * 10.0 ** torch.randint(-18, 18, (200, 1), device="cuda")
+    want = a.double() @ w.double().T
+    got = product(a, w)
+    rms = want.norm() / want.numel() ** 0.5
+    scale = (a.double().norm(dim=1)[:, None] * w.double().norm(dim=1)[None])  # each output against the size of what it sums
+    assert torch.isfinite(rms) and ((got.double() - want).abs() / scale).max().item() < CLOSE
+    a[3, 7], w[5, 100] = float("inf"), float("nan")
+    spoilt = product(a, w)
+    rows, cols = torch.arange(40) != 3, torch.arange(200) != 5
+    assert not torch.isfinite(spoilt[3]).any() and not torch.isfinite(spoilt[:, 5]).any()
+    assert torch.equal(spoilt[rows][:, cols], got[rows][:, cols])
