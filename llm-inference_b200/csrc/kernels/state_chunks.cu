@@ -19,15 +19,16 @@
 //   chunk_walk       a head's chunks one after another, a tile of 16 columns of S per block: U = W + Y S, S <- e S + (G_last K)^T U;
 //   chunk_scan       the same without U: S <- e S + the chunk's own sum, element by element;
 //   chunk_out        all chunks side by side again: O = (e Q) S + A U, from the states left at each chunk's start.
-// Only what the next chunk waits for is in the walk. All numbers stay 32-bit: sums are FMAs where pairs of tokens are made and triangles
-// solved, and products on the tensor cores of numbers taken apart into three bfloat16 ones where a chunk meets the state (`mma_split`).
-// Against 64 bits, outputs and states are as far off as with FMAs throughout (2,048 tokens, 2-norm: a decay per channel 1.76e-7 and 1.53e-7,
-// before 1.92e-7 and 1.61e-7; generalized rule 1.77e-7 and 1.71e-7, before 1.96e-7 and 1.68e-7). Decays enter as products (or sums of their
-// logarithms) from token j on, never as quotients of products from the chunk's start, so strong decays in front of a pair cost it no digits.
+// Only what the next chunk waits for is in the walk. All numbers stay 32-bit: products are FMAs where a token meets its group of eight, and
+// elsewhere tensor-core products of numbers taken apart into three bfloat16 ones (`mma_split`). Against 64 bits, outputs and states are nearer than
+// with FMAs throughout (2,048 tokens, 2-norm: a decay per channel 1.74e-7 and 1.41e-7, before 1.92e-7 and 1.61e-7; generalized rule 1.62e-7
+// and 1.43e-7, before 1.96e-7 and 1.68e-7; without a removal 2.01e-7 and 1.91e-7, before 2.22e-7 and 2.05e-7). Decays enter as products (or
+// sums of their logarithms) from token j on, never as quotients of products from the chunk's start, so strong decays in front of a pair
+// cost it no digits.
 //
-// Measured on a B200 (one request of 2,048 tokens, all three kernels; walk and outputs with FMAs, on the tensor cores): heads of 128 x 128, a
-// decay per channel, 12 of them 230 -> 172 us (prepare 60, walk 135 -> 80, out 35 -> 30), 28 of them 430 -> 319; 24 heads of 64 x 64 under the
-// generalized rule 229 -> 181 us (prepare 97, walk 91 -> 55, out 35 -> 27).
+// Measured on a B200 (one request of 2,048 tokens, all three kernels; FMAs throughout, now): heads of 128 x 128, a decay per channel, 12 of them
+// 230 -> 152 us (prepare 60 -> 43, walk 135 -> 80, out 35 -> 30), 28 of them 430 -> 277; one decay per head 228 -> 152; 24 heads of 64 x 64 under the
+// generalized rule 229 -> 162 us (prepare 97 -> 77, walk 91 -> 55, out 35 -> 27), without a removal 87 -> 72.
 #include <type_traits>
 
 #include "common.cuh"
@@ -74,30 +75,7 @@ __device__ __forceinline__ void stage_rows(float* dst, int dst_ld, const float* 
   }
 }
 
-// Two 32-bit numbers in one register pair, multiplied and added as such (two FMAs an instruction).
-using pair_t = unsigned long long;
-__device__ __forceinline__ pair_t fma_pair(pair_t a, pair_t b, pair_t c) {
-  pair_t d;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
-  return d;
-}
-__device__ __forceinline__ pair_t mul_pair(pair_t a, pair_t b) {
-  pair_t d;
-  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
-  return d;
-}
-__device__ __forceinline__ float sum_pair(pair_t a) {
-  float x, y;
-  asm("mov.b64 {%0, %1}, %2;" : "=f"(x), "=f"(y) : "l"(a));
-  return x + y;
-}
-struct quad_t {  // four neighbouring numbers
-  pair_t lo, hi;
-};
-__device__ __forceinline__ quad_t load_quad(const float* p) {
-  const ulonglong2 v = *reinterpret_cast<const ulonglong2*>(p);
-  return {v.x, v.y};
-}
+__device__ __forceinline__ float from_pair(float give, float keep, int with) { return keep + __shfl_xor_sync(0xffffffffu, give, with); }
 
 // What the preparing kernels hand on, and the walk's result, by (chunk's place, head): rows of `padded_rows(dk)` and `padded_columns(dv)`
 // numbers, whole chunks of C tokens (those past a request's end are zeros in y, kd and x). Each array runs along what its reader multiplies
@@ -171,6 +149,7 @@ struct SplitA {  // a lane's share of A
 };
 struct SplitB {  // of B
   Split lo, hi;
+  __device__ __forceinline__ SplitB() {}
   __device__ __forceinline__ explicit SplitB(float4 v) : lo(split_pair(v.x, v.y)), hi(split_pair(v.z, v.w)) {}
 };
 __device__ __forceinline__ void mma_split(float (&d)[4], const SplitA& a, const SplitB& b) {
@@ -179,162 +158,285 @@ __device__ __forceinline__ void mma_split(float (&d)[4], const SplitA& a, const 
   for (int i = 0; i < 6; ++i) mma_bf16(d, a.part[order[i][0]], b.lo.part[order[i][1]], b.hi.part[order[i][1]]);
 }
 
-// Solves (I + l) x = rhs in place, row after row: x_i = rhs_i - sum_{j < i} l[i][j] x_j.
-__device__ __forceinline__ void substitute(const float* l, float (&x)[C]) {
+// --- what does not depend on the state -------------------------------------------------------------------------------------------
+//
+// One block per (chunk, head, request). Pairs of tokens: the chunk's rows form four groups of eight. Between groups every decay product splits
+// at the group's border, G_ij = (product up to i inside i's group) (whole groups between) (product from j + 1 to the end of j's group),
+// three factors without a quotient, so those pairs are plain products of scaled rows: tiles of eight rows of two left operands by eight
+// of the right one on the tensor cores. Inside a group, where G_ij is a run of products for each j, a warp has a group and a left operand, a lane two
+// channels at a time of all its tokens in registers; the lanes' sums meet by shuffles. With one decay per head pairs are products of the raw
+// rows and G_ij stands beside them, so all pairs are tiles.
+// Columns of [e K | V]: (I + L) X = R in halves of sixteen tokens, X1 = T11 R1, X2 = T22 (R2 - L21 X1), with the two halves' inverses made
+// by a warp, a lane per column; transposed (X^T = R^T T^T, sixteen columns a warp at a time), every result is the next product's operand in
+// the lanes that hold it.
+// What bounds it: instructions (24,000 a warp's worth for a chunk of a head of 128 x 128) and the barriers between its seven phases, three blocks
+// an SM. With operands of pairs out of shared memory for every FMA, a thread per column of the triangular system and sums of the warps
+// through shared memory, two blocks an SM waited for shared memory most of the time: 2,048 tokens of 12 heads of 128 x 128, a decay per channel 60 ->
+// 43 us, one per head 56 -> 39; 24 heads of 64 x 64, the generalized rule 97 -> 77, the rule without a removal 54 -> 39. Two blocks an SM
+// with the same code: 50, 47, 87 and 47.
+constexpr int kGroup = 8, kGroups = C / kGroup;
+constexpr int kBetween = 6;             // pairs of different groups
+constexpr int kTiles = kBetween + kGroups;  // and of a group with itself
+constexpr int kLdT = 20;                // numbers from row to row of an inverse
+
+// left_i . G_ij right_j for i, j of one group (j < i; DIAGONAL: j <= i) into `to` [C][C + 1], by one warp. BEFORE: the left row meets the decays
+// of tokens j + 1 .. i - 1 only.
+template <int ROWS, bool BEFORE, bool DIAGONAL>
+__device__ __forceinline__ void pairs_in_group(const float* left, const float* right, const float* decays, int group, float* to) {
+  constexpr int ld = ROWS + 4, kPairs = DIAGONAL ? 36 : 28;
+  const int lane = threadIdx.x & 31;
+  float acc[36] = {};
+#pragma unroll 1
+  for (int x = 0; x < ROWS / 64; ++x) {
+    const int at = group * kGroup * ld + x * 64 + lane * 2;
+    float2 l[kGroup], g[kGroup], r[kGroup];
 #pragma unroll
-  for (int i = 1; i < C; ++i) {
-    float sum0 = x[i], sum1 = 0.f;
+    for (int i = 0; i < kGroup; ++i) {
+      l[i] = *reinterpret_cast<const float2*>(left + at + i * ld);
+      g[i] = *reinterpret_cast<const float2*>(decays + at + i * ld);
+      r[i] = *reinterpret_cast<const float2*>(right + at + i * ld);
+    }
+#pragma unroll
+    for (int j = 0; j < kGroup; ++j) {
+      float2 p = r[j];
+#pragma unroll
+      for (int i = DIAGONAL ? j : j + 1; i < kGroup; ++i) {
+        const int pair = DIAGONAL ? i * (i + 1) / 2 + j : i * (i - 1) / 2 + j;
+        if (!BEFORE && i > j) p.x *= g[i].x, p.y *= g[i].y;
+        acc[pair] = fmaf(l[i].x, p.x, fmaf(l[i].y, p.y, acc[pair]));
+        if (BEFORE) p.x *= g[i].x, p.y *= g[i].y;
+      }
+    }
+  }
+  // Every lane ends with one of the first 32 sums, and with one of the last four.
+#pragma unroll
+  for (int w = 16; w > 0; w /= 2)
+#pragma unroll
+    for (int k = 0; k < w; ++k) {
+      const bool high = lane & w;
+      acc[k] = from_pair(high ? acc[k] : acc[k + w], high ? acc[k + w] : acc[k], w);
+    }
+  if (DIAGONAL) {
+#pragma unroll
+    for (int w = 2; w > 0; w /= 2)
+#pragma unroll
+      for (int k = 32; k < 32 + w; ++k) {
+        const bool high = lane & w;
+        acc[k] = from_pair(high ? acc[k] : acc[k + w], high ? acc[k + w] : acc[k], w);
+      }
+#pragma unroll
+    for (int w = 4; w < 32; w *= 2) acc[32] = from_pair(acc[32], acc[32], w);
+  }
+  auto store = [&](int pair, float sum) {
+    int i = 0;
+#pragma unroll
+    for (int row = 1; row < kGroup; ++row) i += pair >= row * (row + 1) / 2 ? 1 : 0;
+    const int j = pair - i * (i + 1) / 2;
+    to[(group * kGroup + i + (DIAGONAL ? 0 : 1)) * (C + 1) + group * kGroup + j] = sum;
+  };
+  if (lane < kPairs) store(lane, acc[0]);
+  if (DIAGONAL && lane < 4) store(32 + lane, acc[32]);
+}
+
+// Tile `tile` of the pairs: rows of group gi of both left operands by rows of group gj <= gi of the right one into `to0` and `to1` [C][C + 1], by one
+// warp. DECAYS: gj < gi, rows carry their decays inside their own groups, `whole` holds the groups' decays multiplied.
+template <int ROWS, int LEFTS, bool DECAYS>
+__device__ __forceinline__ void pair_tile(const float* left0, const float* left1, const float* right, const float* whole, int tile, float* to0, float* to1) {
+  constexpr int ld = ROWS + 4, kTogether = 4;
+  const int lane = threadIdx.x & 31, g = lane >> 2, q = lane & 3;
+  int gi = 0;  // tiles (1, 0), (2, 0), (2, 1), .., or with (i, i) too
+#pragma unroll
+  for (int row = 1; row < kGroups; ++row) gi += tile >= row * (row + 1) / 2 ? 1 : 0;
+  const int gj = tile - gi * (gi + 1) / 2;
+  if (DECAYS) ++gi;
+  const int at_left = (gi * kGroup + g) * ld + 4 * q, at_right = (gj * kGroup + g) * ld + 4 * q;
+  float acc[4] = {};
+#pragma unroll 1
+  for (int step = 0; step < ROWS / 16; step += kTogether) {
+    float part[kTogether][4] = {};
+#pragma unroll
+    for (int x = 0; x < kTogether; ++x) {
+      const int c = (step + x) * 16;
+      SplitA a = {};
+      const float4 l0 = *reinterpret_cast<const float4*>(left0 + at_left + c);
+      a.set(0, split_pair(l0.x, l0.y)), a.set(2, split_pair(l0.z, l0.w));
+      if (LEFTS == 2) {
+        const float4 l1 = *reinterpret_cast<const float4*>(left1 + at_left + c);
+        a.set(1, split_pair(l1.x, l1.y)), a.set(3, split_pair(l1.z, l1.w));
+      }
+      float4 r = *reinterpret_cast<const float4*>(right + at_right + c);
+      if (DECAYS) {
+        for (int between = gj + 1; between < gi; ++between) {
+          const float4 w = *reinterpret_cast<const float4*>(whole + between * ROWS + c + 4 * q);
+          r.x *= w.x, r.y *= w.y, r.z *= w.z, r.w *= w.w;
+        }
+      }
+      mma_split(part[x], a, SplitB(r));
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i) acc[i] += (part[0][i] + part[1][i]) + (part[2][i] + part[3][i]);
+  }
+  const int at = (gi * kGroup + g) * (C + 1) + gj * kGroup + 2 * q;
+  to0[at] = acc[0], to0[at + 1] = acc[1];
+  if (LEFTS == 2) to1[at] = acc[2], to1[at + 1] = acc[3];
+}
+
+// (I + l)^-1 of both halves of sixteen tokens on the diagonal of l [C][C], to `inverse` [C][kLdT], by one warp: a lane per column.
+__device__ __forceinline__ void invert_halves(const float* l, float* inverse) {
+  const int lane = threadIdx.x & 31, half = lane & 16, column = lane & 15;
+  float x[16];
+#pragma unroll
+  for (int i = 0; i < 16; ++i) {
+    float sum0 = i == column ? 1.f : 0.f, sum1 = 0.f;
 #pragma unroll
     for (int j = 0; j < i; j += 4) {
-      const float4 row = *reinterpret_cast<const float4*>(l + i * C + j);
+      const float4 row = *reinterpret_cast<const float4*>(l + (half + i) * C + half + j);
       sum0 = fmaf(-row.x, x[j], sum0);
       if (j + 1 < i) sum1 = fmaf(-row.y, x[j + 1], sum1);
       if (j + 2 < i) sum0 = fmaf(-row.z, x[j + 2], sum0);
       if (j + 3 < i) sum1 = fmaf(-row.w, x[j + 3], sum1);
     }
     x[i] = sum0 + sum1;
+    inverse[(half + i) * kLdT + column] = i >= column ? x[i] : 0.f;
   }
 }
 
-// What a thread holds of a column for the chunk's tokens, as `y` lies or side by side; zeros past the request's end.
-__device__ __forceinline__ void store_y(float* to, int row, const float (&x)[C], int n) {
-  to += y_place(0, row);
-#pragma unroll
-  for (int i = 0; i < C; ++i) to[y_place(i, 0)] = i < n ? x[i] : 0.f;
+// Sixteen columns of numbers by token, of which a lane has columns g and g + 8, tokens 4 q .. + 3 of both halves: [half][column].
+struct Columns {
+  float4 v[2][2];
+};
+__device__ __forceinline__ SplitA split_columns(const float4 (&v)[2]) {
+  SplitA a;
+  a.set(0, split_pair(v[0].x, v[0].y)), a.set(1, split_pair(v[1].x, v[1].y));
+  a.set(2, split_pair(v[0].z, v[0].w)), a.set(3, split_pair(v[1].z, v[1].w));
+  return a;
 }
-__device__ __forceinline__ void store_column(float* to, const float (&x)[C], int n) {
+// The same of a triangle that all columns meet: its operands in parts, [tile][part][lane], made once.
+constexpr int kTriangle = 2 * 3 * 32;  // uint2 of sixteen rows by sixteen tokens
+__device__ __forceinline__ void pack_triangle(uint2* to, const float* m, int ld) {
+  const int lane = threadIdx.x & 31, g = lane >> 2, q = lane & 3;
 #pragma unroll
-  for (int i = 0; i < C; i += 4)
-    *reinterpret_cast<float4*>(to + i) = make_float4(i < n ? x[i] : 0.f, i + 1 < n ? x[i + 1] : 0.f, i + 2 < n ? x[i + 2] : 0.f, i + 3 < n ? x[i + 3] : 0.f);
+  for (int t = 0; t < 2; ++t) {
+    const SplitB b(*reinterpret_cast<const float4*>(m + in_sixteen(t, g) * ld + 4 * q));
+#pragma unroll
+    for (int p = 0; p < 3; ++p) to[(t * 3 + p) * 32 + lane] = make_uint2(b.lo.part[p], b.hi.part[p]);
+  }
 }
+__device__ __forceinline__ void times_triangle(float4 (&to)[2], const SplitA& a, const uint2* m) {
+  const int lane = threadIdx.x & 31;
+  float part[2][4] = {};
+#pragma unroll
+  for (int t = 0; t < 2; ++t) {
+    SplitB b;
+#pragma unroll
+    for (int p = 0; p < 3; ++p) {
+      const uint2 word = m[(t * 3 + p) * 32 + lane];
+      b.lo.part[p] = word.x, b.hi.part[p] = word.y;
+    }
+    mma_split(part[t], a, b);
+  }
+  to[0] = make_float4(part[0][0], part[0][1], part[1][0], part[1][1]);
+  to[1] = make_float4(part[0][2], part[0][3], part[1][2], part[1][3]);
+}
+// a (sixteen columns by sixteen tokens) times the transposed sixteen rows of m, `ld` numbers apart.
+__device__ __forceinline__ void times_rows(float4 (&to)[2], const SplitA& a, const float* m, int ld) {
+  const int lane = threadIdx.x & 31, g = lane >> 2, q = lane & 3;
+  float part[2][4] = {};
+#pragma unroll
+  for (int t = 0; t < 2; ++t) mma_split(part[t], a, SplitB(*reinterpret_cast<const float4*>(m + in_sixteen(t, g) * ld + 4 * q)));
+  to[0] = make_float4(part[0][0], part[0][1], part[1][0], part[1][1]);
+  to[1] = make_float4(part[0][2], part[0][3], part[1][2], part[1][3]);
+}
+__device__ __forceinline__ float4 minus(float4 a, float4 b) { return make_float4(a.x - b.x, a.y - b.y, a.z - b.z, a.w - b.w); }
+__device__ __forceinline__ float4 plus(float4 a, float4 b) { return make_float4(a.x + b.x, a.y + b.y, a.z + b.z, a.w + b.w); }
 
-// --- what does not depend on the state -------------------------------------------------------------------------------------------
-//
-// One block per (chunk, head, request). Pairs of tokens: the chunk's rows form four groups of eight. Inside a group a lane has a token
-// j and carries p = G_ij k_j from row to row. Between groups every decay product splits at the group's border, G_ij = (product up
-// to i inside i's group) (whole groups between) (product from j + 1 to the end of j's group), three factors without a quotient, so
-// those pairs are plain products of scaled rows. A warp has an eighth of the channels; the warps' sums meet in shared memory.
-// PER_HEAD: one decay per head, given as its logarithm; pairs are products of the raw rows and G_ij = exp of the sum of logarithms.
-// Columns: a thread per column of [e K | V] solves the triangular system by substitution.
-constexpr int kGroup = 8, kGroups = C / kGroup;
-constexpr int kBetween = 6;  // pairs of groups
-__host__ __device__ constexpr int inside_sums(int lefts) { return kGroup * lefts * 32; }  // numbers that a warp hands on
-__host__ __device__ constexpr int between_sums(int lefts) { return kBetween * 2 * lefts * 32; }
-
-// left_i . G_ij right_j for i, j in one group, over the warp's eighth of the channels: lane j, rows i = 8 (j / 8) + r. BEFORE: the first left
-// row meets the decays of tokens j + 1 .. i - 1 only. Without DECAYS: left_i . right_j.
-template <int ROWS, int LEFTS, bool DECAYS, bool BEFORE>
-__device__ __forceinline__ void pairs_inside(const float* left0, const float* left1, const float* right, const float* decays, float* sums) {
-  constexpr int ld = ROWS + 4, slice = ROWS / kWarps;
-  const int c0 = threadIdx.x / 32 * slice;
-  const int lane = threadIdx.x & 31, own = lane & 7, group = (lane & ~7) * ld;
-  pair_t acc[kGroup][LEFTS];
+__device__ __forceinline__ bool all_finite(float4 v) { return fmaf(v.x, 0.f, fmaf(v.y, 0.f, fmaf(v.z, 0.f, v.w * 0.f))) == 0.f; }
+// What is not finite must not reach the tokens in front of it by way of a zero in a triangle: it goes into the products as a zero, and the
+// tokens from it on are NaN behind them. Lowers `first` to the first such token of the lane's two columns in half h.
+__device__ __forceinline__ void take_out(float4 (&r)[2], int h, int2& first) {
+  if (!__any_sync(0xffffffffu, !all_finite(r[0]) || !all_finite(r[1]))) return;
+  const int q = threadIdx.x & 3;
+  int found[2] = {C, C};
 #pragma unroll
-  for (int r = 0; r < kGroup; ++r)
+  for (int c = 0; c < 2; ++c) {
+    float* v[4] = {&r[c].x, &r[c].y, &r[c].z, &r[c].w};
 #pragma unroll
-    for (int x = 0; x < LEFTS; ++x) acc[r][x] = 0;
-#pragma unroll 2
-  for (int c = c0; c < c0 + slice; c += 4) {
-    const quad_t mine = load_quad(right + lane * ld + c);
-    quad_t p = mine;
-    if (DECAYS) p = {0, 0};
+    for (int i = 3; i >= 0; --i)
+      if (!isfinite(*v[i])) *v[i] = 0.f, found[c] = h * 16 + 4 * q + i;
+    found[c] = min(found[c], __shfl_xor_sync(0xffffffffu, found[c], 1));
+    found[c] = min(found[c], __shfl_xor_sync(0xffffffffu, found[c], 2));
+  }
+  first.x = min(first.x, found[0]), first.y = min(first.y, found[1]);
+}
+// The lane's numbers of tokens from `from` on become NaN, those from n on zeros.
+__device__ __forceinline__ void put_back(Columns& x, int2 from, int n) {
+  if (n == C && !__any_sync(0xffffffffu, min(from.x, from.y) < C)) return;
+  const int q = threadIdx.x & 3;
 #pragma unroll
-    for (int r = 0; r < kGroup; ++r) {
-      const int at = group + r * ld + c;
-      const quad_t a = load_quad(left0 + at);
-      if (BEFORE) acc[r][0] = fma_pair(a.hi, p.hi, fma_pair(a.lo, p.lo, acc[r][0]));
-      if (DECAYS) {
-        const quad_t g = load_quad(decays + at);
-        p.lo = r == own ? mine.lo : mul_pair(p.lo, g.lo);
-        p.hi = r == own ? mine.hi : mul_pair(p.hi, g.hi);
-      }
-      if (!BEFORE) acc[r][0] = fma_pair(a.hi, p.hi, fma_pair(a.lo, p.lo, acc[r][0]));
-      if (LEFTS == 2) {
-        const quad_t b = load_quad(left1 + at);
-        acc[r][LEFTS - 1] = fma_pair(b.hi, p.hi, fma_pair(b.lo, p.lo, acc[r][LEFTS - 1]));
+  for (int h = 0; h < 2; ++h)
+#pragma unroll
+    for (int c = 0; c < 2; ++c) {
+      float* v[4] = {&x.v[h][c].x, &x.v[h][c].y, &x.v[h][c].z, &x.v[h][c].w};
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const int token = h * 16 + 4 * q + i;
+        if (token >= (c == 0 ? from.x : from.y)) *v[i] = NAN;
+        if (token >= n) *v[i] = 0.f;
       }
     }
-  }
-#pragma unroll
-  for (int r = 0; r < kGroup; ++r)
-#pragma unroll
-    for (int x = 0; x < LEFTS; ++x) sums[(r * LEFTS + x) * 32 + lane] = sum_pair(acc[r][x]);
 }
-
-// The same for j in a group b before i's group g, from rows that carry their decays inside their own groups: lane = token 8 b + lane % 8,
-// rows 8 g + 2 (lane / 8) and the next one; `whole` holds the groups' decays multiplied.
-template <int ROWS, int LEFTS, bool DECAYS>
-__device__ __forceinline__ void pairs_between(const float* left0, const float* left1, const float* ends, const float* whole, float* sums) {
-  constexpr int rows = ROWS, ld = ROWS + 4, slice = ROWS / kWarps;
-  const int c0 = threadIdx.x / 32 * slice;
-  const int lane = threadIdx.x & 31, at0 = (lane >> 3) * 2 * ld;
-  const float* right = ends + (lane & 7) * ld;
-  pair_t acc[kBetween][2][LEFTS];
+// (I + l) x = r in place; `triangles`: T11, L21 and T22; `spoilt`: the first token of either column that is not to be read any more; zeros
+// from token n on.
+__device__ __forceinline__ void solve_columns(Columns& r, const uint2* triangles, int2 spoilt, int n) {
+  float4 product[2];
+  take_out(r.v[0], 0, spoilt);
+  times_triangle(r.v[0], split_columns(r.v[0]), triangles);
+  times_triangle(product, split_columns(r.v[0]), triangles + kTriangle);
+  r.v[1][0] = minus(r.v[1][0], product[0]), r.v[1][1] = minus(r.v[1][1], product[1]);
+  take_out(r.v[1], 1, spoilt);
+  times_triangle(r.v[1], split_columns(r.v[1]), triangles + 2 * kTriangle);
+  put_back(r, spoilt, n);
+}
+// To `y` (rows row0 .. + 15 of the state) or to `x` (columns from `to` on).
+__device__ __forceinline__ void store_y(float* y, int row0, const Columns& r) {
+  const int lane = threadIdx.x & 31, g = lane >> 2, q = lane & 3;
+  float* to = y + y_place(4 * q, row0) + g;  // tokens 4 q + i: i / 2 is the tile, i % 2 the next lane's
 #pragma unroll
-  for (int x = 0; x < kBetween; ++x)
+  for (int h = 0; h < 2; ++h)
 #pragma unroll
-    for (int y = 0; y < LEFTS; ++y) acc[x][0][y] = acc[x][1][y] = 0;
-  for (int c = c0; c < c0 + slice; c += 4) {
-    quad_t p[kGroups - 1];
+    for (int c = 0; c < 2; ++c) {
+      const float v[4] = {r.v[h][c].x, r.v[h][c].y, r.v[h][c].z, r.v[h][c].w};
 #pragma unroll
-    for (int b = 0; b < kGroups - 1; ++b) p[b] = load_quad(right + b * kGroup * ld + c);
-    int x = 0;
-#pragma unroll
-    for (int g = 1; g < kGroups; ++g) {
-      if (DECAYS && g > 1) {  // the groups that are now whole ones between
-        const quad_t between = load_quad(whole + (g - 1) * rows + c);
-#pragma unroll
-        for (int b = 0; b < g - 1; ++b) p[b].lo = mul_pair(p[b].lo, between.lo), p[b].hi = mul_pair(p[b].hi, between.hi);
-      }
-      quad_t left[2][LEFTS];
-#pragma unroll
-      for (int r = 0; r < 2; ++r) {
-        const int at = at0 + (g * kGroup + r) * ld + c;
-        left[r][0] = load_quad(left0 + at);
-        if (LEFTS == 2) left[r][LEFTS - 1] = load_quad(left1 + at);
-      }
-#pragma unroll
-      for (int b = 0; b < g; ++b, ++x)
-#pragma unroll
-        for (int r = 0; r < 2; ++r)
-#pragma unroll
-          for (int y = 0; y < LEFTS; ++y) acc[x][r][y] = fma_pair(left[r][y].hi, p[b].hi, fma_pair(left[r][y].lo, p[b].lo, acc[x][r][y]));
+      for (int i = 0; i < 4; ++i) to[h * 256 + i / 2 * 128 + i % 2 * 16 + 8 * c] = v[i];
     }
-  }
-#pragma unroll
-  for (int x = 0; x < kBetween; ++x)
-#pragma unroll
-    for (int r = 0; r < 2; ++r)
-#pragma unroll
-      for (int y = 0; y < LEFTS; ++y) sums[((x * 2 + r) * LEFTS + y) * 32 + lane] = sum_pair(acc[x][r][y]);
 }
-
-// The warps' sums of either kind, `stride` numbers from warp to warp, added up into the [C][C + 1] matrices of the left rows.
-template <int LEFTS, bool INSIDE>
-__device__ __forceinline__ void add_up(const float* sums, int stride, float* to0, float* to1) {
-  for (int idx = threadIdx.x; idx < (INSIDE ? inside_sums(LEFTS) : between_sums(LEFTS)); idx += kThreads) {
-    float sum = 0.f;
+__device__ __forceinline__ void store_x(float* x, const Columns& r) {
+  const int lane = threadIdx.x & 31, g = lane >> 2, q = lane & 3;
 #pragma unroll
-    for (int w = 0; w < kWarps; ++w) sum += sums[w * stride + idx];
-    const int l = idx % 32, y = idx / 32 % LEFTS, o = idx / 32 / LEFTS;
-    int i, j;
-    if (INSIDE) {
-      i = (l & ~7) + o, j = l;
-    } else {
-      const int x = o / 2, g = x == 0 ? 1 : (x < 3 ? 2 : 3), b = x - (g == 1 ? 0 : (g == 2 ? 1 : 3));
-      i = g * kGroup + (l >> 3) * 2 + (o & 1), j = b * kGroup + (l & 7);
+  for (int h = 0; h < 2; ++h)
+#pragma unroll
+    for (int c = 0; c < 2; ++c) *reinterpret_cast<float4*>(x + (g + 8 * c) * C + h * 16 + 4 * q) = r.v[h][c];
+}
+// Columns c0 .. + 15 of the chunk's values: rows v + token * ld, zeros past n tokens and dv columns.
+__device__ __forceinline__ Columns load_values(const float* v, int64_t ld, int c0, int dv, int n) {
+  const int lane = threadIdx.x & 31, g = lane >> 2, q = lane & 3;
+  Columns r;
+#pragma unroll
+  for (int h = 0; h < 2; ++h)
+#pragma unroll
+    for (int c = 0; c < 2; ++c) {
+      const int token = h * 16 + 4 * q, column = c0 + g + 8 * c;
+      const float* at = v + token * ld + column;
+      r.v[h][c] = make_float4(column < dv && token < n ? at[0] : 0.f, column < dv && token + 1 < n ? at[ld] : 0.f,
+                              column < dv && token + 2 < n ? at[2 * ld] : 0.f, column < dv && token + 3 < n ? at[3 * ld] : 0.f);
     }
-    (y == 0 ? to0 : to1)[i * (C + 1) + j] = sum;
-  }
+  return r;
 }
 
-constexpr int kWarpSums = inside_sums(2) + between_sums(2);
-size_t prepare_smem(int rows) {
-  return sizeof(float) * (3 * C * (rows + 4) + kGroups * rows + kWarps * kWarpSums + 2 * C * (C + 1) + C * C + 3 * C);
-}
+size_t prepare_smem(int rows) { return sizeof(float) * (3 * C * (rows + 4) + 2 * kGroups * rows + C * C + 3 * C + 2 * C * (C + 1)); }
 
 template <int ROWS, int W, bool PER_HEAD>
-__global__ void __launch_bounds__(kThreads, 2)
+__global__ void __launch_bounds__(kThreads, ROWS <= 128 ? 3 : 1)
 chunk_prepare_kernel(const float* q, const float* k, const float* v, const float* beta, const float* decay, const int* __restrict__ seq_q_start,
                      const int* __restrict__ seq_q_len, int heads, int kv_heads, int dk, int dv, Scratch to) {
   extern __shared__ __align__(16) float chunk_smem[];
@@ -350,13 +452,16 @@ chunk_prepare_kernel(const float* q, const float* k, const float* v, const float
   float* qs = ks + C * ld;                    // [C][ld]: queries, then likewise
   float* gs = qs + C * ld;                    // [C][ld]: decays, then keys times the decays from the next token to their group's end
   float* whole = gs + C * ld;                 // [groups][rows]: each group's decays multiplied
-  float* ls = whole + kGroups * rows;         // [C][C]
-  float* sums = ls + C * C;                   // [warps][kWarpSums]
-  float* kk = sums + kWarps * kWarpSums;      // [C][C + 1]: k_i . G_ij k_j
-  float* qk = kk + C * (C + 1);               // [C][C + 1]: q_i . G_ij k_j
-  float* bs = qk + C * (C + 1);               // [C]: beta
+  float* front = whole + kGroups * rows;      // [groups][rows]: the decays in front of each group multiplied
+  float* ls = front + kGroups * rows;         // [C][C]
+  float* bs = ls + C * C;                     // [C]: beta
   float* es = bs + C;                         // [C]: PER_HEAD: e_i
   float* fs = es + C;                         // [C]: PER_HEAD: G_last,j
+  float* kk = fs + C;                         // [C][C + 1]: k_i . G_ij k_j
+  float* qk = kk + C * (C + 1);               // [C][C + 1]: q_i . G_ij k_j
+  uint2* triangles = reinterpret_cast<uint2*>(kk);  // [3][kTriangle], behind the pairs
+  float* inverse = kk + 6 * kTriangle;              // [C][kLdT]
+  static_assert(6 * kTriangle + C * kLdT <= 2 * C * (C + 1), "the triangles do not fit where the pairs were");
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   wait_for_predecessor();
   stage_rows<W>(ks, ld, k, first, n, static_cast<int64_t>(kv_heads) * dk, static_cast<int64_t>(kvh) * dk, dk, rows);
@@ -366,9 +471,11 @@ chunk_prepare_kernel(const float* q, const float* k, const float* v, const float
   commit_copies();
   wait_copies<0>();
   __syncthreads();
-  float* mine = sums + warp * kWarpSums;
-  pairs_inside<ROWS, 2, !PER_HEAD, false>(ks, qs, ks, gs, mine);
-  if (!PER_HEAD) {
+  if (PER_HEAD) {
+    for (int tile = warp; tile < kTiles; tile += kWarps) pair_tile<ROWS, 2, false>(ks, qs, ks, nullptr, tile, kk, qk);
+  } else {
+    if (warp < kGroups) pairs_in_group<ROWS, false, false>(ks, ks, gs, warp, kk);
+    else pairs_in_group<ROWS, false, true>(qs, ks, gs, warp - kGroups, qk);
     __syncthreads();
     for (int item = tid; item < kGroups * rows; item += kThreads) {  // a thread per (group, channel)
       const int c = item % rows, at = item / rows * kGroup * ld + c;
@@ -391,70 +498,99 @@ chunk_prepare_kernel(const float* q, const float* k, const float* v, const float
       }
     }
     __syncthreads();
+    if (warp < kBetween) pair_tile<ROWS, 2, true>(ks, qs, gs, whole, warp, kk, qk);
   }
-  pairs_between<ROWS, 2, !PER_HEAD>(ks, qs, PER_HEAD ? ks : gs, whole, mine + inside_sums(2));
   __syncthreads();
-  add_up<2, true>(sums, kWarpSums, kk, qk);
-  add_up<2, false>(sums + inside_sums(2), kWarpSums, kk, qk);
-  __syncthreads();
-  {
+  float* a = to.a + place * C * C + lane;
+  if (!PER_HEAD) {
+#pragma unroll
+    for (int i = warp; i < C; i += kWarps) {
+      ls[i * C + lane] = lane < i ? bs[i] * kk[i * (C + 1) + lane] : 0.f;
+      a[i * C] = lane <= i ? qk[i * (C + 1) + lane] : 0.f;
+    }
+  } else {
     float own = 0.f, d = 0.f, prefix = 0.f, e = 0.f;
-    if (PER_HEAD) own = lane < n ? decay[(first + lane) * heads + head] : 0.f;
-    float* a = to.a + place * C * C + lane;
+    own = lane < n ? decay[(first + lane) * heads + head] : 0.f;
     for (int i = 0; i < C; ++i) {
-      if (PER_HEAD) {  // D_ij of column j = lane, the sum of the logarithms from token j + 1 on, grows with i from zero at i = j
+      {  // D_ij of column j = lane, the sum of the logarithms from token j + 1 on, grows with i from zero at i = j
         const float gi = __shfl_sync(0xffffffffu, own, i);
         d = i > lane ? d + gi : 0.f;
         prefix += gi;
         if (i == lane) e = prefix;
       }
       if ((i & 7) == warp) {
-        const float between = PER_HEAD ? expf(d) : 1.f;
+        const float between = expf(d);
         ls[i * C + lane] = lane < i ? bs[i] * between * kk[i * (C + 1) + lane] : 0.f;
         a[i * C] = lane <= i ? between * qk[i * (C + 1) + lane] : 0.f;
       }
     }
-    if (PER_HEAD && warp == 0) es[lane] = expf(e), fs[lane] = expf(d);  // d is now D_last,j: tokens past n added nothing
+    if (warp == 0) es[lane] = expf(e), fs[lane] = expf(d);  // d is now D_last,j: tokens past n added nothing
   }
   __syncthreads();
-  for (int column = tid; column < rows + columns; column += kThreads) {
-    float x[C];
-    if (column < rows) {
-      float* qt = to.qt + place * C * rows + column;
-      float* kd = to.kd + place * rows * C + kd_place(0, column);
-      float before[kGroups], after[kGroups];  // whole groups in front of and behind a token's own
-      if (!PER_HEAD) {
-        before[0] = after[kGroups - 1] = 1.f;
-#pragma unroll
-        for (int g = 1; g < kGroups; ++g) before[g] = before[g - 1] * whole[(g - 1) * rows + column];
-#pragma unroll
-        for (int g = kGroups - 2; g >= 0; --g) after[g] = after[g + 1] * whole[(g + 1) * rows + column];
-      }
-#pragma unroll
-      for (int i0 = 0; i0 < C; i0 += 4) {
-        float decayed[4];
-#pragma unroll
-        for (int y = 0; y < 4; ++y) {
-          const int i = i0 + y;
-          const float key = ks[i * ld + column], e = PER_HEAD ? es[i] : before[i / kGroup];
-          qt[i * rows] = e * qs[i * ld + column];
-          decayed[y] = i < n ? (PER_HEAD ? fs[i] * key : after[i / kGroup] * gs[i * ld + column]) : 0.f;
-          x[i] = -bs[i] * e * key;
-        }
-        *reinterpret_cast<float4*>(kd + kd_place(i0, 0)) = make_float4(decayed[0], decayed[1], decayed[2], decayed[3]);
-      }
-      to.e[place * rows + column] = PER_HEAD ? es[n - 1] : before[kGroups - 1] * whole[(kGroups - 1) * rows + column];
-    } else {
-      const int c = column - rows;
-      const float* value = v + (first * heads + head) * dv + c;
-#pragma unroll
-      for (int i = 0; i < C; ++i) x[i] = i < n && c < dv ? value[static_cast<int64_t>(i) * heads * dv] : 0.f;
-#pragma unroll
-      for (int i = 0; i < C; ++i) x[i] *= bs[i];
+  if (warp == 0) {
+    invert_halves(ls, inverse);
+    __syncwarp();
+    pack_triangle(triangles, inverse, kLdT), pack_triangle(triangles + 2 * kTriangle, inverse + 16 * kLdT, kLdT);
+  } else if (warp == 1) {
+    pack_triangle(triangles + kTriangle, ls + 16 * C, C);
+  }
+  // Scaled rows: a thread per (half of the chunk, channel). The warp that inverts is the last to come.
+  for (int item = kThreads - 1 - tid; item < 2 * rows; item += kThreads) {
+    const int column = item % rows, half = item / rows;
+    float* qt = to.qt + (place * C + half * 16) * rows + column;
+    float* kd = to.kd + place * rows * C + kd_place(half * 16, column);
+    float before[2], after[2];  // whole groups in front of and behind the half's two
+    if (!PER_HEAD) {
+      before[0] = 1.f, after[1] = 1.f;
+      for (int g = 0; g < 2 * half; ++g) before[0] *= whole[g * rows + column];
+      before[1] = before[0] * whole[2 * half * rows + column];
+      for (int g = 2 * half + 2; g < kGroups; ++g) after[1] *= whole[g * rows + column];
+      after[0] = after[1] * whole[(2 * half + 1) * rows + column];
+      front[2 * half * rows + column] = before[0], front[(2 * half + 1) * rows + column] = before[1];
+      if (half == 1) to.e[place * rows + column] = before[1] * whole[3 * rows + column];
+    } else if (half == 1) {
+      to.e[place * rows + column] = es[n - 1];
     }
-    substitute(ls, x);
-    if (column < rows) store_y(to.y + place * C * rows, column, x, n);
-    else store_column(to.x + (place * columns + column - rows) * C, x, n);
+#pragma unroll
+    for (int i0 = 0; i0 < 16; i0 += 4) {
+      float decayed[4];
+#pragma unroll
+      for (int y = 0; y < 4; ++y) {
+        const int i = half * 16 + i0 + y;
+        qt[(i0 + y) * rows] = (PER_HEAD ? es[i] : before[i0 / kGroup]) * qs[i * ld + column];
+        decayed[y] = i < n ? (PER_HEAD ? fs[i] * ks[i * ld + column] : after[i0 / kGroup] * gs[i * ld + column]) : 0.f;
+      }
+      *reinterpret_cast<float4*>(kd + kd_place(i0, 0)) = make_float4(decayed[0], decayed[1], decayed[2], decayed[3]);
+    }
+  }
+  __syncthreads();
+  for (int tile = warp; tile < (rows + columns) / 16; tile += kWarps) {  // sixteen columns of [-beta e K | beta V]
+    const int g = lane >> 2, q4 = 4 * (lane & 3);
+    Columns r;
+    if (tile < rows / 16) {
+#pragma unroll
+      for (int h = 0; h < 2; ++h)
+#pragma unroll
+        for (int c = 0; c < 2; ++c) {
+          const int column = tile * 16 + g + 8 * c, token = h * 16 + q4;
+          const float4 b = *reinterpret_cast<const float4*>(bs + token), e = PER_HEAD ? *reinterpret_cast<const float4*>(es + token) : b;
+          const float before = PER_HEAD ? 1.f : front[token / kGroup * rows + column];
+          const float* key = ks + token * ld + column;
+          r.v[h][c] = make_float4(-b.x * ((PER_HEAD ? e.x : before) * key[0]), -b.y * ((PER_HEAD ? e.y : before) * key[ld]),
+                                  -b.z * ((PER_HEAD ? e.z : before) * key[2 * ld]), -b.w * ((PER_HEAD ? e.w : before) * key[3 * ld]));
+        }
+    } else {
+      r = load_values(v + (first * heads + head) * dv, static_cast<int64_t>(heads) * dv, (tile - rows / 16) * 16, dv, n);
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const float4 b = *reinterpret_cast<const float4*>(bs + h * 16 + q4);
+#pragma unroll
+        for (int c = 0; c < 2; ++c) r.v[h][c].x *= b.x, r.v[h][c].y *= b.y, r.v[h][c].z *= b.z, r.v[h][c].w *= b.w;
+      }
+    }
+    solve_columns(r, triangles, make_int2(C, C), n);
+    if (tile < rows / 16) store_y(to.y + place * rows * C, tile * 16, r);
+    else store_x(to.x + (place * columns + tile * 16 - rows) * C, r);
   }
 }
 
@@ -464,15 +600,12 @@ chunk_prepare_kernel(const float* q, const float* k, const float* v, const float
 // MEMORY: S <- keep S + put k v^T and n <- keep n + put k with two numbers per head and token, o = S^T r and n . r after the update, r
 // times `scale`: pairs are products of the raw rows, times the keeps between them.
 // One block per (chunk, head, request); the sums of the values (G_last K)^T V go where the chunk's state will be.
-constexpr int kValueTile = 64;
-constexpr int kLdV = kValueTile + 4;
 constexpr int kMaxLinearRows = 128;
 
-__host__ __device__ constexpr int linear_warp_sums(bool general) { return general ? 2 * inside_sums(2) : between_sums(1); }
 size_t linear_prepare_smem(int rows, int rule) {
   const bool general = rule == kGeneralDelta;
-  return sizeof(float) * ((general ? 5 : (rule == kMemory ? 2 : 3)) * C * (rows + 4) + 3 * C + C * kLdV + kGroups * rows + kWarps * linear_warp_sums(general) + (general ? 4 : 1) * C * (C + 1) +
-                          (general ? 2 : 0) * C * C);
+  return sizeof(float) * ((general ? 5 : (rule == kMemory ? 2 : 3)) * C * (rows + 4) + 2 * C + kGroups * rows + (general ? 4 : 1) * C * (C + 1) +
+                          (general ? 2 * C * C : 0));
 }
 
 struct LinearRule {
@@ -490,7 +623,7 @@ struct LinearRule {
 };
 
 template <int ROWS, int W, int RULE>
-__global__ void __launch_bounds__(kThreads, 2)
+__global__ void __launch_bounds__(kThreads, ROWS <= 64 ? 3 : 2)
 linear_chunk_prepare_kernel(LinearRule in, const int* __restrict__ seq_q_start, const int* __restrict__ seq_q_len, int heads, int dk, int dv, Scratch to) {
   extern __shared__ __align__(16) float chunk_smem[];
   let_successor_start();
@@ -502,32 +635,26 @@ linear_chunk_prepare_kernel(LinearRule in, const int* __restrict__ seq_q_start, 
   constexpr int rows = ROWS, ld = ROWS + 4;
   const int columns = padded_columns(dv);
   constexpr bool GENERAL = RULE == kGeneralDelta, MEMORY = RULE == kMemory;
-  constexpr int kSums = linear_warp_sums(GENERAL);
   float* ls = chunk_smem;                                // GENERAL: [C][C]: -N
   float* ms = ls + (GENERAL ? C * C : 0);                // GENERAL: [C][C]: M
   float* rs = ms + (GENERAL ? C * C : 0);                // [C][ld]: r, then times the decays of its group in front of (GENERAL: up to) its token
-  float* ks = rs + C * ld;                               // [C][ld]: k, then times the decays from the next token to its group's end
+  float* ks = rs + C * ld;                               // [C][ld]: k, then times the decays from the next token to its group's, then the chunk's end
   float* gs = ks + C * ld;                               // [C][ld]
   float* us = gs + (MEMORY ? 0 : C * ld);                // GENERAL: [C][ld]: u, then times the decays of its group in front of its token
   float* bb = us + (GENERAL ? C * ld : 0);               // GENERAL: [C][ld]: -au, then as k
-  float* vs = bb + (GENERAL ? C * ld : 0);               // [C][kLdV]: a tile of the values
-  float* whole = vs + C * kLdV;                          // [groups][rows]
-  float* sums = whole + kGroups * rows;                  // [warps][kSums]
-  float* rk = sums + kWarps * kSums;                     // [C][C + 1]: r_i . G k_j
+  float* whole = bb + (GENERAL ? C * ld : 0);            // [groups][rows]
+  float* es = whole + kGroups * rows;                    // MEMORY: [C]: the keeps up to a token, multiplied
+  float* fs = es + C;                                    // MEMORY: [C]: the keeps behind a token times its put
+  float* rk = fs + C;                                    // [C][C + 1]: r_i . G k_j
   float* uk = rk + C * (C + 1);
   float* rb = uk + C * (C + 1);
   float* ub = rb + C * (C + 1);
-  float* es = MEMORY ? uk : ub + (GENERAL ? C * (C + 1) : 0);  // MEMORY: [C]: the keeps up to a token, multiplied
-  float* fs = es + C;                                           // MEMORY: [C]: the keeps behind a token times its put
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  uint2* triangles = reinterpret_cast<uint2*>(rk);       // GENERAL: [3][kTriangle], behind the pairs
+  float* inverse = rk + 6 * kTriangle;                   // GENERAL: [C][kLdT], likewise
+  float* front = gs;                                     // GENERAL: [groups][rows]: the decays in front of each group, behind the decays themselves
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, q = lane & 3;
   const int64_t ld_in = in.ld, at_in = static_cast<int64_t>(head) * dk;
-  auto stage_values = [&](int col0) {
-    for (int r = warp; r < C; r += kWarps)
-      for (int c = lane * W; c < kValueTile; c += 32 * W) {
-        const bool valid = r < n && col0 + c < dv;
-        stage_copy<4 * W>(vs + r * kLdV + c, valid ? in.v + (first + r) * in.v_ld + static_cast<int64_t>(head) * dv + col0 + c : in.v, valid);
-      }
-  };
+  const float* values = in.v + first * in.v_ld + static_cast<int64_t>(head) * dv;
   wait_for_predecessor();
   stage_rows<W>(rs, ld, in.r, first, n, ld_in, at_in, dk, rows);
   stage_rows<W>(ks, ld, in.k, first, n, ld_in, at_in, dk, rows);
@@ -536,61 +663,12 @@ linear_chunk_prepare_kernel(LinearRule in, const int* __restrict__ seq_q_start, 
     stage_rows<W>(us, ld, in.u, first, n, ld_in, at_in, dk, rows);
     stage_rows<W>(bb, ld, in.au, first, n, ld_in, at_in, dk, rows);
   }
-  stage_values(0);
   commit_copies();
   wait_copies<0>();
   __syncthreads();
-  float* mine = sums + warp * kSums;
-  if (GENERAL) {
-    pairs_inside<ROWS, 2, true, true>(us, rs, ks, gs, mine);
-    pairs_inside<ROWS, 2, true, true>(us, rs, bb, gs, mine + inside_sums(2));
-  } else {
-    pairs_inside<ROWS, 1, !MEMORY, !MEMORY>(rs, nullptr, ks, gs, mine);
-  }
-  __syncthreads();
-  if (GENERAL) {
-    add_up<2, true>(sums, kSums, uk, rk);
-    add_up<2, true>(sums + inside_sums(2), kSums, ub, rb);
-  } else {
-    add_up<1, true>(sums, kSums, rk, nullptr);
-  }
-  for (int item = tid; !MEMORY && item < kGroups * rows; item += kThreads) {  // a thread per (group, channel)
-    const int c = item % rows, at = item / rows * kGroup * ld + c;
-    float g[kGroup];
-    float run = 1.f;
-#pragma unroll
-    for (int r = 0; r < kGroup; ++r) {
-      g[r] = item / rows * kGroup + r < n ? gs[at + r * ld] : 1.f;
-      if (GENERAL) us[at + r * ld] *= run;
-      else rs[at + r * ld] *= run;
-      run *= g[r];
-      if (GENERAL) rs[at + r * ld] *= run;
-    }
-    whole[item] = run;
-    run = 1.f;
-#pragma unroll
-    for (int r = kGroup - 1; r >= 0; --r) {
-      ks[at + r * ld] *= run;
-      if (GENERAL) bb[at + r * ld] *= run;
-      run *= g[r];
-    }
-  }
-  __syncthreads();
-  if (GENERAL) {
-    pairs_between<ROWS, 2, true>(us, rs, ks, whole, mine);
+  if (MEMORY) {
+    for (int tile = warp; tile < kTiles; tile += kWarps) pair_tile<ROWS, 1, false>(rs, nullptr, ks, nullptr, tile, rk, nullptr);
     __syncthreads();
-    add_up<2, false>(sums, kSums, uk, rk);
-    __syncthreads();
-    pairs_between<ROWS, 2, true>(us, rs, bb, whole, mine);
-    __syncthreads();
-    add_up<2, false>(sums, kSums, ub, rb);
-  } else {
-    pairs_between<ROWS, 1, !MEMORY>(rs, nullptr, ks, whole, mine);
-    __syncthreads();
-    add_up<1, false>(sums, kSums, rk, nullptr);
-  }
-  __syncthreads();
-  if constexpr (MEMORY) {
     // Column j = lane: the keeps of tokens j + 1 .. i multiplied, from one at i = j on.
     const int64_t at = (first + lane) * heads + head;
     const float keep = lane < n ? in.w[at] : 1.f, put = lane < n ? in.put[at] : 0.f;
@@ -616,115 +694,148 @@ linear_chunk_prepare_kernel(LinearRule in, const int* __restrict__ seq_q_start, 
       }
       to.n[place * rows + c] = sum;
       to.e[place * rows + c] = es[n - 1];
-#pragma unroll
-      for (int g = 0; g < kGroups; ++g) whole[g * rows + c] = 1.f;
     }
     __syncthreads();
-  }
-  for (int i = warp; !MEMORY && i < C; i += kWarps) {
-    const int at = i * (C + 1) + lane;
-    const int64_t row = (place * C + i) * C + lane;
-    if (GENERAL) {  // au came in with its own sign: b = -au
-      ls[i * C + lane] = lane < i ? ub[at] : 0.f;
-      ms[i * C + lane] = lane < i ? uk[at] : 0.f;
-      to.a[row] = lane <= i ? -rb[at] : 0.f;
-      to.av[row] = lane <= i ? rk[at] : 0.f;
-    } else {
-      to.av[row] = lane < i ? rk[at] : (lane == i && i < n ? in.bonus[(first + i) * heads + head] : 0.f);
+  } else {
+    if (warp < kGroups) {
+      // One after the other through the same code: an SM holds about half of this kernel's.
+#pragma unroll 1
+      for (int right = 0; right < (GENERAL ? 2 : 1); ++right)
+        pairs_in_group<ROWS, true, false>(GENERAL ? us : rs, right == 0 ? ks : bb, gs, warp, GENERAL ? (right == 0 ? uk : ub) : rk);
+    } else if (GENERAL) {
+#pragma unroll 1
+      for (int right = 0; right < 2; ++right) pairs_in_group<ROWS, false, true>(rs, right == 0 ? ks : bb, gs, warp - kGroups, right == 0 ? rk : rb);
     }
-  }
-  // Scaled rows: r times all decays in front of (or up to) its token, b times all decays behind its token; a thread per (group, channel).
-  for (int item = tid; !MEMORY && item < kGroups * rows; item += kThreads) {
-    const int c = item % rows, group = item / rows;
-    float before = 1.f, after = 1.f;
+    __syncthreads();
+    for (int item = tid; item < kGroups * rows; item += kThreads) {  // a thread per (group, channel)
+      const int c = item % rows, at = item / rows * kGroup * ld + c;
+      float decays[kGroup];
+      float run = 1.f;
 #pragma unroll
-    for (int g = 0; g < kGroups - 1; ++g) {
-      before *= g < group ? whole[g * rows + c] : 1.f;
-      after *= g + 1 > group ? whole[(g + 1) * rows + c] : 1.f;
+      for (int r = 0; r < kGroup; ++r) {
+        decays[r] = item / rows * kGroup + r < n ? gs[at + r * ld] : 1.f;
+        if (GENERAL) us[at + r * ld] *= run;
+        else rs[at + r * ld] *= run;
+        run *= decays[r];
+        if (GENERAL) rs[at + r * ld] *= run;
+      }
+      whole[item] = run;
+      run = 1.f;
+#pragma unroll
+      for (int r = kGroup - 1; r >= 0; --r) {
+        ks[at + r * ld] *= run;
+        if (GENERAL) bb[at + r * ld] *= run;
+        run *= decays[r];
+      }
     }
-    float* qt = to.qt + (place * C + group * kGroup) * rows + c;
-#pragma unroll
-    for (int r = 0; r < kGroup; ++r) qt[r * rows] = before * rs[(group * kGroup + r) * ld + c];
+    __syncthreads();
     if (GENERAL) {
-      float decayed[kGroup];
+      for (int tile = warp; tile < 2 * kBetween; tile += kWarps) {
+        const bool second = tile >= kBetween;
+        pair_tile<ROWS, 2, true>(us, rs, second ? bb : ks, whole, second ? tile - kBetween : tile, second ? ub : uk, second ? rb : rk);
+      }
+    } else if (warp < kBetween) {
+      pair_tile<ROWS, 1, true>(rs, nullptr, ks, whole, warp, rk, nullptr);
+    }
+    __syncthreads();
+    for (int i = warp; i < C; i += kWarps) {
+      const int at = i * (C + 1) + lane;
+      const int64_t row = (place * C + i) * C + lane;
+      if (GENERAL) {  // au came in with its own sign: b = -au
+        ls[i * C + lane] = lane < i ? ub[at] : 0.f;
+        ms[i * C + lane] = lane < i ? uk[at] : 0.f;
+        to.a[row] = lane <= i ? -rb[at] : 0.f;
+        to.av[row] = lane <= i ? rk[at] : 0.f;
+      } else {
+        to.av[row] = lane < i ? rk[at] : (lane == i && i < n ? in.bonus[(first + i) * heads + head] : 0.f);
+      }
+    }
+    // Scaled rows: r times all decays in front of (or up to) its token, k and b times all decays behind theirs; a thread per (group, channel).
+    for (int item = tid; item < kGroups * rows; item += kThreads) {
+      const int c = item % rows, group = item / rows;
+      float before = 1.f, after = 1.f;
 #pragma unroll
-      for (int r = 0; r < kGroup; ++r) decayed[r] = group * kGroup + r < n ? -after * bb[(group * kGroup + r) * ld + c] : 0.f;
-      float* kd = to.kd + place * rows * C + kd_place(group * kGroup, c);
-      *reinterpret_cast<float4*>(kd) = make_float4(decayed[0], decayed[1], decayed[2], decayed[3]);
-      *reinterpret_cast<float4*>(kd + 4) = make_float4(decayed[4], decayed[5], decayed[6], decayed[7]);
+      for (int x = 0; x < kGroups - 1; ++x) {
+        before *= x < group ? whole[x * rows + c] : 1.f;
+        after *= x + 1 > group ? whole[(x + 1) * rows + c] : 1.f;
+      }
+      float* qt = to.qt + (place * C + group * kGroup) * rows + c;
+#pragma unroll
+      for (int r = 0; r < kGroup; ++r) {
+        const int at = (group * kGroup + r) * ld + c;
+        qt[r * rows] = before * rs[at];
+        ks[at] *= after;
+      }
+      if (GENERAL) {
+        front[item] = before;
+        float decayed[kGroup];
+#pragma unroll
+        for (int r = 0; r < kGroup; ++r) decayed[r] = group * kGroup + r < n ? -after * bb[(group * kGroup + r) * ld + c] : 0.f;
+        float* kd = to.kd + place * rows * C + kd_place(group * kGroup, c);
+        *reinterpret_cast<float4*>(kd) = make_float4(decayed[0], decayed[1], decayed[2], decayed[3]);
+        *reinterpret_cast<float4*>(kd + 4) = make_float4(decayed[4], decayed[5], decayed[6], decayed[7]);
+      }
+      if (group == kGroups - 1) to.e[place * rows + c] = before * whole[item];
+    }
+    __syncthreads();
+    if (GENERAL) {
+      if (warp == 0) {
+        invert_halves(ls, inverse);
+        __syncwarp();
+        pack_triangle(triangles, inverse, kLdT), pack_triangle(triangles + 2 * kTriangle, inverse + 16 * kLdT, kLdT);
+      } else if (warp == 1) {
+        pack_triangle(triangles + kTriangle, ls + 16 * C, C);
+      }
+      __syncthreads();
+      for (int tile = warp; tile < (rows + columns) / 16; tile += kWarps) {  // sixteen columns of [e U | M V]
+        Columns r;
+        int2 spoilt = make_int2(C, C);
+        if (tile < rows / 16) {
+#pragma unroll
+          for (int h = 0; h < 2; ++h)
+#pragma unroll
+            for (int c = 0; c < 2; ++c) {
+              const int column = tile * 16 + g + 8 * c, token = h * 16 + 4 * q;
+              const float before = front[token / kGroup * rows + column];
+              const float* at = us + token * ld + column;
+              r.v[h][c] = make_float4(before * at[0], before * at[ld], before * at[2 * ld], before * at[3 * ld]);
+            }
+        } else {
+          r = load_values(values, in.v_ld, (tile - rows / 16) * 16, dv, n);
+          take_out(r.v[0], 0, spoilt), take_out(r.v[1], 1, spoilt);
+          const SplitA v0 = split_columns(r.v[0]), v1 = split_columns(r.v[1]);
+          float4 more[2];
+          times_rows(r.v[0], v0, ms, C);
+          times_rows(r.v[1], v0, ms + 16 * C, C);
+          times_rows(more, v1, ms + 16 * C + 16, C);
+          r.v[1][0] = plus(r.v[1][0], more[0]), r.v[1][1] = plus(r.v[1][1], more[1]);
+        }
+        solve_columns(r, triangles, spoilt, n);
+        if (tile < rows / 16) store_y(to.y + place * rows * C, tile * 16, r);
+        else store_x(to.x + (place * columns + tile * 16 - rows) * C, r);
+      }
     }
   }
-  for (int c = tid; !MEMORY && c < rows; c += kThreads) to.e[place * rows + c] = whole[c] * whole[rows + c] * whole[2 * rows + c] * whole[3 * rows + c];
-  if (GENERAL) __syncthreads();
-  for (int col0 = 0; col0 < columns; col0 += kValueTile) {
-    if (col0 > 0) {
-      __syncthreads();
-      stage_values(col0);
-      commit_copies();
-      wait_copies<0>();
-      __syncthreads();
-    }
-    if (GENERAL && tid < kValueTile + (col0 == 0 ? rows : 0)) {  // a thread per column of [M V | e U]
-      float x[C];
-      const int c = tid;
-      if (tid < kValueTile) {
-        float value[C];
+  // (G_last K)^T V, transposed: sixteen columns by 32 rows a warp at a time.
+  for (int item = warp; item < columns / 16 * (rows / 32); item += kWarps) {
+    const int col0 = item / (rows / 32) * 16, row0 = item % (rows / 32) * 32;
+    const Columns r = load_values(values, in.v_ld, col0, dv, n);
+    const SplitA left[2] = {split_columns(r.v[0]), split_columns(r.v[1])};
 #pragma unroll
-        for (int i = 0; i < C; ++i) value[i] = vs[i * kLdV + c];
+    for (int block = 0; block < 2; ++block) {
+      float part[2][2][4] = {};  // [tile][half of the tokens]
 #pragma unroll
-        for (int i = 0; i < C; ++i) {
-          float sum0 = 0.f, sum1 = 0.f;
+      for (int t = 0; t < 2; ++t)
 #pragma unroll
-          for (int j = 0; j < i; j += 4) {
-            const float4 row = *reinterpret_cast<const float4*>(ms + i * C + j);
-            sum0 = fmaf(row.x, value[j], sum0);
-            if (j + 1 < i) sum1 = fmaf(row.y, value[j + 1], sum1);
-            if (j + 2 < i) sum0 = fmaf(row.z, value[j + 2], sum0);
-            if (j + 3 < i) sum1 = fmaf(row.w, value[j + 3], sum1);
-          }
-          x[i] = sum0 + sum1;
+        for (int h = 0; h < 2; ++h) {
+          const float* at = ks + (h * 16 + 4 * q) * ld + row0 + block * 16 + in_sixteen(t, g);
+          mma_split(part[t][h], left[h], SplitB(make_float4(at[0], at[ld], at[2 * ld], at[3 * ld])));
         }
-      } else {
-        const int channel = c - kValueTile;
-        float before = 1.f;
+      float* s = to.s + place * columns * rows + s_place(col0, row0 + block * 16, rows) + lane * 4;
 #pragma unroll
-        for (int i = 0; i < C; ++i) {
-          if (i > 0 && i % kGroup == 0) before *= whole[(i / kGroup - 1) * rows + channel];
-          x[i] = before * us[i * ld + channel];
-        }
-      }
-      substitute(ls, x);
-      if (tid >= kValueTile) store_y(to.y + place * C * rows, c - kValueTile, x, n);
-      else if (col0 + c < columns) store_column(to.x + (place * columns + col0 + c) * C, x, n);
-    }
-    // (G_last K)^T V over the tile: four rows by four columns a thread, group after group of tokens.
-    const int rt = (tid & 15) * 4, ct = (tid >> 4) * 4;
-    for (int row = rt; row < rows; row += 64) {
-      float acc[4][4];
-#pragma unroll
-      for (int r = 0; r < 4; ++r) acc[r][0] = acc[r][1] = acc[r][2] = acc[r][3] = 0.f;
-#pragma unroll
-      for (int g = 0; g < kGroups; ++g) {
-        const float4 scale = *reinterpret_cast<const float4*>(whole + g * rows + row);
-        const float f[4] = {scale.x, scale.y, scale.z, scale.w};
-#pragma unroll
-        for (int r = 0; r < 4; ++r) acc[r][0] *= f[r], acc[r][1] *= f[r], acc[r][2] *= f[r], acc[r][3] *= f[r];
-#pragma unroll
-        for (int j = g * kGroup; j < (g + 1) * kGroup; ++j) {
-          const float4 key = *reinterpret_cast<const float4*>(ks + j * ld + row), value = *reinterpret_cast<const float4*>(vs + j * kLdV + ct);
-          const float a[4] = {key.x, key.y, key.z, key.w};
-#pragma unroll
-          for (int r = 0; r < 4; ++r) {
-            acc[r][0] = fmaf(a[r], value.x, acc[r][0]), acc[r][1] = fmaf(a[r], value.y, acc[r][1]);
-            acc[r][2] = fmaf(a[r], value.z, acc[r][2]), acc[r][3] = fmaf(a[r], value.w, acc[r][3]);
-          }
-        }
-      }
-      if (col0 + ct < columns) {
-#pragma unroll
-        for (int c = 0; c < 4; ++c)
-          *reinterpret_cast<float4*>(to.s + place * columns * rows + s_place(col0 + ct + c, row, rows)) = make_float4(acc[0][c], acc[1][c], acc[2][c], acc[3][c]);
-      }
+      for (int c = 0; c < 2; ++c)
+        *reinterpret_cast<float4*>(s + c * 128) = make_float4(part[0][0][2 * c] + part[0][1][2 * c], part[0][0][2 * c + 1] + part[0][1][2 * c + 1],
+                                                              part[1][0][2 * c] + part[1][1][2 * c], part[1][0][2 * c + 1] + part[1][1][2 * c + 1]);
     }
   }
 }
@@ -1026,6 +1137,7 @@ chunk_out_kernel(const int* __restrict__ seq_q_start, const int* __restrict__ se
       bool found = false;
 #pragma unroll
       for (int t = 0; t < 4; ++t) {
+        if (all_finite(right[t])) continue;
         float* numbers[4] = {&right[t].x, &right[t].y, &right[t].z, &right[t].w};
 #pragma unroll
         for (int i = 3; i >= 0; --i)
