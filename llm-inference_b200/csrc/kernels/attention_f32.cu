@@ -1,29 +1,31 @@
 // Attention of prompt portions over the paged cache in 32 bits: the tiled form of the plain kernel (attention_plain.cu).
 //
 // One block takes 32 rows of one kv head, a row being a (token, query head) pair of a request, token by token with the query heads
-// that share the kv head side by side, and walks the request's keys 64 at a time: scores as a 32 x 64 product, the running softmax,
-// then the weighted sum of values as a 32 x head_dim product, everything 32-bit FMAs. Keys and values come by cp.async, the values
-// while the scores are formed and the next keys while the values are summed. A row's result does not depend on what else is in the
-// call beyond the order in which its keys' tiles begin. Windows and a sink (a start value of maximum and sum) are taken; other
-// shapes of scores, kept first keys and single tokens run the plain kernel.
+// that share the kv head side by side, and walks the request's keys 64 at a time. A warp has sixteen of the rows and sixteen of every 64 keys: scores,
+// running softmax and weighted sum of values are its own until the end, when the four parts of the keys meet. Both products are tensor-core
+// products of 32-bit numbers taken apart into three bfloat16 ones (split_mma.cuh); eight warps more take the next tile's keys and values
+// apart, into shared memory as the lanes want them, while this one's are multiplied. Windows and a sink (a start value of
+// maximum and sum) are taken; other shapes of scores, kept first keys and single tokens run the plain kernel.
 //
-// What bounds it: operands out of shared memory, 2 (scores) and 2.7 (values) FMAs per number. The plain kernel reads every key row
-// once per (token, head) and forms one score a thread. Measured on a B200 (500 tokens, 12 heads of 128 on 2 kv heads, one request):
-// 325 -> 88 us; 2,048 tokens 4,545 -> 501 us, behind 4,000 others 22.2 -> 2.4 ms.
-#include <type_traits>
-
+// What bounds it: the tensor core's 1,536 products a tile (3,300 cycles of an SM) and, in turn with them, the taking apart. The plain kernel reads
+// every key row once per (token, head) and forms one score a thread; FMAs over tiles in shared memory read 2 (scores) and 2.7 (values) FMAs'
+// worth a number. Measured on a B200 (500 tokens, 12 heads of 128 on 2 kv heads, one request): plain 325, FMAs 76, now 46 us; 2,048
+// tokens 487 and 415 us, behind 4,000 others 2.4 and 2.0 ms; 8 tokens behind 1,000 others 116 and 79. Error against 64 bits (500 tokens,
+// 2-norm) 6.7e-7 and 2.3e-7.
 #include "common.cuh"
+#include "split_mma.cuh"
 
 namespace {
 
-constexpr int kRows = 32, kKeys = 64, kThreads = 128;
-constexpr int kLdP = kKeys + 4;
-
-__device__ __forceinline__ void stage_copy(float* smem, const float* gmem, bool valid) {
-  const uint32_t s = static_cast<uint32_t>(__cvta_generic_to_shared(smem));
-  const int bytes = valid ? 16 : 0;
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(s), "l"(gmem), "r"(bytes) : "memory");
-}
+constexpr int kRows = 32, kKeys = 64;
+constexpr int kKeyParts = kKeys / 16;                 // warps that share sixteen rows
+constexpr int kWarps = kRows / 16 * kKeyParts;        // that multiply
+constexpr int kApart = 2 * kKeyParts;                 // behind them: that take apart, half the numbers of sixteen keys each
+constexpr int kOwnThreads = kWarps * 32, kThreads = kOwnThreads + kApart * 32;
+constexpr int kChunk = 2;                             // blocks of 16 x 16 numbers on the way in a warp's registers
+// Registers a thread of either kind, out of 512 x 128 at launch.
+constexpr int kOwnRegisters = 168, kApartRegisters = 88;
+static_assert(kThreads == 512 && kOwnRegisters + kApartRegisters <= 2 * 128, "more registers than the block was launched with");
 
 struct PortionParams {
   const float* q;
@@ -40,22 +42,43 @@ struct PortionParams {
   float scale;
 };
 
-constexpr size_t portion_smem(int dim) {
-  return sizeof(float) * (kRows * (dim + 4) + 2 * kKeys * (dim + 4) + kRows * kLdP + kRows) + 2 * kKeys * sizeof(int64_t);
+// Parts of 16 x 16 numbers, a uint4 a part and lane.
+constexpr int kBlock = 3 * 32;
+constexpr size_t portion_smem(int dim) { return sizeof(uint4) * (kRows / 16 + 2 * 2 * kKeyParts) * (dim / 16) * kBlock; }
+
+// Two tiles take turns: barrier `id` is met by the warps that multiply and those that take apart, of which one side only arrives.
+__device__ __forceinline__ void meet(int id) { asm volatile("bar.sync %0, %1;" ::"r"(id), "n"(kThreads) : "memory"); }
+__device__ __forceinline__ void arrive(int id) { asm volatile("bar.arrive %0, %1;" ::"r"(id), "n"(kThreads) : "memory"); }
+__device__ __forceinline__ void meet_own() { asm volatile("bar.sync 5, %0;" ::"n"(kOwnThreads) : "memory"); }
+constexpr int kFull = 1, kEmpty = 3;  // + tile % 2
+
+__device__ __forceinline__ void store_block(uint4* to, const SplitB& first, const SplitB& second) {
+  const int lane = threadIdx.x & 31;
+#pragma unroll
+  for (int p = 0; p < 3; ++p) to[p * 32 + lane] = make_uint4(first.lo.part[p], first.hi.part[p], second.lo.part[p], second.hi.part[p]);
+}
+__device__ __forceinline__ void load_block(const uint4* from, SplitB* to) {
+  const int lane = threadIdx.x & 31;
+#pragma unroll
+  for (int p = 0; p < 3; ++p) {
+    const uint4 word = from[p * 32 + lane];
+    to[0].lo.part[p] = word.x, to[0].hi.part[p] = word.y, to[1].lo.part[p] = word.z, to[1].hi.part[p] = word.w;
+  }
 }
 
 template <int DIM>
-__global__ void __launch_bounds__(kThreads)
+__global__ void __launch_bounds__(kThreads, 1)
 portion_attention_f32_kernel(const PortionParams p) {
-  extern __shared__ __align__(16) float attention_smem[];
-  constexpr int kLd = DIM + 4;
-  constexpr int kColGroups = DIM / 4, kRowGroups = kThreads / kColGroups, kOwnRows = kRows / kRowGroups;  // of the values' product
-  float* qs = attention_smem;         // [kRows][kLd]
-  float* ks = qs + kRows * kLd;       // [kKeys][kLd]
-  float* vs = ks + kKeys * kLd;       // [kKeys][kLd]
-  float* ps = vs + kKeys * kLd;       // [kRows][kLdP]
-  float* alphas = ps + kRows * kLdP;  // [kRows]: factor of the running output; at the end 1 / sum
-  int64_t* offsets = reinterpret_cast<int64_t*>(alphas + kRows);  // [2][kKeys]: rows of two tiles, -1: not to be read
+  extern __shared__ __align__(16) uint4 attention_smem[];
+  constexpr int kSteps = DIM / 16;                        // sixteens of a head's numbers
+  constexpr int kTile = kKeyParts * kSteps * kBlock;      // of keys, or of values
+  constexpr int kLdO = DIM + 4;
+  uint4* qs = attention_smem;                             // [kRows / 16][kSteps][kBlock]
+  uint4* ks = qs + kRows / 16 * kSteps * kBlock;          // [2][kKeyParts][kSteps][kBlock]: tiles of eight keys
+  uint4* vs = ks + 2 * kTile;                             // [2][kKeyParts][kSteps][kBlock]: tiles of eight of a value's numbers
+  __shared__ int64_t offsets[2][kKeys];                   // rows of two tiles, -1: not to be read
+  __shared__ int spoilt[2][kApart];                       // values that are not finite
+  __shared__ float tops[kWarps][16], totals[kWarps][16];
   const int seq = p.first_seq + blockIdx.z, kvh = blockIdx.y;
   const int group = p.q_heads / p.kv_heads;
   const int len = p.seq_q_len[seq], start = p.seq_q_start[seq], begin = p.seq_kv_len[seq] - len;  // begin: position of the first new token
@@ -63,156 +86,224 @@ portion_attention_f32_kernel(const PortionParams p) {
   const int block = row_blocks - 1 - static_cast<int>(blockIdx.x);  // the rows with most keys first
   if (block < 0) return;
   const int row0 = block * kRows, rows = min(kRows, len * group - row0);
-  const int tid = threadIdx.x;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, q = lane & 3;
   const int* table = p.block_table + static_cast<int64_t>(seq) * p.max_pages;
   const int last_pos = begin + (row0 + rows - 1) / group, first_pos = begin + row0 / group;
   const int lo = p.window > 0 ? max(0, first_pos - p.window + 1) : 0;
   const int tiles = (last_pos - lo) / kKeys + 1;
-  auto look_up = [&](int tile) {  // where the tile's rows are
-    if (tid < kKeys) {
-      const int j = lo + tile * kKeys + tid;
-      int64_t offset = -1;
+  const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+  auto query = [&](int r, int c) {
+    const int item = row0 + r, token = item / group, head = kvh * group + item % group;
+    return r < rows && c < p.head_dim ? *reinterpret_cast<const float4*>(p.q + (static_cast<int64_t>(start + token) * p.q_heads + head) * p.head_dim + c) : zero;
+  };
+  for (int item = warp; item < kRows / 16 * kSteps; item += kThreads / 32) {
+    const int r = item / kSteps * 16 + g, c = item % kSteps * 16 + 4 * q;
+    const SplitA a = split_rows(query(r, c), query(r + 8, c));
+#pragma unroll
+    for (int x = 0; x < 3; ++x) qs[(item * 3 + x) * 32 + lane] = make_uint4(a.part[x][0], a.part[x][1], a.part[x][2], a.part[x][3]);
+  }
+  __syncthreads();
+  if (warp >= kWarps) {
+    // ---- take apart: half the numbers of sixteen keys a warp, chunk after chunk ----
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kApartRegisters));
+    constexpr int kChunks = kSteps / 2 / kChunk;
+    const int part = (warp - kWarps) / 2, half = (warp - kWarps) % 2, step0 = half * (kSteps / 2);
+    float4 k_next[kChunk][2], v_next[kChunk][2];
+    int64_t own = -1;  // of key lane % 16: where its row is
+    auto look_up = [&](int tile) {
+      const int j = lo + tile * kKeys + part * 16 + (lane & 15);
+      own = -1;
       if (tile < tiles && j <= last_pos) {
         const int logical = j / p.page_size;
         const int page = logical < p.max_pages ? table[logical] : -1;
         if (page < 0 || page >= p.num_pages) atomicOr(p.err, ERRBIT_BAD_PAGE);
-        else offset = kv_row_offset(page, kvh, j % p.page_size, p.kv_heads, p.page_size, p.head_dim);
+        else own = kv_row_offset(page, kvh, j % p.page_size, p.kv_heads, p.page_size, p.head_dim);
       }
-      offsets[(tile & 1) * kKeys + tid] = offset;
-    }
-  };
-  auto fetch = [&](float* to, const float* arena, int tile) {
-    for (int idx = tid; idx < kKeys * (DIM / 4); idx += kThreads) {
-      const int r = idx / (DIM / 4), c = idx % (DIM / 4) * 4;
-      const int64_t offset = offsets[(tile & 1) * kKeys + r];
-      const bool valid = offset >= 0 && c < p.head_dim;
-      stage_copy(to + r * kLd + c, valid ? arena + offset + c : arena, valid);
-    }
-    asm volatile("cp.async.commit_group;" ::: "memory");
-  };
-  for (int idx = tid; idx < kRows * (DIM / 4); idx += kThreads) {
-    const int r = idx / (DIM / 4), c = idx % (DIM / 4) * 4;
-    const int item = row0 + r, token = item / group, head = kvh * group + item % group;
-    const bool valid = r < rows && c < p.head_dim;
-    stage_copy(qs + r * kLd + c, valid ? p.q + (static_cast<int64_t>(start + token) * p.q_heads + head) * p.head_dim + c : p.q, valid);
-  }
-  look_up(0);
-  __syncthreads();
-  fetch(ks, p.keys, 0);  // its group holds the queries too
-  const int tc = tid & 15, tr = tid >> 4;                  // scores: rows tr, tr + 8, .., keys tc, tc + 16, ..
-  const int cg = tid % kColGroups, rg = tid / kColGroups;  // values: rows rg, rg + kRowGroups, .., dims 4 cg .. + 3
-  float top[4], sum[4];
-  int pos[4], from[4];
+    };
+    int64_t key_at[2], value_at[4];
+    auto spread = [&] {
 #pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const int item = row0 + tr + 8 * i;
-    pos[i] = tr + 8 * i < rows ? begin + item / group : -1;
-    from[i] = p.window > 0 ? pos[i] - p.window + 1 : 0;
-    const float* sink = p.sink ? p.sink + kvh * group + item % group : nullptr;
-    top[i] = sink ? *sink : -INFINITY;
-    sum[i] = sink ? 1.f : 0.f;
-  }
-  float acc[kOwnRows][4];
+      for (int t = 0; t < 2; ++t) key_at[t] = __shfl_sync(0xffffffffu, own, in_sixteen(t, g));
 #pragma unroll
-  for (int i = 0; i < kOwnRows; ++i) acc[i][0] = acc[i][1] = acc[i][2] = acc[i][3] = 0.f;
+      for (int x = 0; x < 4; ++x) value_at[x] = __shfl_sync(0xffffffffu, own, 4 * q + x);
+    };
+    auto fetch = [&](int step, int i) {
+      const int c0 = (step0 + step + i) * 16;
+#pragma unroll
+      for (int t = 0; t < 2; ++t) {
+        const int c = c0 + 4 * q, cv = c0 + 8 * t + g;
+        k_next[i][t] = key_at[t] >= 0 && c < p.head_dim ? *reinterpret_cast<const float4*>(p.keys + key_at[t] + c) : zero;
+        const bool in = cv < p.head_dim;
+        v_next[i][t] = make_float4(in && value_at[0] >= 0 ? p.values[value_at[0] + cv] : 0.f, in && value_at[1] >= 0 ? p.values[value_at[1] + cv] : 0.f,
+                                   in && value_at[2] >= 0 ? p.values[value_at[2] + cv] : 0.f, in && value_at[3] >= 0 ? p.values[value_at[3] + cv] : 0.f);
+      }
+    };
+    look_up(0), spread();
+#pragma unroll
+    for (int i = 0; i < kChunk; ++i) fetch(0, i);
+    for (int tile = 0; tile < tiles; ++tile) {
+      const int b = tile & 1;
+      if (tile >= 2) meet(kEmpty + b);
+      if (half == 0 && lane < 16) offsets[b][part * 16 + lane] = own;
+      bool finite = true;
+#pragma unroll 1
+      for (int chunk = 0; chunk < kChunks; ++chunk) {
+        if (chunk + 1 == kChunks) look_up(tile + 1), spread();
+#pragma unroll
+        for (int i = 0; i < kChunk; ++i) {
+          const int at = b * kTile + (part * kSteps + step0 + chunk * kChunk + i) * kBlock;
+          store_block(ks + at, SplitB(k_next[i][0]), SplitB(k_next[i][1]));
+#pragma unroll
+          for (int t = 0; t < 2; ++t) {
+            float4& v = v_next[i][t];
+            if (all_finite(v)) continue;
+            finite = false;  // zeros for now
+            v.x = isfinite(v.x) ? v.x : 0.f, v.y = isfinite(v.y) ? v.y : 0.f, v.z = isfinite(v.z) ? v.z : 0.f, v.w = isfinite(v.w) ? v.w : 0.f;
+          }
+          store_block(vs + at, SplitB(v_next[i][0]), SplitB(v_next[i][1]));
+          fetch(chunk + 1 < kChunks ? (chunk + 1) * kChunk : 0, i);  // the next chunk's, of the next tile behind a tile's last (past the last one: zeros)
+        }
+      }
+      const bool any = __any_sync(0xffffffffu, !finite);
+      if (lane == 0) spoilt[b][warp - kWarps] = any;
+      arrive(kFull + b);
+    }
+    return;
+  }
+  asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kOwnRegisters));
+  const int own_rows = warp / kKeyParts * 16, own_keys = warp % kKeyParts;
+  int pos[2], from[2];
+  float top[2], sum[2];
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    const int r = own_rows + g + 8 * h, item = row0 + r;
+    pos[h] = r < rows ? begin + item / group : -1;
+    from[h] = p.window > 0 ? pos[h] - p.window + 1 : 0;
+    const float* sink = p.sink && own_keys == 0 ? p.sink + kvh * group + item % group : nullptr;
+    top[h] = sink ? *sink : -INFINITY;
+    sum[h] = sink && q == 0 ? 1.f : 0.f;  // a lane's share
+  }
+  float acc[2 * kSteps][4];
+#pragma unroll
+  for (int i = 0; i < 2 * kSteps; ++i) acc[i][0] = acc[i][1] = acc[i][2] = acc[i][3] = 0.f;
   for (int tile = 0; tile < tiles; ++tile) {
-    asm volatile("cp.async.wait_group 0;" ::: "memory");
-    __syncthreads();  // the keys are there; nobody reads the values any more
-    fetch(vs, p.values, tile);
-    look_up(tile + 1);
-    float s[4][4];
+    const int b = tile & 1;
+    meet(kFull + b);
+    // Scores of sixteen rows and sixteen keys, of which the lane has keys 4 q .. + 3.
+    float score[2][4] = {};
+    {
+      constexpr int kTogether = 2;
+#pragma unroll 1
+      for (int s = 0; s < kSteps; s += kTogether) {
+        float sums[2 * kTogether][4] = {};
+        SplitA own[kTogether];
+        SplitB right[2 * kTogether];
 #pragma unroll
-    for (int i = 0; i < 4; ++i) s[i][0] = s[i][1] = s[i][2] = s[i][3] = 0.f;
-#pragma unroll 4
-    for (int c = 0; c < DIM; c += 4) {
-      float4 a[4], b[4];
+        for (int x = 0; x < kTogether; ++x) {
 #pragma unroll
-      for (int x = 0; x < 4; ++x) {
-        a[x] = *reinterpret_cast<const float4*>(qs + (tr + 8 * x) * kLd + c);
-        b[x] = *reinterpret_cast<const float4*>(ks + (tc + 16 * x) * kLd + c);
+          for (int y = 0; y < 3; ++y) {
+            const uint4 word = qs[((own_rows / 16 * kSteps + s + x) * 3 + y) * 32 + lane];
+            own[x].part[y][0] = word.x, own[x].part[y][1] = word.y, own[x].part[y][2] = word.z, own[x].part[y][3] = word.w;
+          }
+          load_block(ks + b * kTile + (own_keys * kSteps + s + x) * kBlock, right + 2 * x);
+        }
+        mma_split(sums, {&own[0], &own[0], &own[1], &own[1]}, right);
+#pragma unroll
+        for (int t = 0; t < 2; ++t)
+#pragma unroll
+          for (int i = 0; i < 4; ++i) score[t][i] += sums[t][i] + sums[2 + t][i];
       }
-#pragma unroll
-      for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int j = 0; j < 4; ++j)
-          s[i][j] = fmaf(a[i].w, b[j].w, fmaf(a[i].z, b[j].z, fmaf(a[i].y, b[j].y, fmaf(a[i].x, b[j].x, s[i][j]))));
     }
-    const int64_t* tile_rows = offsets + (tile & 1) * kKeys;
+    const int key0 = lo + tile * kKeys + own_keys * 16 + 4 * q;
+    const int64_t* own_offsets = offsets[b] + own_keys * 16 + 4 * q;
+    float weight[2][4], alpha[2];
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
+    for (int h = 0; h < 2; ++h) {
       float best = -INFINITY;
       bool seen[4];
 #pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const int key = lo + tile * kKeys + tc + 16 * j;
-        seen[j] = key <= pos[i] && key >= from[i] && tile_rows[tc + 16 * j] >= 0;
-        s[i][j] = seen[j] ? s[i][j] * p.scale : -INFINITY;
-        best = fmaxf(best, s[i][j]);
+      for (int i = 0; i < 4; ++i) {
+        const int key = key0 + i;
+        seen[i] = key <= pos[h] && key >= from[h] && own_offsets[i] >= 0;
+        weight[h][i] = seen[i] ? score[i >> 1][2 * h + (i & 1)] * p.scale : -INFINITY;
+        best = fmaxf(best, weight[h][i]);
       }
+      best = fmaxf(best, __shfl_xor_sync(0xffffffffu, best, 1));
+      best = fmaxf(best, __shfl_xor_sync(0xffffffffu, best, 2));
+      const float new_top = fmaxf(top[h], best);
+      alpha[h] = top[h] > -INFINITY ? expf(top[h] - new_top) : 0.f;
+      float more = 0.f;
 #pragma unroll
-      for (int o = 8; o > 0; o >>= 1) best = fmaxf(best, __shfl_xor_sync(0xffffffffu, best, o));
-      const float new_top = fmaxf(top[i], best);
-      const float alpha = top[i] > -INFINITY ? expf(top[i] - new_top) : 0.f;
-      float part = 0.f;
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const float weight = seen[j] && new_top > -INFINITY ? expf(s[i][j] - new_top) : 0.f;
-        ps[(tr + 8 * i) * kLdP + tc + 16 * j] = seen[j] ? weight : -0.f;  // a minus sign marks what the row does not see
-        part += weight;
+      for (int i = 0; i < 4; ++i) {
+        weight[h][i] = seen[i] && new_top > -INFINITY ? expf(weight[h][i] - new_top) : 0.f;
+        more += weight[h][i];
       }
-#pragma unroll
-      for (int o = 8; o > 0; o >>= 1) part += __shfl_xor_sync(0xffffffffu, part, o);
-      sum[i] = sum[i] * alpha + part;
-      top[i] = new_top;
-      if (tc == 0) alphas[tr + 8 * i] = alpha;
+      sum[h] = fmaf(sum[h], alpha[h], more);
+      top[h] = new_top;
     }
-    asm volatile("cp.async.wait_group 0;" ::: "memory");
-    __syncthreads();  // weights and values are there, the next tile's rows looked up, the keys read
-    if (tile + 1 < tiles) fetch(ks, p.keys, tile + 1);
+    const SplitA left = split_rows(make_float4(weight[0][0], weight[0][1], weight[0][2], weight[0][3]), make_float4(weight[1][0], weight[1][1], weight[1][2], weight[1][3]));
 #pragma unroll
-    for (int i = 0; i < kOwnRows; ++i) {
-      const float alpha = alphas[rg + kRowGroups * i];
+    for (int s = 0; s < kSteps; s += 2) {
+      SplitB right[4];
+      load_block(vs + b * kTile + (own_keys * kSteps + s) * kBlock, right);
+      load_block(vs + b * kTile + (own_keys * kSteps + s + 1) * kBlock, right + 2);
+      float sums[4][4] = {};
+      mma_split(sums, {&left, &left, &left, &left}, right);
 #pragma unroll
-      for (int x = 0; x < 4; ++x) acc[i][x] *= alpha;
+      for (int n = 0; n < 4; ++n)
+#pragma unroll
+        for (int i = 0; i < 4; ++i) acc[2 * s + n][i] = fmaf(acc[2 * s + n][i], alpha[i >> 1], sums[n][i]);
     }
-    // Where some row does not see some key, such a key's value stays out even if it is not finite.
-    const bool whole = lo + (tile + 1) * kKeys - 1 <= first_pos && (p.window == 0 || lo + tile * kKeys >= last_pos - p.window + 1);
-    auto add_values = [&](auto masked) {
-#pragma unroll 4
-      for (int j = 0; j < kKeys; j += 4) {
-        float4 v[4];
+    if (spoilt[b][2 * own_keys] | spoilt[b][2 * own_keys + 1]) {  // what is not finite reaches the rows that see its key, and no others
+      for (int j = 0; j < 16; ++j) {
+        const int key = lo + tile * kKeys + own_keys * 16 + j;
+        const int64_t offset = offsets[b][own_keys * 16 + j];
+        if (offset < 0) continue;
 #pragma unroll
-        for (int x = 0; x < 4; ++x) v[x] = *reinterpret_cast<const float4*>(vs + (j + x) * kLd + cg * 4);
+        for (int x = 0; x < 2 * kSteps; ++x)
 #pragma unroll
-        for (int i = 0; i < kOwnRows; ++i) {
-          const float4 weight = *reinterpret_cast<const float4*>(ps + (rg + kRowGroups * i) * kLdP + j);
-          const float w[4] = {weight.x, weight.y, weight.z, weight.w};
-#pragma unroll
-          for (int x = 0; x < 4; ++x) {
-            if (decltype(masked)::value && __float_as_int(w[x]) < 0) continue;
-            acc[i][0] = fmaf(w[x], v[x].x, acc[i][0]), acc[i][1] = fmaf(w[x], v[x].y, acc[i][1]);
-            acc[i][2] = fmaf(w[x], v[x].z, acc[i][2]), acc[i][3] = fmaf(w[x], v[x].w, acc[i][3]);
+          for (int i = 0; i < 4; ++i) {
+            const int c = x * 8 + 2 * q + (i & 1), h = i >> 1;
+            if (c < p.head_dim && key <= pos[h] && key >= from[h] && !isfinite(p.values[offset + c])) acc[x][i] = NAN;
           }
-        }
       }
-    };
-    if (whole) add_values(std::false_type{});
-    else add_values(std::true_type{});
+    }
+    if (tile + 2 < tiles) arrive(kEmpty + b);
   }
-  __syncthreads();
-  if (tc == 0) {
+  // The four parts of the keys meet.
 #pragma unroll
-    for (int i = 0; i < 4; ++i) alphas[tr + 8 * i] = sum[i] > 0.f ? 1.f / sum[i] : 0.f;
+  for (int h = 0; h < 2; ++h) {
+    sum[h] += __shfl_xor_sync(0xffffffffu, sum[h], 1);
+    sum[h] += __shfl_xor_sync(0xffffffffu, sum[h], 2);
+    if (q == 0) tops[warp][g + 8 * h] = top[h], totals[warp][g + 8 * h] = sum[h];
   }
-  __syncthreads();
+  meet_own();  // the parts have been read too
+  float* os = reinterpret_cast<float*>(ks);  // [kWarps][16][kLdO]
+  static_assert(sizeof(float) * kWarps * 16 * kLdO <= sizeof(uint4) * 4 * kTile, "the warps' sums do not fit where keys and values were");
 #pragma unroll
-  for (int i = 0; i < kOwnRows; ++i) {
-    const int r = rg + kRowGroups * i;
-    if (r >= rows || cg * 4 >= p.head_dim) continue;
+  for (int x = 0; x < 2 * kSteps; ++x)
+#pragma unroll
+    for (int h = 0; h < 2; ++h)
+      *reinterpret_cast<float2*>(os + (warp * 16 + g + 8 * h) * kLdO + x * 8 + 2 * q) = make_float2(acc[x][2 * h], acc[x][2 * h + 1]);
+  meet_own();
+  for (int idx = tid; idx < rows * (DIM / 4); idx += kOwnThreads) {
+    const int r = idx / (DIM / 4), c = idx % (DIM / 4) * 4;
+    if (c >= p.head_dim) continue;
+    const int first = r / 16 * kKeyParts;
+    float whole_top = -INFINITY, total = 0.f;
+#pragma unroll
+    for (int w = 0; w < kKeyParts; ++w) whole_top = fmaxf(whole_top, tops[first + w][r % 16]);
+    float4 o = zero;
+#pragma unroll
+    for (int w = 0; w < kKeyParts; ++w) {
+      const float t = tops[first + w][r % 16], factor = t > -INFINITY ? expf(t - whole_top) : 0.f;
+      const float4 v = *reinterpret_cast<const float4*>(os + ((first + w) * 16 + r % 16) * kLdO + c);
+      total = fmaf(totals[first + w][r % 16], factor, total);
+      o.x = fmaf(v.x, factor, o.x), o.y = fmaf(v.y, factor, o.y), o.z = fmaf(v.z, factor, o.z), o.w = fmaf(v.w, factor, o.w);
+    }
+    const float inv = total > 0.f ? 1.f / total : 0.f;
     const int item = row0 + r, token = item / group, head = kvh * group + item % group;
-    const float inv = alphas[r];
-    *reinterpret_cast<float4*>(p.out + (static_cast<int64_t>(start + token) * p.q_heads + head) * p.head_dim + cg * 4) =
-        make_float4(acc[i][0] * inv, acc[i][1] * inv, acc[i][2] * inv, acc[i][3] * inv);
+    *reinterpret_cast<float4*>(p.out + (static_cast<int64_t>(start + token) * p.q_heads + head) * p.head_dim + c) = make_float4(o.x * inv, o.y * inv, o.z * inv, o.w * inv);
   }
 }
 

@@ -32,6 +32,7 @@
 #include <type_traits>
 
 #include "common.cuh"
+#include "split_mma.cuh"
 
 namespace {
 
@@ -94,9 +95,6 @@ struct Scratch {
   float* s;   // [chunks][heads][columns x rows]: what the values alone add, then the state in front of each chunk
 };
 
-// Of column g = lane / 4 of an operand B, the token (or row) of sixteen that stands there in tile t (of two): D's layout, in which lane q
-// has columns 2 q and 2 q + 1 of either tile, then gives it four neighbours, 4 q .. + 3.
-__device__ __forceinline__ int in_sixteen(int t, int g) { return 4 * (g >> 1) + 2 * t + (g & 1); }
 // Rows of sixteen are a warp's of the walk. y: by (sixteen rows, sixteen tokens, tile) the lanes' four rows of a token each.
 __device__ __forceinline__ int y_place(int token, int row) {
   const int g = (token & 12) / 2 + (token & 1), tile = token / 16 * 2 + (token >> 1 & 1);
@@ -110,52 +108,6 @@ __device__ __forceinline__ int kd_place(int token, int row) {
 // s: by (sixteen columns, sixteen rows, eight of the columns) the lanes' four rows of a column each.
 __device__ __forceinline__ int s_place(int col, int row, int rows) {
   return col / 16 * (16 * rows) + row / 16 * 256 + (col >> 3 & 1) * 128 + (col & 7) * 16 + (row & 15);
-}
-
-// --- products of 32-bit numbers on the tensor cores ----------------------------------------------------------------------------------
-//
-// A number is the sum of three bfloat16 ones, to its last bit: the nearest, the nearest to what is left, and the rest (8 + 8 + 8 bits). Of the
-// nine products of two such sums the six largest are taken; the others are below 2^-26 of the whole. Products of 8-bit numbers are exact in
-// 32 bits. The tensor core's own sums drop bits below the last, so few are chained: the five small products of a step of 16 first, the large
-// one last, and what is summed beyond one step is added with ordinary rounding. What is not finite becomes NaN.
-struct Split {  // two neighbouring numbers, packed
-  uint32_t part[3];
-};
-__device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
-  uint32_t d;
-  asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(d) : "f"(hi), "f"(lo));
-  return d;
-}
-__device__ __forceinline__ Split split_pair(float x, float y) {
-  Split out;
-#pragma unroll
-  for (int i = 0; i < 3; ++i) {
-    out.part[i] = pack_bf16(x, y);
-    if (i < 2) x -= __uint_as_float(out.part[i] << 16), y -= __uint_as_float(out.part[i] & 0xffff0000u);
-  }
-  return out;
-}
-// D[16][8] += A[16][16] B[16][8]. Of a lane (g = lane / 4, q = lane % 4), over the step's numbers along which is summed, in an order of
-// this file's own: it holds 4 q .. + 3 of them. A: row g 4q, + 1; row g + 8 likewise; row g 4q + 2, + 3; row g + 8 likewise. B: column g
-// 4q, + 1; 4q + 2, + 3. D: row g columns 2q, + 1; row g + 8 likewise.
-__device__ __forceinline__ void mma_bf16(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
-  asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
-      : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
-      : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
-}
-struct SplitA {  // a lane's share of A
-  uint32_t part[3][4];
-  __device__ __forceinline__ void set(int at, const Split& s) { part[0][at] = s.part[0], part[1][at] = s.part[1], part[2][at] = s.part[2]; }
-};
-struct SplitB {  // of B
-  Split lo, hi;
-  __device__ __forceinline__ SplitB() {}
-  __device__ __forceinline__ explicit SplitB(float4 v) : lo(split_pair(v.x, v.y)), hi(split_pair(v.z, v.w)) {}
-};
-__device__ __forceinline__ void mma_split(float (&d)[4], const SplitA& a, const SplitB& b) {
-  constexpr int order[6][2] = {{2, 0}, {0, 2}, {1, 1}, {1, 0}, {0, 1}, {0, 0}};
-#pragma unroll
-  for (int i = 0; i < 6; ++i) mma_bf16(d, a.part[order[i][0]], b.lo.part[order[i][1]], b.hi.part[order[i][1]]);
 }
 
 // --- what does not depend on the state -------------------------------------------------------------------------------------------
@@ -305,12 +257,7 @@ __device__ __forceinline__ void invert_halves(const float* l, float* inverse) {
 struct Columns {
   float4 v[2][2];
 };
-__device__ __forceinline__ SplitA split_columns(const float4 (&v)[2]) {
-  SplitA a;
-  a.set(0, split_pair(v[0].x, v[0].y)), a.set(1, split_pair(v[1].x, v[1].y));
-  a.set(2, split_pair(v[0].z, v[0].w)), a.set(3, split_pair(v[1].z, v[1].w));
-  return a;
-}
+__device__ __forceinline__ SplitA split_columns(const float4 (&v)[2]) { return split_rows(v[0], v[1]); }
 // The same of a triangle that all columns meet: its operands in parts, [tile][part][lane], made once.
 constexpr int kTriangle = 2 * 3 * 32;  // uint2 of sixteen rows by sixteen tokens
 __device__ __forceinline__ void pack_triangle(uint2* to, const float* m, int ld) {
@@ -350,7 +297,6 @@ __device__ __forceinline__ void times_rows(float4 (&to)[2], const SplitA& a, con
 __device__ __forceinline__ float4 minus(float4 a, float4 b) { return make_float4(a.x - b.x, a.y - b.y, a.z - b.z, a.w - b.w); }
 __device__ __forceinline__ float4 plus(float4 a, float4 b) { return make_float4(a.x + b.x, a.y + b.y, a.z + b.z, a.w + b.w); }
 
-__device__ __forceinline__ bool all_finite(float4 v) { return fmaf(v.x, 0.f, fmaf(v.y, 0.f, fmaf(v.z, 0.f, v.w * 0.f))) == 0.f; }
 // What is not finite must not reach the tokens in front of it by way of a zero in a triangle: it goes into the products as a zero, and the
 // tokens from it on are NaN behind them. Lowers `first` to the first such token of the lane's two columns in half h.
 __device__ __forceinline__ void take_out(float4 (&r)[2], int h, int2& first) {
