@@ -115,7 +115,7 @@ _SIGNATURES: dict[str, list] = {
     "b200_moe_sort": [c_void_p, c_int, c_int, c_int, c_int] + [c_void_p] * 4,
     "b200_moe_gate_up": [c_void_p] * 5 + [c_int] * 6 + [c_float, c_void_p, c_int, c_int, c_void_p],
     "b200_moe_down": [c_void_p] * 5 + [c_int] * 4 + [c_void_p, c_int, c_int, c_void_p],
-    "b200_moe_gather_rows": [c_void_p, c_void_p, c_int, c_int, c_int, c_void_p, c_void_p],
+    "b200_moe_gather_rows": [c_void_p] * 3 + [c_int] * 4 + [c_void_p] * 2,
     "b200_moe_product_tcgen05": [c_void_p] * 5 + [c_int] * 8 + [c_float, c_void_p, c_int, c_void_p, c_void_p],
     "b200_moe_combine": [c_void_p] * 4 + [c_int, c_void_p, c_void_p] + [c_int] * 4 + [c_void_p, c_int, c_void_p],
     "b200_squared_relu": [c_void_p, c_int64, c_int, c_void_p],

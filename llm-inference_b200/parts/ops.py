@@ -1429,7 +1429,7 @@ def moe_experts(
     ctx.lib.call("b200_moe_sort", ptr(ids), c_int(slots), c_int(experts), c_int(capacity), c_int(tile), ptr(place_slot), ptr(tile_expert), ptr(num_tiles), ctx.stream)
     if tall and choice == "auto" and bool(ctx.lib.lib.b200_moe_tcgen05_supported(width, ff)):
         sorted_rows = ctx.buffer("moe_sorted_rows", (capacity, width), per_token=False)
-        ctx.lib.call("b200_moe_gather_rows", ptr(h), ptr(place_slot), c_int(capacity), c_int(top), c_int(width), ptr(sorted_rows), ctx.stream)
+        ctx.lib.call("b200_moe_gather_rows", ptr(h), ptr(place_slot), ptr(num_tiles), c_int(tile), c_int(capacity), c_int(top), c_int(width), ptr(sorted_rows), ctx.stream)
         stages = c_int(int(ctx.options.get("moe_stages", 0)))
         ctx.lib.call(
             "b200_moe_product_tcgen05", ptr(w_gate_up), ptr(sorted_rows), ptr(place_slot), ptr(tile_expert), ptr(num_tiles), c_int(max_tiles),
