@@ -11,8 +11,9 @@
 // stage; four warps add up the accumulators, two of which take turns in TMEM. An output's sums are the same whatever the tile, so a row's result
 // does not depend on how many rows are in the call. Operands that are not finite make their row or column NaN.
 //
-// What bounds it: shared memory. Per stage at 128 x 128 the parts are 96 KB written and 192 KB read by the products, 2,300 cycles of an SM where
-// the tensor core needs 1,540; measured 3,290 (2,570 at 128 x 64). Two stages ahead in registers instead of one changed nothing.
+// What bounds it: what an SM takes out of L2, 48 KB a stage at 128 x 64 and 64 KB at 128 x 128. Of 34 us for 500 rows by 2,048 x 1,536, a form
+// that only fetches takes 25, the products and the taking apart the rest. Tried: two stages ahead in registers instead of one, no change; numbers by
+// cp.async and W's parts in TMEM, 36 us (17,920 rows of W, 2,048 of A: 858 against 716).
 // Every wait is bounded; a block that gives up sets the timeout bit, frees its TMEM and leaves.
 #include "common.cuh"
 
