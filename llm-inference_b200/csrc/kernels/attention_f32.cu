@@ -195,7 +195,7 @@ portion_attention_f32_kernel(const PortionParams p) {
       constexpr int kTogether = 2;
 #pragma unroll 1
       for (int s = 0; s < kSteps; s += kTogether) {
-        float sums[2 * kTogether][4] = {};
+        float sums[2 * kTogether][4];
         SplitA own[kTogether];
         SplitB right[2 * kTogether];
 #pragma unroll
@@ -207,7 +207,8 @@ portion_attention_f32_kernel(const PortionParams p) {
           }
           load_block(ks + b * kTile + (own_keys * kSteps + s + x) * kBlock, right + 2 * x);
         }
-        mma_split(sums, {&own[0], &own[0], &own[1], &own[1]}, right);
+#pragma unroll
+        for (int n = 0; n < 2 * kTogether; ++n) mma_split(sums[n], own[n / 2], right[n]);
 #pragma unroll
         for (int t = 0; t < 2; ++t)
 #pragma unroll
@@ -247,8 +248,9 @@ portion_attention_f32_kernel(const PortionParams p) {
       SplitB right[4];
       load_block(vs + b * kTile + (own_keys * kSteps + s) * kBlock, right);
       load_block(vs + b * kTile + (own_keys * kSteps + s + 1) * kBlock, right + 2);
-      float sums[4][4] = {};
-      mma_split(sums, {&left, &left, &left, &left}, right);
+      float sums[4][4];
+#pragma unroll
+      for (int n = 0; n < 4; ++n) mma_split(sums[n], left, right[n]);
 #pragma unroll
       for (int n = 0; n < 4; ++n)
 #pragma unroll

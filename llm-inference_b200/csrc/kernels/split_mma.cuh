@@ -33,6 +33,12 @@ __device__ __forceinline__ void mma_bf16(float (&d)[4], const uint32_t (&a)[4], 
       : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
       : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
+// D = A B.
+__device__ __forceinline__ void mma_bf16_fresh(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+  asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%10, %10, %10, %10};"
+      : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3])
+      : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1), "f"(0.f));
+}
 struct SplitA {  // a lane's share of A
   uint32_t part[3][4];
   __device__ __forceinline__ void set(int at, const Split& s) { part[0][at] = s.part[0], part[1][at] = s.part[1], part[2][at] = s.part[2]; }
@@ -49,18 +55,12 @@ struct SplitB {  // of B
   __device__ __forceinline__ SplitB() {}
   __device__ __forceinline__ explicit SplitB(float4 v) : lo(split_pair(v.x, v.y)), hi(split_pair(v.z, v.w)) {}
 };
+// d = a b, over sixteen numbers.
 __device__ __forceinline__ void mma_split(float (&d)[4], const SplitA& a, const SplitB& b) {
   constexpr int order[6][2] = {{2, 0}, {0, 2}, {1, 1}, {1, 0}, {0, 1}, {0, 0}};
+  mma_bf16_fresh(d, a.part[order[0][0]], b.lo.part[order[0][1]], b.hi.part[order[0][1]]);
 #pragma unroll
-  for (int i = 0; i < 6; ++i) mma_bf16(d, a.part[order[i][0]], b.lo.part[order[i][1]], b.hi.part[order[i][1]]);
-}
-// Four of them side by side, one product of each at a time, since a product waits for the one in front of it of the same sums.
-__device__ __forceinline__ void mma_split(float (&d)[4][4], const SplitA* const (&a)[4], const SplitB (&b)[4]) {
-  constexpr int order[6][2] = {{2, 0}, {0, 2}, {1, 1}, {1, 0}, {0, 1}, {0, 0}};
-#pragma unroll
-  for (int i = 0; i < 6; ++i)
-#pragma unroll
-    for (int n = 0; n < 4; ++n) mma_bf16(d[n], a[n]->part[order[i][0]], b[n].lo.part[order[i][1]], b[n].hi.part[order[i][1]]);
+  for (int i = 1; i < 6; ++i) mma_bf16(d, a.part[order[i][0]], b.lo.part[order[i][1]], b.hi.part[order[i][1]]);
 }
 
 // A product whose result is the next one's A has two tiles of eight columns for sixteen: the one that stands as column g = lane / 4 of tile t.

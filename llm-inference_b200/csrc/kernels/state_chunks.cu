@@ -205,7 +205,7 @@ __device__ __forceinline__ void pair_tile(const float* left0, const float* left1
   float acc[4] = {};
 #pragma unroll 1
   for (int step = 0; step < ROWS / 16; step += kTogether) {
-    float part[kTogether][4] = {};
+    float part[kTogether][4];
 #pragma unroll
     for (int x = 0; x < kTogether; ++x) {
       const int c = (step + x) * 16;
@@ -271,7 +271,7 @@ __device__ __forceinline__ void pack_triangle(uint2* to, const float* m, int ld)
 }
 __device__ __forceinline__ void times_triangle(float4 (&to)[2], const SplitA& a, const uint2* m) {
   const int lane = threadIdx.x & 31;
-  float part[2][4] = {};
+  float part[2][4];
 #pragma unroll
   for (int t = 0; t < 2; ++t) {
     SplitB b;
@@ -288,7 +288,7 @@ __device__ __forceinline__ void times_triangle(float4 (&to)[2], const SplitA& a,
 // a (sixteen columns by sixteen tokens) times the transposed sixteen rows of m, `ld` numbers apart.
 __device__ __forceinline__ void times_rows(float4 (&to)[2], const SplitA& a, const float* m, int ld) {
   const int lane = threadIdx.x & 31, g = lane >> 2, q = lane & 3;
-  float part[2][4] = {};
+  float part[2][4];
 #pragma unroll
   for (int t = 0; t < 2; ++t) mma_split(part[t], a, SplitB(*reinterpret_cast<const float4*>(m + in_sixteen(t, g) * ld + 4 * q)));
   to[0] = make_float4(part[0][0], part[0][1], part[1][0], part[1][1]);
@@ -769,7 +769,7 @@ linear_chunk_prepare_kernel(LinearRule in, const int* __restrict__ seq_q_start, 
     const SplitA left[2] = {split_columns(r.v[0]), split_columns(r.v[1])};
 #pragma unroll
     for (int block = 0; block < 2; ++block) {
-      float part[2][2][4] = {};  // [tile][half of the tokens]
+      float part[2][2][4];  // [tile][half of the tokens]
 #pragma unroll
       for (int t = 0; t < 2; ++t)
 #pragma unroll
@@ -938,10 +938,7 @@ chunk_walk_kernel(const int* __restrict__ seq_q_start, const int* __restrict__ s
       for (int t = 0; t < 2; ++t) left.set(2 * t, split_pair(s[t][0], s[t][1])), left.set(2 * t + 1, split_pair(s[t][2], s[t][3]));
       float acc[4][4];
 #pragma unroll
-      for (int t = 0; t < 4; ++t) {
-        acc[t][0] = acc[t][1] = acc[t][2] = acc[t][3] = 0.f;
-        mma_split(acc[t], left, SplitB(staged(chunk, t)));
-      }
+      for (int t = 0; t < 4; ++t) mma_split(acc[t], left, SplitB(staged(chunk, t)));
       __syncwarp();
 #pragma unroll
       for (int t = 0; t < 4; ++t)
@@ -982,10 +979,7 @@ chunk_walk_kernel(const int* __restrict__ seq_q_start, const int* __restrict__ s
         left.part[p][0] = word.x, left.part[p][1] = word.y, left.part[p][2] = word.z, left.part[p][3] = word.w;
       }
 #pragma unroll
-      for (int t = 0; t < 2; ++t) {
-        sum[t][h][0] = sum[t][h][1] = sum[t][h][2] = sum[t][h][3] = 0.f;
-        mma_split(sum[t][h], left, SplitB(staged(chunk, 4 + 2 * t + h)));
-      }
+      for (int t = 0; t < 2; ++t) mma_split(sum[t][h], left, SplitB(staged(chunk, 4 + 2 * t + h)));
     }
     const float4 ef = *reinterpret_cast<const float4*>(stage_of(chunk) + kDecaysAt + row0);
     const float decays[4] = {ef.x, ef.y, ef.z, ef.w};
@@ -1033,7 +1027,8 @@ chunk_out_kernel(const int* __restrict__ seq_q_start, const int* __restrict__ se
   const int columns = padded_columns(dv);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, q = lane & 3;
   const int col0 = blockIdx.z % tiles * COLS + warp * 32;  // columns col0 + 8 t + g in B, col0 + 8 t + 2 q, + 1 in D
-  const int state_steps = rows / 16, steps = state_steps + (WITH_U ? 2 : 0) + (WITH_V ? 2 : 0);
+  const int state_steps = rows / 16;
+  constexpr int kPairSteps = (WITH_U ? 2 : 0) + (WITH_V ? 2 : 0);
   wait_for_predecessor();
   if (den != nullptr && blockIdx.z % tiles == 0) {  // the normaliser read out as the state is: n . (e q) + the chunk's own pairs
     constexpr int kWarpTokens = C / (COLS / 32), kMost = kMaxLinearRows / 32;
@@ -1056,21 +1051,26 @@ chunk_out_kernel(const int* __restrict__ seq_q_start, const int* __restrict__ se
   }
   if (col0 >= columns) return;
   float4 left[4], right[4];
-  auto fetch = [&](int step) {
-    const bool in_state = step < state_steps, is_u = WITH_U && step < state_steps + 2;
-    const int half = (step - state_steps) & 1;  // of the chunk's tokens, behind the state
-    const float* from_left = in_state ? from.qt + place * C * rows + step * 16 : (is_u ? from.a : from.av) + place * C * C + half * 16;
-    const int ld = in_state ? rows : C;
+  const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+  const float* qt = from.qt + place * C * rows + g * rows + 4 * q;
+  const float* states = from.s + place * columns * rows + s_place(col0, 0, rows) + lane * 4;  // 8 t + g columns on, 16 rows 256 numbers on
+  auto fetch_state = [&](int step) {
 #pragma unroll
-    for (int r = 0; r < 4; ++r) left[r] = *reinterpret_cast<const float4*>(from_left + (8 * r + g) * ld + 4 * q);
+    for (int r = 0; r < 4; ++r) left[r] = *reinterpret_cast<const float4*>(qt + 8 * r * rows + step * 16);
+#pragma unroll
+    for (int t = 0; t < 4; ++t)
+      right[t] = col0 + 8 * t < columns ? *reinterpret_cast<const float4*>(states + t / 2 * 16 * rows + t % 2 * 128 + step * 256) : zero;
+  };
+  auto fetch_pairs = [&](bool is_u, int half) {  // sixteen of the chunk's tokens
+    const float* pairs = (is_u ? from.a : from.av) + place * C * C + half * 16;
+#pragma unroll
+    for (int r = 0; r < 4; ++r) left[r] = *reinterpret_cast<const float4*>(pairs + (8 * r + g) * C + 4 * q);
 #pragma unroll
     for (int t = 0; t < 4; ++t) {
-      const int col = col0 + 8 * t + g;
-      if (in_state || is_u) {
-        const float* at = in_state ? from.s + place * columns * rows + s_place(col, step * 16 + 4 * q, rows) : from.x + (place * columns + col) * C + half * 16 + 4 * q;
-        right[t] = col < columns ? *reinterpret_cast<const float4*>(at) : make_float4(0.f, 0.f, 0.f, 0.f);
+      const int col = col0 + 8 * t + g, token = half * 16 + 4 * q;
+      if (is_u) {
+        right[t] = col < columns ? *reinterpret_cast<const float4*>(from.x + (place * columns + col) * C + token) : zero;
       } else {
-        const int token = half * 16 + 4 * q;
         const float* at = v + (first + token) * v_ld + static_cast<int64_t>(head) * dv + col;
         const bool valid = col < dv;
         right[t] = make_float4(valid && token < n ? at[0] : 0.f, valid && token + 1 < n ? at[v_ld] : 0.f, valid && token + 2 < n ? at[2 * v_ld] : 0.f,
@@ -1083,43 +1083,46 @@ chunk_out_kernel(const int* __restrict__ seq_q_start, const int* __restrict__ se
   for (int m = 0; m < 2; ++m)
 #pragma unroll
     for (int t = 0; t < 4; ++t) acc[m][t][0] = acc[m][t][1] = acc[m][t][2] = acc[m][t][3] = 0.f;
-  int spoilt[4] = {C, C, C, C};  // the first token of a column whose U or V is not finite
-  bool any_spoilt = false;
-  fetch(0);
-  for (int step = 0; step < steps; ++step) {
-    const bool pairs = step >= state_steps;
-    const int half = (step - state_steps) & 1;
-    if (pairs) {
-      bool found = false;
-#pragma unroll
-      for (int t = 0; t < 4; ++t) {
-        if (all_finite(right[t])) continue;
-        float* numbers[4] = {&right[t].x, &right[t].y, &right[t].z, &right[t].w};
-#pragma unroll
-        for (int i = 3; i >= 0; --i)
-          if (!isfinite(*numbers[i])) *numbers[i] = 0.f, spoilt[t] = min(spoilt[t], half * 16 + 4 * q + i), found = true;
-      }
-      any_spoilt |= __any_sync(0xffffffffu, found);
-    }
-    SplitA a[2];
-#pragma unroll
-    for (int r = 0; r < 4; ++r) a[r >> 1].set(r & 1, split_pair(left[r].x, left[r].y)), a[r >> 1].set((r & 1) + 2, split_pair(left[r].z, left[r].w));
-    SplitB b[4] = {SplitB(right[0]), SplitB(right[1]), SplitB(right[2]), SplitB(right[3])};
-    if (step + 1 < steps) fetch(step + 1);
+  auto multiply = [&](int from_m, auto fetch_next) {  // tokens in front of 16 from_m are left out
+    const SplitA a[2] = {split_rows(left[0], left[1]), split_rows(left[2], left[3])};
+    const SplitB b[4] = {SplitB(right[0]), SplitB(right[1]), SplitB(right[2]), SplitB(right[3])};
+    fetch_next();
 #pragma unroll
     for (int m = 0; m < 2; ++m) {
-      if ((m == 0 && pairs && half == 1) || 16 * m >= n) continue;  // tokens behind, or none
+      if (m < from_m || 16 * m >= n) continue;
       float sum[4][4];
 #pragma unroll
-      for (int t = 0; t < 4; ++t) {
-        sum[t][0] = sum[t][1] = sum[t][2] = sum[t][3] = 0.f;
-        mma_split(sum[t], a[m], b[t]);
-      }
+      for (int t = 0; t < 4; ++t) mma_split(sum[t], a[m], b[t]);
 #pragma unroll
       for (int t = 0; t < 4; ++t)
 #pragma unroll
         for (int i = 0; i < 4; ++i) acc[m][t][i] += sum[t][i];
     }
+  };
+  fetch_state(0);
+  for (int step = 0; step < state_steps; ++step)
+    multiply(0, [&] {
+      if (step + 1 < state_steps) fetch_state(step + 1);
+      else fetch_pairs(WITH_U, 0);
+    });
+  int spoilt[4] = {C, C, C, C};  // the first token of a column whose U or V is not finite
+  bool any_spoilt = false;
+#pragma unroll 1
+  for (int pairs = 0; pairs < kPairSteps; ++pairs) {
+    const int half = pairs & 1;
+    bool found = false;
+#pragma unroll
+    for (int t = 0; t < 4; ++t) {
+      if (all_finite(right[t])) continue;
+      float* numbers[4] = {&right[t].x, &right[t].y, &right[t].z, &right[t].w};
+#pragma unroll
+      for (int i = 3; i >= 0; --i)
+        if (!isfinite(*numbers[i])) *numbers[i] = 0.f, spoilt[t] = min(spoilt[t], half * 16 + 4 * q + i), found = true;
+    }
+    any_spoilt |= __any_sync(0xffffffffu, found);
+    multiply(half, [&] {
+      if (pairs + 1 < kPairSteps) fetch_pairs(WITH_U && pairs + 1 < 2, (pairs + 1) & 1);
+    });
   }
   if (any_spoilt) {
 #pragma unroll
