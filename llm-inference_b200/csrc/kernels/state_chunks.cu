@@ -62,17 +62,17 @@ __device__ __forceinline__ void wait_copies() {
   asm volatile("cp.async.wait_group %0;" ::"n"(LEFT) : "memory");
 }
 
-// Rows `first .. first + n` of src [tokens][ld] from column `at` on, `width` numbers each, to dst [C][dst_ld], a warp per row; rows
-// past n and columns from `width` to `padded` become zeros. W numbers a copy.
-template <int W>
-__device__ __forceinline__ void stage_rows(float* dst, int dst_ld, const float* src, int64_t first, int n, int64_t ld, int64_t at, int width, int padded) {
-  const int lane = threadIdx.x & 31;
-  for (int r = threadIdx.x >> 5; r < C; r += kWarps) {
-    const float* from = src + (r < n ? (first + r) * ld + at : 0);
-    for (int c = lane * W; c < padded; c += 32 * W) {
-      const bool valid = r < n && c < width;
-      stage_copy<4 * W>(dst + r * dst_ld + c, valid ? from + c : src, valid);
-    }
+// n rows `from` [..][ld] of `width` numbers to dst [C][ROWS + 4]; rows past n and columns from `width` on become zeros. W numbers a copy.
+template <int ROWS, int W>
+__device__ __forceinline__ void stage_rows(float* dst, const float* from, int n, int64_t ld, int width) {
+  constexpr int kPerRow = ROWS / W, kAtOnce = kThreads / kPerRow;  // rows
+  const int r0 = threadIdx.x / kPerRow, c = threadIdx.x % kPerRow * W;
+  const float* at = from + r0 * ld + c;
+  float* to = dst + r0 * (ROWS + 4) + c;
+#pragma unroll
+  for (int i = 0; i < C / kAtOnce; ++i) {
+    const bool valid = r0 + i * kAtOnce < n && c < width;
+    stage_copy<4 * W>(to + i * kAtOnce * (ROWS + 4), valid ? at + i * kAtOnce * ld : from, valid);
   }
 }
 
@@ -410,9 +410,10 @@ chunk_prepare_kernel(const float* q, const float* k, const float* v, const float
   static_assert(6 * kTriangle + C * kLdT <= 2 * C * (C + 1), "the triangles do not fit where the pairs were");
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   wait_for_predecessor();
-  stage_rows<W>(ks, ld, k, first, n, static_cast<int64_t>(kv_heads) * dk, static_cast<int64_t>(kvh) * dk, dk, rows);
-  stage_rows<W>(qs, ld, q, first, n, static_cast<int64_t>(kv_heads) * dk, static_cast<int64_t>(kvh) * dk, dk, rows);
-  if (!PER_HEAD) stage_rows<W>(gs, ld, decay, first, n, static_cast<int64_t>(heads) * dk, static_cast<int64_t>(head) * dk, dk, rows);
+  const int64_t qk_ld = static_cast<int64_t>(kv_heads) * dk, qk_at = first * qk_ld + static_cast<int64_t>(kvh) * dk;
+  stage_rows<ROWS, W>(ks, k + qk_at, n, qk_ld, dk);
+  stage_rows<ROWS, W>(qs, q + qk_at, n, qk_ld, dk);
+  if (!PER_HEAD) stage_rows<ROWS, W>(gs, decay + (first * heads + head) * dk, n, static_cast<int64_t>(heads) * dk, dk);
   if (tid < C) bs[tid] = tid < n ? beta[(first + tid) * heads + head] : 0.f;
   commit_copies();
   wait_copies<0>();
@@ -599,15 +600,15 @@ linear_chunk_prepare_kernel(LinearRule in, const int* __restrict__ seq_q_start, 
   float* inverse = rk + 6 * kTriangle;                   // GENERAL: [C][kLdT], likewise
   float* front = gs;                                     // GENERAL: [groups][rows]: the decays in front of each group, behind the decays themselves
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, q = lane & 3;
-  const int64_t ld_in = in.ld, at_in = static_cast<int64_t>(head) * dk;
+  const int64_t at_in = first * in.ld + static_cast<int64_t>(head) * dk;
   const float* values = in.v + first * in.v_ld + static_cast<int64_t>(head) * dv;
   wait_for_predecessor();
-  stage_rows<W>(rs, ld, in.r, first, n, ld_in, at_in, dk, rows);
-  stage_rows<W>(ks, ld, in.k, first, n, ld_in, at_in, dk, rows);
-  if (!MEMORY) stage_rows<W>(gs, ld, in.w, first, n, ld_in, at_in, dk, rows);
+  stage_rows<ROWS, W>(rs, in.r + at_in, n, in.ld, dk);
+  stage_rows<ROWS, W>(ks, in.k + at_in, n, in.ld, dk);
+  if (!MEMORY) stage_rows<ROWS, W>(gs, in.w + at_in, n, in.ld, dk);
   if (GENERAL) {
-    stage_rows<W>(us, ld, in.u, first, n, ld_in, at_in, dk, rows);
-    stage_rows<W>(bb, ld, in.au, first, n, ld_in, at_in, dk, rows);
+    stage_rows<ROWS, W>(us, in.u + at_in, n, in.ld, dk);
+    stage_rows<ROWS, W>(bb, in.au + at_in, n, in.ld, dk);
   }
   commit_copies();
   wait_copies<0>();
@@ -1012,7 +1013,8 @@ chunk_walk_kernel(const int* __restrict__ seq_q_start, const int* __restrict__ s
 // --- outputs ---------------------------------------------------------------------------------------------------------------------------
 //
 // One block per (chunk, head, request and COLS columns), 32 columns a warp: O = Qt S (+ A U) (+ Av V) as one product over rows + 32 (+ 32)
-// numbers, 16 at a time, each lane's share of the operands straight from memory one step ahead. Pairs of tokens form a triangle: a token
+// numbers, 16 at a time, each lane's share of the operands straight from memory one step ahead (by asynchronous copies three steps ahead: 4 us
+// slower). Pairs of tokens form a triangle: a token
 // leaves out those behind it. What is not finite there times a pair's zero would not be zero, so it goes into the product as a zero, and the
 // tokens that it does reach are set to NaN behind it.
 template <int COLS, bool WITH_U, bool WITH_V>
