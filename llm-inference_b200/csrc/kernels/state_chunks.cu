@@ -190,11 +190,12 @@ __device__ __forceinline__ void pairs_in_group(const float* left, const float* r
   if (DIAGONAL && lane < 4) store(32 + lane, acc[32]);
 }
 
-// Tile `tile` of the pairs: rows of group gi of both left operands by rows of group gj <= gi of the right one into `to0` and `to1` [C][C + 1], by one
-// warp. DECAYS: gj < gi, rows carry their decays inside their own groups, `whole` holds the groups' decays multiplied.
-template <int ROWS, int LEFTS, bool DECAYS>
-__device__ __forceinline__ void pair_tile(const float* left0, const float* left1, const float* right, const float* whole, int tile, float* to0, float* to1) {
-  constexpr int ld = ROWS + 4, kTogether = 4;
+// Tile `tile` of the pairs: rows of group gi of both left operands by rows of group gj <= gi of RIGHTS right ones into `to` [left][right] [C][C + 1], by
+// one warp. DECAYS: gj < gi, rows carry their decays inside their own groups, `whole` holds the groups' decays multiplied.
+template <int ROWS, int LEFTS, int RIGHTS, bool DECAYS>
+__device__ __forceinline__ void pair_tile(const float* left0, const float* left1, const float* const (&right)[RIGHTS], const float* whole, int tile,
+                                          float* const (&to)[LEFTS][RIGHTS]) {
+  constexpr int ld = ROWS + 4, kTogether = 4 / RIGHTS;
   const int lane = threadIdx.x & 31, g = lane >> 2, q = lane & 3;
   int gi = 0;  // tiles (1, 0), (2, 0), (2, 1), .., or with (i, i) too
 #pragma unroll
@@ -202,35 +203,42 @@ __device__ __forceinline__ void pair_tile(const float* left0, const float* left1
   const int gj = tile - gi * (gi + 1) / 2;
   if (DECAYS) ++gi;
   const int at_left = (gi * kGroup + g) * ld + 4 * q, at_right = (gj * kGroup + g) * ld + 4 * q;
-  float acc[4] = {};
+  float acc[RIGHTS][4] = {};
 #pragma unroll 1
   for (int step = 0; step < ROWS / 16; step += kTogether) {
-    float part[kTogether][4];
+    float part[kTogether][RIGHTS][4];
 #pragma unroll
     for (int x = 0; x < kTogether; ++x) {
       const int c = (step + x) * 16;
-      SplitA a = {};
-      const float4 l0 = *reinterpret_cast<const float4*>(left0 + at_left + c);
-      a.set(0, split_pair(l0.x, l0.y)), a.set(2, split_pair(l0.z, l0.w));
-      if (LEFTS == 2) {
-        const float4 l1 = *reinterpret_cast<const float4*>(left1 + at_left + c);
-        a.set(1, split_pair(l1.x, l1.y)), a.set(3, split_pair(l1.z, l1.w));
-      }
-      float4 r = *reinterpret_cast<const float4*>(right + at_right + c);
+      const float4 none = make_float4(0.f, 0.f, 0.f, 0.f);
+      const SplitA a = split_rows(*reinterpret_cast<const float4*>(left0 + at_left + c), LEFTS == 2 ? *reinterpret_cast<const float4*>(left1 + at_left + c) : none);
+      float4 r[RIGHTS];
+#pragma unroll
+      for (int y = 0; y < RIGHTS; ++y) r[y] = *reinterpret_cast<const float4*>(right[y] + at_right + c);
       if (DECAYS) {
         for (int between = gj + 1; between < gi; ++between) {
           const float4 w = *reinterpret_cast<const float4*>(whole + between * ROWS + c + 4 * q);
-          r.x *= w.x, r.y *= w.y, r.z *= w.z, r.w *= w.w;
+#pragma unroll
+          for (int y = 0; y < RIGHTS; ++y) r[y].x *= w.x, r[y].y *= w.y, r[y].z *= w.z, r[y].w *= w.w;
         }
       }
-      mma_split(part[x], a, SplitB(r));
+#pragma unroll
+      for (int y = 0; y < RIGHTS; ++y) mma_split(part[x][y], a, SplitB(r[y]));
     }
 #pragma unroll
-    for (int i = 0; i < 4; ++i) acc[i] += (part[0][i] + part[1][i]) + (part[2][i] + part[3][i]);
+    for (int y = 0; y < RIGHTS; ++y)
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        if (kTogether == 4) acc[y][i] += (part[0][y][i] + part[1][y][i]) + (part[kTogether / 2][y][i] + part[kTogether - 1][y][i]);
+        else acc[y][i] += part[0][y][i] + part[kTogether - 1][y][i];
+      }
   }
   const int at = (gi * kGroup + g) * (C + 1) + gj * kGroup + 2 * q;
-  to0[at] = acc[0], to0[at + 1] = acc[1];
-  if (LEFTS == 2) to1[at] = acc[2], to1[at + 1] = acc[3];
+#pragma unroll
+  for (int y = 0; y < RIGHTS; ++y) {
+    to[0][y][at] = acc[y][0], to[0][y][at + 1] = acc[y][1];
+    if (LEFTS == 2) to[LEFTS - 1][y][at] = acc[y][2], to[LEFTS - 1][y][at + 1] = acc[y][3];
+  }
 }
 
 // (I + l)^-1 of both halves of sixteen tokens on the diagonal of l [C][C], to `inverse` [C][kLdT], by one warp: a lane per column.
@@ -366,13 +374,23 @@ __device__ __forceinline__ void store_x(float* x, const Columns& r) {
 // Columns c0 .. + 15 of the chunk's values: rows v + token * ld, zeros past n tokens and dv columns.
 __device__ __forceinline__ Columns load_values(const float* v, int64_t ld, int c0, int dv, int n) {
   const int lane = threadIdx.x & 31, g = lane >> 2, q = lane & 3;
+  const float* base = v + 4 * q * ld + c0 + g;
   Columns r;
+  if (n == C && c0 + 16 <= dv) {
+#pragma unroll
+    for (int h = 0; h < 2; ++h)
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int c = 0; c < 2; ++c) (&r.v[h][c].x)[i] = base[(h * 16 + i) * ld + 8 * c];
+    return r;
+  }
 #pragma unroll
   for (int h = 0; h < 2; ++h)
 #pragma unroll
     for (int c = 0; c < 2; ++c) {
       const int token = h * 16 + 4 * q, column = c0 + g + 8 * c;
-      const float* at = v + token * ld + column;
+      const float* at = base + h * 16 * ld + 8 * c;
       r.v[h][c] = make_float4(column < dv && token < n ? at[0] : 0.f, column < dv && token + 1 < n ? at[ld] : 0.f,
                               column < dv && token + 2 < n ? at[2 * ld] : 0.f, column < dv && token + 3 < n ? at[3 * ld] : 0.f);
     }
@@ -419,7 +437,7 @@ chunk_prepare_kernel(const float* q, const float* k, const float* v, const float
   wait_copies<0>();
   __syncthreads();
   if (PER_HEAD) {
-    for (int tile = warp; tile < kTiles; tile += kWarps) pair_tile<ROWS, 2, false>(ks, qs, ks, nullptr, tile, kk, qk);
+    for (int tile = warp; tile < kTiles; tile += kWarps) pair_tile<ROWS, 2, 1, false>(ks, qs, {ks}, nullptr, tile, {{kk}, {qk}});
   } else {
     if (warp < kGroups) pairs_in_group<ROWS, false, false>(ks, ks, gs, warp, kk);
     else pairs_in_group<ROWS, false, true>(qs, ks, gs, warp - kGroups, qk);
@@ -445,7 +463,7 @@ chunk_prepare_kernel(const float* q, const float* k, const float* v, const float
       }
     }
     __syncthreads();
-    if (warp < kBetween) pair_tile<ROWS, 2, true>(ks, qs, gs, whole, warp, kk, qk);
+    if (warp < kBetween) pair_tile<ROWS, 2, 1, true>(ks, qs, {gs}, whole, warp, {{kk}, {qk}});
   }
   __syncthreads();
   float* a = to.a + place * C * C + lane;
@@ -614,7 +632,7 @@ linear_chunk_prepare_kernel(LinearRule in, const int* __restrict__ seq_q_start, 
   wait_copies<0>();
   __syncthreads();
   if (MEMORY) {
-    for (int tile = warp; tile < kTiles; tile += kWarps) pair_tile<ROWS, 1, false>(rs, nullptr, ks, nullptr, tile, rk, nullptr);
+    for (int tile = warp; tile < kTiles; tile += kWarps) pair_tile<ROWS, 1, 1, false>(rs, nullptr, {ks}, nullptr, tile, {{rk}});
     __syncthreads();
     // Column j = lane: the keeps of tokens j + 1 .. i multiplied, from one at i = j on.
     const int64_t at = (first + lane) * heads + head;
@@ -676,13 +694,9 @@ linear_chunk_prepare_kernel(LinearRule in, const int* __restrict__ seq_q_start, 
       }
     }
     __syncthreads();
-    if (GENERAL) {
-      for (int tile = warp; tile < 2 * kBetween; tile += kWarps) {
-        const bool second = tile >= kBetween;
-        pair_tile<ROWS, 2, true>(us, rs, second ? bb : ks, whole, second ? tile - kBetween : tile, second ? ub : uk, second ? rb : rk);
-      }
-    } else if (warp < kBetween) {
-      pair_tile<ROWS, 1, true>(rs, nullptr, ks, whole, warp, rk, nullptr);
+    if (warp < kBetween) {
+      if constexpr (GENERAL) pair_tile<ROWS, 2, 2, true>(us, rs, {ks, bb}, whole, warp, {{uk, ub}, {rk, rb}});
+      else pair_tile<ROWS, 1, 1, true>(rs, nullptr, {ks}, whole, warp, {{rk}});
     }
     __syncthreads();
     for (int i = warp; i < C; i += kWarps) {
