@@ -27,8 +27,8 @@
 // cost it no digits.
 //
 // Measured on a B200 (one request of 2,048 tokens, all three kernels; FMAs throughout, now): heads of 128 x 128, a decay per channel, 12 of them
-// 230 -> 152 us (prepare 60 -> 43, walk 135 -> 80, out 35 -> 30), 28 of them 430 -> 277; one decay per head 228 -> 152; 24 heads of 64 x 64 under the
-// generalized rule 229 -> 162 us (prepare 97 -> 77, walk 91 -> 55, out 35 -> 27), without a removal 87 -> 72.
+// 230 -> 148 us (prepare 60 -> 41, walk 135 -> 80, out 35 -> 22), 28 of them 430 -> 273; one decay per head 228 -> 149; 24 heads of 64 x 64 under the
+// generalized rule 229 -> 145 us (prepare 97 -> 64, walk 91 -> 55, out 35 -> 21), without a removal 87 -> 68.
 #include <type_traits>
 
 #include "common.cuh"
@@ -121,11 +121,11 @@ __device__ __forceinline__ int s_place(int col, int row, int rows) {
 // Columns of [e K | V]: (I + L) X = R in halves of sixteen tokens, X1 = T11 R1, X2 = T22 (R2 - L21 X1), with the two halves' inverses made
 // by a warp, a lane per column; transposed (X^T = R^T T^T, sixteen columns a warp at a time), every result is the next product's operand in
 // the lanes that hold it.
-// What bounds it: instructions (24,000 a warp's worth for a chunk of a head of 128 x 128) and the barriers between its seven phases, three blocks
+// What bounds it: instructions (some 20,000 of a warp for a chunk of a head of 128 x 128) and the barriers between its seven phases, three blocks
 // an SM. With operands of pairs out of shared memory for every FMA, a thread per column of the triangular system and sums of the warps
 // through shared memory, two blocks an SM waited for shared memory most of the time: 2,048 tokens of 12 heads of 128 x 128, a decay per channel 60 ->
-// 43 us, one per head 56 -> 39; 24 heads of 64 x 64, the generalized rule 97 -> 77, the rule without a removal 54 -> 39. Two blocks an SM
-// with the same code: 50, 47, 87 and 47.
+// 41 us, one per head 56 -> 39; 24 heads of 64 x 64, the generalized rule 97 -> 64, the rule without a removal 54 -> 37. (A first form of this one
+// with two blocks an SM: 50, 47, 87 and 47; with three: 43, 39, 77 and 39.)
 constexpr int kGroup = 8, kGroups = C / kGroup;
 constexpr int kBetween = 6;             // pairs of different groups
 constexpr int kTiles = kBetween + kGroups;  // and of a group with itself
