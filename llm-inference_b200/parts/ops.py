@@ -993,8 +993,9 @@ def delta_prepare(
 
 
 # Longest portion that is walked token by token. The recurrences alone, one request, 12 heads of 128 x 128 on a B200, chunks against
-# tokens: 49 and 39 us at 64 tokens, 53 and 52 us at 100, 64 and 87 us at 200, 252 and 731 us at 2,048 (one decay per head within 4 us of
-# the same). A whole mixer called by itself, whose launches bound it at these sizes, with chunks and with tokens: one decay per channel 98
+# tokens: 49 and 39 us at 64 tokens, 53 and 52 us at 100, 64 and 87 us at 200, 148 and 731 us at 2,048 (one decay per head within 4 us of
+# the same). The chunks' figures, here and below, are of their form in 32-bit FMAs, except those at 2,048 tokens of the two delta rules and
+# the generalized one, which are of the form on the tensor cores; the lines were left where they were. A whole mixer called by itself, whose launches bound it at these sizes, with chunks and with tokens: one decay per channel 98
 # and 121 us at 116 tokens, one per head 81 and 75 at 116, 84 and 90 at 160. Beside decoded tokens, which are walked either way, the lines
 # lie at the same lengths: with 63 of them chunks and tokens take 161 and 158 us at 100 tokens and 162 and 174 at 128 (one decay per
 # channel), 147 and 152 at 128 and 157 and 167 at 160 (one per head). Decoded tokens inside the chunks' grids cost more than the
@@ -1008,7 +1009,7 @@ HEAD_DELTA_CHUNK_FROM = 128
 # four launches instead of one bind it, 122 and 140 at 64, 135 and 143 at 100, 139 and 141 at 120, 145 and 140 at 141 (32 heads: 134 and 141
 # at 100, 140 and 141 at 120, 145 and 142 at 141). The line lies where a call by itself breaks even; a step of a whole model that waits for
 # the host (one prompt of up to 400 tokens in a model of 1B) pays each layer in chunks with two further launches, 10 us. Generalized delta rule: 61 and 62 us at
-# 200 tokens in chunks and token by token, 244 and 473 at 2,048; the whole mixer 104 and 91 at 200, 104 and 96 at 230.
+# 200 tokens in chunks and token by token, 145 and 473 at 2,048; the whole mixer 104 and 91 at 200, 104 and 96 at 230.
 LINEAR_CHUNK_FROM = 120
 GENERAL_DELTA_CHUNK_FROM = 256
 # The matrix memory, one request, 12 heads of 128 x 128, with its gates and its output: 55 us in chunks and 53 token by token at 160
