@@ -993,33 +993,35 @@ def delta_prepare(
 
 
 # Longest portion that is walked token by token. The recurrences alone, one request, 12 heads of 128 x 128 on a B200, chunks against
-# tokens: 49 and 39 us at 64 tokens, 53 and 52 us at 100, 64 and 87 us at 200, 148 and 731 us at 2,048 (one decay per head within 4 us of
-# the same). The chunks' figures, here and below, are of their form in 32-bit FMAs, except those at 2,048 tokens of the two delta rules and
-# the generalized one, which are of the form on the tensor cores; the lines were left where they were. A whole mixer called by itself, whose launches bound it at these sizes, with chunks and with tokens: one decay per channel 98
-# and 121 us at 116 tokens, one per head 81 and 75 at 116, 84 and 90 at 160. Beside decoded tokens, which are walked either way, the lines
-# lie at the same lengths: with 63 of them chunks and tokens take 161 and 158 us at 100 tokens and 162 and 174 at 128 (one decay per
-# channel), 147 and 152 at 128 and 157 and 167 at 160 (one per head). Decoded tokens inside the chunks' grids cost more than the
-# portion: 200 of them beside 512 tokens 732 us a layer, walked in front of the chunks 370, all token by token 543.
+# tokens: 25 and 29 us at 64 tokens, 31 and 44 us at 100, 32 and 84 us at 200, 146 and 839 us at 2,048 (one decay per head 26 and
+# 28, 29 and 39, 34 and 71, 148 and 647). A whole mixer called by itself, whose launches bound it at these sizes, with chunks and with tokens: one decay per channel 102
+# and 91 us at 100 tokens, 102 and 120 at 160, one per head 84 and 74 at 100, 85 and 111 at 230. Beside decoded tokens, which are walked either way, the lines
+# lie at the same lengths: with 63 of them chunks and tokens take 165 and 170 us at 120 tokens and 186 and 372 at 512 (one decay per
+# channel), 149 and 149 at 120 and 178 and 328 at 512 (one per head). Decoded tokens inside the chunks' grids cost more than the
+# portion: 200 of them beside 512 tokens twice a layer's time (732 us against 370, walked in front of the chunks; now 343, all token by token 507).
 DELTA_CHUNK_FROM = 112
 HEAD_DELTA_CHUNK_FROM = 128
 
 
 # The same for the rules in which the values enter as they are, one request, 24 heads of 64 x 64. Without a removal the whole mixer, tokens
-# and chunks: on the device 52 and 48 us at 64 tokens, 64 and 55 at 100, 69 and 56 at 120, 88 and 59 at 180; called by itself, when the host's
+# and chunks: on the device 54 and 49 us at 64 tokens, 67 and 55 at 100, 74 and 54 at 128, 86 and 59 at 160; called by itself, when the host's
 # four launches instead of one bind it, 122 and 140 at 64, 135 and 143 at 100, 139 and 141 at 120, 145 and 140 at 141 (32 heads: 134 and 141
 # at 100, 140 and 141 at 120, 145 and 142 at 141). The line lies where a call by itself breaks even; a step of a whole model that waits for
-# the host (one prompt of up to 400 tokens in a model of 1B) pays each layer in chunks with two further launches, 10 us. Generalized delta rule: 61 and 62 us at
-# 200 tokens in chunks and token by token, 145 and 473 at 2,048; the whole mixer 104 and 91 at 200, 104 and 96 at 230.
+# the host (one prompt of up to 400 tokens in a model of 1B) pays each layer in chunks with two further launches, 10 us. Generalized delta rule: 33 and 47 us at
+# 200 tokens in chunks and token by token, 145 and 450 at 2,048; the whole mixer called by itself 108 and 99 at 200, 107 and 97 at 230, 109 and
+# 108 at 300.
 LINEAR_CHUNK_FROM = 120
 GENERAL_DELTA_CHUNK_FROM = 256
-# The matrix memory, one request, 12 heads of 128 x 128, with its gates and its output: 55 us in chunks and 53 token by token at 160
-# tokens, 56 and 54 at 200, 63 and 107 at 512, 219 and 579 at 2,048; the whole mixer 67 and 64 at 230 tokens of 12 heads, 79 and 84 at 300 in
-# two requests.
+# The matrix memory, one request, 12 heads of 128 x 128, with its gates and its output: 41 us in chunks and 52 token by token at 160
+# tokens, 42 and 51 at 200, 49 and 106 at 512, 150 and 579 at 2,048; the whole mixer 57 and 53 at 160 tokens of 12 heads, 58 and 61 at 200, 58
+# and 64 at 230. It would begin to gain at 200; the line was drawn when chunks came level at 250.
 MEMORY_CHUNK_FROM = 256
-# Both of these rules' steps token by token are short, so where enough (request, head) chains stand side by side to fill the SMs, chunks come
-# level only in longer portions. Whole mixers, tokens and chunks: generalized rule, 24 heads, requests of 300 tokens: 4 of them 189 and 198 us,
-# 8 318 and 340, 13 479 and 517; of 512: 4 of them 301 and 294, 8 530 and 532; one of 300 with 80 heads 245 and 241. Matrix memory, 12 heads, of
-# 300: 4 of them 200 and 158, 8 287 and 308, 13 422 and 488; 8 of 512 471 and 470; of 300 with 40 heads: one 213 and 197, 8 1,135 and 1,232.
+# Both of these rules' steps token by token are short, so where enough (request, head) chains stand side by side to fill the SMs, chunks
+# gain less. Whole mixers, tokens and chunks: generalized rule, 24 heads, requests of 130 tokens: 16 of them 266 and 246 us; of 300: 4 of them
+# 189 and 148, 8 318 and 254, 13 480 and 390; of 512: 4 of them 300 and 217, 8 530 and 401; of 300 with 80 heads: one 247 and 195, 8 1,241 and
+# 1,083. Matrix memory, 12 heads, of 130: 16 of them 247 and 229; of 300: 4 of them 209 and 126, 8 290 and 238, 13 424 and 405; 8 of 512 472 and
+# 370; of 300 with 40 heads: one 213 and 159, 8 1,113 and 1,045. The line is where chunks in 32-bit FMAs came level; on the tensor cores they
+# would gain from 300 on.
 MANY_CHAINS, MANY_CHAINS_CHUNK_FROM = 96, 512
 # Scratch grows with the step's tokens (0.13 MB a token at 28 heads of 128 x 128): past this a step takes its heads in parts, and past so
 # many parts it walks its portions token by token, as if they were short, in the memory that takes.
