@@ -221,12 +221,11 @@ portion_attention_f32_kernel(const PortionParams p) {
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
       float best = -INFINITY;
-      bool seen[4];
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
         const int key = key0 + i;
-        seen[i] = key <= pos[h] && key >= from[h] && own_offsets[i] >= 0;
-        weight[h][i] = seen[i] ? score[i >> 1][2 * h + (i & 1)] * p.scale : -INFINITY;
+        const bool seen = key <= pos[h] && key >= from[h] && own_offsets[i] >= 0;
+        weight[h][i] = seen ? score[i >> 1][2 * h + (i & 1)] * p.scale : -INFINITY;
         best = fmaxf(best, weight[h][i]);
       }
       best = fmaxf(best, __shfl_xor_sync(0xffffffffu, best, 1));
@@ -236,7 +235,7 @@ portion_attention_f32_kernel(const PortionParams p) {
       float more = 0.f;
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
-        weight[h][i] = seen[i] && new_top > -INFINITY ? expf(weight[h][i] - new_top) : 0.f;
+        weight[h][i] = weight[h][i] != -INFINITY ? expf(weight[h][i] - new_top) : 0.f;  // a score that is NaN stays, also where no other is seen
         more += weight[h][i];
       }
       sum[h] = fmaf(sum[h], alpha[h], more);

@@ -80,3 +80,41 @@ def test_a_bad_page_is_flagged_and_not_read():
     view = CacheView(0, True, arena, arena, torch.tensor([[1, 9]], dtype=torch.int32, device="cuda"), 3, 2, 64, 0)
     out = ops.portion_attention_f32(ctx, view, q, torch.empty_like(q), 1, 1, 16, 0.25, first_seq=0)
     assert int(ctx.err.item()) == 1 and torch.isfinite(out).all()
+
+
+def attend_one_request(q, keys, values, heads, dim, decode=0):
+    """One request's tokens, all new, one kv head a query head; rows of keys and values in pages of 32."""
+    from llm_inference_b200.cli.microbench import make_ctx
+    from llm_inference_b200.parts import ops
+    from llm_inference_b200.parts.context import CacheView
+
+    n, page = q.shape[0], 32
+    pages = -(-n // page)
+    arenas = [torch.zeros(pages, heads, page, dim, device="cuda") for _ in range(2)]
+    for arena, rows in zip(arenas, (keys, values)):
+        padded = torch.zeros(pages * page, heads, dim, device="cuda")
+        padded[:n] = rows
+        arena.copy_(padded.view(pages, page, heads, dim).transpose(1, 2))
+    ctx = make_ctx(list(range(n)), [0] * n, [0], [n])
+    view = CacheView(0, True, *arenas, torch.arange(pages, dtype=torch.int32, device="cuda")[None], pages, pages, page, 0)
+    rows = q.reshape(n, -1).contiguous()
+    out = ops.portion_attention_f32(ctx, view, rows, torch.full_like(rows, 7.0), heads, heads, dim, dim**-0.5, first_seq=0)
+    assert int(ctx.err.item()) == 0
+    return out.view(n, heads, dim)
+
+
+@pytest.mark.parametrize("operand", ["q", "k"])
+@pytest.mark.parametrize("at", [0, 16, 17, 48, 90])
+@pytest.mark.parametrize("dim", [64, 128])
+def test_a_score_that_is_nan_reaches_its_row(operand, at, dim):
+    """Also where it is the only one that a row has of its sixteen keys (tokens 0, 16 and 48), or all of a row's scores are."""
+    torch.manual_seed(at)
+    n, heads = 100, 2
+    operands = dict(q=torch.randn(n, heads, dim, device="cuda"), k=torch.randn(n, heads, dim, device="cuda"), v=torch.randn(n, heads, dim, device="cuda"))
+    clean = attend_one_request(*operands.values(), heads, dim)
+    operands[operand][at, 1, 3] = float("nan")
+    got = attend_one_request(*operands.values(), heads, dim)
+    reached = torch.zeros(n, heads, dtype=torch.bool, device="cuda")
+    reached[at : at + 1 if operand == "q" else n, 1] = True
+    assert torch.isnan(got[reached]).all()
+    assert torch.equal(got[~reached], clean[~reached])
