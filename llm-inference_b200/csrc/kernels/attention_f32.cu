@@ -66,9 +66,49 @@ __device__ __forceinline__ void load_block(const uint4* from, SplitB* to) {
   }
 }
 
+// One row by one warp, of the numbers themselves, a lane a key and then four of the row's numbers: where a product of parts is not finite, an
+// infinite operand (whose parts are NaN) or a number next to the largest may be the reason, and the row may be finite, or infinite.
+__device__ __noinline__ void attend_row(const PortionParams& p, int seq, int kvh, int token, int head, int pos) {
+  const int lane = threadIdx.x & 31, from = p.window > 0 ? max(0, pos - p.window + 1) : 0;
+  const float* own = p.q + (static_cast<int64_t>(token) * p.q_heads + head) * p.head_dim;
+  const int* table = p.block_table + static_cast<int64_t>(seq) * p.max_pages;
+  float top = p.sink != nullptr ? p.sink[head] : -INFINITY, sum = p.sink != nullptr ? 1.f : 0.f;
+  float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+  for (int key0 = from; key0 <= pos; key0 += 32) {
+    const int key = key0 + lane, logical = key / p.page_size;
+    const int page = key <= pos && logical < p.max_pages ? table[logical] : -1;
+    const int64_t offset = page >= 0 && page < p.num_pages ? kv_row_offset(page, kvh, key % p.page_size, p.kv_heads, p.page_size, p.head_dim) : -1;
+    float score = -INFINITY;
+    if (offset >= 0) {
+      score = 0.f;
+      for (int c = 0; c < p.head_dim; ++c) score = fmaf(own[c], p.keys[offset + c], score);
+      score *= p.scale;
+    }
+    float best = score;
+    for (int o = 16; o > 0; o >>= 1) best = fmaxf(best, __shfl_xor_sync(0xffffffffu, best, o));
+    const float new_top = fmaxf(top, best), alpha = top > -INFINITY ? expf(top - new_top) : 0.f;
+    const float weight = score != -INFINITY ? expf(score - new_top) : 0.f;
+    float more = weight;
+    for (int o = 16; o > 0; o >>= 1) more += __shfl_xor_sync(0xffffffffu, more, o);
+    sum = fmaf(sum, alpha, more);
+    top = new_top;
+    acc = make_float4(acc.x * alpha, acc.y * alpha, acc.z * alpha, acc.w * alpha);
+    for (int j = 0; j < 32; ++j) {
+      const int64_t at = __shfl_sync(0xffffffffu, offset, j);
+      const float w = __shfl_sync(0xffffffffu, weight, j);
+      if (at < 0 || lane * 4 >= p.head_dim) continue;
+      const float4 v = *reinterpret_cast<const float4*>(p.values + at + lane * 4);
+      acc = make_float4(fmaf(w, v.x, acc.x), fmaf(w, v.y, acc.y), fmaf(w, v.z, acc.z), fmaf(w, v.w, acc.w));
+    }
+  }
+  const float inv = sum > 0.f ? 1.f / sum : 0.f;
+  if (lane * 4 < p.head_dim)
+    *reinterpret_cast<float4*>(p.out + (static_cast<int64_t>(token) * p.q_heads + head) * p.head_dim + lane * 4) = make_float4(acc.x * inv, acc.y * inv, acc.z * inv, acc.w * inv);
+}
+
 template <int DIM>
 __global__ void __launch_bounds__(kThreads, 1)
-portion_attention_f32_kernel(const PortionParams p) {
+portion_attention_f32_kernel(const __grid_constant__ PortionParams p) {
   extern __shared__ __align__(16) uint4 attention_smem[];
   constexpr int kSteps = DIM / 16;                        // sixteens of a head's numbers
   constexpr int kTile = kKeyParts * kSteps * kBlock;      // of keys, or of values
@@ -287,6 +327,8 @@ portion_attention_f32_kernel(const PortionParams p) {
     for (int h = 0; h < 2; ++h)
       *reinterpret_cast<float2*>(os + (warp * 16 + g + 8 * h) * kLdO + x * 8 + 2 * q) = make_float2(acc[x][2 * h], acc[x][2 * h + 1]);
   meet_own();
+  static_assert(32 % (DIM / 4) == 0, "a row's numbers are those of one warp");
+  uint32_t odd = 0;  // rows with a result that is not finite
   for (int idx = tid; idx < rows * (DIM / 4); idx += kOwnThreads) {
     const int r = idx / (DIM / 4), c = idx % (DIM / 4) * 4;
     if (c >= p.head_dim) continue;
@@ -304,7 +346,15 @@ portion_attention_f32_kernel(const PortionParams p) {
     }
     const float inv = total > 0.f ? 1.f / total : 0.f;
     const int item = row0 + r, token = item / group, head = kvh * group + item % group;
-    *reinterpret_cast<float4*>(p.out + (static_cast<int64_t>(start + token) * p.q_heads + head) * p.head_dim + c) = make_float4(o.x * inv, o.y * inv, o.z * inv, o.w * inv);
+    o = make_float4(o.x * inv, o.y * inv, o.z * inv, o.w * inv);
+    if (!all_finite(o)) odd |= 1u << r;
+    *reinterpret_cast<float4*>(p.out + (static_cast<int64_t>(start + token) * p.q_heads + head) * p.head_dim + c) = o;
+  }
+  odd = __reduce_or_sync(0xffffffffu, odd);
+  for (; odd != 0; odd &= odd - 1) {
+    const int item = row0 + __ffs(odd) - 1;
+    __syncwarp();
+    attend_row(p, seq, kvh, start + item / group, kvh * group + item % group, begin + item / group);
   }
 }
 

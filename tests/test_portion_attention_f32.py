@@ -118,3 +118,30 @@ def test_a_score_that_is_nan_reaches_its_row(operand, at, dim):
     reached[at : at + 1 if operand == "q" else n, 1] = True
     assert torch.isnan(got[reached]).all()
     assert torch.equal(got[~reached], clean[~reached])
+
+
+@pytest.mark.parametrize("operand,value", [("q", "inf"), ("k", "inf"), ("k", "-inf"), ("v", "inf"), ("v", "-inf"), ("k", "3.4e38"), ("k", "-3.4e38")])
+@pytest.mark.parametrize("at", [0, 16, 31, 75])
+@pytest.mark.parametrize("dim", [24, 128])
+def test_infinite_and_very_large_numbers(operand, value, at, dim):
+    """As 32-bit products and sums have them: signs of infinities, keys that an infinite score takes out, numbers next to the largest."""
+    torch.manual_seed(at + dim)
+    n, heads = 90, 2
+    operands = dict(q=0.3 * torch.randn(n, heads, dim, device="cuda"), k=torch.randn(n, heads, dim, device="cuda"), v=torch.randn(n, heads, dim, device="cuda"))
+    clean = attend_one_request(*operands.values(), heads, dim)
+    operands[operand][at, 1, 5] = float(value)
+    q, k, v = (x.double().transpose(0, 1) for x in operands.values())
+    scores = (q @ k.transpose(1, 2)).float().double() * dim**-0.5  # very large sums overflow 32 bits
+    want = torch.zeros(n, heads, dim, dtype=torch.float64, device="cuda")
+    for t in range(n):
+        seen = scores[:, t, : t + 1]
+        weights = torch.where(seen == -float("inf"), 0.0, torch.exp(seen - seen.max(-1, keepdim=True).values))
+        total = weights.sum(-1, keepdim=True)
+        want[t] = (weights[..., None] * v[:, : t + 1]).sum(1) * torch.where(total > 0, 1 / total, 0.0)
+    got = attend_one_request(*operands.values(), heads, dim).double()
+    assert torch.equal(torch.isnan(got), torch.isnan(want)) and torch.equal(torch.isinf(got), torch.isinf(want))
+    assert torch.equal(got[torch.isinf(want)], want[torch.isinf(want)])
+    finite = torch.isfinite(want)
+    close = 3e-5 + 3e-5 * want[finite].abs()  # as for the portions above
+    assert ((got[finite] - want[finite]).abs() <= close).all()
+    assert torch.equal(got[:at], clean[:at].double())
