@@ -3,7 +3,8 @@
 // A number is the sum of three bfloat16 ones, to its last bit: the nearest, the nearest to what is left, and the rest (8 + 8 + 8 bits). Of the
 // nine products of two such sums the six largest are taken; the others are below 2^-26 of the whole. Products of 8-bit numbers are exact in
 // 32 bits. The tensor core's own sums drop bits below the last, so few are chained: the five small products of a step of 16 first, the large
-// one last, and what is summed beyond one step is added with ordinary rounding. What is not finite becomes NaN.
+// one last, and what is summed beyond one step is added with ordinary rounding. What is not finite becomes NaN;
+// the largest numbers, which bfloat16 would round to infinity, keep the largest bfloat16 as their first part.
 #pragma once
 
 #include "common.cuh"
@@ -16,11 +17,16 @@ __device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
   asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(d) : "f"(hi), "f"(lo));
   return d;
 }
+__device__ __forceinline__ uint32_t pack_bf16_within(float lo, float hi) {  // past the largest number: the largest
+  uint32_t d;
+  asm("cvt.rn.satfinite.bf16x2.f32 %0, %1, %2;" : "=r"(d) : "f"(hi), "f"(lo));
+  return d;
+}
 __device__ __forceinline__ Split split_pair(float x, float y) {
   Split out;
 #pragma unroll
   for (int i = 0; i < 3; ++i) {
-    out.part[i] = pack_bf16(x, y);
+    out.part[i] = i == 0 ? pack_bf16_within(x, y) : pack_bf16(x, y);
     if (i < 2) x -= __uint_as_float(out.part[i] << 16), y -= __uint_as_float(out.part[i] & 0xffff0000u);
   }
   return out;

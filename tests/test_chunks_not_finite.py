@@ -60,3 +60,23 @@ def test_earlier_tokens_keep_their_bits(rule, operand, value, at):
     own = range(RUNS[0]) if at < RUNS[0] else range(RUNS[0], n)
     others = [t for t in range(n) if t < at or t not in own]
     assert torch.isfinite(clean).all() and torch.equal(got[others], clean[others])
+
+
+@pytest.mark.parametrize("rule", ["channel", "head", "general", "wkv", "memory"])
+@pytest.mark.parametrize("operand", ["v", "k", "q"])
+@pytest.mark.parametrize("value", [torch.finfo(torch.float32).max, -3.397e38])
+@pytest.mark.parametrize("at", [41 + 5, 41 + 30, 41 + 66])
+def test_the_largest_numbers_leave_earlier_tokens_alone(rule, operand, value, at):
+    """They are finite: a zero in a triangle of pairs takes them out, although bfloat16 rounds them to infinity."""
+    n = sum(RUNS)
+    torch.manual_seed(at)
+    unit = torch.nn.functional.normalize(torch.randn(2, n, HEADS, DIM, device="cuda"), dim=-1).reshape(2, n, -1)
+    operands = dict(q=unit[0].contiguous(), k=unit[1].contiguous(), v=torch.randn(n, HEADS * DIM, device="cuda"),
+                    beta=torch.rand(n, HEADS, device="cuda"), decay=0.6 + 0.4 * torch.rand(n, HEADS * DIM, device="cuda"))
+    clean = outputs(rule, operands, n)
+    operands[operand] = operands[operand].clone()
+    operands[operand][at] = value
+    got = outputs(rule, operands, n)
+    own = range(RUNS[0], n)
+    others = [t for t in range(n) if t < at or t not in own]
+    assert torch.isfinite(clean).all() and torch.equal(got[others], clean[others])

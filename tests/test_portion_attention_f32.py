@@ -120,7 +120,7 @@ def test_a_score_that_is_nan_reaches_its_row(operand, at, dim):
     assert torch.equal(got[~reached], clean[~reached])
 
 
-@pytest.mark.parametrize("operand,value", [("q", "inf"), ("k", "inf"), ("k", "-inf"), ("v", "inf"), ("v", "-inf"), ("k", "3.4e38"), ("k", "-3.4e38")])
+@pytest.mark.parametrize("operand,value", [("q", "inf"), ("k", "inf"), ("k", "-inf"), ("v", "inf"), ("v", "-inf"), ("v", "3.4e38"), ("k", "3.4e38"), ("k", "-3.4e38")])
 @pytest.mark.parametrize("at", [0, 16, 31, 75])
 @pytest.mark.parametrize("dim", [24, 128])
 def test_infinite_and_very_large_numbers(operand, value, at, dim):
