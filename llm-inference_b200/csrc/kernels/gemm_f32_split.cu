@@ -9,13 +9,14 @@
 // A block computes 128 rows of W by TOKENS rows of A (D[row of W][token]: W is the MMA's 128-row side). Eight warps fetch 32-bit rows, 64
 // numbers a stage, take them apart and store the parts K-major with 128-byte swizzle; one elected thread issues the 24 products of a
 // stage; four warps add up the accumulators, two of which take turns in TMEM. An output's sums are the same whatever the tile, so a row's result
-// does not depend on how many rows are in the call. Operands that are not finite make their row or column NaN.
+// does not depend on how many rows are in the call. Outputs that are not finite are made again as one chain of FMAs (`chain`).
 //
 // What bounds it: what an SM takes out of L2, 48 KB a stage at 128 x 64 and 64 KB at 128 x 128. Of 34 us for 500 rows by 2,048 x 1,536, a form
 // that only fetches takes 25, the products and the taking apart the rest. Tried: two stages ahead in registers instead of one, no change; numbers by
 // cp.async and W's parts in TMEM, 36 us (17,920 rows of W, 2,048 of A: 858 against 716).
 // Every wait is bounded; a block that gives up sets the timeout bit, frees its TMEM and leaves.
 #include "common.cuh"
+#include "split_mma.cuh"
 
 namespace {
 
@@ -97,15 +98,10 @@ __device__ __forceinline__ void tmem_load_16(uint32_t taddr, float (&v)[16]) {
   for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(r[i]);
 }
 
-__device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
-  uint32_t d;
-  asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(d) : "f"(hi), "f"(lo));
-  return d;
-}
 // Eight neighbouring numbers of a row, in parts, to piece `piece` of the row in the three tiles of parts.
 __device__ __forceinline__ void store_parts(unsigned char* tile, uint32_t bytes, int row, int piece, float4 a, float4 b) {
-  float v[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
   unsigned char* to = tile + row * 128 + ((piece ^ (row & 7)) << 4);
+  float v[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
 #pragma unroll
   for (int p = 0; p < kParts; ++p) {
     uint32_t word[4];
@@ -127,9 +123,22 @@ struct SplitProduct {
   int* err;
 };
 
+// An output as the FMA kernel makes it, where the sum of the products of parts is not finite: an infinite operand (whose parts are NaN), or a sum
+// that passes the range on its way, may be the reason, and the output is infinite, or finite after all.
+__device__ __noinline__ float chain(const SplitProduct& p, int m, int n) {
+  const float* a = p.A + static_cast<int64_t>(m) * p.lda;
+  const float* w = p.W + static_cast<int64_t>(n) * p.ldw;
+  float sum = 0.f;
+  for (int k = 0; k < p.K; k += 4) {
+    const float4 x = *reinterpret_cast<const float4*>(a + k), y = *reinterpret_cast<const float4*>(w + k);
+    sum = fmaf(x.w, y.w, fmaf(x.z, y.z, fmaf(x.y, y.y, fmaf(x.x, y.x, sum))));
+  }
+  return sum;
+}
+
 template <int TOKENS>
 __global__ void __launch_bounds__(kThreads, 1)
-gemm_f32_split_kernel(const SplitProduct p) {
+gemm_f32_split_kernel(const __grid_constant__ SplitProduct p) {
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   constexpr int kStages = split_stages(TOKENS);
   constexpr uint32_t kColumns = 2 * TOKENS < 32 ? 32 : 2 * TOKENS;  // of TMEM: two accumulators; a power of two
@@ -256,9 +265,19 @@ gemm_f32_split_kernel(const SplitProduct p) {
     }
     if (have && n < p.N) {
       const float more = p.bias != nullptr ? p.bias[n] : 0.f;
+      uint32_t odd[(TOKENS + 31) / 32] = {};  // tokens whose sum is not finite
 #pragma unroll
-      for (int i = 0; i < TOKENS; ++i)
-        if (m0 + i < p.M) p.C[static_cast<int64_t>(m0 + i) * p.ldc + n] = sum[i] + more;
+      for (int i = 0; i < TOKENS; ++i) {
+        if (m0 + i >= p.M) break;
+        if (!isfinite(sum[i])) odd[i / 32] |= 1u << (i % 32);
+        p.C[static_cast<int64_t>(m0 + i) * p.ldc + n] = sum[i] + more;
+      }
+#pragma unroll
+      for (int word = 0; word < (TOKENS + 31) / 32; ++word)
+        for (; odd[word] != 0; odd[word] &= odd[word] - 1) {
+          const int m = m0 + word * 32 + __ffs(odd[word]) - 1;
+          p.C[static_cast<int64_t>(m) * p.ldc + n] = chain(p, m, n) + more;
+        }
     }
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");

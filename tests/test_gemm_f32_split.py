@@ -66,3 +66,24 @@ def test_sizes_far_apart_and_what_is_not_finite():
     rows, cols = torch.arange(40) != 3, torch.arange(200) != 5
     assert not torch.isfinite(spoilt[3]).any() and not torch.isfinite(spoilt[:, 5]).any()
     assert torch.equal(spoilt[rows][:, cols], got[rows][:, cols])
+
+
+@pytest.mark.parametrize("operand", ["a", "w"])
+@pytest.mark.parametrize("value", ["inf", "-inf", "3.4028234e38", "-3.397e38"])
+@pytest.mark.parametrize("tokens", [16, 32, 64, 128])
+def test_infinite_and_very_large_operands(operand, value, tokens):
+    """As chains of FMAs have them: infinities with their signs, sums of very large numbers where they are finite."""
+    torch.manual_seed(1)
+    m, n, k = 130, 200, 516
+    operands = dict(a=0.5 * torch.rand(m, k, device="cuda") - 0.25, w=torch.rand(n, k, device="cuda") - 0.5)
+    bias = torch.randn(n, device="cuda")
+    clean = product(*operands.values(), bias, tokens)
+    operands[operand][17, 33] = float(value)
+    want = operands["a"].double() @ operands["w"].double().T + bias.double()
+    got = product(*operands.values(), bias, tokens).double()
+    finite = torch.isfinite(want)
+    assert torch.equal(got[~finite], want[~finite]) and torch.isfinite(got[finite]).all()
+    assert ((got - want)[finite].norm() / want[finite].norm()).item() < CLOSE
+    other = torch.ones(m if operand == "a" else n, dtype=torch.bool, device="cuda")
+    other[17] = False
+    assert torch.equal(got[other] if operand == "a" else got[:, other], (clean[other] if operand == "a" else clean[:, other]).double())
