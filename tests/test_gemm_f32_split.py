@@ -87,3 +87,18 @@ def test_infinite_and_very_large_operands(operand, value, tokens):
     other = torch.ones(m if operand == "a" else n, dtype=torch.bool, device="cuda")
     other[17] = False
     assert torch.equal(got[other] if operand == "a" else got[:, other], (clean[other] if operand == "a" else clean[:, other]).double())
+
+
+@pytest.mark.parametrize("small,large", [(-118, 100), (-122, 0), (-130, 60), (-142, 90)])
+@pytest.mark.parametrize("operand", ["a", "w"])
+def test_the_smallest_operands(operand, small, large):
+    """Numbers whose last bits lie below bfloat16's smallest number, from 2^-149 on, beside ordinary and large ones."""
+    torch.manual_seed(2)
+    m, n, k = 33, 200, 320
+    few = torch.randint(1, 1 << 24, (m, k), device="cuda").float() if small > -130 else torch.randint(1, 1 << 7, (m, k), device="cuda").float()
+    tiny = torch.ldexp(few, torch.tensor(small - (24 if small > -130 else 7), device="cuda"))
+    other = torch.ldexp(torch.rand(n, k, device="cuda") + 0.5, torch.tensor(large, device="cuda"))
+    a, w = (tiny, other) if operand == "a" else (other, tiny)
+    want = a.double() @ w.double().T
+    got = product(a.contiguous(), w.contiguous())
+    assert ((got.double() - want).abs() / want).max().item() < CLOSE + 2.0**-149 / want.min().item()
