@@ -235,13 +235,14 @@ __device__ __forceinline__ float block_max(float v, float* scratch) {
 }
 
 // 1 / (1 + e^-x) where many stand in line: the quotient as the hardware's estimate and one step of the Newton-Raphson iteration, in a
-// third of a division's instructions and as good (over 2^28 numbers from -87 to 87 largest error 2.1e-7, mean 2.2e-8, both with a division). Reciprocals that are no normal numbers
-// are zero.
+// third of a division's instructions and as good (over 2^28 numbers from -87 to 87 largest error 2.1e-7, mean 2.2e-8, both with a division). A
+// quarter of the divisor is taken, whose reciprocal is a normal number wherever e^-x is finite; an infinite one becomes 3e38, whose estimate is zero.
 __device__ __forceinline__ float sigmoid_quick(float x) {
-  const float d = 1.f + expf(-x);
-  float r;
+  float d = fmaf(expf(-x), 0.25f, 0.25f), r;
+  asm("min.NaN.f32 %0, %1, %2;" : "=f"(d) : "f"(d), "f"(3e38f));
   asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(d));
-  return d > 8e37f ? r : fmaf(r, fmaf(-d, r, 1.f), r);
+  const float quotient = 0.25f * r;
+  return fmaf(quotient, fmaf(-d, r, 1.f), quotient);
 }
 
 // The gated units of the feed-forwards: silu(gate) * up, or gelu(gate) * up with the tanh form of gelu,
