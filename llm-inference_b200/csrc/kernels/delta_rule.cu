@@ -101,6 +101,9 @@ __global__ void delta_prepare_kernel(const T* proj, int ld, const T* decay_in, i
 // two blocks an SM, and went through a token's rows with a look at its request for every tap: on a B200 2,048 tokens of 4,608 channels took
 // 58 us with a decay per channel and 30 with one per head (3,072 channels), now 29 and 16
 // (with divisions 52 and 26: their code, in line sixteen times, did not fit what an SM holds of it).
+// Heads of more than 256 channels do not fit a warp's registers: the four warps of a block share one, and its numbers wait for their factors where they
+// go (4 heads of 512, 2,048 tokens: 78 us with a decay per channel and 59 with one per head in the form for single tokens, 55 and 41 in the block for all
+// channels, now 40 and 27; 300 tokens 21 and 17, 24 and 20, now 11 and 9; one warp a head 23 and 23).
 constexpr int kWideTokens = 4, kWideTaps = 4, kWideChannels = 128;
 
 struct WidePrepare {
@@ -155,15 +158,19 @@ __device__ __forceinline__ void convolve_wide(float4 (&y)[kWideTokens], const Wi
   }
 }
 
-template <typename T, int QUADS>  // QUADS: a q or k head has up to 128 QUADS channels
+template <typename T, int QUADS>  // QUADS: a q or k head has up to 128 QUADS channels; 0: any number, a block's four warps a head
 __global__ void __launch_bounds__(128, QUADS == 1 ? 6 : 4)
 delta_prepare_wide_kernel(const WidePrepare p, const T* proj, const T* decay_in, const T* conv_state) {
   const int items = p.kv_heads + p.v_pieces + p.decay_pieces + 1;
-  const int64_t warp = static_cast<int64_t>(blockIdx.x) * 4 + (threadIdx.x >> 5);
   // Tokens run fastest: what an SM works on at a time is then of one kind, whose code it holds.
-  const int groups = (p.tokens + kWideTokens - 1) / kWideTokens;
-  const int t0 = static_cast<int>(warp % groups) * kWideTokens, lane = threadIdx.x & 31;
+  const int groups = (p.tokens + kWideTokens - 1) / kWideTokens, lane = threadIdx.x & 31, own = threadIdx.x >> 5;
+  const int64_t warp = static_cast<int64_t>(blockIdx.x) * 4 + own;
+  const int t0 = static_cast<int>((QUADS == 0 ? blockIdx.x : warp) % groups) * kWideTokens;
   int item = static_cast<int>(warp / groups);
+  if (QUADS == 0) {
+    item = blockIdx.x / groups;
+    if (item >= p.kv_heads) item += 3 * (item - p.kv_heads) + own;
+  }
   if (item >= items) return;
   const int count = min(kWideTokens, p.tokens - t0);
   const int qk = p.kv_heads * p.dk, vw = p.heads * p.dv;
@@ -171,9 +178,46 @@ delta_prepare_wide_kernel(const WidePrepare p, const T* proj, const T* decay_in,
   const bool inside = p.token_seq[t0 + count - 1] == seq && t0 - p.seq_q_start[seq] >= kWideTaps - 1;
   wait_for_predecessor();
   let_successor_start();
-  if (item < p.kv_heads) {  // unit vectors, and k . q
+  if (QUADS == 0 && item < p.kv_heads) {
+    float q_ss[kWideTokens] = {}, k_ss[kWideTokens] = {}, dot[kWideTokens] = {};
+    float* q_to = p.q_out + static_cast<int64_t>(t0) * qk + item * p.dk;
+    float* k_to = p.k_out + static_cast<int64_t>(t0) * qk + item * p.dk;
+#pragma unroll 1
+    for (int c = threadIdx.x * 4; c < p.dk; c += 4 * kWideChannels) {
+      float4 q[kWideTokens], k[kWideTokens];
+      convolve_wide<T>(q, p, proj, conv_state, t0, count, inside, item * p.dk + c);
+      convolve_wide<T>(k, p, proj, conv_state, t0, count, inside, qk + item * p.dk + c);
+#pragma unroll
+      for (int i = 0; i < kWideTokens; ++i) {
+        const float4 a = q[i], b = k[i];
+        q_ss[i] = square_sum(a, q_ss[i]), k_ss[i] = square_sum(b, k_ss[i]);
+        dot[i] = fmaf(a.x, b.x, fmaf(a.y, b.y, fmaf(a.z, b.z, fmaf(a.w, b.w, dot[i]))));
+        if (i < count) *reinterpret_cast<float4*>(q_to + static_cast<int64_t>(i) * qk + c) = a, *reinterpret_cast<float4*>(k_to + static_cast<int64_t>(i) * qk + c) = b;
+      }
+    }
+    __shared__ float sums[kWideTokens][3][4];
+#pragma unroll
+    for (int i = 0; i < kWideTokens; ++i) {
+      q_ss[i] = warp_sum(q_ss[i]), k_ss[i] = warp_sum(k_ss[i]), dot[i] = warp_sum(dot[i]);
+      if (lane == 0) sums[i][0][own] = q_ss[i], sums[i][1][own] = k_ss[i], sums[i][2][own] = dot[i];
+    }
+    __syncthreads();
+    const auto whole = [&](int i, int kind) { return (sums[i][kind][0] + sums[i][kind][1]) + (sums[i][kind][2] + sums[i][kind][3]); };
+#pragma unroll 1
+    for (int i = 0; i < count; ++i) {
+      const float q_factor = (1.f / sqrtf(whole(i, 0) + 1e-6f)) * (1.f / sqrtf(static_cast<float>(p.dk))), k_factor = 1.f / sqrtf(whole(i, 1) + 1e-6f);
+      for (int c = threadIdx.x * 4; c < p.dk; c += 4 * kWideChannels) {  // a thread's own numbers again
+        float4* q = reinterpret_cast<float4*>(q_to + static_cast<int64_t>(i) * qk + c);
+        float4* k = reinterpret_cast<float4*>(k_to + static_cast<int64_t>(i) * qk + c);
+        *q = scale_each(*q, q_factor), *k = scale_each(*k, k_factor);
+      }
+      if (p.kq_out != nullptr && threadIdx.x == 0) p.kq_out[static_cast<int64_t>(t0 + i) * p.kv_heads + item] = whole(i, 2) * k_factor * q_factor;
+    }
+    return;
+  }
+  if (QUADS > 0 && item < p.kv_heads) {  // unit vectors, and k . q
     float q_factor[kWideTokens], k_factor[kWideTokens], dot[kWideTokens];
-    float4 q[QUADS][kWideTokens], k[QUADS][kWideTokens];
+    float4 q[QUADS + (QUADS == 0)][kWideTokens], k[QUADS + (QUADS == 0)][kWideTokens];
 #pragma unroll
     for (int x = 0; x < QUADS; ++x) {
       const int c = x * kWideChannels + lane * 4;
@@ -464,7 +508,7 @@ B200_API int b200_delta_prepare(const void* proj, int ld, const void* decay_in, 
   // The wide form from half a block an SM on, with rows, taps and results on 16-byte (bfloat16 rows: 8-byte) boundaries.
   const auto on = [](const void* p, int bytes) { return reinterpret_cast<uintptr_t>(p) % bytes == 0; };
   const int in_bytes = dtype == DTYPE_F32 ? 16 : 8;
-  const bool wide = taps == kWideTaps && tokens >= kWideTokens * b200_sm_count_host() / 2 && ld % 4 == 0 && dk % 4 == 0 && dv % 4 == 0 && dk <= 2 * kWideChannels &&
+  const bool wide = taps == kWideTaps && tokens >= kWideTokens * b200_sm_count_host() / 2 && ld % 4 == 0 && dk % 4 == 0 && dv % 4 == 0 &&
                     on(proj, in_bytes) && on(conv_state, in_bytes) && on(taps_w, 16) && on(q_out, 16) && on(k_out, 16) && on(v_out, 16) &&
                     (kq_out != nullptr || (decay_ld % 4 == 0 && on(decay_in, in_bytes) && on(dt_bias, 16) && on(decay_out, 16)));
   auto launch_wide = [&](auto kernel, auto* typed) {
@@ -472,13 +516,17 @@ B200_API int b200_delta_prepare(const void* proj, int ld, const void* decay_in, 
     const auto pieces = [](int64_t n) { return static_cast<int>((n + kWideChannels - 1) / kWideChannels); };
     const WidePrepare p = {ld, decay_ld, tokens, heads, kv_heads, dk, dv, taps_w, a_log, dt_bias, token_seq, seq_q_start, seq_slot, q_out, k_out, v_out, beta_out,
                            decay_out, kq_out, pieces(static_cast<int64_t>(heads) * dv), kq_out != nullptr ? 0 : pieces(static_cast<int64_t>(heads) * dk)};
-    const int64_t warps = static_cast<int64_t>((tokens + kWideTokens - 1) / kWideTokens) * (kv_heads + p.v_pieces + p.decay_pieces + 1);
-    launch_kernel(kernel, dim3(static_cast<unsigned>((warps + 3) / 4)), dim3(128), 0, stream, p, typed, static_cast<const T*>(decay_in), static_cast<const T*>(conv_state));
+    const int64_t groups = (tokens + kWideTokens - 1) / kWideTokens, pieces_a_group = p.v_pieces + p.decay_pieces + 1;
+    const int64_t blocks = dk > 2 * kWideChannels ? groups * (kv_heads + (pieces_a_group + 3) / 4) : (groups * (kv_heads + pieces_a_group) + 3) / 4;
+    launch_kernel(kernel, dim3(static_cast<unsigned>(blocks)), dim3(128), 0, stream, p, typed, static_cast<const T*>(decay_in), static_cast<const T*>(conv_state));
   };
   if (wide && (dtype == DTYPE_F32 || dtype == DTYPE_BF16)) {
-    const bool one = dk <= kWideChannels;
-    if (dtype == DTYPE_F32) launch_wide(one ? delta_prepare_wide_kernel<float, 1> : delta_prepare_wide_kernel<float, 2>, static_cast<const float*>(proj));
-    else launch_wide(one ? delta_prepare_wide_kernel<__nv_bfloat16, 1> : delta_prepare_wide_kernel<__nv_bfloat16, 2>, static_cast<const __nv_bfloat16*>(proj));
+    const auto form = [&](auto one, auto two, auto any) { return dk <= kWideChannels ? one : (dk <= 2 * kWideChannels ? two : any); };
+    if (dtype == DTYPE_F32)
+      launch_wide(form(delta_prepare_wide_kernel<float, 1>, delta_prepare_wide_kernel<float, 2>, delta_prepare_wide_kernel<float, 0>), static_cast<const float*>(proj));
+    else
+      launch_wide(form(delta_prepare_wide_kernel<__nv_bfloat16, 1>, delta_prepare_wide_kernel<__nv_bfloat16, 2>, delta_prepare_wide_kernel<__nv_bfloat16, 0>),
+                  static_cast<const __nv_bfloat16*>(proj));
     if (int status = b200_check_launch("delta_prepare")) return status;
     if (dtype == DTYPE_F32)
       launch_kernel(conv_state_update_kernel<float>, dim3(seqs, update_blocks), dim3(threads), 0, stream, static_cast<const float*>(proj), ld, channels, taps,

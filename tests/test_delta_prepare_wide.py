@@ -1,5 +1,6 @@
 """The delta rules' convolution, unit vectors, betas and decays over steps long enough for four tokens a block: ragged requests whose
-first tokens reach into their slots, a step that ends inside a block of four, 48 KB of convolved queries and keys."""
+first tokens reach into their slots, a step that ends inside a block of four, heads of up to 128, of up to 256 and of more channels that are no
+whole number of a warp's."""
 
 from __future__ import annotations
 
@@ -12,7 +13,8 @@ from test_state_chunks import device_context, on_device
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("heads,kv_heads,dk,dv,runs", [(12, 12, 128, 128, (301,)), (4, 2, 64, 36, (1, 2, 3, 300, 1)), (3, 1, 20, 8, (4, 297))])
+@pytest.mark.parametrize("heads,kv_heads,dk,dv,runs", [(12, 12, 128, 128, (301,)), (4, 2, 64, 36, (1, 2, 3, 300, 1)), (3, 1, 20, 8, (4, 297)),
+                                                       (2, 2, 132, 8, (298,)), (3, 1, 256, 16, (2, 5, 297)), (2, 1, 260, 8, (1, 299)), (2, 2, 1028, 8, (3, 298))])
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
 @pytest.mark.parametrize("per_head", [False, True])
 def test_against_64_bits(heads, kv_heads, dk, dv, runs, dtype, per_head):
