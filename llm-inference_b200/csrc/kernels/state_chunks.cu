@@ -864,25 +864,28 @@ chunk_scan_kernel(const int* __restrict__ seq_q_start, const int* __restrict__ s
 // One block per (16 columns of the state, head, request), a warp per 16 rows, which it keeps in registers, transposed, as the tensor core
 // leaves them (D: 16 columns x 2 times 8 rows): D's layout is A's, so the state goes into the next chunk's first product without leaving
 // its lanes. That product, U^T = W^T + S^T Y^T, is summed over the warps through shared memory, each warp adding up its share of the sums; S^T <-
-// e S^T + U^T Kd then wants nothing of the other warps. A lane's share of the operands comes by its own asynchronous copies, two chunks ahead,
+// e S^T + U^T Kd then wants nothing of the other warps. A lane's share of the operands comes by its own asynchronous copies, one or two chunks ahead,
 // so that nobody waits for anybody's (loads into registers a chunk ahead did: 101 us where this takes 80, a third of it spent
 // waiting for memory; copies that also go into L1 112).
 // What bounds it: the chain product, sum over warps, product, in turn and once a chunk: 2,400 cycles, of which the tensor core works 830 (heads
 // of 128 x 128). Tried: operands in parts in memory, made where they are prepared, half as many bytes again: 76 us, but 5 us more there;
 // taking them apart while the warps wait for one another: 95 us.
 constexpr int kSumPairs = 8;  // pairs of U^T's numbers that a lane holds: (half of the chunk, pair of four tokens, column g or g + 8)
-__host__ __device__ constexpr int walk_stages(int rows) { return rows <= 128 ? 3 : 2; }  // two blocks fit an SM up to 128 rows
+// Three stages where two blocks then still fit an SM: with what the values add, up to 64 rows (128 rows in three stages had an SM to themselves: generalized
+// rule, 28 heads of 128 x 128, all three kernels, 2,048 tokens 410 us, in two stages 372; 8 requests of 300 tokens 470 and 430).
+__host__ __device__ constexpr int walk_stages(int rows, bool add) { return rows <= (add ? 64 : 128) ? 3 : 2; }
 __host__ __device__ constexpr int own_pairs(int rows) { return rows < 16 * kSumPairs ? 16 * kSumPairs / rows : 1; }  // that a warp adds up
 // Bytes of a stage: per lane four pieces of y, four of kd, two of what the values add and its pairs of W; and e.
 __host__ __device__ constexpr int walk_stage(int rows, bool add) { return 2 * rows * (16 * (add ? 10 : 8) + 8 * own_pairs(rows)) + 4 * rows; }
-constexpr size_t walk_smem(int rows, bool add) { return walk_stages(rows) * walk_stage(rows, add); }
+constexpr size_t walk_smem(int rows, bool add) { return walk_stages(rows, add) * walk_stage(rows, add); }
+static_assert(2 * (walk_smem(128, false) + 5 * 1024) <= 228 * 1024 && 2 * (walk_smem(128, true) + 5 * 1024) <= 228 * 1024, "two blocks of 128 rows do not fit an SM");
 
 template <int ROWS, bool ADD>  // ADD: what the values alone add to S stands where the chunk's state goes
 __global__ void __launch_bounds__(2 * ROWS, ROWS <= 128 ? 2 : 1)
 chunk_walk_kernel(const int* __restrict__ seq_q_start, const int* __restrict__ seq_q_len, const int* __restrict__ seq_slot, int heads, int dk, int dv,
                   Scratch from, float* state) {
   extern __shared__ __align__(16) float chunk_smem[];
-  constexpr int kParts = ROWS / 16, kOwn = own_pairs(ROWS), kLanes = 2 * ROWS, kStages = walk_stages(ROWS);
+  constexpr int kParts = ROWS / 16, kOwn = own_pairs(ROWS), kLanes = 2 * ROWS, kStages = walk_stages(ROWS, ADD);
   constexpr int kPairsAt = (ADD ? 10 : 8) * kLanes * 4, kDecaysAt = kPairsAt + kOwn * kLanes * 2;  // in a stage
   __shared__ uint4 us[2][3][32];  // U^T in parts, as the lanes of every warp want it
   let_successor_start();
