@@ -4,7 +4,7 @@
 // that share the kv head side by side, and walks the request's keys 64 at a time. A warp has sixteen of the rows and sixteen of every 64 keys: scores,
 // running softmax and weighted sum of values are its own until the end, when the four parts of the keys meet. Both products are tensor-core
 // products of 32-bit numbers taken apart into three bfloat16 ones (split_mma.cuh); eight warps more take the next tile's keys and values
-// apart, into shared memory as the lanes want them, while this one's are multiplied. Windows and a sink (a start value of
+// apart, into shared memory as the lanes want them, while this one's are multiplied; where a block has few keys, each warp fetches its own (`few_keys`). Windows and a sink (a start value of
 // maximum and sum) are taken; other shapes of scores, kept first keys and single tokens run the plain kernel.
 //
 // What bounds it: the tensor core's 1,536 products a tile (3,300 cycles of an SM) and, in turn with them, the taking apart. The plain kernel reads
@@ -44,7 +44,9 @@ struct PortionParams {
 
 // Parts of 16 x 16 numbers, a uint4 a part and lane.
 constexpr int kBlock = 3 * 32;
-constexpr size_t portion_smem(int dim) { return sizeof(uint4) * (kRows / 16 + 2 * 2 * kKeyParts) * (dim / 16) * kBlock; }
+constexpr size_t portion_smem(int dim, bool direct) {
+  return direct ? sizeof(float) * kWarps * 16 * (dim + 4) : sizeof(uint4) * (kRows / 16 + 2 * 2 * kKeyParts) * (dim / 16) * kBlock;
+}
 
 // Two tiles take turns: barrier `id` is met by the warps that multiply and those that take apart, of which one side only arrives.
 __device__ __forceinline__ void meet(int id) { asm volatile("bar.sync %0, %1;" ::"r"(id), "n"(kThreads) : "memory"); }
@@ -52,6 +54,9 @@ __device__ __forceinline__ void arrive(int id) { asm volatile("bar.arrive %0, %1
 __device__ __forceinline__ void meet_own() { asm volatile("bar.sync 5, %0;" ::"n"(kOwnThreads) : "memory"); }
 constexpr int kFull = 1, kEmpty = 3;  // + tile % 2
 
+__device__ __forceinline__ float4 finite_part(float4 v) {
+  return make_float4(isfinite(v.x) ? v.x : 0.f, isfinite(v.y) ? v.y : 0.f, isfinite(v.z) ? v.z : 0.f, isfinite(v.w) ? v.w : 0.f);
+}
 __device__ __forceinline__ void store_block(uint4* to, const SplitB& first, const SplitB& second) {
   const int lane = threadIdx.x & 31;
 #pragma unroll
@@ -106,8 +111,8 @@ __device__ __noinline__ void attend_row(const PortionParams& p, int seq, int kvh
     *reinterpret_cast<float4*>(p.out + (static_cast<int64_t>(token) * p.q_heads + head) * p.head_dim + lane * 4) = make_float4(acc.x * inv, acc.y * inv, acc.z * inv, acc.w * inv);
 }
 
-template <int DIM>
-__global__ void __launch_bounds__(kThreads, 1)
+template <int DIM, bool DIRECT>  // DIRECT: no warps that take apart, each fetches what it multiplies by
+__global__ void __launch_bounds__(DIRECT ? kOwnThreads : kThreads, DIRECT ? 2 : 1)
 portion_attention_f32_kernel(const __grid_constant__ PortionParams p) {
   extern __shared__ __align__(16) uint4 attention_smem[];
   constexpr int kSteps = DIM / 16;                        // sixteens of a head's numbers
@@ -136,14 +141,14 @@ portion_attention_f32_kernel(const __grid_constant__ PortionParams p) {
     const int item = row0 + r, token = item / group, head = kvh * group + item % group;
     return r < rows && c < p.head_dim ? *reinterpret_cast<const float4*>(p.q + (static_cast<int64_t>(start + token) * p.q_heads + head) * p.head_dim + c) : zero;
   };
-  for (int item = warp; item < kRows / 16 * kSteps; item += kThreads / 32) {
+  for (int item = warp; item < kRows / 16 * kSteps; item += (DIRECT ? kOwnThreads : kThreads) / 32) {
     const int r = item / kSteps * 16 + g, c = item % kSteps * 16 + 4 * q;
     const SplitA a = split_rows(query(r, c), query(r + 8, c));
 #pragma unroll
     for (int x = 0; x < 3; ++x) qs[(item * 3 + x) * 32 + lane] = make_uint4(a.part[x][0], a.part[x][1], a.part[x][2], a.part[x][3]);
   }
   __syncthreads();
-  if (warp >= kWarps) {
+  if (!DIRECT && warp >= kWarps) {
     // ---- take apart: half the numbers of sixteen keys a warp, chunk after chunk ----
     asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kApartRegisters));
     constexpr int kChunks = kSteps / 2 / kChunk;
@@ -197,8 +202,7 @@ portion_attention_f32_kernel(const __grid_constant__ PortionParams p) {
           for (int t = 0; t < 2; ++t) {
             float4& v = v_next[i][t];
             if (all_finite(v)) continue;
-            finite = false;  // zeros for now
-            v.x = isfinite(v.x) ? v.x : 0.f, v.y = isfinite(v.y) ? v.y : 0.f, v.z = isfinite(v.z) ? v.z : 0.f, v.w = isfinite(v.w) ? v.w : 0.f;
+            finite = false, v = finite_part(v);  // zeros for now
           }
           store_block(vs + at, SplitB(v_next[i][0]), SplitB(v_next[i][1]));
           fetch(chunk + 1 < kChunks ? (chunk + 1) * kChunk : 0, i);  // the next chunk's, of the next tile behind a tile's last (past the last one: zeros)
@@ -210,7 +214,7 @@ portion_attention_f32_kernel(const __grid_constant__ PortionParams p) {
     }
     return;
   }
-  asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kOwnRegisters));
+  if constexpr (!DIRECT) asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kOwnRegisters));
   const int own_rows = warp / kKeyParts * 16, own_keys = warp % kKeyParts;
   int pos[2], from[2];
   float top[2], sum[2];
@@ -228,11 +232,40 @@ portion_attention_f32_kernel(const __grid_constant__ PortionParams p) {
   for (int i = 0; i < 2 * kSteps; ++i) acc[i][0] = acc[i][1] = acc[i][2] = acc[i][3] = 0.f;
   for (int tile = 0; tile < tiles; ++tile) {
     const int b = tile & 1;
-    meet(kFull + b);
+    int64_t row = -1;  // DIRECT: of key lane % 16: where its row is
+    if constexpr (DIRECT) {
+      const int part0 = lo + tile * kKeys + own_keys * 16, j = part0 + (lane & 15);
+      if (part0 > last_pos) break;  // the last tile's last keys
+      if (j <= last_pos) {
+        const int logical = j / p.page_size;
+        const int page = logical < p.max_pages ? table[logical] : -1;
+        if (page < 0 || page >= p.num_pages) atomicOr(p.err, ERRBIT_BAD_PAGE);
+        else row = kv_row_offset(page, kvh, j % p.page_size, p.kv_heads, p.page_size, p.head_dim);
+      }
+    } else {
+      meet(kFull + b);
+    }
     // Scores of sixteen rows and sixteen keys, of which the lane has keys 4 q .. + 3.
     float score[2][4] = {};
     {
       constexpr int kTogether = 2;
+      const float* at[2];
+      float4 next[2 * kTogether];
+      const auto fetch_keys = [&](int s) {
+#pragma unroll
+        for (int n = 0; n < 2 * kTogether; ++n) {
+          const int c = (s + n / 2) * 16 + 4 * q;
+          next[n] = at[n % 2] != nullptr && c < p.head_dim ? *reinterpret_cast<const float4*>(at[n % 2] + c) : zero;
+        }
+      };
+      if constexpr (DIRECT) {
+#pragma unroll
+        for (int t = 0; t < 2; ++t) {
+          const int64_t key_at = __shfl_sync(0xffffffffu, row, in_sixteen(t, g));
+          at[t] = key_at >= 0 ? p.keys + key_at : nullptr;
+        }
+        fetch_keys(0);
+      }
 #pragma unroll 1
       for (int s = 0; s < kSteps; s += kTogether) {
         float sums[2 * kTogether][4];
@@ -245,7 +278,12 @@ portion_attention_f32_kernel(const __grid_constant__ PortionParams p) {
             const uint4 word = qs[((own_rows / 16 * kSteps + s + x) * 3 + y) * 32 + lane];
             own[x].part[y][0] = word.x, own[x].part[y][1] = word.y, own[x].part[y][2] = word.z, own[x].part[y][3] = word.w;
           }
-          load_block(ks + b * kTile + (own_keys * kSteps + s + x) * kBlock, right + 2 * x);
+          if constexpr (!DIRECT) load_block(ks + b * kTile + (own_keys * kSteps + s + x) * kBlock, right + 2 * x);
+        }
+        if constexpr (DIRECT) {
+#pragma unroll
+          for (int n = 0; n < 2 * kTogether; ++n) right[n] = SplitB(next[n]);
+          if (s + kTogether < kSteps) fetch_keys(s + kTogether);
         }
 #pragma unroll
         for (int n = 0; n < 2 * kTogether; ++n) mma_split(sums[n], own[n / 2], right[n]);
@@ -256,7 +294,7 @@ portion_attention_f32_kernel(const __grid_constant__ PortionParams p) {
       }
     }
     const int key0 = lo + tile * kKeys + own_keys * 16 + 4 * q;
-    const int64_t* own_offsets = offsets[b] + own_keys * 16 + 4 * q;
+    const auto own_offset = [&](int i) { return DIRECT ? __shfl_sync(0xffffffffu, row, 4 * q + i) : offsets[b][own_keys * 16 + 4 * q + i]; };
     float weight[2][4], alpha[2];
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
@@ -264,7 +302,7 @@ portion_attention_f32_kernel(const __grid_constant__ PortionParams p) {
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
         const int key = key0 + i;
-        const bool seen = key <= pos[h] && key >= from[h] && own_offsets[i] >= 0;
+        const bool seen = own_offset(i) >= 0 && key <= pos[h] && key >= from[h];
         weight[h][i] = seen ? score[i >> 1][2 * h + (i & 1)] * p.scale : -INFINITY;
         best = fmaxf(best, weight[h][i]);
       }
@@ -282,11 +320,40 @@ portion_attention_f32_kernel(const __grid_constant__ PortionParams p) {
       top[h] = new_top;
     }
     const SplitA left = split_rows(make_float4(weight[0][0], weight[0][1], weight[0][2], weight[0][3]), make_float4(weight[1][0], weight[1][1], weight[1][2], weight[1][3]));
+    float4 v[4];
+    const float* value_at[4];
+    if constexpr (DIRECT) {
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const int64_t at = own_offset(i);
+        value_at[i] = at >= 0 ? p.values + at + g : nullptr;
+      }
+    }
+    const auto fetch_values = [&](int s) {
+#pragma unroll
+      for (int n = 0; n < 4; ++n) {
+        const int c = s * 16 + 8 * n;
+        const bool in = c + g < p.head_dim;
+        v[n] = make_float4(in && value_at[0] ? value_at[0][c] : 0.f, in && value_at[1] ? value_at[1][c] : 0.f, in && value_at[2] ? value_at[2][c] : 0.f,
+                           in && value_at[3] ? value_at[3][c] : 0.f);
+      }
+    };
+    bool finite = true;
+    if constexpr (DIRECT) fetch_values(0);
 #pragma unroll
     for (int s = 0; s < kSteps; s += 2) {
       SplitB right[4];
-      load_block(vs + b * kTile + (own_keys * kSteps + s) * kBlock, right);
-      load_block(vs + b * kTile + (own_keys * kSteps + s + 1) * kBlock, right + 2);
+      if constexpr (DIRECT) {
+#pragma unroll
+        for (int n = 0; n < 4; ++n) {
+          if (!all_finite(v[n])) finite = false, v[n] = finite_part(v[n]);
+          right[n] = SplitB(v[n]);
+        }
+        if (s + 2 < kSteps) fetch_values(s + 2);
+      } else {
+        load_block(vs + b * kTile + (own_keys * kSteps + s) * kBlock, right);
+        load_block(vs + b * kTile + (own_keys * kSteps + s + 1) * kBlock, right + 2);
+      }
       float sums[4][4];
 #pragma unroll
       for (int n = 0; n < 4; ++n) mma_split(sums[n], left, right[n]);
@@ -295,10 +362,10 @@ portion_attention_f32_kernel(const __grid_constant__ PortionParams p) {
 #pragma unroll
         for (int i = 0; i < 4; ++i) acc[2 * s + n][i] = fmaf(acc[2 * s + n][i], alpha[i >> 1], sums[n][i]);
     }
-    if (spoilt[b][2 * own_keys] | spoilt[b][2 * own_keys + 1]) {  // what is not finite reaches the rows that see its key, and no others
+    if (DIRECT ? __any_sync(0xffffffffu, !finite) : spoilt[b][2 * own_keys] | spoilt[b][2 * own_keys + 1]) {  // what is not finite reaches the rows that see its key, and no others
       for (int j = 0; j < 16; ++j) {
         const int key = lo + tile * kKeys + own_keys * 16 + j;
-        const int64_t offset = offsets[b][own_keys * 16 + j];
+        const int64_t offset = DIRECT ? __shfl_sync(0xffffffffu, row, j) : offsets[b][own_keys * 16 + j];
         if (offset < 0) continue;
 #pragma unroll
         for (int x = 0; x < 2 * kSteps; ++x)
@@ -309,7 +376,7 @@ portion_attention_f32_kernel(const __grid_constant__ PortionParams p) {
           }
       }
     }
-    if (tile + 2 < tiles) arrive(kEmpty + b);
+    if (!DIRECT && tile + 2 < tiles) arrive(kEmpty + b);
   }
   // The four parts of the keys meet.
 #pragma unroll
@@ -319,7 +386,7 @@ portion_attention_f32_kernel(const __grid_constant__ PortionParams p) {
     if (q == 0) tops[warp][g + 8 * h] = top[h], totals[warp][g + 8 * h] = sum[h];
   }
   meet_own();  // the parts have been read too
-  float* os = reinterpret_cast<float*>(ks);  // [kWarps][16][kLdO]
+  float* os = reinterpret_cast<float*>(DIRECT ? qs : ks);  // [kWarps][16][kLdO]
   static_assert(sizeof(float) * kWarps * 16 * kLdO <= sizeof(uint4) * 4 * kTile, "the warps' sums do not fit where keys and values were");
 #pragma unroll
   for (int x = 0; x < 2 * kSteps; ++x)
@@ -365,11 +432,24 @@ B200_API int b200_portion_attention_f32_supported(int q_heads, int kv_heads, int
   return kv_heads > 0 && kv_heads <= 65535 && q_heads > 0 && q_heads % kv_heads == 0 && head_dim > 0 && head_dim % 4 == 0 && head_dim <= 128;
 }
 
-// Attention of the requests first_seq .. first_seq + num_seqs of the step (float32 queries, keys, values and outputs).
+// Whether a block's keys are too few for warps that take apart: one block has an SM to itself then, and what it does alone (its look at its
+// request, its queries, its first keys, the join of the parts) is most of it. Without them a warp fetches and takes apart what it multiplies by, which is
+// twice that work, but two blocks share an SM. Both give the same bits. Measured on a B200, with and without, heads of 128 (12 on 2): 192 blocks
+// of one tile of keys 21 and 16 us, 768 57 and 44, 192 of two 21 and 23, 256 36 and 34, 512 of three 66 and 63, 256 of six 63 and 65; heads of 64
+// (8): 128 of one 9.2 and 8.6, 512 25 and 16, 256 of three 15 and 12, 128 15 and 17, 512 of five 30 and 27, 1,024 of nine 92 and 90.
+static bool few_keys(bool narrow, int tokens, int max_kv_len, int group, int kv_heads, int num_seqs, int window) {
+  const int64_t blocks = (static_cast<int64_t>(tokens) * group + static_cast<int64_t>(num_seqs) * (kRows / 2)) / kRows * kv_heads, sms = b200_sm_count_host();
+  const int64_t keys = window > 0 && max_kv_len > window + kRows / group ? window + kRows / group : max_kv_len, tiles = (keys + kKeys - 1) / kKeys;
+  if (narrow) return tiles <= (blocks > 6 * sms ? 9 : (blocks > 2 * sms ? 6 : (blocks > sms ? 3 : 1)));
+  return tiles <= (blocks > 4 * sms ? 4 : (blocks > sms ? 2 : 0));
+}
+
+// Attention of the requests first_seq .. first_seq + num_seqs of the step (float32 queries, keys, values and outputs), which have `tokens` new tokens, at
+// most max_q_len each and max_kv_len with those before. `form`: 1 without warps that take apart, 2 with them; 0: by the sizes.
 B200_API int b200_portion_attention_f32(const float* q, const float* k_arena, const float* v_arena, const int* block_table, int max_pages, int num_pages,
                                         const int* seq_q_start, const int* seq_q_len, const int* seq_kv_len, int first_seq, int num_seqs, int max_q_len,
-                                        const float* sink, float* out, int q_heads, int kv_heads, int head_dim, int page_size, int window, float scale, int* err,
-                                        cudaStream_t stream) {
+                                        const float* sink, float* out, int q_heads, int kv_heads, int head_dim, int page_size, int window, float scale, int tokens, int max_kv_len,
+                                        int form, int* err, cudaStream_t stream) {
   if (num_seqs <= 0 || max_q_len <= 0) return 0;
   B200_REQUIRE(b200_portion_attention_f32_supported(q_heads, kv_heads, head_dim), "portion_attention_f32: shape not taken");
   B200_REQUIRE(page_size > 0 && max_pages > 0 && window >= 0 && num_seqs <= 65535, "portion_attention_f32: bad geometry");
@@ -377,16 +457,18 @@ B200_API int b200_portion_attention_f32(const float* q, const float* k_arena, co
   B200_REQUIRE(aligned(q) && aligned(k_arena) && aligned(v_arena) && aligned(out), "portion_attention_f32: operands must be aligned to 16 bytes");
   const PortionParams p{q, k_arena, v_arena, block_table, seq_q_start, seq_q_len, seq_kv_len, sink, out, err,
                         first_seq, max_pages, num_pages, q_heads, kv_heads, head_dim, page_size, window, scale};
-  const bool narrow = head_dim <= 64;
-  auto kernel = narrow ? portion_attention_f32_kernel<64> : portion_attention_f32_kernel<128>;
+  const bool narrow = head_dim <= 64, direct = form == 0 ? few_keys(narrow, tokens, max_kv_len, q_heads / kv_heads, kv_heads, num_seqs, window) : form == 1;
+  auto kernel = direct ? (narrow ? portion_attention_f32_kernel<64, true> : portion_attention_f32_kernel<128, true>)
+                       : (narrow ? portion_attention_f32_kernel<64, false> : portion_attention_f32_kernel<128, false>);
   static OncePerDevice raised;
   const auto raise = [] {
-    return cudaFuncSetAttribute(portion_attention_f32_kernel<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(portion_smem(64))) == cudaSuccess &&
-           cudaFuncSetAttribute(portion_attention_f32_kernel<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(portion_smem(128))) == cudaSuccess;
+    const auto raise_one = [](auto form_of, size_t bytes) { return cudaFuncSetAttribute(form_of, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(bytes)) == cudaSuccess; };
+    return raise_one(portion_attention_f32_kernel<64, false>, portion_smem(64, false)) && raise_one(portion_attention_f32_kernel<128, false>, portion_smem(128, false)) &&
+           raise_one(portion_attention_f32_kernel<64, true>, portion_smem(64, true)) && raise_one(portion_attention_f32_kernel<128, true>, portion_smem(128, true));
   };
   B200_REQUIRE(raised(raise), "portion_attention_f32: cannot size shared memory");
   const int64_t rows = static_cast<int64_t>(max_q_len) * (q_heads / kv_heads);
   const dim3 grid(static_cast<unsigned>((rows + kRows - 1) / kRows), kv_heads, num_seqs);
-  kernel<<<grid, kThreads, portion_smem(narrow ? 64 : 128), stream>>>(p);
+  kernel<<<grid, direct ? kOwnThreads : kThreads, portion_smem(narrow ? 64 : 128, direct), stream>>>(p);
   return b200_check_launch("portion_attention_f32");
 }

@@ -57,7 +57,7 @@ _SIGNATURES: dict[str, list] = {
     + [c_int, c_int, c_void_p]
     + [c_int] * 7
     + [c_float, c_int, c_float, c_void_p, c_int, c_int, c_void_p, c_void_p, c_int, c_void_p, c_void_p],
-    "b200_portion_attention_f32": [c_void_p] * 4 + [c_int] * 2 + [c_void_p] * 3 + [c_int] * 3 + [c_void_p] * 2 + [c_int] * 5 + [c_float, c_void_p, c_void_p],
+    "b200_portion_attention_f32": [c_void_p] * 4 + [c_int] * 2 + [c_void_p] * 3 + [c_int] * 3 + [c_void_p] * 2 + [c_int] * 5 + [c_float] + [c_int] * 3 + [c_void_p] * 2,
     "b200_gemm_f32": [c_void_p] * 4 + [c_int] * 6 + [c_void_p],
     "b200_gemm_f32_split": [c_void_p] * 4 + [c_int] * 7 + [c_void_p] * 2,
     "b200_paged_flash_attention": [c_void_p] * 8 + [c_int] * 12 + [c_float, c_int, c_int, c_int, c_float, c_void_p, c_int, c_int, c_void_p,

@@ -451,14 +451,15 @@ def portion_attention_f32_takes(ctx: StepContext, cache: CacheView, q: torch.Ten
 
 def portion_attention_f32(ctx: StepContext, cache: CacheView, q: torch.Tensor, out: torch.Tensor, q_heads: int, kv_heads: int, head_dim: int, scale: float,
                           *, first_seq: int, shape: ScoreShape = NO_SHAPE) -> torch.Tensor:
-    """Attention of the requests from ``first_seq`` on (float32)."""
+    """Attention of the requests from ``first_seq`` on, single tokens in front of them (float32). ``options["portion_keys"]``: ``"few"`` or
+    ``"many"`` forces one of the kernel's two forms, which give the same bits."""
     _need(q.is_contiguous() and out.is_contiguous() and q.dtype == torch.float32 == out.dtype == cache.keys.dtype, "portion_attention_f32: bad operands")
     sink = shape.arguments(q_heads)[-1]
     ctx.lib.call(
         "b200_portion_attention_f32", ptr(q), ptr(cache.keys), ptr(cache.values), ptr(cache.block_table), c_int(cache.max_pages), c_int(cache.num_pages),
         ptr(ctx.seq_q_start), ptr(ctx.seq_q_len), ptr(ctx.seq_kv_len), c_int(first_seq), c_int(ctx.num_seqs - first_seq), c_int(ctx.max_q_len),
         sink, ptr(out), c_int(q_heads), c_int(kv_heads), c_int(head_dim), c_int(cache.page_size), c_int(cache.window), c_float(scale),
-        ptr(ctx.err), ctx.stream,
+        c_int(q.shape[0] - first_seq), c_int(ctx.max_kv_len), c_int({"auto": 0, "few": 1, "many": 2}[ctx.options.get("portion_keys", "auto")]), ptr(ctx.err), ctx.stream,
     )
     return out
 

@@ -145,3 +145,27 @@ def test_infinite_and_very_large_numbers(operand, value, at, dim):
     close = 3e-5 + 3e-5 * want[finite].abs()  # as for the portions above
     assert ((got[finite] - want[finite]).abs() <= close).all()
     assert torch.equal(got[:at], clean[:at].double())
+
+
+@pytest.mark.parametrize("q_heads,kv_heads,dim,window,with_sink", [(12, 2, 128, 0, False), (3, 3, 64, 20, True), (16, 1, 100, 0, True), (4, 2, 24, 70, False)])
+def test_both_forms_give_the_same_bits(q_heads, kv_heads, dim, window, with_sink):
+    """The form for few keys a block is chosen by the whole step; a row must not depend on that."""
+    from llm_inference_b200.cli.microbench import make_ctx
+    from llm_inference_b200.parts import ops
+    from llm_inference_b200.parts.context import CacheView
+
+    torch.manual_seed(dim)
+    runs, starts, page = [5, 64, 33, 130, 1, 70], [3, 0, 40, 200, 300, 0], 16
+    pages = -(-max(r + s for r, s in zip(runs, starts)) // page)
+    table = torch.randperm(len(runs) * pages, device="cuda").int().view(len(runs), pages)
+    keys, values = (torch.randn(len(runs) * pages, kv_heads, page, dim, device="cuda") for _ in range(2))
+    keys[7, :, 3], values[11, :, 5, 2], values[12, :, 9] = float("inf"), float("-inf"), torch.finfo(torch.float32).max
+    shape = ops.ScoreShape(sink=torch.randn(q_heads, device="cuda")) if with_sink else ops.NO_SHAPE
+    view = CacheView(0, True, keys, values, table, len(runs) * pages, pages, page, window)
+    q = torch.randn(sum(runs), q_heads * dim, device="cuda")
+    outs = []
+    for form in ("few", "many"):
+        ctx = make_ctx([p for r, s in zip(runs, starts) for p in range(s, s + r)], [i for i, r in enumerate(runs) for _ in range(r)], starts, runs, {"portion_keys": form})
+        outs.append(ops.portion_attention_f32(ctx, view, q, torch.full_like(q, 7.0), q_heads, kv_heads, dim, dim**-0.5, first_seq=0, shape=shape))
+        assert int(ctx.err.item()) == 0
+    assert torch.equal(outs[0].nan_to_num(nan=1e30), outs[1].nan_to_num(nan=1e30)) and torch.isfinite(outs[0]).any()
