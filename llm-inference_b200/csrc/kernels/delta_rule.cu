@@ -98,9 +98,9 @@ __global__ void delta_prepare_kernel(const T* proj, int ld, const T* decay_in, i
 // are read once for the four tokens that want them, and a lane's seven rows are asked for together. Only tokens next to a request's
 // start look into its slot.
 // What bounds it: instructions (exponentials, logarithms, quotients). One block for four tokens of all channels held 128 registers a thread, so
-// two blocks an SM, and went through a token's rows with a look at its request for every tap: on a B200 2,048 tokens of 4,608 channels took
-// 58 us with a decay per channel and 30 with one per head (3,072 channels), now 29 and 16
-// (with divisions 52 and 26: their code, in line sixteen times, did not fit what an SM holds of it).
+// two blocks an SM, and went through a token's rows with a look at its request for every tap: on a B200 2,048 tokens of 12 heads of 128 took, the
+// slots' update with them, 56 us with a decay per channel and 45 with one per head, now 28 and 21
+// (with divisions nearly what they took before: their code, in line sixteen times, does not fit what an SM holds of it).
 // Heads of more than 256 channels do not fit a warp's registers: the four warps of a block share one, and its numbers wait for their factors where they
 // go (4 heads of 512, 2,048 tokens: 78 us with a decay per channel and 59 with one per head in the form for single tokens, 55 and 41 in the block for all
 // channels, now 40 and 27; 300 tokens 21 and 17, 24 and 20, now 11 and 9; one warp a head 23 and 23).

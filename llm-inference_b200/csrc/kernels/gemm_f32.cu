@@ -138,10 +138,13 @@ int launch_tiles(const Product& p, bool wide, cudaStream_t stream) {
 
 // Tiles of 64 x 64 outputs, 8 x 4 a thread, where there are enough of them for every SM; tiles of 16 x 32, 2 x 4 a thread, for few rows and
 // wherever they come to at most three an SM: each tile walks all of K, so a product of few tiles takes the time of one tile's walk, which
-// is the shorter the fewer outputs it has. Measured on a B200 (N x K, rows; us; before: 64 x 64 outputs, 4 x 4 a thread, no copies ahead):
-//   2,048 x 1,536:  1 row 145 -> 52 (64 x 64: 78), 100 rows 155 -> 76 (16 x 32: 69), 500 rows 165 -> 119 (16 x 32: 173), 2,048 rows 461 -> 326
-//   17,920 x 1,536: 16 rows 184 -> 68 (64 x 64: 117), 33 rows 189 -> 117 (16 x 32: 160), 2,048 rows 3,349 -> 2,649 (58 % of the FMA pipe)
-//   1,536 x 8,960:  1 row 831 -> 226, 100 rows 853 -> 305 (64 x 64: 380), 500 rows 856 -> 614, 2,048 rows 2,474 -> 1,588
+// is the shorter the fewer outputs it has. Measured on a B200 (N x K, rows; us; in brackets the other tile), at sizes that the
+// tensor cores do not take:
+//   64 x 1,536:     1 row 38 (64 x 64: 63), 500 rows 39 (65), 2,048 rows 43 (65)
+//   2,048 x 1,537:  1 row 60 (90), 33 rows 63 (90), 100 rows 90 (16 x 32: 83), 500 rows 138 (16 x 32: 224), 2,048 rows 436 (828)
+//   17,920 x 128:   16 rows 6.7 (64 x 64: 10.7), 33 rows 11.1 (16 x 32: 14.3), 500 rows 64 (112), 2,048 rows 236 (435)
+//   4,096 x 64:     1 row 3.1 (64 x 64: 4.3), 33 rows 3.9 (4.6), 100 rows 5.0 (16 x 32: 5.6), 500 rows 10.6 (16), 2,048 rows 31 (55)
+//   12 heads, 512 x 128 each: 16 rows 5.1 (64 x 64: 7.4), 33 rows 7.5 (16 x 32: 6.6), 100 rows 11 (11.5), 2,048 rows 83 (152)
 // Tiles of 128 x 128 and 64 x 128 with 8 x 8 a thread were slower throughout (2,735 and 2,709 us for 2,048 rows of 17,920 x 1,536).
 int launch_product(const Product& p, cudaStream_t stream) {
   const bool wide = p.K % 4 == 0 && p.lda % 4 == 0 && p.ldw % 4 == 0 && p.stride_a % 4 == 0 && p.stride_w % 4 == 0 &&

@@ -1,7 +1,7 @@
 // True 32-bit matrix product on the fifth-generation tensor cores:  C[M,N] = A[M,K] * W[N,K]^T (+ bias[N]), 32-bit operands and result.
 //
 // A number is the sum of three bfloat16 ones to its last bit: the nearest, the nearest to what is left, and the rest (8 + 8 + 8 bits). Of the nine
-// products of two such sums the six largest are taken; the others are below 2^-26 of the whole. Products of 8-bit numbers are exact in 32
+// products of two such sums the six largest are taken; the others come to at most 2^-24 of the whole. Products of 8-bit numbers are exact in 32
 // bits. `tcgen05.mma` drops bits below the last when it adds, so its chains are short: over 64 numbers the twenty small products first, the
 // four large ones last, into an accumulator of their own, which is then added to 32-bit registers with ordinary rounding. Against 64
 // bits results are nearer than those of the FMA kernel (gemm_f32.cu), whose chains are K long: figures at `b200_gemm_f32_split_takes`.

@@ -1,10 +1,12 @@
 // Products of 32-bit numbers on the tensor cores.
 //
 // A number is the sum of three bfloat16 ones, to its last bit: the nearest, the nearest to what is left, and the rest (8 + 8 + 8 bits). Of the
-// nine products of two such sums the six largest are taken; the others are below 2^-26 of the whole. Products of 8-bit numbers are exact in
+// nine products of two such sums the six largest are taken; the others come to at most 2^-24 of the whole (the second part is up to 2^-8 of a number,
+// the third 2^-17), as much as rounding it. Products of 8-bit numbers are exact in
 // 32 bits. The tensor core's own sums drop bits below the last, so few are chained: the five small products of a step of 16 first, the large
-// one last, and what is summed beyond one step is added with ordinary rounding. What is not finite becomes NaN;
-// the largest numbers, which bfloat16 would round to infinity, keep the largest bfloat16 as their first part.
+// one last, and what is summed beyond one step is added with ordinary rounding.
+// At the ends of the range: an infinity, like NaN, becomes NaN; the largest numbers, which bfloat16 would round to infinity, keep the largest bfloat16
+// as their first part and are exact; below 2^-110 the third part falls under bfloat16's smallest number, 2^-133, half of which is then the error of a number.
 #pragma once
 
 #include "common.cuh"

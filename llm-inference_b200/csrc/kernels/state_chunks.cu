@@ -1250,7 +1250,7 @@ bool aligned16(const void* p) { return reinterpret_cast<uintptr_t>(p) % 16 == 0;
 // Heads know nothing of one another, so a scratch that does not hold all of them takes them in as few equal parts as fit, one after the
 // other through the same scratch. Each part costs another walk of the same length with fewer blocks: 2,048 tokens of 28 heads of 128 x 128
 // with one decay per head take 273 us in one part, 320 in two, 395 in three, 487 in four (token by token 815), 24 heads of 64 x 64 under the
-// generalized rule 145, 205, 271 and 328 (450). More than three parts would still gain; three already hold steps of 55,000 tokens of 28 heads.
+// generalized rule 145, 205, 271 and 328 (450). Three hold steps of 55,000 tokens of 28 heads; `ops.py` has why they end there.
 template <typename Pass>
 int part_by_part(const char* name, int rule, const Sizes& z, float* base, int64_t floats, Pass pass) {
   Scratch scratch;

@@ -438,9 +438,11 @@ def paged_attention_plain(
 def portion_attention_f32_takes(ctx: StepContext, cache: CacheView, q: torch.Tensor, q_heads: int, kv_heads: int, head_dim: int, value_head: int,
                                 shape: ScoreShape) -> bool:
     """Whether the step's prompt portions run the tiled 32-bit kernel (csrc/kernels/attention_f32.cu): float32, unshaped scores (a window
-    and a sink are taken). Only portions of a few tokens with few keys stay with the plain kernel, whose blocks start sooner
-    (one request, 12 heads of 128 on 2 kv heads, plain and tiled: 16 tokens 28 and 30 us, 32 tokens 30 and 28, 500 tokens 325 and
-    88; 8 tokens behind 1,000 others 191 and 128)."""
+    and a sink are taken). Only portions of a few tokens with few keys stay with the plain kernel, whose blocks start sooner.
+    One request, 12 heads of 128 on 2 kv heads, plain and tiled: 16 tokens 8.2 and 10.5 us, 32 tokens 9.7 and 10.7, 64 tokens 12.7 and 11.5;
+    16 tokens with 80 keys 13 and 15, 116 keys 16 and 15, 266 keys 36 and 28. 8 heads of 64: 8 tokens 5.6 and 5.9, 32 tokens 7.8 and
+    6.6, 16 tokens with 266 keys 30 and 15. The line is where the tiled kernel's form in FMAs came level; up to it the present one gains
+    from 110 keys (heads of 64: 70) on."""
     return (
         q.dtype == torch.float32 and value_head < 0 and not shape.changes_scores() and shape.sigmoid_bias is None
         and not (cache.window and cache.keep_first) and ctx.num_seqs > ctx.num_decode_seqs
@@ -1027,7 +1029,10 @@ MANY_CHAINS, MANY_CHAINS_CHUNK_FROM = 96, 512
 # Scratch grows with the step's tokens (0.13 MB a token at 28 heads of 128 x 128): past this a step takes its heads in parts, and past so
 # many parts it walks its portions token by token, as if they were short, in the memory that takes.
 CHUNK_SCRATCH_BYTES = 2 << 30
-CHUNK_PARTS = 3  # where chunks in parts stop being faster: state_chunks.cu has the figures
+# Long portions would gain past three parts too (32 requests of 2,048 tokens, 28 heads of 128 x 128, in four: 7.3 ms, token by token 18.7), many short ones
+# beside a long one would not throughout (1,500 of 20 tokens beside one of 2,048: decay per channel in five 10.5 and 12.7 ms, generalized rule, 56
+# heads of 64 x 64, in four 14.2 and 6.8).
+CHUNK_PARTS = 3
 _DELTA, _GENERAL_DELTA, _LINEAR, _MEMORY = 0, 1, 2, 3  # csrc/kernels/state_chunks.cu
 
 

@@ -23,8 +23,9 @@ def product(a, w, bias=None, tokens=0):
     return out
 
 
-# Rounding alone: a part is exact, what is left out of a product below 2^-26 of it, a stage of 64 numbers ends in a handful of roundings (2^-23
-# each, towards zero inside the tensor core), and K / 64 stages add up with ordinary rounding: 2^-22 of the whole at these K, with room.
+# A part is exact; what is left out of a product is at most 2^-24 of it (2 x 2^-8 x 2^-17 and less; its sign changes from product to product unless it is
+# made not to); a stage of 64 numbers ends in four roundings towards zero inside the tensor core (2^-23 each of what has been summed by then: 2.5
+# of them on sums of one sign), and K / 64 stages add up with ordinary rounding. Random signs: 2^-22 and what is left out, 3e-7, with room.
 CLOSE = 5e-7
 
 
@@ -102,3 +103,13 @@ def test_the_smallest_operands(operand, small, large):
     want = a.double() @ w.double().T
     got = product(a.contiguous(), w.contiguous())
     assert ((got.double() - want).abs() / want).max().item() < CLOSE + 2.0**-149 / want.min().item()
+
+
+@pytest.mark.parametrize("k", [256, 516, 1028])
+def test_what_is_left_out_with_one_sign(k):
+    """1 + 2^-8 - 2^-17 splits into parts as large as they get, so every product leaves out its 2^-24, all on the same side."""
+    x = 1 + 2.0**-8 - 2.0**-17
+    got = product(torch.full((40, k), x, device="cuda"), torch.full((150, k), -x, device="cuda"))
+    # left out, the four roundings towards zero of each stage, half an ulp for each of the K / 64 sums
+    bound = 2.0**-24 + 2.5 * 2.0**-23 + (k // 64 + 1) / 2 * 2.0**-24
+    assert ((got.double() + k * x * x).abs() / (k * x * x)).max().item() < bound
