@@ -130,8 +130,9 @@ struct SplitProduct {
   int* err;
 };
 
+__device__ __forceinline__ bool any_nan(float4 v) { return isnan(v.x) || isnan(v.y) || isnan(v.z) || isnan(v.w); }
 // An output as the FMA kernel makes it, where the sum of the products of parts is not finite: an infinite operand (whose parts are NaN), or a sum
-// that passes the range on its way, may be the reason, and the output is infinite, or finite after all.
+// that passes the range on its way, may be the reason, and the output is infinite, or finite after all. Where a row has a NaN it stays NaN.
 __device__ __noinline__ float chain(const SplitProduct& p, int m, int n) {
   const float* a = p.A + static_cast<int64_t>(m) * p.lda;
   const float* w = p.W + static_cast<int64_t>(n) * p.ldw;
@@ -270,22 +271,31 @@ gemm_f32_split_kernel(const __grid_constant__ SplitProduct p) {
       __syncwarp();
       if (lane == 0) mbar_arrive(&sum_empty[b]);
     }
+    uint32_t odd[(TOKENS + 31) / 32] = {};  // tokens whose sum is not finite
+    const float more = p.bias != nullptr && n < p.N ? p.bias[n] : 0.f;
     if (have && n < p.N) {
-      const float more = p.bias != nullptr ? p.bias[n] : 0.f;
-      uint32_t odd[(TOKENS + 31) / 32] = {};  // tokens whose sum is not finite
 #pragma unroll
       for (int i = 0; i < TOKENS; ++i) {
         if (m0 + i >= p.M) break;
         if (!isfinite(sum[i])) odd[i / 32] |= 1u << (i % 32);
         p.C[static_cast<int64_t>(m0 + i) * p.ldc + n] = fmaf(sum[i], kSumScale, more);
       }
-#pragma unroll
-      for (int word = 0; word < (TOKENS + 31) / 32; ++word)
-        for (; odd[word] != 0; odd[word] &= odd[word] - 1) {
-          const int m = m0 + word * 32 + __ffs(odd[word]) - 1;
-          p.C[static_cast<int64_t>(m) * p.ldc + n] = chain(p, m, n) + more;
-        }
     }
+    __syncwarp();
+    bool looked = false, spoilt = false;  // at the lane's row of W; that has a NaN
+#pragma unroll
+    for (int word = 0; word < (TOKENS + 31) / 32; ++word)
+      for (uint32_t any = __reduce_or_sync(0xffffffffu, odd[word]); any != 0; any &= any - 1) {
+        const int bit = __ffs(any) - 1, m = m0 + word * 32 + bit;
+        bool nan = false;
+        for (int k = lane * 4; k < p.K; k += 128) nan |= any_nan(*reinterpret_cast<const float4*>(p.A + static_cast<int64_t>(m) * p.lda + k));
+        if (__any_sync(0xffffffffu, nan) || !(odd[word] >> bit & 1)) continue;  // NaN it stays
+        if (!looked) {
+          looked = true;
+          for (int k = 0; k < p.K; k += 4) spoilt |= any_nan(*reinterpret_cast<const float4*>(p.W + static_cast<int64_t>(n) * p.ldw + k));
+        }
+        if (!spoilt) p.C[static_cast<int64_t>(m) * p.ldc + n] = chain(p, m, n) + more;
+      }
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
