@@ -72,13 +72,17 @@ __device__ __forceinline__ void load_block(const uint4* from, SplitB* to) {
 }
 
 // One row by one warp, of the numbers themselves, a lane a key and then four of the row's numbers: where a product of parts is not finite, an
-// infinite operand (whose parts are NaN) or a number next to the largest may be the reason, and the row may be finite, or infinite.
+// infinite operand (whose parts are NaN) or a number next to the largest may be the reason, and the row may be finite, or infinite. A NaN in its scores
+// leaves the row as it is, NaN.
 __device__ __noinline__ void attend_row(const PortionParams& p, int seq, int kvh, int token, int head, int pos) {
   const int lane = threadIdx.x & 31, from = p.window > 0 ? max(0, pos - p.window + 1) : 0;
   const float* own = p.q + (static_cast<int64_t>(token) * p.q_heads + head) * p.head_dim;
   const int* table = p.block_table + static_cast<int64_t>(seq) * p.max_pages;
   float top = p.sink != nullptr ? p.sink[head] : -INFINITY, sum = p.sink != nullptr ? 1.f : 0.f;
   float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+  bool nan = false;
+  for (int c = lane; c < p.head_dim; c += 32) nan |= isnan(own[c]);
+  if (__any_sync(0xffffffffu, nan)) return;
   for (int key0 = from; key0 <= pos; key0 += 32) {
     const int key = key0 + lane, logical = key / p.page_size;
     const int page = key <= pos && logical < p.max_pages ? table[logical] : -1;
@@ -89,6 +93,7 @@ __device__ __noinline__ void attend_row(const PortionParams& p, int seq, int kvh
       for (int c = 0; c < p.head_dim; ++c) score = fmaf(own[c], p.keys[offset + c], score);
       score *= p.scale;
     }
+    if (__any_sync(0xffffffffu, isnan(score))) return;
     float best = score;
     for (int o = 16; o > 0; o >>= 1) best = fmaxf(best, __shfl_xor_sync(0xffffffffu, best, o));
     const float new_top = fmaxf(top, best), alpha = top > -INFINITY ? expf(top - new_top) : 0.f;
@@ -372,7 +377,7 @@ portion_attention_f32_kernel(const __grid_constant__ PortionParams p) {
 #pragma unroll
           for (int i = 0; i < 4; ++i) {
             const int c = x * 8 + 2 * q + (i & 1), h = i >> 1;
-            if (c < p.head_dim && key <= pos[h] && key >= from[h] && !isfinite(p.values[offset + c])) acc[x][i] = NAN;
+            if (c < p.head_dim && key <= pos[h] && key >= from[h] && !isfinite(p.values[offset + c])) acc[x][i] += p.values[offset + c];
           }
       }
     }
@@ -395,7 +400,7 @@ portion_attention_f32_kernel(const __grid_constant__ PortionParams p) {
       *reinterpret_cast<float2*>(os + (warp * 16 + g + 8 * h) * kLdO + x * 8 + 2 * q) = make_float2(acc[x][2 * h], acc[x][2 * h + 1]);
   meet_own();
   static_assert(32 % (DIM / 4) == 0, "a row's numbers are those of one warp");
-  uint32_t odd = 0;  // rows with a result that is not finite
+  uint32_t odd = 0;  // rows to be made again
   for (int idx = tid; idx < rows * (DIM / 4); idx += kOwnThreads) {
     const int r = idx / (DIM / 4), c = idx % (DIM / 4) * 4;
     if (c >= p.head_dim) continue;
@@ -414,7 +419,8 @@ portion_attention_f32_kernel(const __grid_constant__ PortionParams p) {
     const float inv = total > 0.f ? 1.f / total : 0.f;
     const int item = row0 + r, token = item / group, head = kvh * group + item % group;
     o = make_float4(o.x * inv, o.y * inv, o.z * inv, o.w * inv);
-    if (!all_finite(o)) odd |= 1u << r;
+    // NaN beside a finite sum of weights comes from values and stands.
+    if (!isfinite(total) || isinf(o.x) || isinf(o.y) || isinf(o.z) || isinf(o.w)) odd |= 1u << r;
     *reinterpret_cast<float4*>(p.out + (static_cast<int64_t>(start + token) * p.q_heads + head) * p.head_dim + c) = o;
   }
   odd = __reduce_or_sync(0xffffffffu, odd);

@@ -169,3 +169,17 @@ def test_both_forms_give_the_same_bits(q_heads, kv_heads, dim, window, with_sink
         outs.append(ops.portion_attention_f32(ctx, view, q, torch.full_like(q, 7.0), q_heads, kv_heads, dim, dim**-0.5, first_seq=0, shape=shape))
         assert int(ctx.err.item()) == 0
     assert torch.equal(outs[0].nan_to_num(nan=1e30), outs[1].nan_to_num(nan=1e30)) and torch.isfinite(outs[0]).any()
+
+
+def test_infinities_of_both_signs_and_nan_in_one_column():
+    """Values that are not finite, told apart: NaN beats all, infinities of both signs are NaN, one sign stays, other columns are as they were."""
+    torch.manual_seed(3)
+    n, dim = 80, 64
+    q, k, v = (0.3 * torch.randn(n, 1, dim, device="cuda") for _ in range(3))
+    clean = attend_one_request(q, k, v, 1, dim)
+    inf, nan = float("inf"), float("nan")
+    v[5, 0, 1], v[40, 0, 2], v[7, 0, 3], v[41, 0, 3], v[9, 0, 4], v[9, 0, 4] = inf, -inf, inf, -inf, inf, nan
+    got = attend_one_request(q, k, v, 1, dim)
+    assert (got[5:, 0, 1] == inf).all() and (got[40:, 0, 2] == -inf).all() and (got[7:41, 0, 3] == inf).all()
+    assert torch.isnan(got[41:, 0, 3]).all() and torch.isnan(got[9:, 0, 4]).all()
+    assert torch.equal(got[:5], clean[:5]) and torch.isfinite(got[5:, 0, 5:]).all()
