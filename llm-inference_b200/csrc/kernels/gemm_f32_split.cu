@@ -11,7 +11,7 @@
 // stage; four warps add up the accumulators, two of which take turns in TMEM. An output's sums are the same whatever the tile, so a row's result
 // does not depend on how many rows are in the call. Outputs that are not finite are made again as one chain of FMAs (`chain`).
 //
-// What bounds it: what an SM takes out of L2, 48 KB a stage at 128 x 64 and 64 KB at 128 x 128. Of 34 us for 500 rows by 2,048 x 1,536, a form
+// What bounds it: what an SM takes out of L2, 48 KB a stage at 128 x 64 and 64 KB at 128 x 128. Of 32 us for 500 rows by 2,048 x 1,536, a form
 // that only fetches takes 25, the products and the taking apart the rest. Tried: two stages ahead in registers instead of one, no change; numbers by
 // cp.async and W's parts in TMEM, 36 us (17,920 rows of W, 2,048 of A: 858 against 716).
 // Every wait is bounded; a block that gives up sets the timeout bit, frees its TMEM and leaves.
@@ -179,19 +179,25 @@ gemm_f32_split_kernel(const __grid_constant__ SplitProduct p) {
     const int piece = threadIdx.x & 7, row0 = threadIdx.x >> 3;  // rows row0, row0 + 32, ..
     const bool takes_a = TOKENS * 8 >= kFetchThreads || row0 < TOKENS;
     float4 w[kWItems][2], a[kAItems][2];
-    auto fetch = [&](float4 (&to)[2], const float* from, int64_t ld, int row, bool valid, int step) {
-      const int k = step * kBlockK + piece * 8;
+    const float* w_at = p.W + static_cast<int64_t>(n0 + row0) * p.ldw + piece * 8;  // of the stage that is fetched next
+    const float* a_at = p.A + static_cast<int64_t>(m0 + row0) * p.lda + piece * 8;
+    const int64_t w_step = 32LL * p.ldw, a_step = 32LL * p.lda;
+    const int w_rows = p.N - n0 - row0, a_rows = takes_a ? p.M - m0 - row0 : 0;  // row 32 i is one if above 32 i
+    int left = p.K - piece * 8;
+    auto fetch = [&](float4 (&to)[2], const float* from, bool valid) {
 #pragma unroll
-      for (int h = 0; h < 2; ++h)
-        to[h] = valid && k + 4 * h < p.K ? *reinterpret_cast<const float4*>(from + row * ld + k + 4 * h) : make_float4(0.f, 0.f, 0.f, 0.f);
+      for (int h = 0; h < 2; ++h) to[h] = valid && left > 4 * h ? *reinterpret_cast<const float4*>(from + 4 * h) : make_float4(0.f, 0.f, 0.f, 0.f);
     };
-    auto fetch_stage = [&](int step) {
+    auto fetch_w = [&](int i) { fetch(w[i], w_at + i * w_step, w_rows > 32 * i); };
+    auto fetch_a = [&](int i) { fetch(a[i], a_at + i * a_step, a_rows > 32 * i); };
+    auto go_on = [&] { w_at += kBlockK, a_at += kBlockK, left -= kBlockK; };
+    auto fetch_all = [&] {
 #pragma unroll
-      for (int i = 0; i < kWItems; ++i) fetch(w[i], p.W, p.ldw, n0 + row0 + 32 * i, n0 + row0 + 32 * i < p.N, step);
+      for (int i = 0; i < kWItems; ++i) fetch_w(i);
 #pragma unroll
-      for (int i = 0; i < kAItems; ++i) fetch(a[i], p.A, p.lda, m0 + row0 + 32 * i, takes_a && m0 + row0 + 32 * i < p.M, step);
+      for (int i = 0; i < kAItems; ++i) fetch_a(i);
     };
-    fetch_stage(0);
+    fetch_all(), go_on();
     for (int step = 0; step < steps; ++step) {
       const int s = step % kStages;
       if (step >= kStages && !mbar_wait(&empty_bar[s], (step / kStages - 1) & 1)) {
@@ -199,13 +205,22 @@ gemm_f32_split_kernel(const __grid_constant__ SplitProduct p) {
         break;
       }
       unsigned char* stage = tiles + static_cast<size_t>(s) * stage_bytes(TOKENS);
+      // The next stage's numbers are asked for as soon as registers are free (none past K); behind all stores in blocks of sixteen tokens, since a launch may
+      // have few of those and each then waits for its own stores behind the loads (1 row, 128 x 8,960: 105 us, early 115). Larger tiles are taken
+      // where there are blocks for most SMs (early and behind: 500 rows, 17,920 x 1,536 172 and 182 us, 100 rows, 1,536 x 8,960 127 and 130).
+      constexpr bool kEarly = TOKENS >= 32;
 #pragma unroll
-      for (int i = 0; i < kWItems; ++i) store_parts(stage, part_bytes(kRows), row0 + 32 * i, piece, w[i][0], w[i][1]);
-      if (takes_a) {
-#pragma unroll
-        for (int i = 0; i < kAItems; ++i) store_parts(stage + kParts * part_bytes(kRows), part_bytes(TOKENS), row0 + 32 * i, piece, a[i][0], a[i][1]);
+      for (int i = 0; i < kWItems; ++i) {
+        store_parts(stage, part_bytes(kRows), row0 + 32 * i, piece, w[i][0], w[i][1]);
+        if (kEarly) fetch_w(i);
       }
-      if (step + 1 < steps) fetch_stage(step + 1);
+#pragma unroll
+      for (int i = 0; i < kAItems; ++i) {
+        if (takes_a) store_parts(stage + kParts * part_bytes(kRows), part_bytes(TOKENS), row0 + 32 * i, piece, a[i][0], a[i][1]);
+        if (kEarly) fetch_a(i);
+      }
+      if (kEarly) go_on();
+      else if (step + 1 < steps) fetch_all(), go_on();
       asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
       __syncwarp();
       if (lane == 0) mbar_arrive(&full_bar[s]);
